@@ -255,3 +255,89 @@ def tolerance(case):
   if case["kind"] == "fp8" and case["p_format"] == "e4m3":
     return {"rel": 3e-2, "max": 0.6}
   return {"rel": 1e-2, "max": 0.2}
+
+
+# ----------------------------------------------------------------------------------------------
+# the same results in 64 bits
+# ----------------------------------------------------------------------------------------------
+_EXACT_ELEMENTS = 1 << 27  # scores held at a time: 1 GiB each of logits, probabilities and their gradients
+
+
+def _wide(t, c):
+  """One operand in 64 bits as [B, H, S, D]; e4m3 values times the scale of their 128-token tile."""
+  if isinstance(t, fp8.Fp8Tensor):
+    return t.data.double() * t.scale.double().repeat_interleave(fp8.SCALE_TILE, dim=2)[..., None]
+  t = t.detach().double()
+  return t.transpose(1, 2) if c["kind"] == "op" else t
+
+
+def _keep(c, state, b, rows, lo, hi):
+  """Which keys lo .. hi the query rows of batch row b see: bool [rows, hi - lo]."""
+  q_at = (rows + (c["kv_len"] - c["q_len"]))[:, None]
+  k_at = torch.arange(lo, hi, device=rows.device)[None, :]
+  if c["mask"] == "prefix":
+    return state["mask"][rows, lo:hi]
+  if c["mask"] == "full":
+    return torch.ones((rows.numel(), hi - lo), dtype=torch.bool, device=rows.device)
+  keep = k_at <= q_at
+  if c["mask"] == "local":
+    keep &= k_at >= q_at - c["window"]
+  if c["docs"]:
+    ids = state["segments"].q[b]
+    keep &= ids[rows][:, None] == ids[lo:hi][None, :]
+  return keep
+
+
+def exact(case, seed):
+  """What ``run`` returns for these inputs, from dense attention in 64 bits, a block of query rows at a time."""
+  c = dict(case)
+  state = prepare(c, seed)
+  q, k, v = (_wide(state[n], c) for n in ("q", "k", "v"))
+  grads = c["kind"] in ("train", "op")
+  offset, group, dev = c["kv_len"] - c["q_len"], c["q_heads"] // c["kv_heads"], q.device
+  out = torch.zeros((c["batch"], c["q_heads"], c["q_len"], c["d_v"]), dtype=torch.float64, device=dev)
+  if grads:
+    do = _wide(state["do"], c)
+    dq, dk, dv = torch.zeros_like(q), torch.zeros_like(k), torch.zeros_like(v)
+  for b in range(c["batch"]):
+    first = 0
+    while first < c["q_len"]:
+      n = min(c["q_len"] - first, max(128, _EXACT_ELEMENTS // (c["q_heads"] * c["kv_len"])))
+      rows = torch.arange(first, first + n, device=dev)
+      lo = max(0, first + offset - c["window"]) if c["mask"] == "local" else 0
+      hi = c["kv_len"] if c["mask"] in ("full", "prefix") else first + n + offset
+      # heads as [kv heads, group * rows]: the q heads of one kv head are rows of one product
+      qb = q[b, :, first:first + n].reshape(c["kv_heads"], group * n, c["d"])
+      kb, vb = k[b, :, lo:hi], v[b, :, lo:hi]
+      keep = _keep(c, state, b, rows, lo, hi)
+      x = (qb @ kb.transpose(1, 2)).mul_(state["scale"]).view(c["kv_heads"], group, n, hi - lo)
+      slope = None
+      if c["soft_cap"]:
+        x.div_(c["soft_cap"]).tanh_()
+        slope = 1 - x * x if grads else None
+        x.mul_(c["soft_cap"])
+      x.masked_fill_(~keep, -math.inf)
+      top = x.amax(-1, keepdim=True)
+      sink = state["sinks"].double().view(c["kv_heads"], group, 1, 1) if c["sinks"] else None
+      if sink is not None:
+        top = torch.maximum(top, sink)
+      x.sub_(top).exp_()
+      total = x.sum(-1, keepdim=True)
+      if sink is not None:
+        total = total + torch.exp(sink - top)
+      p = x.div_(total).view(c["kv_heads"], group * n, hi - lo)
+      ob = p @ vb
+      out[b, :, first:first + n] = ob.view(c["q_heads"], n, c["d_v"])
+      if grads:
+        dob = do[b, :, first:first + n].reshape(c["kv_heads"], group * n, c["d_v"])
+        dv[b, :, lo:hi] += p.transpose(1, 2) @ dob
+        ds = (dob @ vb.transpose(1, 2)).sub_((ob * dob).sum(-1, keepdim=True)).mul_(p).mul_(state["scale"])
+        if slope is not None:
+          ds.mul_(slope.view_as(ds))
+        dq[b, :, first:first + n] = (ds @ kb).view(c["q_heads"], n, c["d"])
+        dk[b, :, lo:hi] += ds.transpose(1, 2) @ qb
+      first += n
+  lay = (lambda t: t.transpose(1, 2).contiguous()) if c["kind"] == "op" else (lambda t: t)
+  if not grads:
+    return lay(out)
+  return {"out": lay(out), "dq": lay(dq), "dk": lay(dk), "dv": lay(dv)}
