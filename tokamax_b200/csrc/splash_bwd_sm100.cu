@@ -201,7 +201,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (warp >= 8) {
    setmaxnreg_dec<kIssueRegs>();
    if (warp == 8) {
-    if (lane == 0 && n_ent > 0) {
+    if (n_ent > 0 && elect_one()) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_do);
       tma_prefetch_desc(&tm_k);
@@ -232,7 +232,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
     }
   } else if (warp == 9) {
-    if (lane == 0 && n_ent > 0) {
+    if (n_ent > 0 && elect_one()) {
       constexpr uint32_t idesc_kk = make_idesc_bf16(kTile, kTile, false, false);
       // N of dQ += dS K: dq's columns — 128, or 64 when q / k have at most 64
       const uint32_t idesc_mn = make_idesc_bf16(kTile, p.d_qk <= 64 ? 64 : kHeadDim, false, true);
@@ -626,7 +626,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
   } else if (warp >= 16) {
    if (warp == kDkvTmaWarp) {
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0 && elect_one()) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_do);
       tma_prefetch_desc(&tm_k);
@@ -667,7 +667,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
     }
   } else if (warp == kDkvMmaWarp) {
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0 && elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kTile, false, false);
       // N of the accumulating MMAs = the gradient's columns: 128, or 64 when the tensor has at most 64
       const uint32_t idesc_dv = make_idesc_bf16(kTile, p.d_v <= 64 ? 64 : kHeadDim, false, true);

@@ -142,7 +142,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
    setmaxnreg_dec<kIssueRegs>();
    if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0 && elect_one()) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_do);
       tma_prefetch_desc(&tm_k);
@@ -210,7 +210,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     }
    } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0 && elect_one()) {
       constexpr uint32_t idesc_kk = make_idesc_bf16(kTile, kTile, false, false);
       const uint32_t a1_addr = smem_u32(a1_smem), a2_addr = smem_u32(a2_smem);
       const uint32_t held_addr = smem_u32(held_smem), pass_addr = smem_u32(pass_smem);

@@ -117,7 +117,7 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
 
   if (warp == 8) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
@@ -153,7 +153,7 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     }
   } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(kTile, kTile, false, false);
       const uint32_t q_addr = smem_u32(q_smem);
       const uint32_t ring_addr = smem_u32(ring);
