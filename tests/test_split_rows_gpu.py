@@ -1,0 +1,124 @@
+"""Grids that leave SMs idle: schedule rows shared by a cluster of CTAs, against the CPU oracle.
+
+A few heads and long rows, so that the launchers take 2 .. 8 CTAs a row: every way of forming a
+row's entries (causal offset, window, segments, table mask), odd numbers of query tiles, parts of
+unequal length, rows without a live key in some part, sinks (counted once) and a fixed maximum.
+Bounds: those of test_splash_gpu.py, but for outputs of rows with one large weight.
+"""
+import dataclasses
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import attention_ref
+from tokamax_b200 import fp8
+from tokamax_b200 import splash_attention_kernel as splash
+from tokamax_b200 import splash_attention_mask as mask_lib
+
+pytestmark = pytest.mark.gpu
+
+DEV = torch.device("cuda:0")
+
+
+def _mk(seed, *shape):
+  g = torch.Generator().manual_seed(seed)
+  return torch.randn(*shape, generator=g).to(torch.bfloat16)
+
+
+def _dense(mask):
+  return np.asarray(mask[(slice(0, mask.shape[0]), slice(0, mask.shape[1]))]).astype(np.bool_)
+
+
+def _table(sq, skv):
+  m = np.random.default_rng(3).random((sq, skv)) < 0.4
+  m[:, : skv // 2] &= (np.arange(sq) % 3 != 0)[:, None]  # rows whose keys are all in the second half
+  m[5] = False  # and one without any
+  return m
+
+
+CASES = {
+    "causal": (lambda sq, skv: mask_lib.CausalMask((sq, skv), skv - sq), {}),
+    "window": (lambda sq, skv: mask_lib.LocalMask((sq, skv), (skv // 3, 0), skv - sq), {}),
+    "full_sinks": (lambda sq, skv: mask_lib.FullMask((sq, skv)), dict(sinks=True)),
+    "segments": (lambda sq, skv: mask_lib.FullMask((sq, skv)), dict(segments=True, sinks=True)),
+    "table": (_table, {}),
+    "soft_cap": (lambda sq, skv: mask_lib.CausalMask((sq, skv), skv - sq), dict(cap=20.0, sinks=True)),
+    "fixed_max": (lambda sq, skv: mask_lib.FullMask((sq, skv)), dict(fixed=6.0, sinks=True)),
+}
+
+
+@pytest.mark.parametrize("sq,skv,hq,hkv", [(128, 4096, 2, 1), (256, 1280, 3, 3), (384, 2944, 4, 2), (1024, 1024, 4, 2)])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_forward_and_gradients(name, sq, skv, hq, hkv):
+  make, opt = CASES[name]
+  mask = make(sq, skv)
+  dense = mask if isinstance(mask, np.ndarray) else _dense(mask)
+  d = 64 if name == "window" else 128
+  q, k, v, do = _mk(0, 1, hq, sq, d), _mk(1, 1, hkv, skv, d), _mk(2, 1, hkv, skv, d), _mk(3, 1, hq, sq, d)
+  # a jump of the row maximum between parts: the keys of the last tiles carry larger logits
+  k[:, :, -256:] *= 4
+  config = splash.SplashConfig.get_default()
+  if "cap" in opt:
+    config = dataclasses.replace(config, attn_logits_soft_cap=opt["cap"])
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1, save_residuals=True, config=config)
+  sinks = torch.linspace(-1.0, 3.0, hq) if opt.get("sinks") else None
+  seg = None
+  if opt.get("segments"):
+    seg = ((torch.arange(sq) * 3 // sq)[None].int(), (torch.arange(skv) * 3 // skv)[None].int())
+  scale = 1 / math.sqrt(d)
+  qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+  out, res = kernel(qd, kd, vd, None if seg is None else splash.SegmentIds(*(s.to(DEV) for s in seg)),
+                    None if sinks is None else sinks.to(DEV), logits_scale=scale,
+                    max_logit_value=opt.get("fixed"))
+  out.backward(do.to(DEV))
+  kernel.check_errors()
+  ref = [attention_ref.attention_reference(q[0], k[0], v[0], dense, None if seg is None else (seg[0][0], seg[1][0]),
+                                           scale=scale, attn_logits_soft_cap=opt.get("cap"), sinks=sinks)]
+  ro, rlse, rmax = ref[0]
+  live = rlse > -1e30
+  # P and the result are rounded to bf16: half an ulp (2^-9) of sum p |v| each, and sum p |v| <= max |v|
+  # (with one large weight a row keeps all of it)
+  assert (out[0].float().cpu() - ro)[live].abs().max().item() <= 2.0 ** -8 * v.abs().max().item()
+  assert torch.all(out[0].float().cpu()[~live] == 0)
+  assert (res["logsumexp"][0].cpu() - rlse)[live].abs().max().item() <= 1e-3
+  if "fixed" not in opt:
+    assert (res["max_logits"][0].cpu() - rmax)[live].abs().max().item() <= 1e-3 * max(1.0, rmax[live].abs().max().item())
+  ro, rlse = torch.where(live[..., None], ro, 0.0), torch.where(live, rlse, float("inf"))
+  grads = attention_ref.attention_reference_vjp(do[0], q[0], k[0], v[0], dense,
+                                                None if seg is None else (seg[0][0], seg[1][0]), ro, rlse, scale=scale,
+                                                attn_logits_soft_cap=opt.get("cap"))
+  for got, want in zip((qd.grad, kd.grad, vd.grad), grads):
+    assert ((got[0].float().cpu() - want).norm() / want.norm()).item() <= 1e-2
+
+
+@pytest.mark.parametrize("p_format,rel", [("e4m3", 3e-2), ("f16", 5e-3)])
+@pytest.mark.parametrize("sq,skv", [(128, 4096), (384, 2944)])
+def test_e4m3_forward(p_format, rel, sq, skv):
+  q, k, v = (fp8.quantize_e4m3(_mk(i, 1, 2, n, 128).to(DEV)) for i, n in ((0, sq), (1, skv), (2, skv)))
+  mask = mask_lib.CausalMask((sq, skv), skv - sq)
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1)
+  scale = 1 / math.sqrt(128)
+  out, res = fp8.splash_fwd_fp8(kernel, q, k, v, logits_scale=scale, save_residuals=True, p_format=p_format)
+  kernel.check_errors()
+  deq = [fp8.dequantize_e4m3(t, torch.float32).cpu()[0] for t in (q, k, v)]
+  ro, rlse, _ = attention_ref.attention_reference(*deq, _dense(mask), scale=scale)
+  assert ((out[0].float().cpu() - ro).norm() / ro.norm()).item() <= rel
+  assert (res["logsumexp"][0].cpu() - rlse).abs().max().item() <= 1e-3
+
+
+def test_parts_without_a_live_key():
+  """Only the last tile of a long row is live: every other part of the cluster ends with sum 0."""
+  sq, skv = 256, 4096
+  q, k, v = _mk(0, 1, 2, sq, 128), _mk(1, 1, 2, skv, 128), _mk(2, 1, 2, skv, 128)
+  live_everywhere = np.ones((sq, skv), np.bool_)
+  ids = torch.zeros(1, skv, dtype=torch.int32)
+  ids[:, 1:-1] = 1  # tiles stay in the schedule, their keys belong to another segment
+  kernel = splash.make_splash_mha(mask_lib.FullMask((sq, skv)), q_seq_shards=1, save_residuals=True)
+  qs = torch.zeros(1, sq, dtype=torch.int32)
+  out, res = kernel(q.to(DEV), k.to(DEV), v.to(DEV), splash.SegmentIds(qs.to(DEV), ids.to(DEV)), logits_scale=0.1)
+  kernel.check_errors()
+  ro, rlse, _ = attention_ref.attention_reference(q[0], k[0], v[0], live_everywhere, (qs[0], ids[0]), scale=0.1)
+  assert (out[0].float().cpu() - ro).abs().max().item() <= 1e-2
+  assert (res["logsumexp"][0].cpu() - rlse).abs().max().item() <= 1e-3

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "splash_common.cuh"
+#include "splash_split.cuh"
 
 namespace sb {
 
@@ -42,6 +43,7 @@ struct FwdParams {
   int pm_bq, pm_bkv;
   SplashMaskFn fn;
   int q_len, kv_len, q_heads, kv_heads, n_q_tiles, n_rows;
+  int n_split;                 // CTAs of a cluster that share a schedule row (1: no clusters)
   int n_groups, chunk_groups;  // (batch, q head) pairs; how many of them share a launch chunk
   float scale, scale_log2, mask_value;
   uint32_t* err;

@@ -34,6 +34,7 @@
 
 #include "splash_common.cuh"
 #include "splash_fwd_params.cuh"
+#include "splash_split.cuh"
 
 namespace sb {
 
@@ -52,9 +53,14 @@ struct FwdBarriers {
   uint32_t early_exit;
 };
 
-constexpr int fwd_smem_bytes(bool fp8, bool p16 = false) {
-  return (2 + kFwdStages) * (fp8 ? kFp8TileBytes : kTileBytes) + (p16 ? 2 * kTileBytes : 0) /*f16 V tiles*/ +
-         1024 /*barriers*/ + 1024 /*alignment slack*/;
+// kSplit: a CTA's part of the result lies over the operand tiles: 32 x 256 words of 16 bytes, one more row of statistics
+constexpr int kPartBytes = (kHeadDim / 4 + 1) * 2 * kTile * 16;
+__host__ __device__ constexpr int fwd_operand_bytes(bool fp8, bool p16, bool split) {
+  const int tiles = (2 + kFwdStages) * (fp8 ? kFp8TileBytes : kTileBytes) + (p16 ? 2 * kTileBytes : 0) /*f16 V tiles*/;
+  return split && tiles < kPartBytes ? kPartBytes : tiles;
+}
+__host__ __device__ constexpr int fwd_smem_bytes(bool fp8, bool p16, bool split) {
+  return fwd_operand_bytes(fp8, p16, split) + 1024 /*barriers*/ + 1024 /*alignment slack*/;
 }
 
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
@@ -84,12 +90,32 @@ __device__ __forceinline__ void e4m3x4_to_f16x4(uint32_t in, uint32_t& out01, ui
       : "r"(in));
 }
 
+// logsumexp and max_logits of one row: `m` and `l` its maximum in use (log2 units) and sum, `m_true` its true maximum
+template <bool kFp8, bool kSoftCap>
+__device__ __forceinline__ void store_row_stats(const FwdParams& p, int batch, int head, int q_row, bool live, float m,
+                                                float l, float m_true, float sink2, bool fixed_max) {
+  const int64_t stat = ((int64_t)batch * p.q_heads + head) * p.q_len + q_row;
+  if (p.lse) p.lse[stat] = live ? (m + log2f(l)) * kLn2 : p.mask_value;
+  if (p.maxl) {
+    float mv = kFp8 ? m_true * kLn2 : m_true * (kSoftCap ? p.soft_cap : p.scale);
+    if (p.sinks != nullptr) mv = fmaxf(mv, sink2 * kLn2);
+    if (fixed_max) mv = m * kLn2;
+    p.maxl[stat] = live ? mv : p.mask_value;
+  }
+}
+
 // kFp8: e4m3 q / k / v with one scale per 128-token tile.  kP16 (with kFp8): the probabilities stay
 // 16 bits wide — q k^T runs on the e4m3 tiles as they are, each V tile is converted once to f16 in
 // shared memory (exact: e4m3 values are f16 values) by the two otherwise idle warps, and p v runs as
 // an f16 MMA.  That variant meets the bf16 kernel's output bound; the all-e4m3 one does not (P
 // rounded to 3 mantissa bits) but spends half the tensor time on p v.
-template <bool kFp8, bool kSoftCap, bool kP16 = false>
+//
+// kSplit: a cluster of 2 .. 8 CTAs shares one schedule row, each taking its part of the row's kv tiles
+// as if the row held nothing else.  Afterwards every CTA leaves its O (fp32), maximum and sum in its
+// own shared memory (the ring is free by then), and the cluster adds them up over distributed shared
+// memory, each CTA a share of the columns: no scratch in global memory, no second launch, and the
+// order of the additions is fixed.  For grids that leave SMs idle; split_for() holds the rule.
+template <bool kFp8, bool kSoftCap, bool kP16, bool kSplit>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                   const __grid_constant__ CUtensorMap tm_v, const FwdParams p) {
@@ -101,23 +127,30 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   static_assert(!kP16 || kFp8, "the f16-P variant is a variant of the e4m3 forward");
   uint8_t* kv_smem = smem + 2 * kTB;                       // ring
   uint8_t* vc_smem = smem + (2 + kFwdStages) * kTB;        // kP16: two f16 images of V tiles
-  FwdBarriers* bars = reinterpret_cast<FwdBarriers*>(smem + (2 + kFwdStages) * kTB + (kP16 ? 2 * kTileBytes : 0));
+  FwdBarriers* bars = reinterpret_cast<FwdBarriers*>(smem + fwd_operand_bytes(kFp8, kP16, kSplit));
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const CtaWork work = cta_work(p.row_order, p.n_rows, p.n_groups, p.chunk_groups, true);
+  const unsigned rank = kSplit ? cluster_rank() : 0u;
+  const CtaWork work = cta_work_at(kSplit ? blockIdx.x / p.n_split : blockIdx.x, p.row_order, p.n_rows, p.n_groups,
+                                   p.chunk_groups, true);
   const int row = work.row;
   const int head = work.group % p.q_heads;
   const int batch = work.group / p.q_heads;
   const int kv_head = head / (p.q_heads / p.kv_heads);
-  const int ebeg = p.row_ptr[row];
-  const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + row] : p.row_ptr[row + 1];
+  int ebeg = p.row_ptr[row];
+  int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + row] : p.row_ptr[row + 1];
+  if constexpr (kSplit) {
+    const int n = eend - ebeg;
+    eend = ebeg + (int)((int64_t)n * (rank + 1) / p.n_split);
+    ebeg += (int)((int64_t)n * rank / p.n_split);
+  }
   const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
   const int qt0 = row * 2;
 
   if (threadIdx.x == 0) {
     bars->early_exit = *reinterpret_cast<volatile uint32_t*>(p.err);
-    bars->abort_flag = 0;
+    bars->abort_flag = kSplit ? bars->early_exit : 0u;  // (read by the other CTAs of the cluster)
     for (int i = 0; i < 2; ++i) {
       mbar_init(&bars->q_full[i], 1);
       mbar_init(&bars->s_full[i], 1);
@@ -136,7 +169,13 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_fence_init();
   }
   __syncthreads();
-  if (bars->early_exit != 0) return;  // an earlier CTA already reported a fault
+  if (bars->early_exit != 0) {  // an earlier CTA already reported a fault
+    if constexpr (kSplit) {  // the others may not have seen it: no CTA leaves while its shared memory may be read
+      cluster_sync();
+      cluster_sync();
+    }
+    return;
+  }
 
   if (warp == 9) {
     tmem_alloc(&bars->tmem_base, 512);
@@ -386,10 +425,11 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const bool fixed_max = p.max_logit_value != nullptr;
     float sink2 = -INFINITY;  // sink logit in log2 units
     if (p.sinks != nullptr) sink2 = p.sinks[head] * kLog2e;
+    const bool own_sink = p.sinks != nullptr && rank == 0;  // one CTA of a cluster counts it
     if (fixed_max) {
       m_used = p.max_logit_value[head] * kLog2e;
-      if (p.sinks != nullptr) l = ex2(sink2 - m_used);
-    } else if (p.sinks != nullptr) {
+      if (own_sink) l = ex2(sink2 - m_used);
+    } else if (own_sink) {
       m_used = sink2;
       l = 1.f;
     }
@@ -610,7 +650,78 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       ok = mbar_wait(&bars->o_done[i], 0, ab, 0x500u + i);
       ok = __all_sync(0xffffffffu, ok);
     }
-    if (ok && valid) {
+    if constexpr (kSplit) {
+      // this CTA's part of the row, [column / 4][row of the pair] in 16-byte words, then its statistics
+      if (ok && valid) {
+        tc_fence_after();
+        float4* part = reinterpret_cast<float4*>(smem) + threadIdx.x;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint32_t v[32];
+          if (started) {
+            tmem_ld32(t_o + g * 32, v);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = 0u;
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            part[(g * 8 + j) * 2 * kTile] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                        __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+        }
+        part[kHeadDim / 4 * 2 * kTile] = make_float4(m_used, l, m_true, 0.f);
+      }
+      tc_fence_before();
+      cluster_sync();  // (with the same call of the third warpgroup below)
+      bool good = valid;
+      float weight[kMaxSplit];
+      float top = -INFINITY, sum = 0.f, m_all = kMaskedLogit;
+#pragma unroll
+      for (int s = 0; s < kMaxSplit; ++s) {
+        weight[s] = 0.f;
+        if (s < p.n_split) good = good && cluster_ld_u32(cluster_addr(&bars->abort_flag, s)) == 0u;
+      }
+      if (good) {
+        const float4* part = reinterpret_cast<const float4*>(smem) + threadIdx.x;
+        float4 st[kMaxSplit];
+#pragma unroll
+        for (int s = 0; s < kMaxSplit; ++s) {
+          st[s] = make_float4(-INFINITY, 0.f, kMaskedLogit, 0.f);
+          if (s < p.n_split) st[s] = cluster_ld_v4(cluster_addr(part + kHeadDim / 4 * 2 * kTile, s));
+          if (st[s].y != 0.f) top = fmaxf(top, st[s].x);  // (a part without a live key has sum 0; NaN counts)
+          m_all = fmaxf(m_all, st[s].z);
+        }
+#pragma unroll
+        for (int s = 0; s < kMaxSplit; ++s) {
+          if (st[s].y != 0.f) weight[s] = ex2(st[s].x - top);
+          sum = fmaf(st[s].y, weight[s], sum);
+        }
+        const bool live = sum > 0.f;
+        const float inv = live ? (kFp8 ? v_ref * 0.015625f / sum : 1.0f / sum) : 0.f;
+        __nv_bfloat16* orow = p.o + (int64_t)batch * p.o_sb + (int64_t)head * p.o_sh + (int64_t)q_row * p.o_ss;
+        uint4* o4 = reinterpret_cast<uint4*>(orow);
+        uint4* peer4 = p.o_peer.ptrs ? reinterpret_cast<uint4*>(peer_row(p.o_peer, batch, head, q_row)) : nullptr;
+        for (int c = rank; c * 8 < p.d_v; c += p.n_split) {  // eight columns at a time, shared out over the cluster
+          float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+#pragma unroll
+          for (int s = 0; s < kMaxSplit; ++s) {
+            if (s >= p.n_split) break;
+            const float4 u = cluster_ld_v4(cluster_addr(part + (2 * c) * 2 * kTile, s));
+            const float4 w = cluster_ld_v4(cluster_addr(part + (2 * c + 1) * 2 * kTile, s));
+            x.x = fmaf(u.x, weight[s], x.x), x.y = fmaf(u.y, weight[s], x.y);
+            x.z = fmaf(u.z, weight[s], x.z), x.w = fmaf(u.w, weight[s], x.w);
+            y.x = fmaf(w.x, weight[s], y.x), y.y = fmaf(w.y, weight[s], y.y);
+            y.z = fmaf(w.z, weight[s], y.z), y.w = fmaf(w.w, weight[s], y.w);
+          }
+          const uint4 w = make_uint4(pack_bf16(x.x * inv, x.y * inv), pack_bf16(x.z * inv, x.w * inv),
+                                     pack_bf16(y.x * inv, y.y * inv), pack_bf16(y.z * inv, y.w * inv));
+          o4[c] = w;
+          if (peer4) peer4[c] = w;
+        }
+        if (rank == 0) store_row_stats<kFp8, kSoftCap>(p, batch, head, q_row, live, top, sum, m_all, sink2, fixed_max);
+      }
+    } else if (ok && valid) {
       tc_fence_after();
       __nv_bfloat16* orow = p.o + (int64_t)batch * p.o_sb + (int64_t)head * p.o_sh +
                             (int64_t)q_row * p.o_ss;
@@ -643,18 +754,15 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           }
         }
       }
-      const int64_t stat = ((int64_t)batch * p.q_heads + head) * p.q_len + q_row;
-      if (p.lse) p.lse[stat] = live ? (m_used + log2f(l)) * kLn2 : p.mask_value;
-      if (p.maxl) {
-        float mv = kFp8 ? m_true * kLn2 : m_true * (kSoftCap ? p.soft_cap : p.scale);
-        if (p.sinks != nullptr) mv = fmaxf(mv, sink2 * kLn2);
-        if (fixed_max) mv = m_used * kLn2;
-        p.maxl[stat] = live ? mv : p.mask_value;
-      }
+      store_row_stats<kFp8, kSoftCap>(p, batch, head, q_row, live, m_used, l, m_true, sink2, fixed_max);
     }
   }
 
   // ---- teardown
+  if constexpr (kSplit) {
+    if (warp >= 8) cluster_sync();  // the parts are in place
+    cluster_sync();                 // they have been read
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 9) {
@@ -766,34 +874,43 @@ static int launch_fwd_common(const SplashFwdArgs& a, const float* q_scale, const
   p.chunk_groups = chunk_groups_for(Skv * kv_row_bytes / (Hq / Hkv), p.n_groups, Hq / Hkv);
   if (wide) return launch_fwd_wide(tm_q, tm_k, tm_v, p, soft_cap, stream);
   if ((int64_t)p.n_rows * p.n_groups > 0x7fffffffll) return SPLASH_ERR_TOO_LARGE;
-  dim3 grid((unsigned)(p.n_rows * p.n_groups), 1u, 1u);
+  using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FwdParams);
+  static const Kernel kernels[2][4] = {
+      {splash_fwd_kernel<false, false, false, false>, splash_fwd_kernel<true, false, false, false>,
+       splash_fwd_kernel<false, true, false, false>, splash_fwd_kernel<true, false, true, false>},
+      {splash_fwd_kernel<false, false, false, true>, splash_fwd_kernel<true, false, false, true>,
+       splash_fwd_kernel<false, true, false, true>, splash_fwd_kernel<true, false, true, true>}};
+  const int variant = fp8 ? (p16 ? 3 : 1) : (soft_cap ? 2 : 0);
+  // row lengths: a schedule row is 256 query rows
+  const RowWork rw = estimate_row_work(a.mask_fn, a.q_sequence == nullptr, p.n_rows, 2 * kTile, p.n_kv_tiles,
+                                       (int64_t)p.n_rows * p.n_groups);
+  p.n_split = 1;
+  if (rw.longest > 0.f) {
+    const ClusterCapacity* cap = cluster_capacity((const void*)kernels[1][variant], variant, kFwdThreads,
+                                                  fwd_smem_bytes(fp8, p16, true));
+    if (cap == nullptr) return SPLASH_ERR_CUDA;
+    p.n_split = split_for((int64_t)p.n_rows * p.n_groups, rw, *cap);
+  }
+  const bool split = p.n_split > 1;
+  const Kernel kernel = kernels[split][variant];
+  const int smem = fwd_smem_bytes(fp8, p16, split);
   // The dynamic shared-memory attribute is per device and per kernel variant: set once, under a
   // lock (calls may come from several threads).
-  const int variant = fp8 ? (p16 ? 3 : 1) : (soft_cap ? 2 : 0);
-  const int smem = fwd_smem_bytes(fp8, fp8 && p16);
-  const void* fn = fp8 ? (p16 ? (const void*)splash_fwd_kernel<true, false, true> : (const void*)splash_fwd_kernel<true, false>)
-                       : (soft_cap ? (const void*)splash_fwd_kernel<false, true> : (const void*)splash_fwd_kernel<false, false>);
-  {
+  if (!split) {
     static std::mutex attr_mu;
     static bool attr_done[64][4] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SPLASH_ERR_CUDA;
     std::lock_guard<std::mutex> lock(attr_mu);
     if (!attr_done[dev][variant]) {
-      if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      if (cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
         return SPLASH_ERR_CUDA;
       attr_done[dev][variant] = true;
     }
   }
-  if (fp8 && p16)
-    splash_fwd_kernel<true, false, true><<<grid, kFwdThreads, smem, stream>>>(tm_q, tm_k, tm_v, p);
-  else if (fp8)
-    splash_fwd_kernel<true, false><<<grid, kFwdThreads, smem, stream>>>(tm_q, tm_k, tm_v, p);
-  else if (soft_cap)
-    splash_fwd_kernel<false, true><<<grid, kFwdThreads, smem, stream>>>(tm_q, tm_k, tm_v, p);
-  else
-    splash_fwd_kernel<false, false><<<grid, kFwdThreads, smem, stream>>>(tm_q, tm_k, tm_v, p);
-  return cudaGetLastError() == cudaSuccess ? SPLASH_OK : SPLASH_ERR_CUDA;
+  const cudaError_t err = launch_clusters(kernel, (unsigned)(p.n_rows * p.n_groups), p.n_split, kFwdThreads, smem, stream,
+                                          tm_q, tm_k, tm_v, p);
+  return err == cudaSuccess ? SPLASH_OK : SPLASH_ERR_CUDA;
 }
 
 int launch_fwd(const SplashFwdArgs& a, cudaStream_t stream) {

@@ -1,0 +1,139 @@
+// Sharing one schedule row between the CTAs of a cluster: when, between how many, and the launch.
+//
+// The kernels keep one CTA on an SM, so a grid of few long rows leaves SMs idle for the whole launch
+// (512 query rows of 32 heads against 16384 keys: 64 CTAs of 128 steps on 148 SMs).  Measured, one CTA
+// a row -> shared: that forward 240 -> 138.5 us (two CTAs a row); causal 2 x 1024, 8 heads (64 CTAs of 2 .. 8
+// steps, two a row) 24.7 -> 20.9; 256 x 256, 8 heads (2 steps a row) stays whole.
+#pragma once
+
+#include <mutex>
+
+#include "splash_common.cuh"
+
+namespace sb {
+
+constexpr int kMaxSplit = 8;  // portable cluster size
+
+// Steps (128-column tiles) of the longest row and of the average one, from the mask function; a table
+// mask, or rows in another order than their index, count as full.  Segment ids can only shorten rows.
+struct RowWork {
+  float longest, mean;
+};
+struct ClusterCapacity {
+  int clusters[kMaxSplit + 1];  // [n]: clusters of n CTAs that are resident at the same time; [1]: CTAs
+};
+
+constexpr int kSplitMaxCtas = 1024;  // grids above this fill the chip several times over
+
+// rows of `row_span` query rows (transposed = false) or key tiles (true) over `n_steps_full` tiles of the other side
+inline RowWork estimate_row_work(const SplashMaskFn& fn, bool in_order, int n_rows, int row_span, int n_tiles,
+                                 int64_t n_ctas, bool transposed = false) {
+  RowWork w{0.f, 0.f};
+  if (n_ctas > kSplitMaxCtas) return w;
+  w.longest = w.mean = (float)n_tiles;
+  if (!in_order || (fn.kind != SPLASH_MASK_CAUSAL && fn.kind != SPLASH_MASK_LOCAL)) return w;
+  int64_t sum = 0, most = 0;
+  for (int r = 0; r < n_rows; ++r) {
+    // the row sees columns lo .. hi of the other side
+    const int64_t first = (int64_t)r * row_span, last = first + row_span - 1;
+    int64_t lo = 0, hi = (int64_t)n_tiles * kTile - 1;
+    const int64_t left = fn.kind == SPLASH_MASK_LOCAL && fn.has_left ? fn.left : -1;
+    const int64_t right = fn.kind == SPLASH_MASK_CAUSAL ? 0 : (fn.has_right ? fn.right : -1);
+    const bool has_right = fn.kind == SPLASH_MASK_CAUSAL || fn.has_right;
+    const bool has_left = fn.kind == SPLASH_MASK_LOCAL && fn.has_left;
+    if (!transposed) {  // query i sees keys i + offset - left .. i + offset + right
+      if (has_left && first + fn.offset - left > lo) lo = first + fn.offset - left;
+      if (has_right && last + fn.offset + right < hi) hi = last + fn.offset + right;
+    } else {            // key j is seen by queries j - offset - right .. j - offset + left
+      if (has_right && first - fn.offset - right > lo) lo = first - fn.offset - right;
+      if (has_left && last - fn.offset + left < hi) hi = last - fn.offset + left;
+    }
+    const int64_t n = hi < lo ? 0 : hi / kTile - lo / kTile + 1;
+    sum += n;
+    if (n > most) most = n;
+  }
+  w.longest = (float)most;
+  w.mean = n_rows > 0 ? (float)sum / n_rows : 0.f;
+  return w;
+}
+
+// CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (prologue, epilogue; one more
+// for the addition across the cluster).  While everything is resident the longest row sets the time; beyond that the
+// total work over the slots, and half a row for the uneven end.
+inline int split_for(int64_t rows, const RowWork& w, const ClusterCapacity& cap) {
+  constexpr float kFixed = 3.f, kMerge = 1.f;
+  auto time = [&](int n) {
+    const float fixed = kFixed + (n > 1 ? kMerge : 0.f);
+    const float longest = w.longest / n + fixed, mean = w.mean / n + fixed;
+    if (rows <= cap.clusters[n]) return longest;
+    return (float)rows * mean / cap.clusters[n] + 0.5f * longest;
+  };
+  int best = 1;
+  float least = 0.9f * time(1);  // a split has to gain a tenth
+  for (int n = 2; n <= kMaxSplit && n * 2 <= w.longest; ++n)
+    if (cap.clusters[n] > 0 && time(n) < least) {
+      least = time(n);
+      best = n;
+    }
+  return best;
+}
+
+// What fits on the current device, asked once per kernel and device; also sets the kernel's shared-memory size.
+inline const ClusterCapacity* cluster_capacity(const void* kernel, int variant, int threads, int smem) {
+  static std::mutex mu;
+  static ClusterCapacity table[64][16];
+  static bool known[64][16] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || variant < 0 || variant >= 16) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  ClusterCapacity& c = table[dev][variant];
+  if (!known[dev][variant]) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return nullptr;
+    c.clusters[0] = 0;
+    c.clusters[1] = sms;
+    for (int n = 2; n <= kMaxSplit; ++n) {
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = (unsigned)n;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.gridDim = dim3((unsigned)(n * sms));
+      cfg.blockDim = dim3((unsigned)threads);
+      cfg.dynamicSmemBytes = (size_t)smem;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int count = 0;
+      if (cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) != cudaSuccess) {
+        (void)cudaGetLastError();
+        count = 0;
+      }
+      c.clusters[n] = count;
+    }
+    known[dev][variant] = true;
+  }
+  return &c;
+}
+
+template <typename... Params, typename... Args>
+inline cudaError_t launch_clusters(void (*kernel)(Params...), unsigned rows, int n_split, int threads, int smem,
+                                   cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(rows * (unsigned)n_split);
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  if (n_split > 1) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)n_split;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+  }
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+}  // namespace sb
