@@ -1,7 +1,7 @@
 """Grids that leave SMs idle: schedule rows shared by a cluster of CTAs, against the CPU oracle.
 
 A few heads and long rows, so that the launchers take 2 .. 8 CTAs a row: every way of forming a
-row's entries (causal offset, window, segments, table mask), odd numbers of query tiles, parts of
+row's entries (causal offset, window, table mask; segment ids, whose rows stay whole), odd numbers of query tiles, parts of
 unequal length, rows without a live key in some part, sinks (counted once) and a fixed maximum.
 Bounds: those of test_splash_gpu.py, but for outputs of rows with one large weight.
 """
@@ -93,6 +93,43 @@ def test_forward_and_gradients(name, sq, skv, hq, hkv):
     assert ((got[0].float().cpu() - want).norm() / want.norm()).item() <= 1e-2
 
 
+@pytest.mark.parametrize("repeatable", [False, True])
+@pytest.mark.parametrize("name", sorted(CASES))
+def test_gradients_of_one_kv_head(name, repeatable):
+  """Few kv tiles, many steps each (q heads x q tiles): the dkv kernels share the tiles."""
+  make, opt = CASES[name]
+  sq, skv, hq, d = 1152, 640, 8, 64 if name == "window" else 128
+  mask = make(sq, skv)
+  dense = mask if isinstance(mask, np.ndarray) else _dense(mask)
+  q, k, v, do = _mk(0, 1, hq, sq, d), _mk(1, 1, 1, skv, d), _mk(2, 1, 1, skv, d), _mk(3, 1, hq, sq, d)
+  config = splash.SplashConfig.get_default()
+  if "cap" in opt:
+    config = dataclasses.replace(config, attn_logits_soft_cap=opt["cap"])
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1, config=config, repeatable_dq=repeatable)
+  seg = None
+  if opt.get("segments"):
+    seg = ((torch.arange(sq) * 3 // sq)[None].int(), (torch.arange(skv) * 3 // skv)[None].int())
+  scale = 1 / math.sqrt(d)
+  got = []
+  for _ in range(2):
+    qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+    out = kernel(qd, kd, vd, None if seg is None else splash.SegmentIds(*(s.to(DEV) for s in seg)), logits_scale=scale)
+    out.backward(do.to(DEV))
+    got.append((qd.grad, kd.grad, vd.grad))
+  kernel.check_errors()
+  assert torch.equal(got[0][1], got[1][1]) and torch.equal(got[0][2], got[1][2])  # dk, dv: always repeatable
+  assert not repeatable or torch.equal(got[0][0], got[1][0])
+  pair = None if seg is None else (seg[0][0], seg[1][0])
+  ro, rlse, _ = attention_ref.attention_reference(q[0], k[0], v[0], dense, pair, scale=scale,
+                                                  attn_logits_soft_cap=opt.get("cap"))
+  live = rlse > -1e30
+  ro, rlse = torch.where(live[..., None], ro, 0.0), torch.where(live, rlse, float("inf"))
+  grads = attention_ref.attention_reference_vjp(do[0], q[0], k[0], v[0], dense, pair, ro, rlse, scale=scale,
+                                                attn_logits_soft_cap=opt.get("cap"))
+  for g, want in zip(got[0], grads):
+    assert ((g[0].float().cpu() - want).norm() / want.norm()).item() <= 1e-2
+
+
 @pytest.mark.parametrize("p_format,rel", [("e4m3", 3e-2), ("f16", 5e-3)])
 @pytest.mark.parametrize("sq,skv", [(128, 4096), (384, 2944)])
 def test_e4m3_forward(p_format, rel, sq, skv):
@@ -109,16 +146,14 @@ def test_e4m3_forward(p_format, rel, sq, skv):
 
 
 def test_parts_without_a_live_key():
-  """Only the last tile of a long row is live: every other part of the cluster ends with sum 0."""
+  """Every row is live in one tile only, every tile in some row: most parts of a cluster end with sum 0."""
   sq, skv = 256, 4096
+  dense = np.zeros((sq, skv), np.bool_)
+  dense[np.arange(sq), (np.arange(sq) * 128 + 17) % skv] = True
   q, k, v = _mk(0, 1, 2, sq, 128), _mk(1, 1, 2, skv, 128), _mk(2, 1, 2, skv, 128)
-  live_everywhere = np.ones((sq, skv), np.bool_)
-  ids = torch.zeros(1, skv, dtype=torch.int32)
-  ids[:, 1:-1] = 1  # tiles stay in the schedule, their keys belong to another segment
-  kernel = splash.make_splash_mha(mask_lib.FullMask((sq, skv)), q_seq_shards=1, save_residuals=True)
-  qs = torch.zeros(1, sq, dtype=torch.int32)
-  out, res = kernel(q.to(DEV), k.to(DEV), v.to(DEV), splash.SegmentIds(qs.to(DEV), ids.to(DEV)), logits_scale=0.1)
+  kernel = splash.make_splash_mha(dense, q_seq_shards=1, save_residuals=True)
+  out, res = kernel(q.to(DEV), k.to(DEV), v.to(DEV), logits_scale=0.1)
   kernel.check_errors()
-  ro, rlse, _ = attention_ref.attention_reference(q[0], k[0], v[0], live_everywhere, (qs[0], ids[0]), scale=0.1)
+  ro, rlse, _ = attention_ref.attention_reference(q[0], k[0], v[0], dense, scale=0.1)
   assert (out[0].float().cpu() - ro).abs().max().item() <= 1e-2
   assert (res["logsumexp"][0].cpu() - rlse).abs().max().item() <= 1e-3

@@ -882,10 +882,10 @@ static int launch_fwd_common(const SplashFwdArgs& a, const float* q_scale, const
        splash_fwd_kernel<false, true, false, true>, splash_fwd_kernel<true, false, true, true>}};
   const int variant = fp8 ? (p16 ? 3 : 1) : (soft_cap ? 2 : 0);
   // row lengths: a schedule row is 256 query rows
-  const RowWork rw = estimate_row_work(a.mask_fn, a.q_sequence == nullptr, p.n_rows, 2 * kTile, p.n_kv_tiles,
+  const RowWork rw = estimate_row_work(a.mask_fn, p.n_rows, 2 * kTile, p.n_kv_tiles,
                                        (int64_t)p.n_rows * p.n_groups);
   p.n_split = 1;
-  if (rw.longest > 0.f) {
+  if (a.q_segment_ids == nullptr && a.q_sequence == nullptr && rw.longest > 0.f) {
     const ClusterCapacity* cap = cluster_capacity((const void*)kernels[1][variant], variant, kFwdThreads,
                                                   fwd_smem_bytes(fp8, p16, true));
     if (cap == nullptr) return SPLASH_ERR_CUDA;

@@ -2,8 +2,8 @@
 //
 // The kernels keep one CTA on an SM, so a grid of few long rows leaves SMs idle for the whole launch
 // (512 query rows of 32 heads against 16384 keys: 64 CTAs of 128 steps on 148 SMs).  Measured, one CTA
-// a row -> shared: that forward 240 -> 138.5 us (two CTAs a row); causal 2 x 1024, 8 heads (64 CTAs of 2 .. 8
-// steps, two a row) 24.7 -> 20.9; 256 x 256, 8 heads (2 steps a row) stays whole.
+// a row -> shared: that forward 240 -> 138 us (two CTAs a row); dkv of causal 2 x 4096, 16 q heads
+// on one kv head, d 64 (64 CTAs of 16 .. 512 steps) 745 -> 245 (eight a tile).
 #pragma once
 
 #include <mutex>
@@ -15,7 +15,10 @@ namespace sb {
 constexpr int kMaxSplit = 8;  // portable cluster size
 
 // Steps (128-column tiles) of the longest row and of the average one, from the mask function; a table
-// mask, or rows in another order than their index, count as full.  Segment ids can only shorten rows.
+// mask counts as full.  Not asked for calls with q_sequence either: a shard of the query rows gives the
+// bits that the whole gives while both leave their rows whole.  Not asked for calls with segment
+// ids: they cut rows at places that only the device knows, and a schedule filtered by them gives bit for
+// bit what an unfiltered one gives only while no row is cut into parts by its number of entries.
 struct RowWork {
   float longest, mean;
 };
@@ -26,12 +29,12 @@ struct ClusterCapacity {
 constexpr int kSplitMaxCtas = 1024;  // grids above this fill the chip several times over
 
 // rows of `row_span` query rows (transposed = false) or key tiles (true) over `n_steps_full` tiles of the other side
-inline RowWork estimate_row_work(const SplashMaskFn& fn, bool in_order, int n_rows, int row_span, int n_tiles,
+inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_span, int n_tiles,
                                  int64_t n_ctas, bool transposed = false) {
   RowWork w{0.f, 0.f};
   if (n_ctas > kSplitMaxCtas) return w;
   w.longest = w.mean = (float)n_tiles;
-  if (!in_order || (fn.kind != SPLASH_MASK_CAUSAL && fn.kind != SPLASH_MASK_LOCAL)) return w;
+  if (fn.kind != SPLASH_MASK_CAUSAL && fn.kind != SPLASH_MASK_LOCAL) return w;
   int64_t sum = 0, most = 0;
   for (int r = 0; r < n_rows; ++r) {
     // the row sees columns lo .. hi of the other side
@@ -59,9 +62,12 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, bool in_order, int n_ro
 
 // CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (prologue, epilogue; one more
 // for the addition across the cluster).  While everything is resident the longest row sets the time; beyond that the
-// total work over the slots, and half a row for the uneven end.
+// total work over the slots, and half a row for the uneven end.  Rows below 16 steps stay whole: little
+// is left to gain there (causal 2 x 1024, 8 heads, 64 CTAs of 2 .. 8 steps: 24.7 us, 20.9 with two CTAs a row),
+// and short sequences give the same bits whatever else is in the launch.
 inline int split_for(int64_t rows, const RowWork& w, const ClusterCapacity& cap) {
-  constexpr float kFixed = 3.f, kMerge = 1.f;
+  constexpr float kFixed = 3.f, kMerge = 1.f, kFewest = 16.f;
+  if (w.longest < kFewest) return 1;
   auto time = [&](int n) {
     const float fixed = kFixed + (n > 1 ? kMerge : 0.f);
     const float longest = w.longest / n + fixed, mean = w.mean / n + fixed;

@@ -192,7 +192,8 @@ class _DeviceTables:
     if q_seq is not None and n_shards > 1:  # global q indices of this shard's rows
       q_seq = np.asarray(q_seq)[shard * q_len:(shard + 1) * q_len]
     self.q_sequence = None
-    if q_seq is not None and not np.array_equal(np.asarray(q_seq), np.arange(q_len, dtype=np.int32)):
+    # (the first shard keeps its indices too: with them the kernels leave every shard's rows whole, as one)
+    if q_seq is not None and (n_shards > 1 or not np.array_equal(np.asarray(q_seq), np.arange(q_len, dtype=np.int32))):
       self.q_sequence = torch.from_numpy(np.ascontiguousarray(q_seq, dtype=np.int32)).to(device)
 
   def _upload(self, state, pid, bq, bkv, kind, pmb, device) -> _native.SplashDeviceSchedule:
