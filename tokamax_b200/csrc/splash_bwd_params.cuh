@@ -34,6 +34,7 @@ struct BwdParams {
   int q_len, kv_len, q_heads, kv_heads, n_rows;
   int d_qk, d_v;               // real columns of q / k / dq / dk and of v / o / do / dv (<= 128)
   int nk_qk, nk_v;             // K = 16 slices with real columns in contractions over d_qk / d_v
+  int n_split;                 // dkv kernel: CTAs of a cluster that share a kv tile (1: no clusters)
   int n_groups, chunk_groups;  // (batch, head) pairs of the grid; how many share a launch chunk
   // soft-cap variants: logits = cap * tanh(scale * q k^T / cap); dS gains the factor 1 - tanh^2
   float soft_cap, softcap_a;   // cap; scale / cap

@@ -30,6 +30,7 @@
 
 #include "splash_common.cuh"
 #include "splash_bwd_params.cuh"
+#include "splash_split.cuh"
 
 namespace sb {
 
@@ -515,7 +516,15 @@ struct DkvBarriers {
 };
 static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 
-template <bool kSoftCap, bool kFuseDq>
+//
+// kSplit: a cluster of 2 .. 8 CTAs shares one kv tile, each taking a run of its steps (q head, q tile).
+// At the end every CTA leaves its dK and dV (fp32) in its own shared memory and the cluster adds them
+// up over distributed shared memory in rank order, each CTA a share of the columns: no atomics, still
+// bitwise repeatable.  For grids that leave SMs idle; split_for() holds the rule.
+constexpr int kDkvPartWords = 2 * kHeadDim / 4 * kTile;  // 16-byte words: [dk, dv column / 4][kv row]
+static_assert(kDkvPartWords * 16 <= (3 + kBwdStages) * kTileBytes, "the parts lie over the operand tiles");
+
+template <bool kSoftCap, bool kFuseDq, bool kSplit>
 __global__ void __launch_bounds__(kFuseDq ? kFusedThreads : kDkvThreads, 1)
 splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -531,7 +540,9 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const CtaWork work = cta_work(p.row_order, p.n_rows, p.n_groups, p.chunk_groups, false);
+  const unsigned rank = kSplit ? cluster_rank() : 0u;
+  const CtaWork work = cta_work_at(kSplit ? blockIdx.x / p.n_split : blockIdx.x, p.row_order, p.n_rows, p.n_groups,
+                                   p.chunk_groups, false);
   const int kv_tile = work.row;
   const int kv_head = work.group % p.kv_heads;
   const int batch = work.group / p.kv_heads;
@@ -540,7 +551,16 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + kv_tile] : p.row_ptr[kv_tile + 1];
   const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
   const int n_ent = eend - ebeg;
-  const int n_steps = n_ent * group;
+  // steps of this CTA: (q head g of the group, entry e) pairs in that order, from (first_g, first_e)
+  int n_steps = n_ent * group, first_g = 0, first_e = ebeg;
+  if constexpr (kSplit) {
+    const int total = n_steps, from = (int)((int64_t)total * rank / p.n_split);
+    n_steps = (int)((int64_t)total * (rank + 1) / p.n_split) - from;
+    if (n_ent > 0) {
+      first_g = from / n_ent;
+      first_e = ebeg + from % n_ent;
+    }
+  }
 
   if (threadIdx.x == 0) {
     // The operand tiles need a 1024-byte aligned base for the 128-byte swizzle; there is no
@@ -555,7 +575,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       bad = 2u;
     }
     bars->early_exit = bad;
-    bars->abort_flag = 0;
+    bars->abort_flag = kSplit ? bad : 0u;  // (read by the other CTAs of the cluster)
     mbar_init(&bars->stat_full[0], 1);
     mbar_init(&bars->stat_full[1], 1);
     for (int s = 0; s < kBwdStages; ++s) {
@@ -573,7 +593,13 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_fence_init();
   }
   __syncthreads();
-  if (bars->early_exit != 0) return;
+  if (bars->early_exit != 0) {
+    if constexpr (kSplit) {  // the others may not have seen it: no CTA leaves while its shared memory may be read
+      cluster_sync();
+      cluster_sync();
+    }
+    return;
+  }
   if (warp == kDkvMmaWarp) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
@@ -596,10 +622,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int n_q_tiles = p.q_len / kTile;
     bool ok = true;
     uint32_t n = 0;
-    for (int g = 0; g < group && ok; ++g) {
+    for (int g = first_g, e = first_e; n < (uint32_t)n_steps && ok; ++g, e = ebeg) {
       const int head = kv_head * group + g;
       float* head_base = p.dq_acc + ((int64_t)batch * p.q_heads + head) * n_q_tiles * (int64_t)kDqTileFloats + r * 4;
-      for (int e = ebeg; e < eend && ok; ++e, ++n) {
+      for (; e < eend && (!kSplit || n < (uint32_t)n_steps) && ok; ++e, ++n) {
         float* dst = head_base + (int64_t)entries[e].x * kDqTileFloats;
         ok = mbar_wait(&bars->dq_full, n & 1u, ab, 0x3600u);
         ok = __all_sync(0xffffffffu, ok);
@@ -641,10 +667,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (v2) tma_load_4d(v_smem + kHalfBytes, &tm_v, &bars->stat_full[1], 64, kv_tile * kTile, kv_head, batch);
       uint32_t it = 0;
       bool ok = true;
-      for (int g = 0; g < group && ok; ++g) {
+      for (int g = first_g, e = first_e; it < 2u * (uint32_t)n_steps && ok; ++g, e = ebeg) {
         const int head = kv_head * group + g;
         const int64_t stat_base = ((int64_t)batch * p.q_heads + head) * p.q_len;
-        for (int e = ebeg; e < eend && ok; ++e) {
+        for (; e < eend && (!kSplit || it < 2u * (uint32_t)n_steps) && ok; ++e) {
           const int qt = entries[e].x;
           for (int which = 0; which < 2 && ok; ++which, ++it) {
             const uint32_t s = it % kBwdStages;
@@ -787,9 +813,9 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     bool ok = true;
     int n = 0;
 
-    for (int g = 0; g < group && ok; ++g) {
-      int4 ent_next = n_ent > 0 ? entries[ebeg] : make_int4(0, 0, 0, 0);
-      for (int e = ebeg; e < eend && ok; ++e, ++n) {
+    for (int g = first_g, e = first_e; n < n_steps && ok; ++g, e = ebeg) {
+      int4 ent_next = entries[e];
+      for (; e < eend && (!kSplit || n < n_steps) && ok; ++e, ++n) {
         const int4 ent = ent_next;
         if (e + 1 < eend) ent_next = entries[e + 1];
         const int st = ent.y & 3;
@@ -932,7 +958,55 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
                         (int64_t)kv_row * p.out0_ss + cq * 32;
     __nv_bfloat16* dv = p.out1 + (int64_t)batch * p.out1_sb + (int64_t)kv_head * p.out1_sh +
                         (int64_t)kv_row * p.out1_ss + cq * 32;
-    if (n_steps > 0) {
+    if constexpr (kSplit) {
+      if (n_steps > 0 && ok) {
+        ok = mbar_wait(&bars->acc_done, 0, ab, 0x3500u);
+        ok = __all_sync(0xffffffffu, ok);
+      }
+      float4* part = reinterpret_cast<float4*>(smem) + r;
+      if (ok) {
+        tc_fence_after();
+#pragma unroll
+        for (int which = 0; which < 2; ++which) {  // dk, dv: columns cq * 32 .. + 31
+          uint32_t v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0u;
+          if (n_steps > 0) {
+            tmem_ld32(tmem + lane_addr + (2 + which) * kTile + cq * 32, v);
+            tmem_ld_wait();
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            part[(which * (kHeadDim / 4) + cq * 8 + j) * kTile] =
+                make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]),
+                            __uint_as_float(v[4 * j + 3]));
+        }
+      }
+      tc_fence_before();
+      cluster_sync();  // (with the same call of the other warps below)
+      bool good = true;
+      for (int s = 0; s < p.n_split; ++s) good = good && cluster_ld_u32(cluster_addr(&bars->abort_flag, s)) == 0u;
+      if (good) {
+        // groups of eight columns (16 of dk, 16 of dv) shared out over the cluster's warps; lane = row
+        for (int c = (int)rank * 4 + cq; c < 2 * kHeadDim / 8; c += 4 * p.n_split) {
+          const int which = c / (kHeadDim / 8), col = (c % (kHeadDim / 8)) * 8;
+          if (col >= (which ? p.d_v : p.d_qk)) continue;
+          float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+          for (int s = 0; s < p.n_split; ++s) {
+            const float4 u = cluster_ld_v4(cluster_addr(part + (2 * c) * kTile, s));
+            const float4 w = cluster_ld_v4(cluster_addr(part + (2 * c + 1) * kTile, s));
+            x.x += u.x, x.y += u.y, x.z += u.z, x.w += u.w;
+            y.x += w.x, y.y += w.y, y.z += w.z, y.w += w.w;
+          }
+          const float mul = which ? 1.0f : p.scale;
+          const uint4 w = make_uint4(pack_bf16(x.x * mul, x.y * mul), pack_bf16(x.z * mul, x.w * mul),
+                                     pack_bf16(y.x * mul, y.y * mul), pack_bf16(y.z * mul, y.w * mul));
+          const SplashPeerOutput& peer = which ? p.out1_peer : p.out0_peer;
+          *reinterpret_cast<uint4*>((which ? dv : dk) - cq * 32 + col) = w;
+          if (peer.ptrs) *reinterpret_cast<uint4*>(peer_row(peer, batch, kv_head, kv_row) + col) = w;
+        }
+      }
+    } else if (n_steps > 0) {
       if (ok) {
         ok = mbar_wait(&bars->acc_done, 0, ab, 0x3500u);
         ok = __all_sync(0xffffffffu, ok);
@@ -961,6 +1035,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
   }
 
+  if constexpr (kSplit) {
+    if (warp >= 16) cluster_sync();  // the parts are in place
+    cluster_sync();                  // they have been read
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == kDkvMmaWarp) {
@@ -1112,8 +1190,8 @@ int launch_bwd(const SplashBwdArgs& a, cudaStream_t stream) {
   const bool soft_cap = a.soft_cap != 0.f;
   if (soft_cap && !(a.soft_cap > 0.f)) return SPLASH_ERR_INVALID_ARGUMENT;
   auto* dq_kernel = soft_cap ? splash_dq_kernel<true> : splash_dq_kernel<false>;
-  auto* dkv_kernel = fused ? (soft_cap ? splash_dkv_kernel<true, true> : splash_dkv_kernel<false, true>)
-                           : (soft_cap ? splash_dkv_kernel<true, false> : splash_dkv_kernel<false, false>);
+  auto* dkv_kernel = fused ? (soft_cap ? splash_dkv_kernel<true, true, false> : splash_dkv_kernel<false, true, false>)
+                           : (soft_cap ? splash_dkv_kernel<true, false, false> : splash_dkv_kernel<false, false, false>);
   const int dkv_smem = kDkvSmemBytes;
   // function attributes are per device: remember which devices have been set up
   {
@@ -1207,10 +1285,26 @@ int launch_bwd(const SplashBwdArgs& a, cudaStream_t stream) {
   // (fused: plus the fp32 dQ image of those heads, which the reds keep in L2)
   p.chunk_groups = chunk_groups_for((Hq / Hkv) * Sq * kHeadDim * (fused ? 8 : 4), p.n_groups, 1);
   if ((int64_t)p.n_rows * p.n_groups > 0x7fffffffll) return SPLASH_ERR_TOO_LARGE;
-  if (mask & 4u)
-    dkv_kernel<<<dim3((unsigned)(p.n_rows * p.n_groups), 1u, 1u), fused ? kFusedThreads : kDkvThreads, dkv_smem,
-                 stream>>>(tm_q, tm_do, tm_k, tm_v, p);
-  if (cudaGetLastError() != cudaSuccess) return SPLASH_ERR_CUDA;
+  if (mask & 4u) {
+    const int64_t n_ctas = (int64_t)p.n_rows * p.n_groups;
+    const int threads = fused ? kFusedThreads : kDkvThreads;
+    RowWork rw = estimate_row_work(a.mask_fn, p.n_rows, kTile, (int)(Sq / kTile), n_ctas, true);
+    p.n_split = 1;
+    if (a.q_segment_ids == nullptr && a.q_sequence == nullptr && rw.longest > 0.f) {
+      auto* split_kernel = fused ? (soft_cap ? splash_dkv_kernel<true, true, true> : splash_dkv_kernel<false, true, true>)
+                                 : (soft_cap ? splash_dkv_kernel<true, false, true> : splash_dkv_kernel<false, false, true>);
+      rw.longest *= (float)(Hq / Hkv);  // a kv tile walks every q head of its group
+      rw.mean *= (float)(Hq / Hkv);
+      const ClusterCapacity* cap = cluster_capacity((const void*)split_kernel, 4 + (soft_cap ? 1 : 0) + (fused ? 2 : 0),
+                                                    threads, dkv_smem);
+      if (cap == nullptr) return SPLASH_ERR_CUDA;
+      p.n_split = split_for(n_ctas, rw, *cap);
+      if (p.n_split > 1) dkv_kernel = split_kernel;
+    }
+    if (launch_clusters(dkv_kernel, (unsigned)n_ctas, p.n_split, threads, dkv_smem, stream, tm_q, tm_do, tm_k, tm_v, p) !=
+        cudaSuccess)
+      return SPLASH_ERR_CUDA;
+  }
   if (fused && (mask & 2u)) {
     DqConvertParams cp;
     cp.acc = dq_acc;
