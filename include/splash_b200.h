@@ -209,6 +209,9 @@ int splash_segment_schedule(const SplashDeviceSchedule* in, int32_t kind, const 
  * bool or int8 array), 16-byte aligned rows (`row_stride_bytes` a multiple of 16); writes the state
  * of every 128x128 tile (0 empty, 1 partial, 2 full) to `states` [q_len / 128, kv_len / 128].
  *
+ * splash_mask_prepare: the same states, and in the same pass a dense copy of the mask (`copy`, [q_len,
+ * kv_len]) and its transpose (`transposed`, [kv_len, q_len]), both 16-byte aligned.
+ *
  * splash_dynamic_schedule: turns `states` into a schedule of `kind` (as in splash_schedule_build)
  * inside `workspace` (splash_dynamic_schedule_bytes bytes, 256-byte aligned): rows at a fixed
  * stride with `row_end` replicated for `batch` rows.  `partial_blocks` is what the attention
@@ -219,6 +222,8 @@ int splash_segment_schedule(const SplashDeviceSchedule* in, int32_t kind, const 
  * ---------------------------------------------------------------------------------------- */
 int splash_mask_tile_states(const void* mask, int64_t row_stride_bytes, int64_t q_len, int64_t kv_len,
                             int32_t* states, void* cuda_stream);
+int splash_mask_prepare(const void* mask, int64_t row_stride_bytes, int64_t q_len, int64_t kv_len, void* copy,
+                        void* transposed, int32_t* states, void* cuda_stream);
 size_t splash_dynamic_schedule_bytes(int64_t q_len, int64_t kv_len, int32_t kind, int64_t batch);
 int splash_dynamic_schedule(const int32_t* states, int64_t q_len, int64_t kv_len, int32_t kind, int64_t batch,
                             const void* partial_blocks, void* workspace, size_t workspace_bytes,

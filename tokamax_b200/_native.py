@@ -217,6 +217,8 @@ _PROTOTYPES = {
                                           C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_size_t,
                                           C.POINTER(SplashDeviceSchedule), C.c_void_p]),
     "splash_mask_tile_states": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p]),
+    "splash_mask_prepare": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p,
+                                      C.c_void_p]),
     "splash_dynamic_schedule_bytes": (C.c_size_t, [C.c_int64, C.c_int64, C.c_int32, C.c_int64]),
     "splash_dynamic_schedule": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_int64, C.c_void_p,
                                           C.c_void_p, C.c_size_t, C.POINTER(SplashDeviceSchedule), C.c_void_p]),

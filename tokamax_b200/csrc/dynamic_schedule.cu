@@ -51,6 +51,52 @@ splash_mask_tile_state_kernel(const uint8_t* __restrict__ mask, int64_t row_stri
   }
 }
 
+// The same states, and on the way the two images of the mask that the attention kernels read: a copy
+// and its transpose.  One CTA per tile: the tile's 128 rows of 128 bytes pass through shared memory
+// as 32-bit words (skewed by the group of four rows, so that rows and columns of words are both free of bank
+// conflicts); 4 x 4 byte blocks are transposed with byte permutes and leave as whole 128-byte rows.
+// HBM-bound: a byte read and two written per mask element; 4096 x 4096 in 10.7 us (4.7 TB/s), where copy (7 us), states
+// (6 us) and a byte-wise strided transpose (66 us) were three passes before.
+constexpr int kPrepThreads = 256;
+__global__ void __launch_bounds__(kPrepThreads)
+splash_mask_prepare_kernel(const uint8_t* __restrict__ mask, int64_t row_stride, int q_len, int kv_len,
+                           uint8_t* __restrict__ copy, uint8_t* __restrict__ transposed, int32_t* __restrict__ states) {
+  const int kt = blockIdx.x, qt = blockIdx.y;
+  __shared__ uint32_t tile[kTile * 32];
+  auto word = [&](int r, int c) -> uint32_t& { return tile[r * 32 + ((c + (r >> 2)) & 31)]; };
+  bool any = false, all = true;
+#pragma unroll
+  for (int i = 0; i < kTile * 8 / kPrepThreads; ++i) {
+    const int idx = i * kPrepThreads + threadIdx.x, r = idx >> 3, c = (idx & 7) * 4;
+    const int64_t q = (int64_t)qt * kTile + r;
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(mask + q * row_stride + (int64_t)kt * kTile) + (idx & 7));
+    *(reinterpret_cast<uint4*>(copy + q * kv_len + (int64_t)kt * kTile) + (idx & 7)) = v;
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      word(r, c + j) = w[j];
+      any |= w[j] != 0u;
+      all &= ((w[j] - 0x01010101u) & ~w[j] & 0x80808080u) == 0u;  // no zero byte in the word
+    }
+  }
+  const int tile_any = __syncthreads_or(any);
+  const int tile_all = __syncthreads_and(all);
+  if (threadIdx.x == 0) states[(int64_t)qt * (kv_len / kTile) + kt] = tile_any ? (tile_all ? 2 : 1) : 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int i = 0; i < 32 / (kPrepThreads / 32); ++i) {
+    const int c = i * (kPrepThreads / 32) + warp;  // word column: four keys; lane: four queries
+    const uint32_t a = word(4 * lane, c), b = word(4 * lane + 1, c), d = word(4 * lane + 2, c), e = word(4 * lane + 3, c);
+    const uint32_t ab_lo = __byte_perm(a, b, 0x5140), ab_hi = __byte_perm(a, b, 0x7362);  // a0 b0 a1 b1 / a2 b2 a3 b3
+    const uint32_t de_lo = __byte_perm(d, e, 0x5140), de_hi = __byte_perm(d, e, 0x7362);
+    const uint32_t out[4] = {__byte_perm(ab_lo, de_lo, 0x5410), __byte_perm(ab_lo, de_lo, 0x7632),
+                             __byte_perm(ab_hi, de_hi, 0x5410), __byte_perm(ab_hi, de_hi, 0x7632)};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      reinterpret_cast<uint32_t*>(transposed + ((int64_t)kt * kTile + 4 * c + j) * q_len + (int64_t)qt * kTile)[lane] = out[j];
+  }
+}
+
 // One CTA per schedule row: compacts the live tiles of the row, in order, into its fixed-stride
 // slot.  kind 0: row = pair of q tiles, entries = kv tiles; kind 1: row = q tile; kind 2: row = kv
 // tile, entries = q tiles.  Partial tiles get block id 0 (the whole mask is the one block).
@@ -128,6 +174,22 @@ int splash_mask_tile_states(const void* mask, int64_t row_stride_bytes, int64_t 
   sb::splash_mask_tile_state_kernel<<<dim3((unsigned)nkv, (unsigned)nq), sb::kDynThreads, 0,
                                       static_cast<cudaStream_t>(cuda_stream)>>>(
       static_cast<const uint8_t*>(mask), row_stride_bytes, (int)nkv, states);
+  return cudaGetLastError() == cudaSuccess ? SPLASH_OK : SPLASH_ERR_CUDA;
+}
+
+int splash_mask_prepare(const void* mask, int64_t row_stride_bytes, int64_t q_len, int64_t kv_len, void* copy,
+                        void* transposed, int32_t* states, void* cuda_stream) {
+  if (mask == nullptr || states == nullptr || copy == nullptr || transposed == nullptr) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (q_len <= 0 || kv_len <= 0 || q_len % sb::kTile != 0 || kv_len % sb::kTile != 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (row_stride_bytes < kv_len || row_stride_bytes % 16 != 0 || (reinterpret_cast<uintptr_t>(mask) & 15u) != 0 ||
+      (reinterpret_cast<uintptr_t>(copy) & 15u) != 0 || (reinterpret_cast<uintptr_t>(transposed) & 15u) != 0)
+    return SPLASH_ERR_INVALID_ARGUMENT;
+  const int64_t nq = q_len / sb::kTile, nkv = kv_len / sb::kTile;
+  if (nq > 65535 || q_len > 0x7fffffffll || kv_len > 0x7fffffffll) return SPLASH_ERR_TOO_LARGE;
+  sb::splash_mask_prepare_kernel<<<dim3((unsigned)nkv, (unsigned)nq), sb::kPrepThreads, 0,
+                                   static_cast<cudaStream_t>(cuda_stream)>>>(
+      static_cast<const uint8_t*>(mask), row_stride_bytes, (int)q_len, (int)kv_len, static_cast<uint8_t*>(copy),
+      static_cast<uint8_t*>(transposed), states);
   return cudaGetLastError() == cudaSuccess ? SPLASH_OK : SPLASH_ERR_CUDA;
 }
 

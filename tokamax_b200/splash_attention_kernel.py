@@ -234,16 +234,17 @@ class _DynamicDeviceTables:
       raise NotImplementedError(f"mask sides must be multiples of {_TILE} on B200, got {tuple(mask.shape)}")
     # Snapshot: the kernels read the mask in place on every call, so a copy is kept; a caller who
     # updates its tensor afterwards builds a new kernel object.
-    m = mask.contiguous().view(torch.uint8).clone()
-    mt = m.t().contiguous()
-    if mt.data_ptr() % 16:
-      mt = mt.clone()
+    src = mask.view(torch.uint8)
+    if src.stride(1) != 1 or src.stride(0) < kv_len or src.stride(0) % 16 or src.data_ptr() % 16:
+      src = src.clone(memory_format=torch.contiguous_format)  # rows the kernel cannot read in place
+    m = torch.empty((q_len, kv_len), dtype=torch.uint8, device=device)
+    mt = torch.empty((kv_len, q_len), dtype=torch.uint8, device=device)
     states = torch.empty((q_len // _TILE, kv_len // _TILE), dtype=torch.int32, device=device)
     stream = C.c_void_p(torch.cuda.current_stream(device).cuda_stream)
     self.keep = [m, mt, states]
     with torch.cuda.device(device):
-      _native.check(lib.splash_mask_tile_states(m.data_ptr(), m.stride(0), q_len, kv_len, states.data_ptr(), stream),
-                    "splash_mask_tile_states")
+      _native.check(lib.splash_mask_prepare(src.data_ptr(), src.stride(0), q_len, kv_len, m.data_ptr(), mt.data_ptr(),
+                                            states.data_ptr(), stream), "splash_mask_prepare")
       scheds = []
       for kind, blocks in ((0, m), (1, m), (2, mt)):
         nbytes = lib.splash_dynamic_schedule_bytes(q_len, kv_len, kind, batch)
