@@ -64,6 +64,11 @@ int check_e4m3_tensor(const SplashTensor& t) {
 int make_tile_tensor_map(CUtensorMap* out, const SplashTensor& t, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return SPLASH_ERR_NO_DEVICE;
+  // The encoder is a driver call and needs a current context.  A thread that has made no runtime call
+  // of its own (autograd's, for a first backward small enough to find its memory cached) has none, although
+  // its device is right; cudaSetDevice binds it.
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return SPLASH_ERR_CUDA;
   const bool fp8 = t.dtype == SPLASH_F8E4M3;
   const cuuint64_t esize = fp8 ? 1u : 2u;
   const cuuint64_t dims[4] = {(cuuint64_t)t.size[3], (cuuint64_t)t.size[2], (cuuint64_t)t.size[1],
