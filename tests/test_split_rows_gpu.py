@@ -157,3 +157,52 @@ def test_parts_without_a_live_key():
   ro, rlse, _ = attention_ref.attention_reference(q[0], k[0], v[0], dense, scale=0.1)
   assert (out[0].float().cpu() - ro).abs().max().item() <= 1e-2
   assert (res["logsumexp"][0].cpu() - rlse).abs().max().item() <= 1e-3
+
+
+INF = float("inf")
+
+
+def _dead_rows(kind):
+  """Masks whose query rows have live keys in no part of a cluster, in one part only, or in all."""
+  if kind == "shifted":  # the first half of the rows sees nothing and has no schedule entry at all
+    return mask_lib.CausalMask((4096, 2048), -2048)
+  m = np.zeros((512, 4096), np.bool_)
+  m[0:128, 2048:] = True        # query tile 0 is live in the second half of the keys,
+  m[::3] = False                # but for every third row;
+  m[200, 128 * 5 + 3] = True    # tile 1 has one live row, in a single key tile (fewer entries than parts);
+  m[256:384, :] = True          # tile 3, of a live pair, is dead
+  return m
+
+
+@pytest.mark.parametrize("form", ["bf16", "e4m3", "f16"])
+@pytest.mark.parametrize("kind", ["shifted", "table"])
+def test_infinite_sinks(kind, form):
+  """A sink of -inf is a head without one and +inf takes all the weight: dead rows come out 0, also where
+  the part that counts the sink holds no live key.  Their logsumexp is the sink, but for a sink of -inf in
+  tiles that hold other rows' keys: there it is the mask value, as for any row without a live key."""
+  mask = _dead_rows(kind)
+  dense = mask if isinstance(mask, np.ndarray) else _dense(mask)
+  sq, skv = dense.shape
+  q, k, v = _mk(0, 1, 3, sq, 128), _mk(1, 1, 1, skv, 128), _mk(2, 1, 1, skv, 128)
+  sinks = torch.tensor([-INF, INF, 0.5])
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1, save_residuals=True)
+  if form == "bf16":
+    out, res = kernel(q.to(DEV), k.to(DEV), v.to(DEV), None, sinks.to(DEV), logits_scale=0.09)
+    rel = 5e-3
+  else:
+    qkv = [fp8.quantize_e4m3(t.to(DEV)) for t in (q, k, v)]
+    out, res = fp8.splash_fwd_fp8(kernel, *qkv, sinks=sinks.to(DEV), logits_scale=0.09, save_residuals=True, p_format=form)
+    q, k, v = (fp8.dequantize_e4m3(t, torch.float32).cpu() for t in qkv)
+    rel = 3e-2 if form == "e4m3" else 5e-3
+  kernel.check_errors()
+  out, lse = out[0].float().cpu(), res["logsumexp"][0].cpu()
+  live = torch.from_numpy(dense.any(-1))
+  assert torch.all(out[:, ~live] == 0) and torch.all(out[1] == 0)
+  visited = live.view(-1, 128).any(-1).repeat_interleave(128)
+  assert torch.all(lse[0, ~visited] == -INF) and torch.all(lse[1] == INF)
+  assert torch.all(lse[0, visited & ~live] == max(kernel.mask_value, -3.0e38))
+  assert (lse[2, ~live] - 0.5).abs().max().item() <= 1e-5
+  for head, sink in ((0, None), (2, sinks[2:])):
+    ro, rlse, _ = attention_ref.attention_reference(q[0, head:head + 1], k[0], v[0], dense, scale=0.09, sinks=sink)
+    assert ((out[head] - ro[0])[live].norm() / ro[0][live].norm()).item() <= rel
+    assert (lse[head] - rlse[0])[live].abs().max().item() <= 1e-3

@@ -689,12 +689,13 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int s = 0; s < kMaxSplit; ++s) {
           st[s] = make_float4(-INFINITY, 0.f, kMaskedLogit, 0.f);
           if (s < p.n_split) st[s] = cluster_ld_v4(cluster_addr(part + kHeadDim / 4 * 2 * kTile, s));
-          if (st[s].y != 0.f) top = fmaxf(top, st[s].x);  // (a part without a live key has sum 0; NaN counts)
+          top = fmaxf(top, st[s].x);  // (-inf: nothing seen; the floor: dead keys only, as in a row left whole)
           m_all = fmaxf(m_all, st[s].z);
         }
 #pragma unroll
         for (int s = 0; s < kMaxSplit; ++s) {
-          if (st[s].y != 0.f) weight[s] = ex2(st[s].x - top);
+          // (a part at the maximum weighs 1, also where that is infinite: a sink of -inf or +inf)
+          if (st[s].y != 0.f) weight[s] = st[s].x == top ? 1.f : ex2(st[s].x - top);
           sum = fmaf(st[s].y, weight[s], sum);
         }
         const bool live = sum > 0.f;
