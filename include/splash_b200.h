@@ -145,7 +145,8 @@ void splash_maskinfo_free(SplashMaskInfoOut* out);
  * bits 0-1 and of sub-tile 1 in bits 2-3 (0 skip, 1 partial, 2 full); bits 4 / 5, written by
  * splash_segment_schedule only: sub-tile 0 / 1 lies inside one segment (every token of its q tile
  * and of its kv tile carries the same id), so the kernels need not compare ids element by element;
- * [2]/[3] partial-block id of sub-tile 0/1 (-1 if none).
+ * [2]/[3] partial-block id of sub-tile 0/1 (-1 if none).  The entries of a row are in ascending order
+ * of [0], each tile once; the kernels rely on it.
  * ---------------------------------------------------------------------------------------- */
 typedef struct SplashScheduleOut {
   int32_t* row_ptr;   /* [n_rows + 1] */

@@ -206,3 +206,29 @@ def test_infinite_sinks(kind, form):
     ro, rlse, _ = attention_ref.attention_reference(q[0, head:head + 1], k[0], v[0], dense, scale=0.09, sinks=sink)
     assert ((out[head] - ro[0])[live].norm() / ro[0][live].norm()).item() <= rel
     assert (lse[head] - rlse[0])[live].abs().max().item() <= 1e-3
+
+
+def test_listed_tiles_without_a_live_key_change_nothing():
+  """One mask as tables cut with blocks of 128 and of 512 tokens (whose partial blocks list tiles that are
+  empty) and as a device tensor: the parts of a row hold the same live tiles, so every bit agrees."""
+  sq, skv = 512, 4096
+  rng = np.random.default_rng(11)
+  dense = rng.random((sq, skv)) < 0.5
+  dense &= np.kron(rng.random((sq // 128, skv // 128)) < 0.6, np.ones((128, 128))).astype(np.bool_)
+  dense[np.arange(sq), np.arange(sq) * 8] = True
+  q, k, v, do = _mk(0, 1, 4, sq, 128), _mk(1, 1, 1, skv, 128), _mk(2, 1, 1, skv, 128), _mk(3, 1, 4, sq, 128)
+  kw = dict(save_residuals=True, repeatable_dq=True)
+  blocks = lambda b: dataclasses.replace(splash.SplashConfig.get_default(), block_q=b, block_kv=b, block_kv_compute=b,
+                                         block_q_dkv=b, block_kv_dkv=b, block_kv_dkv_compute=b)
+  got = []
+  for kernel in (splash.make_splash_mha(dense, q_seq_shards=1, config=blocks(128), **kw),
+                 splash.make_splash_mha(dense, q_seq_shards=1, config=blocks(512), **kw),
+                 splash.make_dynamic_splash_mha(torch.from_numpy(dense).to(DEV), **kw)):
+    qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+    out, res = kernel(qd, kd, vd, logits_scale=0.09)
+    out.backward(do.to(DEV))
+    kernel.check_errors()
+    got.append((out, res["logsumexp"], qd.grad, kd.grad, vd.grad))
+  for other in got[1:]:
+    for a, b in zip(got[0], other):
+      assert torch.equal(a, b)

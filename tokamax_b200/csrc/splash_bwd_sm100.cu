@@ -515,11 +515,13 @@ struct DkvBarriers {
   uint32_t tmem_base;
   uint32_t abort_flag;
   uint32_t early_exit;
+  uint32_t n_steps;   // kSplit: steps of this CTA
+  int4 step[kBwdStages / 2];  // kSplit: schedule entries of the steps in the ring, covered by their Q slots' barriers
 };
 static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 
 //
-// kSplit: a cluster of 2 .. 8 CTAs shares one kv tile, each taking a run of its steps (q head, q tile).
+// kSplit: a cluster of 2 .. 8 CTAs shares one kv tile, each taking its part of the steps (q head, q tile), see PartWalk.
 // At the end every CTA leaves its dK and dV (fp32) in its own shared memory and the cluster adds them
 // up over distributed shared memory in rank order, each CTA a share of the columns: no atomics, still
 // bitwise repeatable.  For grids that leave SMs idle; split_for() holds the rule.
@@ -553,16 +555,11 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + kv_tile] : p.row_ptr[kv_tile + 1];
   const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
   const int n_ent = eend - ebeg;
-  // steps of this CTA: (q head g of the group, entry e) pairs in that order, from (first_g, first_e)
-  int n_steps = n_ent * group, first_g = 0, first_e = ebeg;
-  if constexpr (kSplit) {
-    const int total = n_steps, from = (int)((int64_t)total * rank / p.n_split);
-    n_steps = (int)((int64_t)total * (rank + 1) / p.n_split) - from;
-    if (n_ent > 0) {
-      first_g = from / n_ent;
-      first_e = ebeg + from % n_ent;
-    }
-  }
+  // steps of this CTA: (q head g of the group, entry e) pairs in that order
+  const PartWalk<kSplit> walk(entries, ebeg, eend, p.n_split);
+  const int offset0 = walk.offset((int)rank);  // of head 0's part; a tile less for each further head
+  auto offset_behind = [&](int offset) { return kSplit ? (offset == 0 ? p.n_split : offset) - 1 : 0; };
+  int n_steps = n_ent * group;  // (kSplit: counted below)
 
   if (threadIdx.x == 0) {
     // The operand tiles need a 1024-byte aligned base for the 128-byte swizzle; there is no
@@ -578,6 +575,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
     bars->early_exit = bad;
     bars->abort_flag = kSplit ? bad : 0u;  // (read by the other CTAs of the cluster)
+    bars->n_steps = 0;
     mbar_init(&bars->stat_full[0], 1);
     mbar_init(&bars->stat_full[1], 1);
     for (int s = 0; s < kBwdStages; ++s) {
@@ -602,6 +600,15 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
     return;
   }
+  if constexpr (kSplit) {
+    unsigned mine = 0;
+    for (int e = ebeg + (int)threadIdx.x; e < eend; e += (int)blockDim.x) {
+      const int part = (entries[e].x - walk.first_tile) % p.n_split;
+      for (int g = 0, o = offset0; g < group; ++g, o = offset_behind(o)) mine += part == o;
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0) atomicAdd(&bars->n_steps, mine);
+  }
   if (warp == kDkvMmaWarp) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
@@ -609,6 +616,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if constexpr (kSplit) n_steps = (int)bars->n_steps;
   const uint32_t tmem = bars->tmem_base;
   AbortCtx ab{&bars->abort_flag, p.err};
 
@@ -624,10 +632,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int n_q_tiles = p.q_len / kTile;
     bool ok = true;
     uint32_t n = 0;
-    for (int g = first_g, e = first_e; n < (uint32_t)n_steps && ok; ++g, e = ebeg) {
+    for (int g = 0, o = offset0; n < (uint32_t)n_steps && ok; ++g, o = offset_behind(o)) {
       const int head = kv_head * group + g;
       float* head_base = p.dq_acc + ((int64_t)batch * p.q_heads + head) * n_q_tiles * (int64_t)kDqTileFloats + r * 4;
-      for (; e < eend && (!kSplit || n < (uint32_t)n_steps) && ok; ++e, ++n) {
+      for (int e = walk.first(o); e < eend && ok; e = walk.next(e), ++n) {
         float* dst = head_base + (int64_t)entries[e].x * kDqTileFloats;
         ok = mbar_wait(&bars->dq_full, n & 1u, ab, 0x3600u);
         ok = __all_sync(0xffffffffu, ok);
@@ -669,10 +677,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (v2) tma_load_4d(v_smem + kHalfBytes, &tm_v, &bars->stat_full[1], 64, kv_tile * kTile, kv_head, batch);
       uint32_t it = 0;
       bool ok = true;
-      for (int g = first_g, e = first_e; it < 2u * (uint32_t)n_steps && ok; ++g, e = ebeg) {
+      for (int g = 0, o = offset0; it < 2u * (uint32_t)n_steps && ok; ++g, o = offset_behind(o)) {
         const int head = kv_head * group + g;
         const int64_t stat_base = ((int64_t)batch * p.q_heads + head) * p.q_len;
-        for (; e < eend && (!kSplit || it < 2u * (uint32_t)n_steps) && ok; ++e) {
+        for (int e = walk.first(o); e < eend && ok; e = walk.next(e)) {
           const int qt = entries[e].x;
           for (int which = 0; which < 2 && ok; ++which, ++it) {
             const uint32_t s = it % kBwdStages;
@@ -682,6 +690,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             const CUtensorMap* tm = which == 0 ? &tm_q : &tm_do;
             const bool two = which == 0 ? qk2 : v2;
             const uint32_t tile_bytes = two ? kTileBytes : kHalfBytes;
+            if (kSplit && which == 0) bars->step[s / 2] = entries[e];
             mbar_arrive_expect_tx(&bars->ring_full[s], which == 0 ? tile_bytes + 2 * kTile * 4 : tile_bytes);
             tma_load_4d(dst, tm, &bars->ring_full[s], 0, qt * kTile, head, batch);
             if (two) tma_load_4d(dst + kHalfBytes, tm, &bars->ring_full[s], 64, qt * kTile, head, batch);
@@ -815,18 +824,21 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     bool ok = true;
     int n = 0;
 
-    for (int g = first_g, e = first_e; n < n_steps && ok; ++g, e = ebeg) {
-      int4 ent_next = entries[e];
-      for (; e < eend && (!kSplit || n < n_steps) && ok; ++e, ++n) {
-        const int4 ent = ent_next;
-        if (e + 1 < eend) ent_next = entries[e + 1];
-        const int st = ent.y & 3;
+    // (kSplit: one run through this CTA's steps, whose entries the TMA warp leaves in shared memory)
+    for (int g = 0; n < n_steps && ok; ++g) {
+      int4 ent_next = make_int4(0, 0, 0, 0);
+      if constexpr (!kSplit) ent_next = entries[ebeg];
+      for (int e = ebeg; (kSplit ? n < n_steps : e < eend) && ok; ++e, ++n) {
+        int4 ent = ent_next;
+        if (!kSplit && e + 1 < eend) ent_next = entries[e + 1];
         const uint32_t ph = (uint32_t)n & 1u;
-        const int q0 = ent.x * kTile + cq * 32;  // first q column of this thread's 32
         const uint32_t itq = 2u * (uint32_t)n;
         ok = mbar_wait(&bars->ring_full[itq % kBwdStages], (itq / kBwdStages) & 1u, ab, 0x3420u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
+        if constexpr (kSplit) ent = bars->step[(itq % kBwdStages) / 2];
+        const int st = ent.y & 3;
+        const int q0 = ent.x * kTile + cq * 32;  // first q column of this thread's 32
         const float4* nl4 = reinterpret_cast<const float4*>(stats + ((itq % kBwdStages) / 2) * 2 * kTile + cq * 32);
         const float4* dl4 = nl4 + kTile / 4;
 

@@ -138,14 +138,11 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int head = work.group % p.q_heads;
   const int batch = work.group / p.q_heads;
   const int kv_head = head / (p.q_heads / p.kv_heads);
-  int ebeg = p.row_ptr[row];
-  int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + row] : p.row_ptr[row + 1];
-  if constexpr (kSplit) {
-    const int n = eend - ebeg;
-    eend = ebeg + (int)((int64_t)n * (rank + 1) / p.n_split);
-    ebeg += (int)((int64_t)n * rank / p.n_split);
-  }
+  const int ebeg = p.row_ptr[row];
+  const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + row] : p.row_ptr[row + 1];
   const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
+  const PartWalk<kSplit> walk(entries, ebeg, eend, p.n_split);  // the entries of this CTA
+  const int efirst = walk.first(walk.offset((int)rank));
   const int qt0 = row * 2;
 
   if (threadIdx.x == 0) {
@@ -198,7 +195,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       static_assert(kFwdStages % 2 == 0, "V tiles must keep to the odd ring slots");
       const int t = (warp - 10) * 32 + lane;
       uint32_t n = 0;
-      for (int e = ebeg; e < eend; ++e, ++n) {
+      for (int e = efirst; e < eend; e = walk.next(e), ++n) {
         const uint32_t it = 2 * n + 1, s = it % kFwdStages, j = n & 1u;
         bool ok = mbar_wait(&bars->kv_full[s], (it / kFwdStages) & 1u, ab, 0x600u + s);
         if (ok) ok = mbar_wait(&bars->vc_empty[j], ((n >> 1) & 1u) ^ 1u, ab, 0x610u + j);
@@ -244,7 +241,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
       uint32_t it = 0;
       bool ok = true;
-      for (int e = ebeg; e < eend && ok; ++e) {
+      for (int e = efirst; e < eend && ok; e = walk.next(e)) {
         const int col = entries[e].x;
         for (int kv = 0; kv < 2 && ok; ++kv, ++it) {
           const uint32_t s = it % kFwdStages;
@@ -330,10 +327,11 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       };
 
       const int n_ent = eend - ebeg;
+      int e = efirst;
       uint32_t pcnt[2] = {0, 0};
       bool started[2] = {false, false};
-      if (n_ent > 0 && ok) {
-        const int4 e0 = entries[ebeg];
+      if (efirst < eend && ok) {
+        const int4 e0 = entries[efirst];
         ok = mbar_wait(&bars->kv_full[0], 0, ab, 0x300u);
         if (ok) {
           mma_issue_fence();
@@ -342,10 +340,11 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           tc_commit(&bars->kv_empty[0]);
         }
         int4 nxt = e0;
-        for (int n = 0; n < n_ent && ok; ++n) {
+        for (int n = 0; (kSplit ? e < eend : n < n_ent) && ok; ++n) {
           const int4 cur = nxt;
-          const bool has_next = n + 1 < n_ent;
-          if (has_next) nxt = entries[ebeg + n + 1];
+          if constexpr (kSplit) e = walk.next(e);
+          const bool has_next = kSplit ? e < eend : n + 1 < n_ent;
+          if (has_next) nxt = entries[kSplit ? e : ebeg + n + 1];
           const uint32_t itv = 2 * n + 1, itk = 2 * n + 2;
           const uint32_t vslot = itv % kFwdStages, kslot = itk % kFwdStages;
           const uint32_t vc = n & 1u;  // kP16: which f16 image holds this step's V
@@ -437,19 +436,35 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     bool started = false;
     bool ok = true;
 
-    int4 ent_next = ebeg < eend ? entries[ebeg] : make_int4(0, 0, 0, 0);
+    int4 ent_next = efirst < eend ? entries[efirst] : make_int4(0, 0, 0, 0);
     float ks_next = 1.f, vs_next = 1.f;
     if constexpr (kFp8) {
-      if (ebeg < eend) {
+      if (efirst < eend) {
         ks_next = __ldg(k_scale + ent_next.x);
         vs_next = __ldg(v_scale + ent_next.x);
       }
     }
-    for (int e = ebeg; e < eend; ++e) {
+    int e_last = 0, x_due = ent_next.x, e_probe = efirst;
+    for (int e = efirst; e < eend; e = kSplit ? e_probe : e + 1) {
+      if constexpr (kSplit) {
+        if (ent_next.x != x_due) {  // a gap in the row
+          e = walk.find(e_last + 1, x_due);
+          if (e >= eend) break;
+          ent_next = entries[e];
+          if constexpr (kFp8) {
+            ks_next = __ldg(k_scale + ent_next.x);
+            vs_next = __ldg(v_scale + ent_next.x);
+          }
+        }
+        e_last = e;
+        x_due = ent_next.x + walk.n;
+        e_probe = walk.probe(e, x_due);
+      }
+      const int e_next = kSplit ? e_probe : e + 1;
       const int4 ent = ent_next;
       const float ks = ks_next, vs = vs_next;
-      if (e + 1 < eend) {  // fetched a step ahead of its use
-        ent_next = entries[e + 1];
+      if (e_next < eend) {  // fetched a step ahead of its use
+        ent_next = entries[e_next];
         if constexpr (kFp8) {
           ks_next = __ldg(k_scale + ent_next.x);
           vs_next = __ldg(v_scale + ent_next.x);

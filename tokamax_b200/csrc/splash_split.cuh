@@ -123,6 +123,61 @@ inline const ClusterCapacity* cluster_capacity(const void* kernel, int variant, 
   return &c;
 }
 
+// Which steps of a row belong to which CTA of its cluster: those whose place along the walked axis (forward:
+// the kv tile; dkv: the q tile plus the q head's number in its group) is the CTA's rank modulo the CTAs.
+// Neighbours fall to different CTAs, so whole rows, windows and what is left of a diagonal all part evenly;
+// and the part of a step depends on nothing but its place: tiles that are listed though they hold no live
+// key (a partial block of several tiles, the other tile of a pair) leave every sum as it is without them.
+// The entries of a row come in ascending order, mostly without a gap; that the entry n further on is the
+// tile n further on shows it in one load.
+template <bool kSplit>
+struct PartWalk {
+  const int4* entries;
+  int beg, end, n;
+  int first_tile, last_tile;
+
+  __device__ __forceinline__ PartWalk(const int4* list, int from, int to, int parts) : entries(list), beg(from), end(to), n(parts) {
+    first_tile = beg < end ? entries[beg].x : 0;
+    last_tile = beg < end ? entries[end - 1].x : -1;
+  }
+  // tiles from the row's first one on to the first that is `residue` modulo n
+  __device__ __forceinline__ int offset(int residue) const {
+    const int d = (residue - first_tile) % n;
+    return d < 0 ? d + n : d;
+  }
+  // the entry of tile `x`, or of the next one of the same part, looked for from `e` on (`end`: none)
+  __device__ __forceinline__ int find(int e, int x) const {
+    for (; e < end; ++e) {
+      const int ahead = entries[e].x - x;
+      if (ahead >= 0 && ahead % n == 0) return e;
+    }
+    return end;
+  }
+  // the first entry of the part that begins `offset` tiles behind the row's first
+  __device__ __forceinline__ int first(int offset) const {
+    const int x = first_tile + offset;
+    if (x > last_tile) return end;
+    return beg + offset < end && entries[beg + offset].x == x ? beg + offset : find(beg, x);
+  }
+  // the entry behind `e` in its part
+  __device__ __forceinline__ int next(int e) const {
+    const int x = entries[e].x + n;
+    if (x > last_tile) return end;
+    return e + n < end && entries[e + n].x == x ? e + n : find(e + 1, x);
+  }
+  // For loops that fetch an entry a step ahead of its use: where tile x = (tile of `e`) + n is if the row has no
+  // gap before it (`end`: the row ends before x).  Where another tile is found there: find(e + 1, x).
+  __device__ __forceinline__ int probe(int e, int x) const { return x > last_tile ? end : min(e + n, end - 1); }
+};
+template <>
+struct PartWalk<false> {  // the whole row
+  int beg;
+  __device__ __forceinline__ PartWalk(const int4*, int from, int, int) : beg(from) {}
+  __device__ __forceinline__ int offset(int) const { return 0; }
+  __device__ __forceinline__ int first(int) const { return beg; }
+  __device__ __forceinline__ int next(int e) const { return e + 1; }
+};
+
 template <typename... Params, typename... Args>
 inline cudaError_t launch_clusters(void (*kernel)(Params...), unsigned rows, int n_split, int threads, int smem,
                                    cudaStream_t stream, const Args&... args) {
