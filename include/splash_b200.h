@@ -286,6 +286,22 @@ typedef struct SplashFwdArgs {
 
 int splash_fwd(const SplashFwdArgs* args, void* cuda_stream);
 
+/* The call that a launch is a share of.  In a small grid a row is shared between CTAs, its sums are formed in
+ * parts, and the last bits of o, logsumexp, dk and dv depend on how many there are; which depends on the batch
+ * and the heads of the launch.  A launch that is told of the others shares its rows as one launch of the
+ * whole call would, so that its results are bit for bit the whole call's.  Zero-initialise. */
+typedef struct SplashShards {
+  int32_t head_shards; /* the call's heads lie in this many equal launches, each with its own kv heads (0, 1: in one) */
+} SplashShards;
+/* splash_fwd as one of such launches; shards == NULL: splash_fwd. */
+int splash_fwd_shard(const SplashFwdArgs* args, const SplashShards* shards, void* cuda_stream);
+
+/* How many CTAs share a schedule row in the launch splash_fwd_shard would make, or a kv tile in
+ * splash_bwd_shard's dkv kernel (1: none; the grid fills the GPU, or its rows are short).  Reads the tensors'
+ * sizes, mask_fn and which pointers are set, nothing on the device.  `clusters` [9]: how many clusters of n
+ * CTAs the GPU holds at a time ([1]: CTAs); NULL: those of the current device.  Negative: a SplashStatus. */
+int splash_fwd_row_parts(const SplashFwdArgs* args, const SplashShards* shards, const int32_t* clusters);
+
 /* Forward for e4m3 inputs (inference prefill).  No counterpart in the reference, whose splash path
  * rejects everything but bf16 / f32 (pallas_mosaic_tpu_common.py:40-42); the contract is the bf16
  * forward above run on the dequantised tensors.
@@ -309,12 +325,14 @@ typedef struct SplashFwdFp8Args {
 } SplashFwdFp8Args;
 
 int splash_fwd_fp8(const SplashFwdFp8Args* args, void* cuda_stream);
+int splash_fwd_fp8_shard(const SplashFwdFp8Args* args, const SplashShards* shards, void* cuda_stream);
 
 /* ------------------------------------------------------------------------------------------
  * Backward.  Replaces `_splash_attention_bwd` + `_splash_attention_bwd_dkv` +
  * `_flash_attention_dkv_kernel` (splash_attention_kernel.py:1871-1947, :1462-1868, :1234-1459):
  * di = sum(o * do), then dq (q-tile stationary) and dk/dv (kv-tile stationary, the q heads of a
- * kv head summed inside one CTA in fp32 — no atomics, bitwise repeatable).
+ * kv head summed in fp32 inside one CTA, or in a small grid inside a cluster of CTAs in a fixed order — no
+ * atomics, bitwise repeatable).
  * Workspace: splash_bwd_workspace_bytes(batch, q_heads, q_len) bytes, 256-byte aligned.
  * ---------------------------------------------------------------------------------------- */
 typedef struct SplashBwdArgs {
@@ -359,6 +377,8 @@ typedef enum SplashBwdFlags {
 size_t splash_bwd_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len);
 size_t splash_bwd_fused_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len);
 int splash_bwd(const SplashBwdArgs* args, void* cuda_stream);
+int splash_bwd_shard(const SplashBwdArgs* args, const SplashShards* shards, void* cuda_stream);
+int splash_bwd_row_parts(const SplashBwdArgs* args, const SplashShards* shards, const int32_t* clusters); /* as for splash_fwd */
 
 /* Ring attention (ring_attention_kernel.py:150-158): folds one ring step's partial result
  * (o_i bf16 [n_rows, 128], its logsumexp lse_i [n_rows]) into the running fp32 pair in place:

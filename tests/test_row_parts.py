@@ -1,0 +1,112 @@
+"""How many CTAs share a schedule row: the launchers' rule, asked on the host with given capacities.
+
+GPU (marked): results of calls on a share of the heads are the whole call's, bit for bit, at sizes
+whose rows are shared.
+"""
+import ctypes as C
+import math
+
+import pytest
+import torch
+
+from tokamax_b200 import _native
+from tokamax_b200 import splash_attention_kernel as splash
+from tokamax_b200 import splash_attention_mask as mask_lib
+
+# clusters of n CTAs that 148 SMs hold at a time: in one piece, in GPCs of 16 and 18 SMs, in pairs of SMs lost to each
+CAPACITIES = [
+    [0, 148, 74, 49, 37, 29, 24, 21, 18],
+    [0, 148, 74, 48, 36, 27, 24, 18, 18],
+    [0, 148, 72, 44, 33, 26, 20, 16, 15],
+]
+
+
+def _sizes(tensor, *shape):
+  for i, n in enumerate(shape):
+    tensor.size[i] = n
+
+
+def _args(mask, batch, hq, hkv, sq, skv, head_shards=0, d=128, d_v=128):
+  """Forward and backward arguments as far as the rule reads them, for 1 / head_shards of the heads, and SplashShards."""
+  fa, ba = _native.SplashFwdArgs(), _native.SplashBwdArgs()
+  n = max(head_shards, 1)
+  for a in (fa, ba):
+    _sizes(a.q, batch, hq // n, sq, d)
+    _sizes(a.k, batch, hkv // n, skv, d)
+    _sizes(a.v, batch, hkv // n, skv, d_v)
+    a.mask_fn = splash._mask_fn_struct(getattr(mask, "interval_rule", None))  # pylint: disable=protected-access
+  return fa, ba, _native.SplashShards(head_shards=head_shards)
+
+
+def _parts(*args, clusters=None, **kw):
+  fa, ba, shards = _args(*args, **kw)
+  lib = _native.lib()
+  table = None if clusters is None else C.byref((C.c_int32 * 9)(*clusters))
+  return (lib.splash_fwd_row_parts(C.byref(fa), C.byref(shards), table),
+          lib.splash_bwd_row_parts(C.byref(ba), C.byref(shards), table))
+
+
+@pytest.mark.parametrize("clusters", CAPACITIES)
+@pytest.mark.parametrize("batch,hq,hkv,s,shards", [(1, 8, 4, 2048, 2), (1, 8, 4, 2048, 4), (2, 16, 16, 4096, 8),
+                                                   (1, 64, 8, 8192, 8), (1, 8, 8, 16384, 8)])
+def test_head_shards_are_shared_out_as_the_whole_call(batch, hq, hkv, s, shards, clusters):
+  mask = mask_lib.CausalMask((s, s))
+  whole = _parts(mask, batch, hq, hkv, s, s, clusters=clusters)
+  assert min(whole) >= 1
+  assert _parts(mask, batch, hq, hkv, s, s, head_shards=shards, clusters=clusters) == whole
+  if (hq, s, shards) == (8, 2048, 2):  # a rank's launch by itself would be cut otherwise
+    assert _parts(mask, batch, hq // 2, hkv // 2, s, s, clusters=clusters) != whole and min(whole) > 1
+
+
+def test_row_parts_refuses_what_it_cannot_read():
+  lib = _native.lib()
+  mask = mask_lib.CausalMask((2048, 2048))
+  assert lib.splash_fwd_row_parts(None, None, None) == -1 and lib.splash_bwd_row_parts(None, None, None) == -1
+  assert lib.splash_fwd_shard(None, None, None) == -1 and lib.splash_bwd_shard(None, None, None) == -1
+  assert lib.splash_fwd_fp8_shard(None, None, None) == -1
+  assert _parts(mask, 0, 8, 4, 2048, 2048, clusters=CAPACITIES[0]) == (-1, -1)
+  assert _parts(mask, 1, 8, 4, 2000, 2048, clusters=CAPACITIES[0]) == (-1, -1)
+  assert _parts(mask, 1, 8, 4, 2048, 2048, clusters=[0] * 9) == (-1, -1)
+  assert _parts(mask, 1, 8, 4, 2048, 2048, d=192, clusters=CAPACITIES[0]) == (1, 1)  # two-panel kernels
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1)
+  assert kernel.head_shards == 1 and kernel.head_shard(4).head_shard(2).head_shards == 8
+  for bad in (0, -1, 1 << 16):
+    with pytest.raises(ValueError):
+      kernel.head_shard(bad)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("repeatable", [True, False])
+@pytest.mark.parametrize("name,b,hq,hkv,sq,skv,shards", [("causal", 1, 8, 4, 2048, 2048, 2), ("causal", 1, 8, 4, 2048, 2048, 4),
+                                                         ("window", 2, 4, 2, 384, 4096, 2), ("full", 1, 12, 2, 256, 2176, 2)])
+def test_shares_of_the_heads_give_the_whole_calls_bits(name, b, hq, hkv, sq, skv, shards, repeatable):
+  dev = torch.device("cuda:0")
+  mask = {"causal": lambda: mask_lib.CausalMask((sq, skv), skv - sq),
+          "window": lambda: mask_lib.LocalMask((sq, skv), (skv * 3 // 4, 0), skv - sq),
+          "full": lambda: mask_lib.FullMask((sq, skv))}[name]()
+  g = torch.Generator().manual_seed(7)
+  mk = lambda h, s: torch.randn(b, h, s, 128, generator=g).to(torch.bfloat16).to(dev)
+  q, k, v, do = mk(hq, sq), mk(hkv, skv), mk(hkv, skv), mk(hq, sq)
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1, save_residuals=True, repeatable_dq=repeatable)
+
+  def call(kern, *tensors):
+    *qkv, d_o = (t.clone() for t in tensors)
+    qkv = [t.requires_grad_(True) for t in qkv]
+    out, res = kern(*qkv, logits_scale=1 / math.sqrt(128))
+    out.backward(d_o)
+    return (out, res["logsumexp"], res["max_logits"], *(t.grad for t in qkv))
+
+  whole = call(kernel, q, k, v, do)
+  # the case tests what it says only where rows are shared, and a share by itself would not do
+  assert max(_parts(mask, b, hq, hkv, sq, skv)) > 1
+  assert _parts(mask, b, hq, hkv, sq, skv, head_shards=shards) == _parts(mask, b, hq, hkv, sq, skv)
+  assert _parts(mask, b, hq // shards, hkv // shards, sq, skv) != _parts(mask, b, hq, hkv, sq, skv)
+  for rank in range(shards):
+    heads = lambda t: t[:, rank * t.shape[1] // shards:(rank + 1) * t.shape[1] // shards]  # noqa: B023
+    share = call(kernel.head_shard(shards), *map(heads, (q, k, v, do)))
+    for i, (got, want) in enumerate(zip(share, map(heads, whole))):
+      if i == 3 and not repeatable:  # the fused backward's dq: fp32 sums in varying order
+        assert ((got.float() - want.float()).norm() / want.float().norm()).item() <= 1e-3
+      else:
+        assert torch.equal(got, want)
+  kernel.check_errors()

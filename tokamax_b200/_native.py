@@ -153,6 +153,10 @@ class SplashFwdArgs(C.Structure):
   ]
 
 
+class SplashShards(C.Structure):
+  _fields_ = [("head_shards", C.c_int32)]
+
+
 class SplashFwdFp8Args(C.Structure):
   _fields_ = [
       ("base", SplashFwdArgs),
@@ -223,6 +227,11 @@ _PROTOTYPES = {
     "splash_dynamic_schedule": (C.c_int, [C.c_void_p, C.c_int64, C.c_int64, C.c_int32, C.c_int64, C.c_void_p,
                                           C.c_void_p, C.c_size_t, C.POINTER(SplashDeviceSchedule), C.c_void_p]),
     "splash_fwd": (C.c_int, [C.POINTER(SplashFwdArgs), C.c_void_p]),
+    "splash_fwd_shard": (C.c_int, [C.POINTER(SplashFwdArgs), C.POINTER(SplashShards), C.c_void_p]),
+    "splash_fwd_row_parts": (C.c_int, [C.POINTER(SplashFwdArgs), C.POINTER(SplashShards), C.POINTER(C.c_int32 * 9)]),
+    "splash_fwd_fp8_shard": (C.c_int, [C.POINTER(SplashFwdFp8Args), C.POINTER(SplashShards), C.c_void_p]),
+    "splash_bwd_shard": (C.c_int, [C.POINTER(SplashBwdArgs), C.POINTER(SplashShards), C.c_void_p]),
+    "splash_bwd_row_parts": (C.c_int, [C.POINTER(SplashBwdArgs), C.POINTER(SplashShards), C.POINTER(C.c_int32 * 9)]),
     "splash_fwd_fp8": (C.c_int, [C.POINTER(SplashFwdFp8Args), C.c_void_p]),
     "splash_ring_merge": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_void_p]),
     "splash_bwd_workspace_bytes": (C.c_size_t, [C.c_int64, C.c_int64, C.c_int64]),

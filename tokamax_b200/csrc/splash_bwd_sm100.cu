@@ -1125,7 +1125,41 @@ size_t bwd_fused_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len) 
   return base + (size_t)batch * (size_t)q_heads * (size_t)q_len * kHeadDim * sizeof(float);
 }
 
-int launch_bwd(const SplashBwdArgs& a, cudaStream_t stream) {
+using DkvKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
+static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap) {
+  static const DkvKernel kernels[2][2][2] = {
+      {{splash_dkv_kernel<false, false, false>, splash_dkv_kernel<true, false, false>},
+       {splash_dkv_kernel<false, true, false>, splash_dkv_kernel<true, true, false>}},
+      {{splash_dkv_kernel<false, false, true>, splash_dkv_kernel<true, false, true>},
+       {splash_dkv_kernel<false, true, true>, splash_dkv_kernel<true, true, true>}}};
+  return kernels[split][fused][soft_cap];
+}
+
+// CTAs that share a kv tile of this call's dkv kernel (head dims up to 128)
+static int dkv_split(const SplashBwdArgs& a, const SplashShards& shards, bool fused, const int32_t* clusters) {
+  if (a.q_segment_ids != nullptr || a.q_sequence != nullptr) return 1;
+  const int64_t n_rows = a.k.size[2] / kTile;
+  RowWork rw = estimate_row_work(a.mask_fn, (int)n_rows, kTile, (int)(a.q.size[2] / kTile),
+                                 n_rows * a.k.size[0] * a.k.size[1] * (shards.head_shards > 1 ? shards.head_shards : 1), true);
+  rw.longest *= (float)(a.q.size[1] / a.k.size[1]);  // a kv tile walks every q head of its group
+  rw.mean *= (float)(a.q.size[1] / a.k.size[1]);
+  const bool soft_cap = a.soft_cap != 0.f;
+  return row_parts(rw, clusters, [&] {
+    return cluster_capacity((const void*)dkv_kernel_for(true, fused, soft_cap), 4 + (soft_cap ? 1 : 0) + (fused ? 2 : 0),
+                            fused ? kFusedThreads : kDkvThreads, kDkvSmemBytes);
+  });
+}
+
+int bwd_row_parts(const SplashBwdArgs& a, const SplashShards& shards, const int32_t* clusters) {
+  for (int i = 0; i < 4; ++i)
+    if (a.q.size[i] <= 0 || a.k.size[i] <= 0 || a.v.size[i] <= 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (a.q.size[2] % kTile != 0 || a.k.size[2] % kTile != 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (a.mask_fn.kind == SPLASH_MASK_CHUNKED && a.mask_fn.chunk <= 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (a.q.size[3] > kHeadDim || a.v.size[3] > kHeadDim) return 1;
+  return dkv_split(a, shards, (a.flags & SPLASH_BWD_FUSED_DQ) != 0, clusters);
+}
+
+int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t stream) {
   int st;
   const SplashTensor* ts[8] = {&a.q, &a.k, &a.v, &a.o, &a.d_o, &a.dq, &a.dk, &a.dv};
   for (int i = 0; i < 8; ++i)
@@ -1203,8 +1237,7 @@ int launch_bwd(const SplashBwdArgs& a, cudaStream_t stream) {
   const bool soft_cap = a.soft_cap != 0.f;
   if (soft_cap && !(a.soft_cap > 0.f)) return SPLASH_ERR_INVALID_ARGUMENT;
   auto* dq_kernel = soft_cap ? splash_dq_kernel<true> : splash_dq_kernel<false>;
-  auto* dkv_kernel = fused ? (soft_cap ? splash_dkv_kernel<true, true, false> : splash_dkv_kernel<false, true, false>)
-                           : (soft_cap ? splash_dkv_kernel<true, false, false> : splash_dkv_kernel<false, false, false>);
+  DkvKernel dkv_kernel = dkv_kernel_for(false, fused, soft_cap);
   const int dkv_smem = kDkvSmemBytes;
   // function attributes are per device: remember which devices have been set up
   {
@@ -1301,19 +1334,9 @@ int launch_bwd(const SplashBwdArgs& a, cudaStream_t stream) {
   if (mask & 4u) {
     const int64_t n_ctas = (int64_t)p.n_rows * p.n_groups;
     const int threads = fused ? kFusedThreads : kDkvThreads;
-    RowWork rw = estimate_row_work(a.mask_fn, p.n_rows, kTile, (int)(Sq / kTile), n_ctas, true);
-    p.n_split = 1;
-    if (a.q_segment_ids == nullptr && a.q_sequence == nullptr && rw.longest > 0.f) {
-      auto* split_kernel = fused ? (soft_cap ? splash_dkv_kernel<true, true, true> : splash_dkv_kernel<false, true, true>)
-                                 : (soft_cap ? splash_dkv_kernel<true, false, true> : splash_dkv_kernel<false, false, true>);
-      rw.longest *= (float)(Hq / Hkv);  // a kv tile walks every q head of its group
-      rw.mean *= (float)(Hq / Hkv);
-      const ClusterCapacity* cap = cluster_capacity((const void*)split_kernel, 4 + (soft_cap ? 1 : 0) + (fused ? 2 : 0),
-                                                    threads, dkv_smem);
-      if (cap == nullptr) return SPLASH_ERR_CUDA;
-      p.n_split = split_for(n_ctas, rw, *cap);
-      if (p.n_split > 1) dkv_kernel = split_kernel;
-    }
+    p.n_split = dkv_split(a, shards, fused, nullptr);
+    if (p.n_split < 0) return p.n_split;
+    if (p.n_split > 1) dkv_kernel = dkv_kernel_for(true, fused, soft_cap);
     if (launch_clusters(dkv_kernel, (unsigned)n_ctas, p.n_split, threads, dkv_smem, stream, tm_q, tm_do, tm_k, tm_v, p) !=
         cudaSuccess)
       return SPLASH_ERR_CUDA;
@@ -1369,7 +1392,7 @@ int launch_bwd_static_scratch(const SplashBwdArgs& a, cudaStream_t stream) {
   b.flags &= ~(uint32_t)SPLASH_BWD_FUSED_DQ;  // the array holds the two per-row terms only
   b.workspace = scratch;
   b.workspace_bytes = bwd_workspace_bytes(B, Hq, Sq);  // <= sizeof(g_static_scratch) by the row check
-  return launch_bwd(b, stream);
+  return launch_bwd(b, SplashShards{}, stream);
 }
 
 }  // namespace sb

@@ -790,7 +790,38 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 // ------------------------------------------------------------------------------------------
 // host launcher
 // ------------------------------------------------------------------------------------------
-static int launch_fwd_common(const SplashFwdArgs& a, const float* q_scale, const float* k_scale,
+using FwdKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FwdParams);
+static FwdKernel fwd_kernel(bool split, int variant) {
+  static const FwdKernel kernels[2][4] = {
+      {splash_fwd_kernel<false, false, false, false>, splash_fwd_kernel<true, false, false, false>,
+       splash_fwd_kernel<false, true, false, false>, splash_fwd_kernel<true, false, true, false>},
+      {splash_fwd_kernel<false, false, false, true>, splash_fwd_kernel<true, false, false, true>,
+       splash_fwd_kernel<false, true, false, true>, splash_fwd_kernel<true, false, true, true>}};
+  return kernels[split][variant];
+}
+
+// CTAs that share a schedule row (256 query rows) of this call; the 128-wide kernels only
+static int fwd_split(const SplashFwdArgs& a, const SplashShards& shards, int variant, const int32_t* clusters) {
+  if (a.q_segment_ids != nullptr || a.q_sequence != nullptr) return 1;
+  const int64_t n_rows = (a.q.size[2] / kTile + 1) / 2;
+  const RowWork rw = estimate_row_work(a.mask_fn, (int)n_rows, 2 * kTile, (int)(a.k.size[2] / kTile),
+                                       n_rows * a.q.size[0] * a.q.size[1] * (shards.head_shards > 1 ? shards.head_shards : 1));
+  return row_parts(rw, clusters, [&] {
+    return cluster_capacity((const void*)fwd_kernel(true, variant), variant, kFwdThreads,
+                            fwd_smem_bytes(variant & 1, variant == 3, true));
+  });
+}
+
+int fwd_row_parts(const SplashFwdArgs& a, const SplashShards& shards, const int32_t* clusters) {
+  for (int i = 0; i < 4; ++i)
+    if (a.q.size[i] <= 0 || a.k.size[i] <= 0 || a.v.size[i] <= 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (a.q.size[2] % kTile != 0 || a.k.size[2] % kTile != 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (a.mask_fn.kind == SPLASH_MASK_CHUNKED && a.mask_fn.chunk <= 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  if (a.q.size[3] > kHeadDim || a.v.size[3] > kHeadDim) return 1;
+  return fwd_split(a, shards, a.q.dtype == SPLASH_F8E4M3 ? 1 : (a.soft_cap != 0.f ? 2 : 0), clusters);
+}
+
+static int launch_fwd_common(const SplashFwdArgs& a, const SplashShards& shards, const float* q_scale, const float* k_scale,
                              const float* v_scale, bool fp8, bool p16, cudaStream_t stream) {
   int st;
   const bool soft_cap = a.soft_cap != 0.f;
@@ -890,25 +921,11 @@ static int launch_fwd_common(const SplashFwdArgs& a, const float* q_scale, const
   p.chunk_groups = chunk_groups_for(Skv * kv_row_bytes / (Hq / Hkv), p.n_groups, Hq / Hkv);
   if (wide) return launch_fwd_wide(tm_q, tm_k, tm_v, p, soft_cap, stream);
   if ((int64_t)p.n_rows * p.n_groups > 0x7fffffffll) return SPLASH_ERR_TOO_LARGE;
-  using Kernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, FwdParams);
-  static const Kernel kernels[2][4] = {
-      {splash_fwd_kernel<false, false, false, false>, splash_fwd_kernel<true, false, false, false>,
-       splash_fwd_kernel<false, true, false, false>, splash_fwd_kernel<true, false, true, false>},
-      {splash_fwd_kernel<false, false, false, true>, splash_fwd_kernel<true, false, false, true>,
-       splash_fwd_kernel<false, true, false, true>, splash_fwd_kernel<true, false, true, true>}};
   const int variant = fp8 ? (p16 ? 3 : 1) : (soft_cap ? 2 : 0);
-  // row lengths: a schedule row is 256 query rows
-  const RowWork rw = estimate_row_work(a.mask_fn, p.n_rows, 2 * kTile, p.n_kv_tiles,
-                                       (int64_t)p.n_rows * p.n_groups);
-  p.n_split = 1;
-  if (a.q_segment_ids == nullptr && a.q_sequence == nullptr && rw.longest > 0.f) {
-    const ClusterCapacity* cap = cluster_capacity((const void*)kernels[1][variant], variant, kFwdThreads,
-                                                  fwd_smem_bytes(fp8, p16, true));
-    if (cap == nullptr) return SPLASH_ERR_CUDA;
-    p.n_split = split_for((int64_t)p.n_rows * p.n_groups, rw, *cap);
-  }
+  p.n_split = fwd_split(a, shards, variant, nullptr);
+  if (p.n_split < 0) return p.n_split;
   const bool split = p.n_split > 1;
-  const Kernel kernel = kernels[split][variant];
+  const FwdKernel kernel = fwd_kernel(split, variant);
   const int smem = fwd_smem_bytes(fp8, p16, split);
   // The dynamic shared-memory attribute is per device and per kernel variant: set once, under a
   // lock (calls may come from several threads).
@@ -929,13 +946,13 @@ static int launch_fwd_common(const SplashFwdArgs& a, const float* q_scale, const
   return err == cudaSuccess ? SPLASH_OK : SPLASH_ERR_CUDA;
 }
 
-int launch_fwd(const SplashFwdArgs& a, cudaStream_t stream) {
-  return launch_fwd_common(a, nullptr, nullptr, nullptr, false, false, stream);
+int launch_fwd(const SplashFwdArgs& a, const SplashShards& shards, cudaStream_t stream) {
+  return launch_fwd_common(a, shards, nullptr, nullptr, nullptr, false, false, stream);
 }
 
-int launch_fwd_fp8(const SplashFwdFp8Args& a, cudaStream_t stream) {
+int launch_fwd_fp8(const SplashFwdFp8Args& a, const SplashShards& shards, cudaStream_t stream) {
   if (a.flags & ~(uint32_t)SPLASH_FP8_P_F16) return SPLASH_ERR_INVALID_ARGUMENT;
-  return launch_fwd_common(a.base, a.q_scale, a.k_scale, a.v_scale, true, (a.flags & SPLASH_FP8_P_F16) != 0, stream);
+  return launch_fwd_common(a.base, shards, a.q_scale, a.k_scale, a.v_scale, true, (a.flags & SPLASH_FP8_P_F16) != 0, stream);
 }
 
 }  // namespace sb

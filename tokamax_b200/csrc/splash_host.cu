@@ -8,10 +8,12 @@
 
 namespace sb {
 
-int launch_fwd(const SplashFwdArgs& a, cudaStream_t stream);
-int launch_fwd_fp8(const SplashFwdFp8Args& a, cudaStream_t stream);
-int launch_bwd(const SplashBwdArgs& a, cudaStream_t stream);
+int launch_fwd(const SplashFwdArgs& a, const SplashShards& shards, cudaStream_t stream);
+int launch_fwd_fp8(const SplashFwdFp8Args& a, const SplashShards& shards, cudaStream_t stream);
+int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t stream);
 int launch_bwd_static_scratch(const SplashBwdArgs& a, cudaStream_t stream);
+int fwd_row_parts(const SplashFwdArgs& a, const SplashShards& shards, const int32_t* clusters);
+int bwd_row_parts(const SplashBwdArgs& a, const SplashShards& shards, const int32_t* clusters);
 size_t bwd_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len);
 size_t bwd_fused_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len);
 
@@ -116,14 +118,30 @@ int splash_probe_bounded_wait(uint32_t* error_record, int64_t limit_cycles, uint
   return cudaGetLastError() == cudaSuccess ? SPLASH_OK : SPLASH_ERR_CUDA;
 }
 
-int splash_fwd(const SplashFwdArgs* args, void* cuda_stream) {
+static SplashShards shards_or_none(const SplashShards* shards) { return shards != nullptr ? *shards : SplashShards{}; }
+
+int splash_fwd_shard(const SplashFwdArgs* args, const SplashShards* shards, void* cuda_stream) {
   if (args == nullptr) return SPLASH_ERR_INVALID_ARGUMENT;
-  return sb::launch_fwd(*args, static_cast<cudaStream_t>(cuda_stream));
+  return sb::launch_fwd(*args, shards_or_none(shards), static_cast<cudaStream_t>(cuda_stream));
+}
+
+int splash_fwd(const SplashFwdArgs* args, void* cuda_stream) { return splash_fwd_shard(args, nullptr, cuda_stream); }
+
+int splash_fwd_row_parts(const SplashFwdArgs* args, const SplashShards* shards, const int32_t* clusters) {
+  return args == nullptr ? SPLASH_ERR_INVALID_ARGUMENT : sb::fwd_row_parts(*args, shards_or_none(shards), clusters);
+}
+
+int splash_bwd_row_parts(const SplashBwdArgs* args, const SplashShards* shards, const int32_t* clusters) {
+  return args == nullptr ? SPLASH_ERR_INVALID_ARGUMENT : sb::bwd_row_parts(*args, shards_or_none(shards), clusters);
+}
+
+int splash_fwd_fp8_shard(const SplashFwdFp8Args* args, const SplashShards* shards, void* cuda_stream) {
+  if (args == nullptr) return SPLASH_ERR_INVALID_ARGUMENT;
+  return sb::launch_fwd_fp8(*args, shards_or_none(shards), static_cast<cudaStream_t>(cuda_stream));
 }
 
 int splash_fwd_fp8(const SplashFwdFp8Args* args, void* cuda_stream) {
-  if (args == nullptr) return SPLASH_ERR_INVALID_ARGUMENT;
-  return sb::launch_fwd_fp8(*args, static_cast<cudaStream_t>(cuda_stream));
+  return splash_fwd_fp8_shard(args, nullptr, cuda_stream);
 }
 
 size_t splash_bwd_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len) {
@@ -134,10 +152,12 @@ size_t splash_bwd_fused_workspace_bytes(int64_t batch, int64_t q_heads, int64_t 
   return sb::bwd_fused_workspace_bytes(batch, q_heads, q_len);
 }
 
-int splash_bwd(const SplashBwdArgs* args, void* cuda_stream) {
+int splash_bwd_shard(const SplashBwdArgs* args, const SplashShards* shards, void* cuda_stream) {
   if (args == nullptr) return SPLASH_ERR_INVALID_ARGUMENT;
-  return sb::launch_bwd(*args, static_cast<cudaStream_t>(cuda_stream));
+  return sb::launch_bwd(*args, shards_or_none(shards), static_cast<cudaStream_t>(cuda_stream));
 }
+
+int splash_bwd(const SplashBwdArgs* args, void* cuda_stream) { return splash_bwd_shard(args, nullptr, cuda_stream); }
 
 int splash_bwd_static_scratch(const SplashBwdArgs* args, void* cuda_stream) {
   if (args == nullptr) return SPLASH_ERR_INVALID_ARGUMENT;

@@ -15,12 +15,13 @@ namespace sb {
 constexpr int kMaxSplit = 8;  // portable cluster size
 
 // Steps (128-column tiles) of the longest row and of the average one, from the mask function; a table
-// mask counts as full.  Not asked for calls with q_sequence either: a shard of the query rows gives the
-// bits that the whole gives while both leave their rows whole.  Not asked for calls with segment
-// ids: they cut rows at places that only the device knows, and a schedule filtered by them gives bit for
-// bit what an unfiltered one gives only while no row is cut into parts by its number of entries.
+// mask counts as full, whether it comes from the host or from the device: so both give the same bits.
+// Not asked for calls with q_sequence: a shard of the query rows gives the bits that the whole gives
+// while both leave their rows whole.  Nor for calls with segment ids, which cut rows at places that only
+// the device knows.
 struct RowWork {
-  float longest, mean;
+  float longest, mean;  // 0: rows are left whole
+  int64_t ctas;         // rows of the call (of all launches that make it up)
 };
 struct ClusterCapacity {
   int clusters[kMaxSplit + 1];  // [n]: clusters of n CTAs that are resident at the same time; [1]: CTAs
@@ -31,7 +32,7 @@ constexpr int kSplitMaxCtas = 1024;  // grids above this fill the chip several t
 // rows of `row_span` query rows (transposed = false) or key tiles (true) over `n_steps_full` tiles of the other side
 inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_span, int n_tiles,
                                  int64_t n_ctas, bool transposed = false) {
-  RowWork w{0.f, 0.f};
+  RowWork w{0.f, 0.f, n_ctas};
   if (n_ctas > kSplitMaxCtas) return w;
   w.longest = w.mean = (float)n_tiles;
   if (fn.kind != SPLASH_MASK_CAUSAL && fn.kind != SPLASH_MASK_LOCAL) return w;
@@ -65,14 +66,14 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
 // total work over the slots, and half a row for the uneven end.  Rows below 16 steps stay whole: little
 // is left to gain there (causal 2 x 1024, 8 heads, 64 CTAs of 2 .. 8 steps: 24.7 us, 20.9 with two CTAs a row),
 // and short sequences give the same bits whatever else is in the launch.
-inline int split_for(int64_t rows, const RowWork& w, const ClusterCapacity& cap) {
+inline int split_for(const RowWork& w, const ClusterCapacity& cap) {
   constexpr float kFixed = 3.f, kMerge = 1.f, kFewest = 16.f;
   if (w.longest < kFewest) return 1;
   auto time = [&](int n) {
     const float fixed = kFixed + (n > 1 ? kMerge : 0.f);
     const float longest = w.longest / n + fixed, mean = w.mean / n + fixed;
-    if (rows <= cap.clusters[n]) return longest;
-    return (float)rows * mean / cap.clusters[n] + 0.5f * longest;
+    if (w.ctas <= cap.clusters[n]) return longest;
+    return (float)w.ctas * mean / cap.clusters[n] + 0.5f * longest;
   };
   int best = 1;
   float least = 0.9f * time(1);  // a split has to gain a tenth
@@ -82,6 +83,20 @@ inline int split_for(int64_t rows, const RowWork& w, const ClusterCapacity& cap)
       best = n;
     }
   return best;
+}
+
+// The number for a call whose capacity the caller gives (clusters[n], n = 1 .. 8) or `device` knows.
+template <typename Device>
+inline int row_parts(const RowWork& w, const int32_t* clusters, Device device) {
+  if (!(w.longest > 0.f)) return 1;
+  if (clusters == nullptr) {
+    const ClusterCapacity* cap = device();
+    return cap == nullptr ? SPLASH_ERR_CUDA : split_for(w, *cap);
+  }
+  ClusterCapacity cap;
+  for (int n = 0; n <= kMaxSplit; ++n) cap.clusters[n] = clusters[n];
+  if (cap.clusters[1] <= 0) return SPLASH_ERR_INVALID_ARGUMENT;
+  return split_for(w, cap);
 }
 
 // What fits on the current device, asked once per kernel and device; also sets the kernel's shared-memory size.

@@ -125,7 +125,8 @@ def splash_fwd_fp8(kernel: _k.SplashAttentionKernel, q: Fp8Tensor, k: Fp8Tensor,
   args.flags = _native.FP8_P_F16 if p_format == "f16" else 0
   stream = torch.cuda.current_stream(qd.device).cuda_stream
   with torch.cuda.device(qd.device):
-    _native.check(_native.lib().splash_fwd_fp8(C.byref(args), C.c_void_p(stream)), "splash_fwd_fp8")
+    _native.check(_native.lib().splash_fwd_fp8_shard(C.byref(args), C.byref(kernel._shards), C.c_void_p(stream)),  # pylint: disable=protected-access
+                  "splash_fwd_fp8")
   for t in keep + [q_seg, kv_seg, sinks_f32]:
     if t is not None:
       t.record_stream(torch.cuda.current_stream(qd.device))

@@ -16,6 +16,7 @@ there is no PyTorch or CPU fallback — an unsupported configuration raises
 from __future__ import annotations
 
 import contextlib
+import copy
 import ctypes as C
 import dataclasses
 import enum
@@ -358,7 +359,7 @@ def splash_forward(kernel, q, k, v, q_seg, kv_seg, scale, sinks, max_logit, shar
   if o_peer is not None:
     args.o_peer = o_peer
   with _on(q.device):
-    _native.check(_native.lib().splash_fwd(C.byref(args), _raw_stream(q.device)), "splash_fwd")
+    _native.check(_native.lib().splash_fwd_shard(C.byref(args), C.byref(kernel._shards), _raw_stream(q.device)), "splash_fwd")  # pylint: disable=protected-access
   return q, k, v, o, lse, max_logits, sinks_f32
 
 
@@ -438,7 +439,7 @@ def splash_backward(kernel: "SplashAttentionKernel", q, k, v, o, lse, d_o, q_seg
   if peers is not None:
     args.dq_peer, args.dk_peer, args.dv_peer = peers
   with _on(q.device):
-    _native.check(lib.splash_bwd(C.byref(args), _raw_stream(q.device)), "splash_bwd")
+    _native.check(lib.splash_bwd_shard(C.byref(args), C.byref(kernel._shards), _raw_stream(q.device)), "splash_bwd")  # pylint: disable=protected-access
   n = q.shape[0] * q.shape[1] * q.shape[2]
   neg_di = workspace[:4 * n].view(torch.float32).view(q.shape[0], q.shape[1], q.shape[2])
   return dq, dk, dv, neg_di
@@ -465,6 +466,7 @@ class SplashAttentionKernel:
     self._dynamic_mask = dynamic_mask
     self._device_tables: dict = {}
     self._mask_fn = _mask_fn_struct(kwargs.get("mask_function_rule"))
+    self._shards = _native.SplashShards(head_shards=self.head_shards)
 
   def _dynamic_info(self, is_dkv: bool) -> MaskInfo:
     cfg = self.config
@@ -499,6 +501,8 @@ class SplashAttentionKernel:
   # kernel.py:2023-2053 hands shard i of them to device i under shard_map); a call then takes the
   # q rows of ONE shard ([.., q_len / shards, 128], `q_shard=i`) against all keys.
   q_seq_shards = property(lambda self: int(self.kwargs.get("q_seq_shards", 1)))
+  # > 1: a call works on one of that many equal head shards of a call (see head_shard)
+  head_shards = property(lambda self: int(self.kwargs.get("head_shards", 1)))
 
   def with_options(self, **kwargs) -> "SplashAttentionKernel":
     """A kernel object for the same mask with some keyword options replaced (``repeatable_dq``,
@@ -506,6 +510,21 @@ class SplashAttentionKernel:
     other = SplashAttentionKernel(self._fwd_mask_info, self._dkv_mask_info, dynamic_mask=self._dynamic_mask,
                                   **dict(self.kwargs, **kwargs))
     other._device_tables = self._device_tables  # pylint: disable=protected-access
+    return other
+
+  def head_shard(self, shards: int) -> "SplashAttentionKernel":
+    """This kernel for calls on ``1 / shards`` of the heads (one rank's of a head-sharded scheme).
+
+    A call too small to fill the GPU is shared out between SMs, in parts whose number, and with it the
+    last bits of its results, depends on the call's size.  The object returned here shares a shard's
+    rows out as the call on all heads does, so that the shards' results are the whole's bit for bit
+    (dq with ``repeatable_dq``, as ever).  Device tables and the error record are shared with this one.
+    """
+    if shards < 1 or shards * self.head_shards > 0xffff:
+      raise ValueError(f"cannot cut the heads into {shards * self.head_shards} shards")
+    other = copy.copy(self)
+    other.kwargs = dict(self.kwargs, head_shards=shards * self.head_shards)
+    other._shards = _native.SplashShards(head_shards=other.head_shards)
     return other
 
   def _tables(self, device: torch.device, batch: int = 1, shard: int = 0):

@@ -10,8 +10,9 @@ The reference has no all-to-all; its context-parallel wrapper is ring attention
 (tokamax/_src/ops/experimental/tpu/splash_attention/ring_attention_kernel.py:68-293).  The
 contract kept here is the one its tests state for sharded execution
 (ring_attention_kernel_test.py:136-172): the sharded result equals the unsharded splash call on
-the gathered inputs.  Because the kernels are deterministic and each rank computes whole heads,
-the result is bitwise equal to a single-GPU run of the same heads.
+the gathered inputs.  Because the kernels are deterministic, each rank computes whole heads, and a
+rank's launch shares its rows out between SMs as the launch on all heads does
+(``SplashAttentionKernel.head_shard``), the result is bitwise equal to a single-GPU run on all heads.
 
 Layout: tensors are ``[batch, heads, seq, head_dim]``.  An exchange is ONE collective
 (``all_to_all_single``, which NCCL runs as a single grouped transfer over NVLink): the send buffer is
@@ -235,8 +236,9 @@ class _FusedUlysses(torch.autograd.Function):
   def forward(ctx, q, k, v, owner, segment_ids, logits_scale):
     from tokamax_b200 import splash_attention_kernel as splash  # pylint: disable=g-import-not-at-top
 
-    engine, kernel = owner.engine, owner.attention
+    engine = owner.engine
     rank, world = _world(engine.group)
+    kernel = owner.local_attention(world)
     needs_grad = any(ctx.needs_input_grad[:3])
     slot = engine.acquire(needs_grad)
     q_h = engine.exchange(q, True, f"q{slot}", (True, False))
@@ -322,7 +324,8 @@ class UlyssesSplashAttention:
 
   Args:
     attention: a ``SplashAttentionKernel`` built for the FULL (unsharded) mask, or any callable
-      ``(q, k, v, segment_ids, *, logits_scale) -> out`` over ``[batch, heads, seq, dim]``.
+      ``(q, k, v, segment_ids, *, logits_scale) -> out`` over ``[batch, heads, seq, dim]``.  (One that
+      wraps a kernel object wraps ``kernel.head_shard(P)`` to keep the bits of the unsharded call.)
     group: process group spanning the context-parallel ranks (default: the world).
     exchange: "nccl" (default: one ``all_to_all_single`` per tensor), "peer" (:class:`PeerExchange`:
       own copy kernel over symmetric memory; CUDA + NVLink peers only) or "fused" ("peer", and the
@@ -388,9 +391,14 @@ class UlyssesSplashAttention:
     seg_full = None
     if segment_ids is not None:
       seg_full = base.SegmentIds(self._gather_seq(segment_ids.q), self._gather_seq(segment_ids.kv))
-    o_h = self.attention(q_h, k_h, v_h, seg_full, logits_scale=logits_scale)
+    o_h = self.local_attention(world)(q_h, k_h, v_h, seg_full, logits_scale=logits_scale)
     out = head_to_seq(o_h, self.group, engine, tags[3])
     return out.clone() if engine is not None else out  # the caller's tensor must outlive the buffer's next use
+
+  def local_attention(self, world: int) -> Callable:
+    """What runs on one rank's heads; a kernel object as one of ``world`` head shards."""
+    head_shard = getattr(self.attention, "head_shard", None)
+    return self.attention if head_shard is None or world == 1 else head_shard(world)
 
   def _can_fuse(self, q_h, v_h) -> bool:
     from tokamax_b200 import splash_attention_kernel as splash  # pylint: disable=g-import-not-at-top
