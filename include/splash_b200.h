@@ -292,6 +292,9 @@ int splash_fwd(const SplashFwdArgs* args, void* cuda_stream);
  * whole call would, so that its results are bit for bit the whole call's.  Zero-initialise. */
 typedef struct SplashShards {
   int32_t head_shards; /* the call's heads lie in this many equal launches, each with its own kv heads (0, 1: in one) */
+  int32_t q_shards;    /* its query rows lie in this many launches of q_len rows, in order: q_sequence[i], where it
+                          is given, is the row's number in the call (0, 1: in one; rows of a launch whose
+                          q_sequence says otherwise are not shared) */
 } SplashShards;
 /* splash_fwd as one of such launches; shards == NULL: splash_fwd. */
 int splash_fwd_shard(const SplashFwdArgs* args, const SplashShards* shards, void* cuda_stream);

@@ -1,11 +1,12 @@
 """How many CTAs share a schedule row: the launchers' rule, asked on the host with given capacities.
 
-GPU (marked): results of calls on a share of the heads are the whole call's, bit for bit, at sizes
-whose rows are shared.
+GPU (marked), at sizes whose rows are shared: results of calls on a share of the heads are the whole
+call's, bit for bit, and so are o, logsumexp and dq of calls on a share of the query rows.
 """
 import ctypes as C
 import math
 
+import numpy as np
 import pytest
 import torch
 
@@ -26,16 +27,18 @@ def _sizes(tensor, *shape):
     tensor.size[i] = n
 
 
-def _args(mask, batch, hq, hkv, sq, skv, head_shards=0, d=128, d_v=128):
-  """Forward and backward arguments as far as the rule reads them, for 1 / head_shards of the heads, and SplashShards."""
+def _args(mask, batch, hq, hkv, sq, skv, head_shards=0, q_shards=0, d=128, d_v=128):
+  """Forward and backward arguments as far as the rule reads them, for 1 / head_shards of the heads and
+  1 / q_shards of the query rows (not the first ones), and SplashShards."""
   fa, ba = _native.SplashFwdArgs(), _native.SplashBwdArgs()
   n = max(head_shards, 1)
   for a in (fa, ba):
-    _sizes(a.q, batch, hq // n, sq, d)
+    a.mask_fn = splash._mask_fn_struct(getattr(mask, "interval_rule", None))  # pylint: disable=protected-access
+    _sizes(a.q, batch, hq // n, sq // max(q_shards, 1), d)
+    a.q_sequence = 4096 if q_shards > 1 and a.mask_fn.kind else None  # (an address nobody reads)
     _sizes(a.k, batch, hkv // n, skv, d)
     _sizes(a.v, batch, hkv // n, skv, d_v)
-    a.mask_fn = splash._mask_fn_struct(getattr(mask, "interval_rule", None))  # pylint: disable=protected-access
-  return fa, ba, _native.SplashShards(head_shards=head_shards)
+  return fa, ba, _native.SplashShards(head_shards, q_shards)
 
 
 def _parts(*args, clusters=None, **kw):
@@ -56,6 +59,29 @@ def test_head_shards_are_shared_out_as_the_whole_call(batch, hq, hkv, s, shards,
   assert _parts(mask, batch, hq, hkv, s, s, head_shards=shards, clusters=clusters) == whole
   if (hq, s, shards) == (8, 2048, 2):  # a rank's launch by itself would be cut otherwise
     assert _parts(mask, batch, hq // 2, hkv // 2, s, s, clusters=clusters) != whole and min(whole) > 1
+
+
+@pytest.mark.parametrize("clusters", CAPACITIES)
+@pytest.mark.parametrize("sq,skv,shards", [(2048, 4096, 2), (768, 4096, 2), (1920, 8192, 5), (512, 16384, 4)])
+def test_query_shards_are_shared_out_as_the_whole_call(sq, skv, shards, clusters):
+  for mask in (mask_lib.CausalMask((sq, skv), skv - sq), mask_lib.LocalMask((sq, skv), (skv // 2, 0), skv - sq),
+               mask_lib.FullMask((sq, skv))):
+    whole, _ = _parts(mask, 1, 8, 4, sq, skv, clusters=clusters)
+    assert whole > 1 and _parts(mask, 1, 8, 4, sq, skv, q_shards=shards, clusters=clusters)[0] == whole
+
+
+def test_query_shards_say_whether_their_rows_are_in_order():
+  s, cpu = 512, torch.device("cpu")
+  kernel = splash.make_splash_mha(mask_lib.CausalMask((s, s)), q_seq_shards=2)
+  first, second = (splash._DeviceTables(kernel, cpu, i) for i in range(2))  # pylint: disable=protected-access
+  assert first.q_shards == second.q_shards == 2 and first.q_sequence is None
+  assert second.q_sequence.tolist() == list(range(s // 2, s))
+  mask = mask_lib.CausalMask((s, s))
+  mask.q_sequence = np.concatenate([np.arange(256), np.arange(256, 512)[::-1]]).astype(np.int32)
+  kernel = splash.make_splash_mha(mask, q_seq_shards=2)
+  for i in range(2):  # rows of another order: not shared, in either shard
+    tables = splash._DeviceTables(kernel, cpu, i)  # pylint: disable=protected-access
+    assert tables.q_shards == 1 and tables.q_sequence.tolist() == mask.q_sequence[256 * i:256 * (i + 1)].tolist()
 
 
 def test_row_parts_refuses_what_it_cannot_read():
@@ -110,3 +136,34 @@ def test_shares_of_the_heads_give_the_whole_calls_bits(name, b, hq, hkv, sq, skv
       else:
         assert torch.equal(got, want)
   kernel.check_errors()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name", ["causal", "window", "full", "table"])
+@pytest.mark.parametrize("sq,skv,shards", [(1024, 4096, 4), (768, 2944, 2)])  # 3 q tiles a shard: other pairs than the whole's
+def test_shares_of_the_query_rows_give_the_whole_calls_bits(name, sq, skv, shards):
+  dev = torch.device("cuda:0")
+  table = np.random.default_rng(5).random((sq, skv)) < 0.3
+  table[:, 512:1024] = False
+  mask = {"causal": lambda: mask_lib.CausalMask((sq, skv), skv - sq),
+          "window": lambda: mask_lib.LocalMask((sq, skv), (skv * 3 // 4, 0), skv - sq),
+          "full": lambda: mask_lib.FullMask((sq, skv)), "table": lambda: mask_lib.NumpyMask(table)}[name]()
+  g = torch.Generator().manual_seed(9)
+  mk = lambda h, s: torch.randn(1, h, s, 128, generator=g).to(torch.bfloat16).to(dev)
+  q, k, v, do = mk(4, sq), mk(2, skv), mk(2, skv), mk(4, sq)
+  kw = dict(save_residuals=True, repeatable_dq=True)
+  whole, cut = (splash.make_splash_mha(mask, q_seq_shards=n, **kw) for n in (1, shards))
+  assert _parts(mask, 1, 4, 2, sq, skv)[0] > 1
+
+  def call(kern, rows, **kwargs):
+    qi = q[:, :, rows].clone().requires_grad_(True)
+    out, res = kern(qi, k, v, logits_scale=0.09, **kwargs)
+    out.backward(do[:, :, rows])
+    kern.check_errors()
+    return out, qi.grad, res["logsumexp"][..., None], res["max_logits"][..., None]
+
+  want = call(whole, slice(0, sq))
+  for i in range(shards):
+    rows = slice(i * sq // shards, (i + 1) * sq // shards)
+    for got, ref in zip(call(cut, rows, q_shard=i), want):
+      assert torch.equal(got, ref[:, :, rows])

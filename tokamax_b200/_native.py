@@ -154,7 +154,7 @@ class SplashFwdArgs(C.Structure):
 
 
 class SplashShards(C.Structure):
-  _fields_ = [("head_shards", C.c_int32)]
+  _fields_ = [("head_shards", C.c_int32), ("q_shards", C.c_int32)]
 
 
 class SplashFwdFp8Args(C.Structure):

@@ -1138,6 +1138,9 @@ static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap) {
 // CTAs that share a kv tile of this call's dkv kernel (head dims up to 128)
 static int dkv_split(const SplashBwdArgs& a, const SplashShards& shards, bool fused, const int32_t* clusters) {
   if (a.q_segment_ids != nullptr || a.q_sequence != nullptr) return 1;
+  // a shard of the query rows: its dk / dv are one summand of the call's, there are no bits to keep; where the
+  // mask is a function, the first shard (whose rows need no q_sequence) leaves its kv tiles whole as the others do
+  if (shards.q_shards > 1 && a.mask_fn.kind != SPLASH_MASK_TABLE) return 1;
   const int64_t n_rows = a.k.size[2] / kTile;
   RowWork rw = estimate_row_work(a.mask_fn, (int)n_rows, kTile, (int)(a.q.size[2] / kTile),
                                  n_rows * a.k.size[0] * a.k.size[1] * (shards.head_shards > 1 ? shards.head_shards : 1), true);

@@ -802,8 +802,9 @@ static FwdKernel fwd_kernel(bool split, int variant) {
 
 // CTAs that share a schedule row (256 query rows) of this call; the 128-wide kernels only
 static int fwd_split(const SplashFwdArgs& a, const SplashShards& shards, int variant, const int32_t* clusters) {
-  if (a.q_segment_ids != nullptr || a.q_sequence != nullptr) return 1;
-  const int64_t n_rows = (a.q.size[2] / kTile + 1) / 2;
+  const int64_t q_shards = shards.q_shards > 1 ? shards.q_shards : 1;
+  if (a.q_segment_ids != nullptr || (a.q_sequence != nullptr && q_shards == 1)) return 1;
+  const int64_t n_rows = (a.q.size[2] / kTile * q_shards + 1) / 2;
   const RowWork rw = estimate_row_work(a.mask_fn, (int)n_rows, 2 * kTile, (int)(a.k.size[2] / kTile),
                                        n_rows * a.q.size[0] * a.q.size[1] * (shards.head_shards > 1 ? shards.head_shards : 1));
   return row_parts(rw, clusters, [&] {

@@ -16,9 +16,8 @@ constexpr int kMaxSplit = 8;  // portable cluster size
 
 // Steps (128-column tiles) of the longest row and of the average one, from the mask function; a table
 // mask counts as full, whether it comes from the host or from the device: so both give the same bits.
-// Not asked for calls with q_sequence: a shard of the query rows gives the bits that the whole gives
-// while both leave their rows whole.  Nor for calls with segment ids, which cut rows at places that only
-// the device knows.
+// Not asked for calls whose rows come in an order of their own (q_sequence), nor for calls with segment ids,
+// which cut rows at places that only the device knows.
 struct RowWork {
   float longest, mean;  // 0: rows are left whole
   int64_t ctas;         // rows of the call (of all launches that make it up)

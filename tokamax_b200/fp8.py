@@ -125,7 +125,7 @@ def splash_fwd_fp8(kernel: _k.SplashAttentionKernel, q: Fp8Tensor, k: Fp8Tensor,
   args.flags = _native.FP8_P_F16 if p_format == "f16" else 0
   stream = torch.cuda.current_stream(qd.device).cuda_stream
   with torch.cuda.device(qd.device):
-    _native.check(_native.lib().splash_fwd_fp8_shard(C.byref(args), C.byref(kernel._shards), C.c_void_p(stream)),  # pylint: disable=protected-access
+    _native.check(_native.lib().splash_fwd_fp8_shard(C.byref(args), _k._shards(kernel, tables), C.c_void_p(stream)),  # pylint: disable=protected-access
                   "splash_fwd_fp8")
   for t in keep + [q_seg, kv_seg, sinks_f32]:
     if t is not None:

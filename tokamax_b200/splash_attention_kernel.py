@@ -191,13 +191,13 @@ class _DeviceTables:
         pmb_t = np.ascontiguousarray(np.swapaxes(np.asarray(fwd.partial_mask_blocks), -1, -2))
       self.dkv = self._upload(state, pid, cfg.block_q, cfg.block_kv, 2, pmb_t, device)
     self.error_record = torch.zeros(4, dtype=torch.int32, device=device)
-    q_seq = fwd.q_sequence
-    if q_seq is not None and n_shards > 1:  # global q indices of this shard's rows
-      q_seq = np.asarray(q_seq)[shard * q_len:(shard + 1) * q_len]
+    q_seq = None if fwd.q_sequence is None else np.asarray(fwd.q_sequence)
+    in_order = q_seq is None or np.array_equal(q_seq, np.arange(len(q_seq), dtype=np.int32))
+    self.q_shards = n_shards if in_order else 1  # (launches that share their rows as one launch of the call does)
     self.q_sequence = None
-    # (the first shard keeps its indices too: with them the kernels leave every shard's rows whole, as one)
-    if q_seq is not None and (n_shards > 1 or not np.array_equal(np.asarray(q_seq), np.arange(q_len, dtype=np.int32))):
-      self.q_sequence = torch.from_numpy(np.ascontiguousarray(q_seq, dtype=np.int32)).to(device)
+    if q_seq is not None and not (in_order and shard == 0):  # global q indices of this shard's rows
+      rows = np.ascontiguousarray(q_seq[shard * q_len:(shard + 1) * q_len], dtype=np.int32)
+      self.q_sequence = torch.from_numpy(rows).to(device)
 
   def _upload(self, state, pid, bq, bkv, kind, pmb, device) -> _native.SplashDeviceSchedule:
     row_ptr, entries, row_order = _build_schedule(state, pid, bq, bkv, kind)
@@ -262,6 +262,7 @@ class _DynamicDeviceTables:
     self.tile_states = states
     self.error_record = torch.zeros(4, dtype=torch.int32, device=device)
     self.q_sequence = None
+    self.q_shards = 1
 
 
 def _segment_schedule(sched: _native.SplashDeviceSchedule, kind: int, q_seg, kv_seg, q_len: int, kv_len: int):
@@ -309,6 +310,13 @@ def _usable(t: torch.Tensor) -> torch.Tensor:
   """Returns ``t`` if the kernels can read it in place, else a contiguous copy."""
   ok = t.stride(-1) == 1 and all(s % 8 == 0 for s in t.stride()[:-1]) and t.data_ptr() % 16 == 0
   return t if ok else t.contiguous()
+
+
+def _shards(kernel, tables):
+  """The call of which a launch of ``kernel`` on these tables is a share (None: it is the call)."""
+  if kernel.head_shards == 1 and tables.q_shards == 1:
+    return None
+  return C.byref(_native.SplashShards(kernel.head_shards, tables.q_shards))
 
 
 def _mask_fn_struct(mask_function_rule) -> _native.SplashMaskFn:
@@ -359,7 +367,7 @@ def splash_forward(kernel, q, k, v, q_seg, kv_seg, scale, sinks, max_logit, shar
   if o_peer is not None:
     args.o_peer = o_peer
   with _on(q.device):
-    _native.check(_native.lib().splash_fwd_shard(C.byref(args), C.byref(kernel._shards), _raw_stream(q.device)), "splash_fwd")  # pylint: disable=protected-access
+    _native.check(_native.lib().splash_fwd_shard(C.byref(args), _shards(kernel, tables), _raw_stream(q.device)), "splash_fwd")
   return q, k, v, o, lse, max_logits, sinks_f32
 
 
@@ -439,7 +447,7 @@ def splash_backward(kernel: "SplashAttentionKernel", q, k, v, o, lse, d_o, q_seg
   if peers is not None:
     args.dq_peer, args.dk_peer, args.dv_peer = peers
   with _on(q.device):
-    _native.check(lib.splash_bwd_shard(C.byref(args), C.byref(kernel._shards), _raw_stream(q.device)), "splash_bwd")  # pylint: disable=protected-access
+    _native.check(lib.splash_bwd_shard(C.byref(args), _shards(kernel, tables), _raw_stream(q.device)), "splash_bwd")
   n = q.shape[0] * q.shape[1] * q.shape[2]
   neg_di = workspace[:4 * n].view(torch.float32).view(q.shape[0], q.shape[1], q.shape[2])
   return dq, dk, dv, neg_di
@@ -466,7 +474,6 @@ class SplashAttentionKernel:
     self._dynamic_mask = dynamic_mask
     self._device_tables: dict = {}
     self._mask_fn = _mask_fn_struct(kwargs.get("mask_function_rule"))
-    self._shards = _native.SplashShards(head_shards=self.head_shards)
 
   def _dynamic_info(self, is_dkv: bool) -> MaskInfo:
     cfg = self.config
@@ -524,7 +531,6 @@ class SplashAttentionKernel:
       raise ValueError(f"cannot cut the heads into {shards * self.head_shards} shards")
     other = copy.copy(self)
     other.kwargs = dict(self.kwargs, head_shards=shards * self.head_shards)
-    other._shards = _native.SplashShards(head_shards=other.head_shards)
     return other
 
   def _tables(self, device: torch.device, batch: int = 1, shard: int = 0):
