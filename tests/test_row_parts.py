@@ -84,6 +84,17 @@ def test_query_shards_say_whether_their_rows_are_in_order():
     assert tables.q_shards == 1 and tables.q_sequence.tolist() == mask.q_sequence[256 * i:256 * (i + 1)].tolist()
 
 
+@pytest.mark.parametrize("chunk,span", [(512, 6), (1000, 10), (4096, 32), (8192, 64), (20000, 64)])
+def test_chunked_rows_count_the_keys_they_see(chunk, span):
+  """A row of a chunked mask is a chunk long at most; as many steps of a causal mask are shared alike."""
+  s = 8192
+  got = _parts(mask_lib.ChunkedCausalMask((s, s), chunk), 1, 2, 2, s, s, clusters=CAPACITIES[1])
+  causal = _parts(mask_lib.CausalMask((s, s)), 1, 2, 2, s, s, clusters=CAPACITIES[1])
+  assert got == (1, 1) if span < 16 else min(got) > 1
+  if chunk >= s:
+    assert got == causal
+
+
 def test_row_parts_refuses_what_it_cannot_read():
   lib = _native.lib()
   mask = mask_lib.CausalMask((2048, 2048))

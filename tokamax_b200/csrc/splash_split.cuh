@@ -34,7 +34,7 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
   RowWork w{0.f, 0.f, n_ctas};
   if (n_ctas > kSplitMaxCtas) return w;
   w.longest = w.mean = (float)n_tiles;
-  if (fn.kind != SPLASH_MASK_CAUSAL && fn.kind != SPLASH_MASK_LOCAL) return w;
+  if (fn.kind == SPLASH_MASK_TABLE) return w;
   int64_t sum = 0, most = 0;
   for (int r = 0; r < n_rows; ++r) {
     // the row sees columns lo .. hi of the other side
@@ -44,7 +44,15 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
     const int64_t right = fn.kind == SPLASH_MASK_CAUSAL ? 0 : (fn.has_right ? fn.right : -1);
     const bool has_right = fn.kind == SPLASH_MASK_CAUSAL || fn.has_right;
     const bool has_left = fn.kind == SPLASH_MASK_LOCAL && fn.has_left;
-    if (!transposed) {  // query i sees keys i + offset - left .. i + offset + right
+    if (fn.kind == SPLASH_MASK_CHUNKED) {  // query i sees keys (i / chunk) * chunk .. i
+      if (!transposed) {
+        lo = first / fn.chunk * fn.chunk;
+        if (last < hi) hi = last;
+      } else {
+        lo = first;
+        if ((last / fn.chunk + 1) * fn.chunk - 1 < hi) hi = (last / fn.chunk + 1) * fn.chunk - 1;
+      }
+    } else if (!transposed) {  // query i sees keys i + offset - left .. i + offset + right
       if (has_left && first + fn.offset - left > lo) lo = first + fn.offset - left;
       if (has_right && last + fn.offset + right < hi) hi = last + fn.offset + right;
     } else {            // key j is seen by queries j - offset - right .. j - offset + left
