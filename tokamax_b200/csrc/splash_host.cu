@@ -22,19 +22,39 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+typedef CUresult (*CtxGetCurrentFn)(CUcontext*);
+
+template <typename Fn>
+static Fn driver_entry(const char* name) {
+  void* sym = nullptr;
+  cudaDriverEntryPointQueryResult qres;
+  if (cudaGetDriverEntryPoint(name, &sym, cudaEnableDefault, &qres) == cudaSuccess && qres == cudaDriverEntryPointSuccess)
+    return reinterpret_cast<Fn>(sym);
+  return nullptr;
+}
+
 static EncodeTiledFn get_encode_fn() {
   static std::mutex mu;
   static EncodeTiledFn fn = nullptr;
   std::lock_guard<std::mutex> lock(mu);
-  if (fn == nullptr) {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres) ==
-            cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(sym);
-  }
+  if (fn == nullptr) fn = driver_entry<EncodeTiledFn>("cuTensorMapEncodeTiled");
   return fn;
+}
+
+// The encoder is a driver call and needs a current context.  A thread that has made no runtime call of its own
+// (autograd's, for a first backward small enough to find its memory cached) has none, although its device is
+// right: cudaSetDevice binds the device's.  A context that is current, the caller's own perhaps, stays.
+static bool have_context() {
+  static std::mutex mu;
+  static CtxGetCurrentFn get_current = nullptr;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (get_current == nullptr) get_current = driver_entry<CtxGetCurrentFn>("cuCtxGetCurrent");
+  }
+  CUcontext current = nullptr;
+  if (get_current != nullptr && get_current(&current) == CUDA_SUCCESS && current != nullptr) return true;
+  int dev = 0;
+  return cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
 }
 
 int check_bf16_tensor(const SplashTensor& t) {
@@ -66,11 +86,7 @@ int check_e4m3_tensor(const SplashTensor& t) {
 int make_tile_tensor_map(CUtensorMap* out, const SplashTensor& t, int box_rows) {
   EncodeTiledFn enc = get_encode_fn();
   if (enc == nullptr) return SPLASH_ERR_NO_DEVICE;
-  // The encoder is a driver call and needs a current context.  A thread that has made no runtime call
-  // of its own (autograd's, for a first backward small enough to find its memory cached) has none, although
-  // its device is right; cudaSetDevice binds it.
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return SPLASH_ERR_CUDA;
+  if (!have_context()) return SPLASH_ERR_CUDA;
   const bool fp8 = t.dtype == SPLASH_F8E4M3;
   const cuuint64_t esize = fp8 ? 1u : 2u;
   const cuuint64_t dims[4] = {(cuuint64_t)t.size[3], (cuuint64_t)t.size[2], (cuuint64_t)t.size[1],
