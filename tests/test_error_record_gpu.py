@@ -1,4 +1,5 @@
-"""The device error record: a bounded wait that runs out, and what a raised record does.
+"""The device error record: a bounded wait that runs out, and what a raised record does; and launches that
+the runtime refuses.
 
 Every device-side wait in the kernels is bounded; one that runs out writes the 4-word error record
 and the kernel returns.  splash_probe_bounded_wait makes that happen on purpose in a one-thread
@@ -69,3 +70,46 @@ def test_a_raised_error_record_stops_later_kernels_and_check_errors_clears_it():
   out.backward(do)
   kernel.check_errors()
   assert torch.isfinite(out.float()).all() and torch.isfinite(qd.grad.float()).all()
+
+
+_REFUSED = """
+import ctypes as C
+import torch
+from tokamax_b200 import _native
+from tokamax_b200 import splash_attention_kernel as splash
+from tokamax_b200 import splash_attention_mask as mask_lib
+lib, cuda = _native.lib(), C.CDLL("libcuda.so.1")
+q = torch.randn(1, 2, 2048, 128, device="cuda").to(torch.bfloat16)
+mask = torch.ones(256, 256, dtype=torch.bool, device="cuda")
+states = torch.empty(4, dtype=torch.int32, device="cuda")
+for s in (256, 2048):  # rows left whole, rows shared
+  kernel, x = splash.make_splash_mha(mask_lib.FullMask((s, s)), q_seq_shards=1), q[:, :, :s].contiguous()
+  want, spare = kernel(x, x, x), kernel(x, x, x)
+  del spare  # (memory for the calls below, which cannot ask for any under a capture)
+  torch.cuda.synchronize()
+  stream, graph = C.c_void_p(), C.c_void_p()
+  # a launch on the legacy stream while a stream that waits for it is being captured is refused
+  assert cuda.cuStreamCreate(C.byref(stream), 0) == 0 and cuda.cuStreamBeginCapture_v2(stream, 0) == 0
+  try:
+    kernel(x, x, x)
+    status = 0
+  except _native.SplashError as e:
+    status = e.status
+  cuda.cuStreamEndCapture(stream, C.byref(graph))
+  assert cuda.cuStreamDestroy_v2(stream) == 0
+  assert status == -3, status
+  assert lib.splash_mask_tile_states(mask.data_ptr(), 256, 256, 256, states.data_ptr(), None) == 0, "an old error"
+  assert torch.equal(kernel(x, x, x), want) and states.tolist() == [2, 2, 2, 2]
+print("fine")
+"""
+
+
+def test_a_refused_launch_leaves_no_error_behind():
+  """The call that fails reports it; the next one, which checks the runtime's last error, is not to."""
+  import os
+  import subprocess
+  import sys
+
+  root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+  r = subprocess.run([sys.executable, "-c", _REFUSED], cwd=root, capture_output=True, text=True, timeout=300)
+  assert r.returncode == 0 and "fine" in r.stdout, r.stderr[-2000:]

@@ -118,8 +118,10 @@ inline const ClusterCapacity* cluster_capacity(const void* kernel, int variant, 
   if (!known[dev][variant]) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) {
+      (void)cudaGetLastError();
       return nullptr;
+    }
     c.clusters[0] = 0;
     c.clusters[1] = sms;
     for (int n = 2; n <= kMaxSplit; ++n) {
@@ -216,7 +218,9 @@ inline cudaError_t launch_clusters(void (*kernel)(Params...), unsigned rows, int
     cfg.attrs = attr;
     cfg.numAttrs = 1;
   }
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (err != cudaSuccess) (void)cudaGetLastError();  // reported here: the next call's check is not to find it
+  return err;
 }
 
 }  // namespace sb
