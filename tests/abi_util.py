@@ -50,3 +50,31 @@ def fwd_bwd(lib, kernel, q, k, v, do, scale, *, fused=False, error_record=None, 
   _native.check(lib.splash_bwd(C.byref(ba), stream), "splash_bwd")
   torch.cuda.synchronize(dev)
   return o, lse, dq, dk, dv
+
+
+def _sizes(tensor, *shape):
+  for i, n in enumerate(shape):
+    tensor.size[i] = n
+
+
+def _row_args(mask, batch, hq, hkv, sq, skv, head_shards=0, q_shards=0, d=128, d_v=128):
+  """Forward and backward arguments as far as the rule reads them, for 1 / head_shards of the heads and
+  1 / q_shards of the query rows (not the first ones), and SplashShards."""
+  fa, ba = _native.SplashFwdArgs(), _native.SplashBwdArgs()
+  n = max(head_shards, 1)
+  for a in (fa, ba):
+    a.mask_fn = splash._mask_fn_struct(getattr(mask, "interval_rule", None))  # pylint: disable=protected-access
+    _sizes(a.q, batch, hq // n, sq // max(q_shards, 1), d)
+    a.q_sequence = 4096 if q_shards > 1 and a.mask_fn.kind else None  # (an address nobody reads)
+    _sizes(a.k, batch, hkv // n, skv, d)
+    _sizes(a.v, batch, hkv // n, skv, d_v)
+  return fa, ba, _native.SplashShards(head_shards, q_shards)
+
+
+def row_parts(*args, clusters=None, **kw):
+  """CTAs that share a schedule row of the forward, a kv tile of dkv; ``clusters``: None asks the current device."""
+  fa, ba, shards = _row_args(*args, **kw)
+  lib = _native.lib()
+  table = None if clusters is None else C.byref((C.c_int32 * 9)(*clusters))
+  return (lib.splash_fwd_row_parts(C.byref(fa), C.byref(shards), table),
+          lib.splash_bwd_row_parts(C.byref(ba), C.byref(shards), table))

@@ -3,7 +3,6 @@
 GPU (marked), at sizes whose rows are shared: results of calls on a share of the heads are the whole
 call's, bit for bit, and so are o, logsumexp and dq of calls on a share of the query rows.
 """
-import ctypes as C
 import math
 
 import numpy as np
@@ -13,6 +12,7 @@ import torch
 from tokamax_b200 import _native
 from tokamax_b200 import splash_attention_kernel as splash
 from tokamax_b200 import splash_attention_mask as mask_lib
+from abi_util import row_parts
 
 # clusters of n CTAs that 148 SMs hold at a time: in one piece, in GPCs of 16 and 18 SMs, in pairs of SMs lost to each
 CAPACITIES = [
@@ -22,43 +22,16 @@ CAPACITIES = [
 ]
 
 
-def _sizes(tensor, *shape):
-  for i, n in enumerate(shape):
-    tensor.size[i] = n
-
-
-def _args(mask, batch, hq, hkv, sq, skv, head_shards=0, q_shards=0, d=128, d_v=128):
-  """Forward and backward arguments as far as the rule reads them, for 1 / head_shards of the heads and
-  1 / q_shards of the query rows (not the first ones), and SplashShards."""
-  fa, ba = _native.SplashFwdArgs(), _native.SplashBwdArgs()
-  n = max(head_shards, 1)
-  for a in (fa, ba):
-    a.mask_fn = splash._mask_fn_struct(getattr(mask, "interval_rule", None))  # pylint: disable=protected-access
-    _sizes(a.q, batch, hq // n, sq // max(q_shards, 1), d)
-    a.q_sequence = 4096 if q_shards > 1 and a.mask_fn.kind else None  # (an address nobody reads)
-    _sizes(a.k, batch, hkv // n, skv, d)
-    _sizes(a.v, batch, hkv // n, skv, d_v)
-  return fa, ba, _native.SplashShards(head_shards, q_shards)
-
-
-def _parts(*args, clusters=None, **kw):
-  fa, ba, shards = _args(*args, **kw)
-  lib = _native.lib()
-  table = None if clusters is None else C.byref((C.c_int32 * 9)(*clusters))
-  return (lib.splash_fwd_row_parts(C.byref(fa), C.byref(shards), table),
-          lib.splash_bwd_row_parts(C.byref(ba), C.byref(shards), table))
-
-
 @pytest.mark.parametrize("clusters", CAPACITIES)
 @pytest.mark.parametrize("batch,hq,hkv,s,shards", [(1, 8, 4, 2048, 2), (1, 8, 4, 2048, 4), (2, 16, 16, 4096, 8),
                                                    (1, 64, 8, 8192, 8), (1, 8, 8, 16384, 8)])
 def test_head_shards_are_shared_out_as_the_whole_call(batch, hq, hkv, s, shards, clusters):
   mask = mask_lib.CausalMask((s, s))
-  whole = _parts(mask, batch, hq, hkv, s, s, clusters=clusters)
+  whole = row_parts(mask, batch, hq, hkv, s, s, clusters=clusters)
   assert min(whole) >= 1
-  assert _parts(mask, batch, hq, hkv, s, s, head_shards=shards, clusters=clusters) == whole
+  assert row_parts(mask, batch, hq, hkv, s, s, head_shards=shards, clusters=clusters) == whole
   if (hq, s, shards) == (8, 2048, 2):  # a rank's launch by itself would be cut otherwise
-    assert _parts(mask, batch, hq // 2, hkv // 2, s, s, clusters=clusters) != whole and min(whole) > 1
+    assert row_parts(mask, batch, hq // 2, hkv // 2, s, s, clusters=clusters) != whole and min(whole) > 1
 
 
 @pytest.mark.parametrize("clusters", CAPACITIES)
@@ -66,8 +39,8 @@ def test_head_shards_are_shared_out_as_the_whole_call(batch, hq, hkv, s, shards,
 def test_query_shards_are_shared_out_as_the_whole_call(sq, skv, shards, clusters):
   for mask in (mask_lib.CausalMask((sq, skv), skv - sq), mask_lib.LocalMask((sq, skv), (skv // 2, 0), skv - sq),
                mask_lib.FullMask((sq, skv))):
-    whole, _ = _parts(mask, 1, 8, 4, sq, skv, clusters=clusters)
-    assert whole > 1 and _parts(mask, 1, 8, 4, sq, skv, q_shards=shards, clusters=clusters)[0] == whole
+    whole, _ = row_parts(mask, 1, 8, 4, sq, skv, clusters=clusters)
+    assert whole > 1 and row_parts(mask, 1, 8, 4, sq, skv, q_shards=shards, clusters=clusters)[0] == whole
 
 
 def test_query_shards_say_whether_their_rows_are_in_order():
@@ -88,8 +61,8 @@ def test_query_shards_say_whether_their_rows_are_in_order():
 def test_chunked_rows_count_the_keys_they_see(chunk, span):
   """A row of a chunked mask is a chunk long at most; as many steps of a causal mask are shared alike."""
   s = 8192
-  got = _parts(mask_lib.ChunkedCausalMask((s, s), chunk), 1, 2, 2, s, s, clusters=CAPACITIES[1])
-  causal = _parts(mask_lib.CausalMask((s, s)), 1, 2, 2, s, s, clusters=CAPACITIES[1])
+  got = row_parts(mask_lib.ChunkedCausalMask((s, s), chunk), 1, 2, 2, s, s, clusters=CAPACITIES[1])
+  causal = row_parts(mask_lib.CausalMask((s, s)), 1, 2, 2, s, s, clusters=CAPACITIES[1])
   assert got == (1, 1) if span < 16 else min(got) > 1
   if chunk >= s:
     assert got == causal
@@ -101,10 +74,10 @@ def test_row_parts_refuses_what_it_cannot_read():
   assert lib.splash_fwd_row_parts(None, None, None) == -1 and lib.splash_bwd_row_parts(None, None, None) == -1
   assert lib.splash_fwd_shard(None, None, None) == -1 and lib.splash_bwd_shard(None, None, None) == -1
   assert lib.splash_fwd_fp8_shard(None, None, None) == -1
-  assert _parts(mask, 0, 8, 4, 2048, 2048, clusters=CAPACITIES[0]) == (-1, -1)
-  assert _parts(mask, 1, 8, 4, 2000, 2048, clusters=CAPACITIES[0]) == (-1, -1)
-  assert _parts(mask, 1, 8, 4, 2048, 2048, clusters=[0] * 9) == (-1, -1)
-  assert _parts(mask, 1, 8, 4, 2048, 2048, d=192, clusters=CAPACITIES[0]) == (1, 1)  # two-panel kernels
+  assert row_parts(mask, 0, 8, 4, 2048, 2048, clusters=CAPACITIES[0]) == (-1, -1)
+  assert row_parts(mask, 1, 8, 4, 2000, 2048, clusters=CAPACITIES[0]) == (-1, -1)
+  assert row_parts(mask, 1, 8, 4, 2048, 2048, clusters=[0] * 9) == (-1, -1)
+  assert row_parts(mask, 1, 8, 4, 2048, 2048, d=192, clusters=CAPACITIES[0]) == (1, 1)  # two-panel kernels
   kernel = splash.make_splash_mha(mask, q_seq_shards=1)
   assert kernel.head_shards == 1 and kernel.head_shard(4).head_shard(2).head_shards == 8
   for bad in (0, -1, 1 << 16):
@@ -115,7 +88,7 @@ def test_row_parts_refuses_what_it_cannot_read():
 @pytest.mark.gpu
 @pytest.mark.parametrize("repeatable", [True, False])
 @pytest.mark.parametrize("name,b,hq,hkv,sq,skv,shards", [("causal", 1, 8, 4, 2048, 2048, 2), ("causal", 1, 8, 4, 2048, 2048, 4),
-                                                         ("window", 2, 4, 2, 384, 4096, 2), ("full", 1, 12, 2, 256, 2176, 2)])
+                                                         ("window", 2, 4, 2, 384, 4096, 2), ("full", 1, 32, 8, 256, 4096, 2)])
 def test_shares_of_the_heads_give_the_whole_calls_bits(name, b, hq, hkv, sq, skv, shards, repeatable):
   dev = torch.device("cuda:0")
   mask = {"causal": lambda: mask_lib.CausalMask((sq, skv), skv - sq),
@@ -135,9 +108,9 @@ def test_shares_of_the_heads_give_the_whole_calls_bits(name, b, hq, hkv, sq, skv
 
   whole = call(kernel, q, k, v, do)
   # the case tests what it says only where rows are shared, and a share by itself would not do
-  assert max(_parts(mask, b, hq, hkv, sq, skv)) > 1
-  assert _parts(mask, b, hq, hkv, sq, skv, head_shards=shards) == _parts(mask, b, hq, hkv, sq, skv)
-  assert _parts(mask, b, hq // shards, hkv // shards, sq, skv) != _parts(mask, b, hq, hkv, sq, skv)
+  assert max(row_parts(mask, b, hq, hkv, sq, skv)) > 1
+  assert row_parts(mask, b, hq, hkv, sq, skv, head_shards=shards) == row_parts(mask, b, hq, hkv, sq, skv)
+  assert row_parts(mask, b, hq // shards, hkv // shards, sq, skv) != row_parts(mask, b, hq, hkv, sq, skv)
   for rank in range(shards):
     heads = lambda t: t[:, rank * t.shape[1] // shards:(rank + 1) * t.shape[1] // shards]  # noqa: B023
     share = call(kernel.head_shard(shards), *map(heads, (q, k, v, do)))
@@ -164,7 +137,7 @@ def test_shares_of_the_query_rows_give_the_whole_calls_bits(name, sq, skv, shard
   q, k, v, do = mk(4, sq), mk(2, skv), mk(2, skv), mk(4, sq)
   kw = dict(save_residuals=True, repeatable_dq=True)
   whole, cut = (splash.make_splash_mha(mask, q_seq_shards=n, **kw) for n in (1, shards))
-  assert _parts(mask, 1, 4, 2, sq, skv)[0] > 1
+  assert row_parts(mask, 1, 4, 2, sq, skv)[0] > 1
 
   def call(kern, rows, **kwargs):
     qi = q[:, :, rows].clone().requires_grad_(True)

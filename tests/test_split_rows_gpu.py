@@ -1,9 +1,10 @@
 """Grids that leave SMs idle: schedule rows shared by a cluster of CTAs, against the CPU oracle.
 
-A few heads and long rows, so that the launchers take 2 .. 8 CTAs a row: every way of forming a
-row's entries (causal offset, window, table mask; segment ids, whose rows stay whole), odd numbers of query tiles, parts of
-unequal length, rows without a live key in some part, sinks (counted once) and a fixed maximum.
-Bounds: those of test_splash_gpu.py, but for outputs of rows with one large weight.
+Few heads, and rows that are shared where the test says so: every way of forming a row's entries (causal
+offset, window, chunks, table mask; segment ids, whose rows stay whole), odd numbers of query tiles, parts
+of unequal length, rows without a live key in some part, sinks (counted once) and a fixed maximum; every
+number of parts, 2 .. 8; second destinations; a record that holds an error.
+Bounds: those of test_splash_gpu.py, and for outputs what rounding P and the result to bf16 gives.
 """
 import dataclasses
 import math
@@ -12,7 +13,9 @@ import numpy as np
 import pytest
 import torch
 
+import abi_util
 from oracle import attention_ref
+from tokamax_b200 import _native
 from tokamax_b200 import fp8
 from tokamax_b200 import splash_attention_kernel as splash
 from tokamax_b200 import splash_attention_mask as mask_lib
@@ -38,6 +41,13 @@ def _table(sq, skv):
   return m
 
 
+def _out_bound(ro, q, k, v, dense, seg, **kw):
+  """P and the result are rounded to bf16, 8 significant bits, so each is off by up to 2^-8 of itself: an output
+  by 2^-8 (sum p |v| + |o|), and a fiftieth of that for everything held in fp32."""
+  spread, _, _ = attention_ref.attention_reference(q, k, v.abs(), dense, seg, **kw)
+  return 1.02 * 2.0 ** -8 * (spread + ro.abs()) + 1e-6
+
+
 CASES = {
     "causal": (lambda sq, skv: mask_lib.CausalMask((sq, skv), skv - sq), {}),
     "window": (lambda sq, skv: mask_lib.LocalMask((sq, skv), (skv // 3, 0), skv - sq), {}),
@@ -56,6 +66,9 @@ def test_forward_and_gradients(name, sq, skv, hq, hkv):
   mask = make(sq, skv)
   dense = mask if isinstance(mask, np.ndarray) else _dense(mask)
   d = 64 if name == "window" else 128
+  # rows of 16 key tiles and more are shared, kv tiles of 16 (q tile, head) steps and more; none with segment ids
+  parts = abi_util.row_parts(mask, 1, hq, hkv, sq, skv, d=d, d_v=d)
+  assert (parts[0] > 1) == (skv > 2048 and name != "window") and (parts[1] > 1) == (sq == 1024 and name != "window")
   q, k, v, do = _mk(0, 1, hq, sq, d), _mk(1, 1, hkv, skv, d), _mk(2, 1, hkv, skv, d), _mk(3, 1, hq, sq, d)
   # a jump of the row maximum between parts: the keys of the last tiles carry larger logits
   k[:, :, -256:] *= 4
@@ -78,9 +91,9 @@ def test_forward_and_gradients(name, sq, skv, hq, hkv):
                                            scale=scale, attn_logits_soft_cap=opt.get("cap"), sinks=sinks)]
   ro, rlse, rmax = ref[0]
   live = rlse > -1e30
-  # P and the result are rounded to bf16 (8 significant bits: half an ulp is up to 2^-8 of the value), and
-  # sum p |v| <= max |v|; with one large weight a row reaches it
-  assert (out[0].float().cpu() - ro)[live].abs().max().item() <= 2 * 2.0 ** -8 * v.abs().max().item()
+  bound = _out_bound(ro, q[0], k[0], v[0], dense, None if seg is None else (seg[0][0], seg[1][0]), scale=scale,
+                     attn_logits_soft_cap=opt.get("cap"), sinks=sinks)
+  assert torch.all(((out[0].float().cpu() - ro).abs() <= bound)[live])
   assert torch.all(out[0].float().cpu()[~live] == 0)
   assert (res["logsumexp"][0].cpu() - rlse)[live].abs().max().item() <= 1e-3
   if "fixed" not in opt:
@@ -232,3 +245,114 @@ def test_listed_tiles_without_a_live_key_change_nothing():
   for other in got[1:]:
     for a, b in zip(got[0], other):
       assert torch.equal(a, b)
+
+
+def _heads_for(which, n, mask, sq, skv, group):
+  """A number of kv heads for which this GPU's launchers take n parts (forward: which = 0, dkv: 1)."""
+  heads = [h for h in range(1, 73) if abi_util.row_parts(mask, 1, group * h, h, sq, skv)[which] == n]
+  if not heads:
+    pytest.skip(f"no call of this mask is cut in {n} parts on this GPU")
+  return heads[0]
+
+
+@pytest.mark.parametrize("n", range(2, 9))
+def test_every_number_of_parts_forward(n):
+  """Head dims 80 and 120, a last row pair of one tile, sinks, rows that end inside a part's first or last tile."""
+  sq, skv = 384, 4096
+  mask = mask_lib.LocalMask((sq, skv), (3000, 0), skv - sq)
+  h = _heads_for(0, n, mask, sq, skv, 1)
+  q, k, v = _mk(0, 1, h, sq, 80), _mk(1, 1, h, skv, 80), _mk(2, 1, h, skv, 120)
+  sinks = torch.linspace(-1.0, 2.0, h)
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1, save_residuals=True)
+  out, res = kernel(q.to(DEV), k.to(DEV), v.to(DEV), None, sinks.to(DEV), logits_scale=0.1)
+  kernel.check_errors()
+  dense = _dense(mask)
+  ro, rlse, rmax = attention_ref.attention_reference(q[0], k[0], v[0], dense, scale=0.1, sinks=sinks)
+  bound = _out_bound(ro, q[0], k[0], v[0], dense, None, scale=0.1, sinks=sinks)
+  assert torch.all((out[0].float().cpu() - ro).abs() <= bound)
+  assert (res["logsumexp"][0].cpu() - rlse).abs().max().item() <= 1e-3
+  assert (res["max_logits"][0].cpu() - rmax).abs().max().item() <= 1e-3
+
+
+@pytest.mark.parametrize("n", range(2, 9))
+@pytest.mark.parametrize("repeatable", [False, True])
+def test_every_number_of_parts_backward(n, repeatable):
+  """Nine q tiles of three q heads on a kv head: the parts begin at another tile for every head."""
+  sq, skv, group = 1152, 384, 3
+  mask = mask_lib.FullMask((sq, skv))
+  h = _heads_for(1, n, mask, sq, skv, group)
+  q, k, v, do = _mk(0, 1, group * h, sq, 80), _mk(1, 1, h, skv, 80), _mk(2, 1, h, skv, 120), _mk(3, 1, group * h, sq, 120)
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1, repeatable_dq=repeatable)
+  qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+  kernel(qd, kd, vd, logits_scale=0.1).backward(do.to(DEV))
+  kernel.check_errors()
+  wants = attention_ref.fwd_bwd(q, k, v, do, _dense(mask), scale=0.1)[3:]
+  for got, want in zip((qd.grad, kd.grad, vd.grad), wants):
+    assert ((got.float().cpu() - want).norm() / want.norm()).item() <= 1e-2
+
+
+def test_chunked_rows():
+  s, hq, hkv = 4096, 2, 1
+  mask = mask_lib.ChunkedCausalMask((s, s), 2500)  # chunks that end inside a tile; rows of 1 .. 20 key tiles
+  assert min(abi_util.row_parts(mask, 1, hq, hkv, s, s)) > 1
+  q, k, v, do = _mk(0, 1, hq, s, 128), _mk(1, 1, hkv, s, 128), _mk(2, 1, hkv, s, 128), _mk(3, 1, hq, s, 128)
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1)
+  qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+  out = kernel(qd, kd, vd, logits_scale=0.09)
+  out.backward(do.to(DEV))
+  kernel.check_errors()
+  dense = _dense(mask)
+  ro, _, _, *wants = attention_ref.fwd_bwd(q, k, v, do, dense, scale=0.09)
+  assert torch.all((out.float().cpu() - ro).abs() <= _out_bound(ro[0], q[0], k[0], v[0], dense, None, scale=0.09))
+  for got, want in zip((qd.grad, kd.grad, vd.grad), wants):
+    assert ((got.float().cpu() - want).norm() / want.norm()).item() <= 1e-2
+
+
+def test_second_destinations():
+  """Rows of shared tiles arrive in the buffers of the ranks that own them as they do in the local tensor
+  (two local buffers stand in for two ranks'), and nothing else is touched."""
+  hq, hkv, s, d, world, rank = 4, 2, 4096, 128, 2, 1
+  q, k, v, do = (_mk(i, 1, h, s, d).to(DEV) for i, h in enumerate((hq, hkv, hkv, hq)))
+  mask = mask_lib.CausalMask((s, s))
+  assert min(abi_util.row_parts(mask, 1, hq, hkv, s, s)) > 1
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1)
+  s_loc = s // world
+
+  def receive(heads):
+    bufs = [torch.full((1, heads * world, s_loc, d), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(world)]
+    ptrs = torch.tensor([t.data_ptr() for t in bufs], dtype=torch.int64, device=DEV)
+    po = _native.SplashPeerOutput()
+    po.ptrs, po.base_bytes, po.rows_per_peer = ptrs.data_ptr(), 0, s_loc
+    po.stride_b, po.stride_h, po.stride_s, po.head0 = heads * world * s_loc * d, s_loc * d, d, rank * heads
+    return bufs, ptrs, po
+
+  recv = [receive(h) for h in (hq, hq, hkv, hkv)]
+  _, _, _, o, lse, _, _ = splash.splash_forward(kernel, q, k, v, None, None, 0.09, None, None, 0, o_peer=recv[0][2])
+  grads = splash.splash_backward(kernel, q, k, v, o, lse, do, None, None, 0.09, 0, peers=tuple(r[2] for r in recv[1:]))[:3]
+  kernel.check_errors()
+  assert torch.equal(o, kernel(q, k, v, logits_scale=0.09))
+  for (bufs, _, _), local in zip(recv, (o, *grads)):
+    heads = local.shape[1]
+    for peer, buf in enumerate(bufs):
+      assert torch.equal(buf[:, rank * heads:], local[:, :, peer * s_loc:(peer + 1) * s_loc])
+      assert (buf[:, :rank * heads] == 7.0).all()
+
+
+def test_a_raised_error_record_stops_shared_rows():
+  """Every CTA of a cluster that finds an error in the record passes the cluster's barriers and writes nothing."""
+  s, hq, hkv = 4096, 4, 2
+  mask = mask_lib.CausalMask((s, s))
+  assert min(abi_util.row_parts(mask, 1, hq, hkv, s, s)) > 1
+  kernel = splash.make_splash_mha(mask, q_seq_shards=1)
+  q, k, v, do = (_mk(i, 1, h, s, 128).to(DEV) for i, h in enumerate((hq, hkv, hkv, hq)))
+  tables = kernel._tables(DEV, 1)  # pylint: disable=protected-access
+  tables.error_record[0] = 1
+  for fused in (False, True):
+    o, lse, dq, dk, dv = abi_util.fwd_bwd(_native.lib(), kernel, q, k, v, do, 0.09, fused=fused, fill=7.0)
+    for name, t in (("o", o), ("lse", lse), ("dk", dk), ("dv", dv)):
+      assert (t == 7.0).all(), name
+  with pytest.raises(_native.SplashError):
+    kernel.check_errors()
+  out = kernel(q, k, v, logits_scale=0.09)
+  kernel.check_errors()
+  assert torch.isfinite(out.float()).all()
