@@ -127,3 +127,45 @@ def test_device_mask_info_is_available_on_request_and_bad_masks_are_rejected():
   assert lib.splash_dynamic_schedule(None, 256, 256, 0, 1, None, None, 0, C.byref(out), None) == -1
   with pytest.raises(ValueError):
     splash._DynamicDeviceTables(torch.zeros(256, 256, device=DEV), 1)  # pylint: disable=protected-access
+
+
+def _views(q_len, kv_len, dtype):
+  """The same kind of mask in every layout a caller may hold: (name, tensor on the device)."""
+  g = torch.Generator().manual_seed(4)
+  tiles = torch.randint(0, 3, (q_len // 128 + 1, kv_len // 128 + 2), generator=g).repeat_interleave(128, 0).repeat_interleave(128, 1)
+  some = torch.rand(tiles.shape, generator=g) < 0.5
+  keep = ((tiles == 2) | ((tiles == 1) & some))
+  # any byte but 0 keeps a key: -128 .. 127 for int8
+  big = keep if dtype == torch.bool else torch.where(keep, torch.randint(1, 256, keep.shape, generator=g), 0).to(torch.uint8).view(dtype)
+  big = big.to(DEV)
+  yield "dense", big[:q_len, :kv_len].contiguous()
+  yield "columns of a wider mask", big[:q_len, 128:128 + kv_len]
+  yield "columns that are not 16-byte aligned", big[:q_len, 1:1 + kv_len]
+  yield "rows that are not 16-byte aligned", big.flatten()[:q_len * (kv_len + 8)].view(q_len, kv_len + 8)[:, :kv_len]
+  yield "transposed", big[:q_len, :kv_len].t().contiguous().t()
+  yield "rows of a mask twice as wide", big.flatten()[:q_len * kv_len].view(q_len // 2, 2 * kv_len).repeat(2, 1)[:, :kv_len]
+  yield "one row for all", big[:1, :kv_len].expand(q_len, kv_len)
+
+
+@pytest.mark.parametrize("dtype", [torch.bool, torch.int8, torch.uint8])
+@pytest.mark.parametrize("q_len,kv_len", [(128, 128), (256, 640), (640, 256)])
+def test_masks_of_every_layout_are_prepared_alike(q_len, kv_len, dtype):
+  """The copy, its transpose and the tile states; the states also from the entry point that makes only them."""
+  lib = _native.lib()
+  for name, view in _views(q_len, kv_len, dtype):
+    tables = splash._DynamicDeviceTables(view, batch=1)  # pylint: disable=protected-access
+    copy, transposed, states = tables.keep[:3]
+    raw = view.contiguous().view(torch.uint8).cpu().numpy()
+    np.testing.assert_array_equal(copy.cpu().numpy(), raw, err_msg=name)
+    np.testing.assert_array_equal(transposed.cpu().numpy(), raw.T, err_msg=name)
+    blocks = (raw != 0).reshape(q_len // 128, 128, kv_len // 128, 128).swapaxes(1, 2)
+    want = blocks.any(axis=(-1, -2)).astype(np.int32) + blocks.all(axis=(-1, -2)).astype(np.int32)
+    np.testing.assert_array_equal(states.cpu().numpy(), want, err_msg=name)
+    only = torch.full_like(states, -1)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib.splash_mask_tile_states(copy.data_ptr(), kv_len, q_len, kv_len, only.data_ptr(), stream) == 0
+    assert torch.equal(only, states), name
+  # the entry point itself takes rows of 16-byte multiples at 16-byte aligned addresses only
+  at = copy.data_ptr()
+  for mask_at, stride, rows in ((at + 1, kv_len, q_len), (at, kv_len + 8, q_len), (at, kv_len - 16, q_len), (at, kv_len, 100), (None, kv_len, q_len)):
+    assert lib.splash_mask_prepare(mask_at, stride, rows, kv_len, copy.data_ptr(), transposed.data_ptr(), states.data_ptr(), None) == -1
