@@ -2,8 +2,8 @@
 //
 // The kernels keep one CTA on an SM, so a grid of few long rows leaves SMs idle for the whole launch
 // (512 query rows of 32 heads against 16384 keys: 64 CTAs of 128 steps on 148 SMs).  Measured, one CTA
-// a row -> shared: that forward 240 -> 138 us (two CTAs a row); dkv of causal 2 x 4096, 16 q heads
-// on one kv head, d 64 (64 CTAs of 16 .. 512 steps) 745 -> 245 (eight a tile).
+// a row -> shared: that forward 240 -> 135 us (two CTAs a row); dkv of causal 2 x 4096, 16 q heads
+// on one kv head, d 64 (64 CTAs of 16 .. 512 steps) 745 -> 244 (eight a tile).
 #pragma once
 
 #include <mutex>
@@ -70,9 +70,10 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
 
 // CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (prologue, epilogue; one more
 // for the addition across the cluster).  While everything is resident the longest row sets the time; beyond that the
-// total work over the slots, and half a row for the uneven end.  Rows below 16 steps stay whole: little
-// is left to gain there (causal 2 x 1024, 8 heads, 64 CTAs of 2 .. 8 steps: 24.7 us, 20.9 with two CTAs a row),
-// and short sequences give the same bits whatever else is in the launch.
+// total work over the slots, and half a row for the uneven end.  Rows below 16 steps stay whole although the
+// rule would share some (causal 2 x 1024, 8 heads, 64 CTAs of 2 .. 8 steps: 24.7 us, 20.9 with two CTAs a row),
+// so that the bits of short rows do not depend on the batch and the heads beside them: in the forward those
+// of fewer than 2048 keys, in dkv kv tiles of fewer than 16 (q tile, q head of the group) steps.
 inline int split_for(const RowWork& w, const ClusterCapacity& cap) {
   constexpr float kFixed = 3.f, kMerge = 1.f, kFewest = 16.f;
   if (w.longest < kFewest) return 1;
