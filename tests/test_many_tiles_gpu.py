@@ -1,0 +1,66 @@
+"""Grids that hold several tiles for every SM.
+
+The CTAs of the kernels take over one tile after the other (operand rings, barrier phases and TMEM carry on
+from tile to tile), so a call that fills the chip several times takes other paths than the small calls the
+oracle is compared with.  Every head of such a call must get the bits of a call on that head alone.
+"""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+from tokamax_b200 import splash_attention_kernel as splash
+from tokamax_b200 import splash_attention_mask as mask_lib
+
+pytestmark = pytest.mark.gpu
+DEV = torch.device("cuda:0")
+
+
+def _run(kernel, q, k, v, do, seg, scale):
+  q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
+  out, res = kernel(q, k, v, seg, logits_scale=scale)
+  dq, dk, dv = torch.autograd.grad(out, (q, k, v), do)
+  return {"out": out.detach(), "lse": res["logsumexp"], "dq": dq, "dk": dk, "dv": dv}
+
+
+def _mask(kind, s):
+  if kind == "window":
+    return mask_lib.LocalMask((s, s), (300, 0), 0)
+  if kind == "table":  # rows of tiles without a live block among them
+    m = np.tril(np.ones((s, s), np.bool_))
+    m[512:768] = False
+    m[:, 640:896] = False
+    return mask_lib.NumpyMask(m)
+  return mask_lib.CausalMask((s, s))
+
+
+# 13 tiles of 22 (batch, kv head) pairs: 286 CTAs and more for at most 148 SMs; an odd number of steps in rings of
+# two, three and four slots
+@pytest.mark.parametrize("d_qk,d_v", [(192, 128), (256, 256), (160, 160), (64, 192), (256, 72), (136, 200)])
+@pytest.mark.parametrize("kind,soft_cap,segments", [("causal", None, False), ("window", 20.0, True), ("table", None, False)])
+def test_heads_above_128_of_a_large_call_are_those_of_small_calls(d_qk, d_v, kind, soft_cap, segments):
+  b, hkv, group, s = 2, 11, 2, 1664
+  g = torch.Generator(device=DEV).manual_seed(d_qk + 3 * d_v)
+  mk = lambda h, d: torch.randn(b, h, s, d, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v, do = mk(hkv * group, d_qk), mk(hkv, d_qk), mk(hkv, d_v), mk(hkv * group, d_v)
+  seg = None
+  if segments:
+    ids = torch.zeros((b, s), dtype=torch.int32, device=DEV)
+    ids[0, 700:], ids[1, 130:], ids[1, 1500:] = 1, 1, 2
+    seg = splash.SegmentIds(q=ids, kv=ids)
+  config = splash.SplashConfig.get_default()
+  if soft_cap:
+    config = splash.dataclasses.replace(config, attn_logits_soft_cap=soft_cap)
+  kernel = splash.make_splash_mha(_mask(kind, s), config=config, q_seq_shards=1, save_residuals=True)
+  scale = 1 / math.sqrt(d_qk)
+  whole = _run(kernel, q, k, v, do, seg, scale)
+  kernel.check_errors()
+  for h in range(0, hkv, 5):
+    heads = slice(h * group, (h + 1) * group)
+    part = _run(kernel, q[:, heads].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous(),
+                do[:, heads].contiguous(), seg, scale)
+    kernel.check_errors()
+    for name in part:
+      mine = whole[name][:, heads if name in ("out", "lse", "dq") else slice(h, h + 1)]
+      assert torch.equal(mine, part[name]), (name, h)

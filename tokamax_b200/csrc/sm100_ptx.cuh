@@ -139,6 +139,33 @@ __device__ __forceinline__ uint32_t cluster_ld_u32(uint32_t addr) {
 }
 
 // ----------------------------------------------------------------------------------------
+// cluster launch control: a running CTA takes over the next one that has not been launched yet
+// ----------------------------------------------------------------------------------------
+// Asks for it; the answer (16 bytes, 16-byte aligned shared memory) completes 16 bytes on `bar`.  No further
+// request may follow one that was refused.
+__device__ __forceinline__ void clc_request(void* answer, uint64_t* bar) {
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+          smem_u32(answer)),
+      "r"(smem_u32(bar))
+      : "memory");
+}
+// blockIdx.x of the CTA whose work this one takes over, or -1: none is left.
+__device__ __forceinline__ int clc_block(const void* answer) {
+  int block;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 r;\n\t"
+      "ld.shared.b128 r, [%1];\n\t"
+      "mov.s32 %0, -1;\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n\t}\n"
+      : "=r"(block)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return block;
+}
+
+// ----------------------------------------------------------------------------------------
 // TMA (tiled, no multicast)
 // ----------------------------------------------------------------------------------------
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {

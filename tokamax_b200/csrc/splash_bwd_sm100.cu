@@ -1171,7 +1171,7 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   const int64_t Hkv = a.k.size[1], Skv = a.k.size[2];
   // head dims below 128 are read in place (zero-extended by the TMA boxes), see splash_fwd
   const int64_t Dv = a.v.size[3];
-  // head dims above 128 (up to 256): three passes over 128-column panels, splash_bwd_wide_sm100.cu
+  // head dims above 128 (up to 256): passes of their own, splash_bwd_wide_sm100.cu
   if (D > 2 * kHeadDim || Dv > 2 * kHeadDim) return SPLASH_ERR_UNSUPPORTED;
   const bool wide = D > kHeadDim || Dv > kHeadDim;
   if (D % 8 != 0 || Dv % 8 != 0) return SPLASH_ERR_INVALID_ARGUMENT;
@@ -1206,8 +1206,9 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   if (!(a.scale > 0.f) || !(a.scale < 1.0e30f)) return SPLASH_ERR_INVALID_ARGUMENT;
 
   CUtensorMap tm_q, tm_do, tm_k, tm_v;
-  if ((st = make_tile_tensor_map(&tm_q, a.q, kTile)) || (st = make_tile_tensor_map(&tm_do, a.d_o, kTile)) ||
-      (st = make_tile_tensor_map(&tm_k, a.k, kTile)) || (st = make_tile_tensor_map(&tm_v, a.v, kTile)))
+  const int box_rows = wide ? kSub : kTile;
+  if ((st = make_tile_tensor_map(&tm_q, a.q, box_rows)) || (st = make_tile_tensor_map(&tm_do, a.d_o, box_rows)) ||
+      (st = make_tile_tensor_map(&tm_k, a.k, box_rows)) || (st = make_tile_tensor_map(&tm_v, a.v, box_rows)))
     return st;
 
   const uint32_t mask = a.launch_mask == 0 ? 7u : a.launch_mask;
