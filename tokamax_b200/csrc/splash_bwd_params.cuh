@@ -70,49 +70,9 @@ __device__ __forceinline__ void store_row_half(__nv_bfloat16* dst, const uint32_
   }
 }
 
-// 32 columns of the rows of a warp's 32 TMEM lanes (lane = row, `v` its columns), starting at column `col0` of a
-// tensor of `cols` columns.  A lane storing its own row would touch 32 lines with every instruction; four lanes
-// exchange their 16-byte chunks first, so that one instruction writes 64 contiguous bytes of eight rows.
-// `row0`: the warp's first row, at column 0.
-__device__ __forceinline__ void store_rows32(__nv_bfloat16* row0, int64_t row_stride, const uint32_t (&v)[32], float mul,
-                                             int col0, int cols) {
-  const int lane = threadIdx.x & 31;
-  uint4 c[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j)
-    c[j] = make_uint4(pack_bf16(__uint_as_float(v[8 * j + 0]) * mul, __uint_as_float(v[8 * j + 1]) * mul),
-                      pack_bf16(__uint_as_float(v[8 * j + 2]) * mul, __uint_as_float(v[8 * j + 3]) * mul),
-                      pack_bf16(__uint_as_float(v[8 * j + 4]) * mul, __uint_as_float(v[8 * j + 5]) * mul),
-                      pack_bf16(__uint_as_float(v[8 * j + 6]) * mul, __uint_as_float(v[8 * j + 7]) * mul));
-  // 4 x 4 transpose over the lanes 4 a .. 4 a + 3: chunk b of row 4 a + i ends in lane 4 a + b as c[i]
-  auto swap = [&](uint4& lo, uint4& hi, int bit) {
-    const bool up = (lane & bit) != 0;
-    uint4 x = up ? lo : hi;
-    x.x = __shfl_xor_sync(0xffffffffu, x.x, bit);
-    x.y = __shfl_xor_sync(0xffffffffu, x.y, bit);
-    x.z = __shfl_xor_sync(0xffffffffu, x.z, bit);
-    x.w = __shfl_xor_sync(0xffffffffu, x.w, bit);
-    if (up)
-      lo = x;
-    else
-      hi = x;
-  };
-  swap(c[0], c[1], 1);
-  swap(c[2], c[3], 1);
-  swap(c[0], c[2], 2);
-  swap(c[1], c[3], 2);
-  const int col = col0 + (lane & 3) * 8;
-  if (col < cols) {
-    __nv_bfloat16* dst = row0 + (int64_t)(lane & ~3) * row_stride + col;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(dst + i * row_stride) = c[i];
-  }
-}
-
 // Backward for head dims above 128 (defined in splash_bwd_wide_sm100.cu).  `p` carries the fields
 // that do not depend on the pass; the launcher fills outputs and schedules per pass.
 // The tensor maps have boxes of kSub rows.
-constexpr int kSub = 64;
 int launch_bwd_wide(const CUtensorMap& tm_q, const CUtensorMap& tm_do, const CUtensorMap& tm_k,
                     const CUtensorMap& tm_v, const BwdParams& base, const SplashBwdArgs& a, bool soft_cap,
                     uint32_t launch_mask, cudaStream_t stream);

@@ -47,15 +47,14 @@ namespace sb {
 
 enum WidePass { kWideDq = 0, kWideDkv = 1, kWideDk = 2, kWideDv = 3 };
 
-constexpr int kSubHalfBytes = kSub * 128;    // 64 columns of a streamed tile (kSub rows): 8 KiB
-constexpr int kWideThreads = 576;            // 16 compute warps, TMA warp, MMA warp
+constexpr int kWideThreads = 576;  // 16 compute warps, TMA warp, MMA warp
 constexpr int kWideTmaWarp = 16;
 constexpr int kWideMmaWarp = 17;
 constexpr int kWideMaxSlots = 4;
-constexpr int kWideTileBytes = 7 * kTileBytes;                       // operand tiles
-constexpr int kWideStatsBytes = kWideMaxSlots * 2 * kSub * 4;        // a slot: -lse log2(e), -di of its query rows
+constexpr int kWideTileBytes = 7 * kTileBytes;  // operand tiles
+constexpr int kWideStatsBytes = kWideMaxSlots * 2 * kSub * 4;  // a slot: -lse log2(e), -di of its query rows
 constexpr int kWideSmemBytes = kWideTileBytes + kWideStatsBytes + 512;
-constexpr int kWideBothColumns = 512 - 3 * kSub;                     // dk and dv columns that one pass can hold
+constexpr int kWideBothColumns = 512 - 3 * kSub;  // dk and dv columns that one pass can hold
 
 struct WideParams {
   BwdParams b;
@@ -85,23 +84,6 @@ struct WideBwdBarriers {
   uint32_t early_exit;
 };
 static_assert(sizeof(WideBwdBarriers) <= 512, "barrier block");
-
-// A position in a ring: slot and the parity of its use.
-struct RingPos {
-  uint32_t slot, phase;
-  __device__ __forceinline__ void advance(uint32_t by, uint32_t slots) {  // by <= slots
-    slot += by;
-    if (slot >= slots) {
-      slot -= slots;
-      phase ^= 1u;
-    }
-  }
-  __device__ __forceinline__ void skip(uint32_t by, uint32_t slots) {  // any number
-    slot += by;
-    phase ^= (slot / slots) & 1u;
-    slot %= slots;
-  }
-};
 
 // kOneS (dq, dk): one S buffer, for head dims whose output and stationary operand leave no columns for a second.
 template <int kPass, bool kSoftCap, bool kOneS>

@@ -15,6 +15,8 @@ constexpr int kTile = 128;          // q and kv tile edge the MMAs work on
 constexpr int kHeadDim = 128;       // head dimension of the bf16 kernels
 constexpr int kTileBytes = kTile * kHeadDim * 2;   // one bf16 operand tile: 32 KiB
 constexpr int kHalfBytes = kTileBytes / 2;         // one 64-column (128-byte) swizzle half
+constexpr int kSub = 64;                           // rows of a streamed tile of the kernels for head dims above 128
+constexpr int kSubHalfBytes = kSub * 128;          // 64 of its columns: 8 KiB
 constexpr float kMaskedLogit = -1.0e30f;           // raw logit given to masked positions
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
@@ -77,6 +79,62 @@ inline int chunk_groups_for(int64_t bytes_per_group, int64_t n_groups, int64_t a
   if (g > n_groups) g = n_groups;
   return (int)g;
 }
+
+// 32 columns of the rows of a warp's 32 TMEM lanes (lane = row, `v` its columns), starting at column `col0` of a
+// tensor of `cols` columns.  A lane storing its own row would touch 32 lines with every instruction; four lanes
+// exchange their 16-byte chunks first, so that one instruction writes 64 contiguous bytes of eight rows.
+// `row0`: the warp's first row, at column 0.
+__device__ __forceinline__ void store_rows32(__nv_bfloat16* row0, int64_t row_stride, const uint32_t (&v)[32], float mul,
+                                             int col0, int cols) {
+  const int lane = threadIdx.x & 31;
+  uint4 c[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    c[j] = make_uint4(pack_bf16(__uint_as_float(v[8 * j + 0]) * mul, __uint_as_float(v[8 * j + 1]) * mul),
+                      pack_bf16(__uint_as_float(v[8 * j + 2]) * mul, __uint_as_float(v[8 * j + 3]) * mul),
+                      pack_bf16(__uint_as_float(v[8 * j + 4]) * mul, __uint_as_float(v[8 * j + 5]) * mul),
+                      pack_bf16(__uint_as_float(v[8 * j + 6]) * mul, __uint_as_float(v[8 * j + 7]) * mul));
+  // 4 x 4 transpose over the lanes 4 a .. 4 a + 3: chunk b of row 4 a + i ends in lane 4 a + b as c[i]
+  auto swap = [&](uint4& lo, uint4& hi, int bit) {
+    const bool up = (lane & bit) != 0;
+    uint4 x = up ? lo : hi;
+    x.x = __shfl_xor_sync(0xffffffffu, x.x, bit);
+    x.y = __shfl_xor_sync(0xffffffffu, x.y, bit);
+    x.z = __shfl_xor_sync(0xffffffffu, x.z, bit);
+    x.w = __shfl_xor_sync(0xffffffffu, x.w, bit);
+    if (up)
+      lo = x;
+    else
+      hi = x;
+  };
+  swap(c[0], c[1], 1);
+  swap(c[2], c[3], 1);
+  swap(c[0], c[2], 2);
+  swap(c[1], c[3], 2);
+  const int col = col0 + (lane & 3) * 8;
+  if (col < cols) {
+    __nv_bfloat16* dst = row0 + (int64_t)(lane & ~3) * row_stride + col;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(dst + i * row_stride) = c[i];
+  }
+}
+
+// A position in a ring: slot and the parity of its use.
+struct RingPos {
+  uint32_t slot, phase;
+  __device__ __forceinline__ void advance(uint32_t by, uint32_t slots) {  // by <= slots
+    slot += by;
+    if (slot >= slots) {
+      slot -= slots;
+      phase ^= 1u;
+    }
+  }
+  __device__ __forceinline__ void skip(uint32_t by, uint32_t slots) {  // any number
+    slot += by;
+    phase ^= (slot / slots) & 1u;
+    slot %= slots;
+  }
+};
 
 // Address of row `s` of local head `h` in the rank that owns it (see SplashPeerOutput).
 __device__ __forceinline__ __nv_bfloat16* peer_row(const SplashPeerOutput& po, int batch, int h, int s) {

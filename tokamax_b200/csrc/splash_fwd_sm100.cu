@@ -845,8 +845,8 @@ static int launch_fwd_common(const SplashFwdArgs& a, const SplashShards& shards,
   // Head dims: the MMA tile is 128 wide.  bf16 tensors with fewer columns (a multiple of 8, so rows
   // stay 16-byte aligned) are read in place — the TMA boxes reach past the row's end and the part
   // outside the tensor arrives as zeros, which change neither q k^T nor p v — and only the real
-  // columns of the output are stored.  Head dims above 128 (up to 256) go to the forward that works
-  // on two 128-column panels (splash_fwd_wide_sm100.cu); e4m3 takes 128 only.
+  // columns of the output are stored.  Head dims above 128 (up to 256) go to a forward of their
+  // own (splash_fwd_wide_sm100.cu); e4m3 takes 128 only.
   const int64_t Dv = a.v.size[3];
   constexpr int64_t kMaxWideDim = 2 * kHeadDim;
   if (D > kMaxWideDim || Dv > kMaxWideDim || (fp8 && (D != kHeadDim || Dv != kHeadDim))) return SPLASH_ERR_UNSUPPORTED;
@@ -870,8 +870,9 @@ static int launch_fwd_common(const SplashFwdArgs& a, const SplashShards& shards,
   if (!(a.scale > 0.f) || !(a.scale < 1.0e30f)) return SPLASH_ERR_INVALID_ARGUMENT;
 
   CUtensorMap tm_q, tm_k, tm_v;
-  if ((st = make_tile_tensor_map(&tm_q, a.q, kTile)) || (st = make_tile_tensor_map(&tm_k, a.k, kTile)) ||
-      (st = make_tile_tensor_map(&tm_v, a.v, kTile)))
+  const int box_rows = wide ? kSub : kTile;
+  if ((st = make_tile_tensor_map(&tm_q, a.q, box_rows)) || (st = make_tile_tensor_map(&tm_k, a.k, box_rows)) ||
+      (st = make_tile_tensor_map(&tm_v, a.v, box_rows)))
     return st;
 
   FwdParams p;
