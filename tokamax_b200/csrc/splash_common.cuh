@@ -80,21 +80,18 @@ inline int chunk_groups_for(int64_t bytes_per_group, int64_t n_groups, int64_t a
   return (int)g;
 }
 
-// 32 columns of the rows of a warp's 32 TMEM lanes (lane = row, `v` its columns), starting at column `col0` of a
-// tensor of `cols` columns.  A lane storing its own row would touch 32 lines with every instruction; four lanes
-// exchange their 16-byte chunks first, so that one instruction writes 64 contiguous bytes of eight rows.
-// `row0`: the warp's first row, at column 0.
-__device__ __forceinline__ void store_rows32(__nv_bfloat16* row0, int64_t row_stride, const uint32_t (&v)[32], float mul,
-                                             int col0, int cols) {
+// 32 columns of the rows of a warp's 32 TMEM lanes (lane = row, `v` its columns), times `mul`, as bf16.  A lane storing
+// its own row would touch 32 lines with every instruction (a CTA's 128 x 128 outputs: 4000 cycles); four lanes
+// exchange their 16-byte chunks first, so that one instruction writes 64 contiguous bytes of eight rows.  The lane
+// gets columns 8 (lane mod 4) .. + 7 of rows 4 (lane / 4) + i as c[i].
+__device__ __forceinline__ void exchange_rows32(const uint32_t (&v)[32], float mul, uint4 (&c)[4]) {
   const int lane = threadIdx.x & 31;
-  uint4 c[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j)
     c[j] = make_uint4(pack_bf16(__uint_as_float(v[8 * j + 0]) * mul, __uint_as_float(v[8 * j + 1]) * mul),
                       pack_bf16(__uint_as_float(v[8 * j + 2]) * mul, __uint_as_float(v[8 * j + 3]) * mul),
                       pack_bf16(__uint_as_float(v[8 * j + 4]) * mul, __uint_as_float(v[8 * j + 5]) * mul),
                       pack_bf16(__uint_as_float(v[8 * j + 6]) * mul, __uint_as_float(v[8 * j + 7]) * mul));
-  // 4 x 4 transpose over the lanes 4 a .. 4 a + 3: chunk b of row 4 a + i ends in lane 4 a + b as c[i]
   auto swap = [&](uint4& lo, uint4& hi, int bit) {
     const bool up = (lane & bit) != 0;
     uint4 x = up ? lo : hi;
@@ -111,6 +108,13 @@ __device__ __forceinline__ void store_rows32(__nv_bfloat16* row0, int64_t row_st
   swap(c[2], c[3], 1);
   swap(c[0], c[2], 2);
   swap(c[1], c[3], 2);
+}
+// The same, stored from column `col0` on of a tensor of `cols` columns.  `row0`: the warp's first row, at column 0.
+__device__ __forceinline__ void store_rows32(__nv_bfloat16* row0, int64_t row_stride, const uint32_t (&v)[32], float mul,
+                                             int col0, int cols) {
+  const int lane = threadIdx.x & 31;
+  uint4 c[4];
+  exchange_rows32(v, mul, c);
   const int col = col0 + (lane & 3) * 8;
   if (col < cols) {
     __nv_bfloat16* dst = row0 + (int64_t)(lane & ~3) * row_stride + col;
@@ -143,6 +147,23 @@ __device__ __forceinline__ __nv_bfloat16* peer_row(const SplashPeerOutput& po, i
   uint8_t* base = reinterpret_cast<uint8_t*>(po.ptrs[peer]) + po.base_bytes;
   return reinterpret_cast<__nv_bfloat16*>(base) + (int64_t)batch * po.stride_b + (int64_t)(po.head0 + h) * po.stride_h +
          local * po.stride_s;
+}
+// Rows seq0 .. seq0 + 31 of head `h`, 32 columns of them (see exchange_rows32), into `out` and into the ranks that own
+// them.
+__device__ __forceinline__ void store_rows32_peer(__nv_bfloat16* row0, int64_t row_stride, const SplashPeerOutput& po, int batch,
+                                                  int h, int seq0, const uint32_t (&v)[32], float mul, int col0, int cols) {
+  const int lane = threadIdx.x & 31;
+  uint4 c[4];
+  exchange_rows32(v, mul, c);
+  const int col = col0 + (lane & 3) * 8;
+  if (col < cols) {
+    __nv_bfloat16* dst = row0 + (int64_t)(lane & ~3) * row_stride + col;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      *reinterpret_cast<uint4*>(dst + i * row_stride) = c[i];
+      if (po.ptrs) *reinterpret_cast<uint4*>(peer_row(po, batch, h, seq0 + (lane & ~3) + i) + col) = c[i];
+    }
+  }
 }
 inline int check_peer_output(const SplashPeerOutput& po, int64_t rows, int64_t head_dim) {
   if (po.ptrs == nullptr) return SPLASH_OK;

@@ -13,6 +13,12 @@
 // The two tiles ping-pong: while the softmax of tile 0 runs on the SIMT lanes, the tensor core
 // computes QK^T of tile 1 and PV of the previous step.
 //
+// A CTA stays for several rows of the schedule: the producer takes over CTAs that have not been launched yet (cluster
+// launch control), posts their rows and goes on loading; q k^T of the next row runs while the softmax warps
+// store this one's outputs, 64 bytes of eight rows an instruction.  A CTA a row, each lane storing its own row, spent
+// 10000 cycles between the loops of two rows.  Window 1024, 2 x 6016, 64 / 8 heads, d 64 (10 steps a row): 478 -> 451 us;
+// causal 4 x 8192, 32 / 8 heads (33 steps on average) 2.20 -> 2.12 ms; 32768 e4m3 (129 steps) no difference.
+//
 // Online softmax keeps a possibly stale running maximum: O and l are rescaled only when the
 // new row maximum exceeds the one in use by more than 2^8, which keeps the TMEM round trip of
 // O off the common path.  logsumexp is exact regardless (it is formed from the maximum in use
@@ -39,13 +45,19 @@
 namespace sb {
 
 struct FwdBarriers {
+  uint64_t answer[2];  // cluster launch control: what the request for the next row returned
+  int4 work[2];        // rows in the order they are worked on: schedule row (-1: none left), group, first and last entry
+  uint64_t answer_full;
+  uint64_t work_full[2], work_empty[2];
   uint64_t q_full[2];
+  uint64_t q_free;       // every q k^T of a row has completed
   uint64_t kv_full[kFwdStages];
   uint64_t kv_empty[kFwdStages];
   uint64_t s_full[2];
   uint64_t p_half[2];    // the first 64 key columns of P are in TMEM (the first half of the p v MMAs may go)
   uint64_t p_full[2];
   uint64_t o_done[2];
+  uint64_t o_free[2];    // a tile's O has been read
   uint64_t vc_full[2];   // e4m3 with f16 P: a V tile has been converted to f16
   uint64_t vc_empty[2];  //                  the p v MMAs that read it have completed
   uint32_t tmem_base;
@@ -132,18 +144,13 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const unsigned rank = kSplit ? cluster_rank() : 0u;
-  const CtaWork work = cta_work_at(kSplit ? blockIdx.x / p.n_split : blockIdx.x, p.row_order, p.n_rows, p.n_groups,
-                                   p.chunk_groups, true);
-  const int row = work.row;
-  const int head = work.group % p.q_heads;
-  const int batch = work.group / p.q_heads;
-  const int kv_head = head / (p.q_heads / p.kv_heads);
-  const int ebeg = p.row_ptr[row];
-  const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + row] : p.row_ptr[row + 1];
-  const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
-  const PartWalk<kSplit> walk(entries, ebeg, eend, p.n_split);  // the entries of this CTA
-  const int efirst = walk.first(walk.offset((int)rank));
-  const int qt0 = row * 2;
+  // schedule row, group, first and last entry of a block of the grid
+  auto row_of = [&](unsigned block) {
+    const CtaWork work = cta_work_at(block, p.row_order, p.n_rows, p.n_groups, p.chunk_groups, true);
+    const int ebeg = p.row_ptr[work.row];
+    const int eend = p.row_end ? p.row_end[(int64_t)(work.group / p.q_heads) * p.n_rows + work.row] : p.row_ptr[work.row + 1];
+    return make_int4(work.row, work.group, ebeg, eend < ebeg ? ebeg : eend);
+  };
 
   if (threadIdx.x == 0) {
     bars->early_exit = *reinterpret_cast<volatile uint32_t*>(p.err);
@@ -154,6 +161,9 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       mbar_init(&bars->p_half[i], 4);  // one arrival per softmax warp
       mbar_init(&bars->p_full[i], 4);
       mbar_init(&bars->o_done[i], 1);
+      mbar_init(&bars->o_free[i], 4);
+      mbar_init(&bars->work_full[i], 1);
+      mbar_init(&bars->work_empty[i], kP16 ? 11 : 9);  // softmax warps, the issuing and the converting ones
       mbar_init(&bars->vc_full[i], 2);   // one arrival per converting warp
       mbar_init(&bars->vc_empty[i], 1);
     }
@@ -163,6 +173,8 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       // odd slots and, in the f16-P variant, are released by the two warps that convert them
       mbar_init(&bars->kv_empty[s], (kP16 && (s & 1)) ? 2 : 1);
     }
+    mbar_init(&bars->answer_full, 1);
+    mbar_init(&bars->q_free, 1);
     mbar_fence_init();
   }
   __syncthreads();
@@ -184,6 +196,27 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const uint32_t tmem = bars->tmem_base;
   AbortCtx ab{&bars->abort_flag, p.err};
 
+  // The rows this CTA works on, in order: its own, then those it takes over (the producer posts both).  A CTA of a
+  // cluster has the cluster's row and no other.
+  RingPos work_pos{0, 0};
+  bool first_work = true;
+  auto next_work = [&](int4& w, bool warp_wide) {  // by a whole warp, or by a thread for its warp
+    if constexpr (kSplit) {
+      if (!first_work) return false;
+      first_work = false;
+      w = row_of(blockIdx.x / p.n_split);
+      return true;
+    }
+    bool ok = mbar_wait(&bars->work_full[work_pos.slot], work_pos.phase, ab, 0x700u + work_pos.slot);
+    if (warp_wide) ok = __all_sync(0xffffffffu, ok);
+    if (!ok) return false;
+    w = bars->work[work_pos.slot];
+    if (warp_wide) __syncwarp();
+    if (!warp_wide || lane == 0) mbar_arrive(&bars->work_empty[work_pos.slot]);
+    work_pos.advance(1, 2);
+    return w.x >= 0;
+  };
+
   if (warp >= 8) {
    setmaxnreg_dec<kIssueRegs>();
    if (warp >= 10) {
@@ -195,11 +228,17 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       static_assert(kFwdStages % 2 == 0, "V tiles must keep to the odd ring slots");
       const int t = (warp - 10) * 32 + lane;
       uint32_t n = 0;
-      for (int e = efirst; e < eend; e = walk.next(e), ++n) {
+      bool ok = true;
+      int4 w;
+      while (ok && next_work(w, true)) {
+       const int eend = w.w;
+       const PartWalk<kSplit> walk(p.entries + (int64_t)(w.y / p.q_heads) * p.entries_per_batch, w.z, eend, p.n_split);
+       for (int e = walk.first(walk.offset((int)rank)); e < eend; e = walk.next(e), ++n) {
         const uint32_t it = 2 * n + 1, s = it % kFwdStages, j = n & 1u;
-        bool ok = mbar_wait(&bars->kv_full[s], (it / kFwdStages) & 1u, ab, 0x600u + s);
+        ok = mbar_wait(&bars->kv_full[s], (it / kFwdStages) & 1u, ab, 0x600u + s);
         if (ok) ok = mbar_wait(&bars->vc_empty[j], ((n >> 1) & 1u) ^ 1u, ab, 0x610u + j);
-        if (!__all_sync(0xffffffffu, ok)) break;
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
         const uint8_t* raw = kv_smem + s * kTB;
         uint8_t* dst = vc_smem + j * kTileBytes;
 #pragma unroll 4
@@ -222,6 +261,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           mbar_arrive(&bars->vc_full[j]);
           mbar_arrive(&bars->kv_empty[s]);
         }
+       }
       }
     }
    } else if (warp == 8) {
@@ -230,31 +270,66 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       tma_prefetch_desc(&tm_q);
       tma_prefetch_desc(&tm_k);
       tma_prefetch_desc(&tm_v);
-      for (int i = 0; i < 2; ++i) {
-        if (qt0 + i < p.n_q_tiles) {
-          uint8_t* dst = q_smem + i * kTB;
-          const bool two = !kFp8 && p.d_qk > 64;  // bf16 tiles are two 64-column halves
-          mbar_arrive_expect_tx(&bars->q_full[i], (kFp8 || two) ? kTB : kHalfBytes);
-          tma_load_4d(dst, &tm_q, &bars->q_full[i], 0, (qt0 + i) * kTile, head, batch);
-          if (two) tma_load_4d(dst + kHalfBytes, &tm_q, &bars->q_full[i], 64, (qt0 + i) * kTile, head, batch);
-        }
-      }
       uint32_t it = 0;
+      uint32_t stepped = 0;  // rows with steps so far
+      uint32_t asked = 0;
       bool ok = true;
-      for (int e = efirst; e < eend && ok; e = walk.next(e)) {
-        const int col = entries[e].x;
-        for (int kv = 0; kv < 2 && ok; ++kv, ++it) {
-          const uint32_t s = it % kFwdStages;
-          const uint32_t ph = (it / kFwdStages) & 1u;
-          ok = mbar_wait(&bars->kv_empty[s], ph ^ 1u, ab, 0x100u + s);
+      int block = (int)(kSplit ? blockIdx.x / p.n_split : blockIdx.x);
+      for (;;) {
+        int4 w = make_int4(-1, 0, 0, 0);
+        if (block >= 0) w = row_of((unsigned)block);
+        if constexpr (!kSplit) {
+          ok = mbar_wait(&bars->work_empty[work_pos.slot], work_pos.phase ^ 1u, ab, 0x710u + work_pos.slot);
           if (!ok) break;
-          uint8_t* dst = kv_smem + s * kTB;
-          const CUtensorMap* tm = kv == 0 ? &tm_k : &tm_v;
-          const bool two = !kFp8 && (kv == 0 ? p.d_qk : p.d_v) > 64;
-          mbar_arrive_expect_tx(&bars->kv_full[s], (kFp8 || two) ? kTB : kHalfBytes);
-          tma_load_4d(dst, tm, &bars->kv_full[s], 0, col * kTile, kv_head, batch);
-          if (two) tma_load_4d(dst + kHalfBytes, tm, &bars->kv_full[s], 64, col * kTile, kv_head, batch);
+          bars->work[work_pos.slot] = w;
+          mbar_arrive(&bars->work_full[work_pos.slot]);
+          work_pos.advance(1, 2);
         }
+        if (block < 0) break;
+        const int qt0 = 2 * w.x, head = w.y % p.q_heads, batch = w.y / p.q_heads, eend = w.w;
+        const int kv_head = head / (p.q_heads / p.kv_heads);
+        const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
+        const PartWalk<kSplit> walk(entries, w.z, eend, p.n_split);  // the entries of this CTA
+        const int efirst = walk.first(walk.offset((int)rank));
+        if (efirst < eend) {
+          if (stepped > 0) ok = mbar_wait(&bars->q_free, (stepped - 1) & 1u, ab, 0x110u);
+          if (!ok) break;
+          for (int i = 0; i < 2; ++i) {
+            if (qt0 + i < p.n_q_tiles) {
+              uint8_t* dst = q_smem + i * kTB;
+              const bool two = !kFp8 && p.d_qk > 64;  // bf16 tiles are two 64-column halves
+              mbar_arrive_expect_tx(&bars->q_full[i], (kFp8 || two) ? kTB : kHalfBytes);
+              tma_load_4d(dst, &tm_q, &bars->q_full[i], 0, (qt0 + i) * kTile, head, batch);
+              if (two) tma_load_4d(dst + kHalfBytes, &tm_q, &bars->q_full[i], 64, (qt0 + i) * kTile, head, batch);
+            }
+          }
+          ++stepped;
+        }
+        for (int e = efirst; e < eend && ok; e = walk.next(e)) {
+          const int col = entries[e].x;
+          for (int kv = 0; kv < 2 && ok; ++kv, ++it) {
+            const uint32_t s = it % kFwdStages;
+            const uint32_t ph = (it / kFwdStages) & 1u;
+            ok = mbar_wait(&bars->kv_empty[s], ph ^ 1u, ab, 0x100u + s);
+            if (!ok) break;
+            uint8_t* dst = kv_smem + s * kTB;
+            const CUtensorMap* tm = kv == 0 ? &tm_k : &tm_v;
+            const bool two = !kFp8 && (kv == 0 ? p.d_qk : p.d_v) > 64;
+            mbar_arrive_expect_tx(&bars->kv_full[s], (kFp8 || two) ? kTB : kHalfBytes);
+            tma_load_4d(dst, tm, &bars->kv_full[s], 0, col * kTile, kv_head, batch);
+            if (two) tma_load_4d(dst + kHalfBytes, tm, &bars->kv_full[s], 64, col * kTile, kv_head, batch);
+          }
+        }
+        if (!ok || kSplit) break;
+        // The next row.  Asked for when all of this one is on its way, two steps ahead of the MMAs, and no earlier: what a
+        // CTA has taken over, no other can take that is done before it.
+        mbar_arrive_expect_tx(&bars->answer_full, 16);
+        clc_request(bars->answer, &bars->answer_full);
+        ok = mbar_wait(&bars->answer_full, asked & 1u, ab, 0x120u);
+        if (!ok) break;
+        ++asked;
+        block = clc_block(bars->answer);
+        fence_proxy_async_smem();  // read before the next answer overwrites it
       }
     }
   } else if (warp == 9) {
@@ -273,10 +348,6 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const uint32_t q_addr = smem_u32(q_smem);
       const uint32_t vc_addr = smem_u32(vc_smem);
       const uint32_t kv_addr = smem_u32(kv_smem);
-      bool ok = true;
-      for (int i = 0; i < 2 && ok; ++i)
-        if (qt0 + i < p.n_q_tiles) ok = mbar_wait(&bars->q_full[i], 0, ab, 0x200u + i);
-
       // S_i = Q_i K^T : both operands K-major.  bf16: eight K=16 slices across two swizzle
       // halves; e4m3: four K=32 slices inside the single 128-byte-wide tile.
       auto issue_qk = [&](int i, uint32_t slot) {
@@ -326,39 +397,55 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
       };
 
-      const int n_ent = eend - ebeg;
-      int e = efirst;
       uint32_t pcnt[2] = {0, 0};
-      bool started[2] = {false, false};
-      if (efirst < eend && ok) {
+      uint32_t qcnt[2] = {0, 0};   // Q tiles so far
+      uint32_t it0 = 0;            // ring slots of the rows before this one
+      uint32_t stepped = 0;        // rows with steps so far
+      bool ok = true;
+      int4 w;
+      while (ok && next_work(w, false)) {
+        const int4* entries = p.entries + (int64_t)(w.y / p.q_heads) * p.entries_per_batch;
+        const int ebeg = w.z, eend = w.w;
+        const PartWalk<kSplit> walk(entries, ebeg, eend, p.n_split);
+        const int efirst = walk.first(walk.offset((int)rank));
+        if (efirst >= eend) continue;
+        const int n_ent = eend - ebeg;
+        int e = efirst;
+        bool started[2] = {false, false};
         const int4 e0 = entries[efirst];
-        ok = mbar_wait(&bars->kv_full[0], 0, ab, 0x300u);
-        if (ok) {
-          mma_issue_fence();
-          for (int i = 0; i < 2; ++i)
-            if ((e0.y >> (2 * i)) & 3) issue_qk(i, 0);
-          tc_commit(&bars->kv_empty[0]);
-        }
+        for (int i = 0; i < 2 && ok; ++i)
+          if (2 * w.x + i < p.n_q_tiles) ok = mbar_wait(&bars->q_full[i], qcnt[i]++ & 1u, ab, 0x200u + i);
+        if (ok) ok = mbar_wait(&bars->kv_full[it0 % kFwdStages], (it0 / kFwdStages) & 1u, ab, 0x300u);
+        if (!ok) break;
+        mma_issue_fence();
+        for (int i = 0; i < 2; ++i)
+          if ((e0.y >> (2 * i)) & 3) issue_qk(i, it0 % kFwdStages);
+        tc_commit(&bars->kv_empty[it0 % kFwdStages]);
         int4 nxt = e0;
-        for (int n = 0; (kSplit ? e < eend : n < n_ent) && ok; ++n) {
+        uint32_t n = 0;
+        for (bool more = true; more && ok; ++n) {
           const int4 cur = nxt;
           if constexpr (kSplit) e = walk.next(e);
-          const bool has_next = kSplit ? e < eend : n + 1 < n_ent;
-          if (has_next) nxt = entries[kSplit ? e : ebeg + n + 1];
-          const uint32_t itv = 2 * n + 1, itk = 2 * n + 2;
+          const bool has_next = kSplit ? e < eend : (int)n + 1 < n_ent;
+          more = has_next;
+          if (has_next) nxt = entries[kSplit ? e : ebeg + (int)n + 1];
+          const uint32_t itv = it0 + 2 * n + 1, itk = it0 + 2 * n + 2;
           const uint32_t vslot = itv % kFwdStages, kslot = itk % kFwdStages;
-          const uint32_t vc = n & 1u;  // kP16: which f16 image holds this step's V
+          const uint32_t step = it0 / 2 + n, vc = step & 1u;  // kP16: which f16 image holds this step's V
           if constexpr (kP16)
-            ok = mbar_wait(&bars->vc_full[vc], (n >> 1) & 1u, ab, 0x340u + vc);
+            ok = mbar_wait(&bars->vc_full[vc], (step >> 1) & 1u, ab, 0x340u + vc);
           else
             ok = mbar_wait(&bars->kv_full[vslot], (itv / kFwdStages) & 1u, ab, 0x310u + vslot);
           if (ok && has_next)
             ok = mbar_wait(&bars->kv_full[kslot], (itk / kFwdStages) & 1u, ab, 0x320u + kslot);
           if (!ok) break;
           mma_issue_fence();
+          if (!kSplit && !has_next) tc_commit(&bars->q_free);
           for (int i = 0; i < 2 && ok; ++i) {
             if ((cur.y >> (2 * i)) & 3) {
-              ok = mbar_wait(&bars->p_half[i], pcnt[i] & 1u, ab, 0x350u + i);
+              if (!kSplit && !started[i] && stepped > 0)  // the previous row's O has left its columns
+                ok = mbar_wait(&bars->o_free[i], (stepped - 1) & 1u, ab, 0x360u + i);
+              ok = ok && mbar_wait(&bars->p_half[i], pcnt[i] & 1u, ab, 0x350u + i);
               if (!ok) break;
               mma_issue_fence();
               issue_pv(i, kP16 ? vc : vslot, started[i], 0);
@@ -370,13 +457,18 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               started[i] = true;
             }
             if (i == 1) tc_commit(kP16 ? &bars->vc_empty[vc] : &bars->kv_empty[vslot]);
+            if (!kSplit && !has_next) tc_commit(&bars->o_done[i]);
             if (has_next && ((nxt.y >> (2 * i)) & 3)) issue_qk(i, kslot);
           }
           if (ok && has_next) tc_commit(&bars->kv_empty[kslot]);
         }
+        if constexpr (kSplit) {  // the parts go over the operand tiles: not before both tiles' MMAs have read them
+          tc_commit(&bars->o_done[0]);
+          tc_commit(&bars->o_done[1]);
+        }
+        it0 += 2 * n;
+        ++stepped;
       }
-      tc_commit(&bars->o_done[0]);
-      tc_commit(&bars->o_done[1]);
     }
    }
   } else {
@@ -385,17 +477,27 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int i = warp >> 2;           // q tile within the pair
     const int wq = warp & 3;           // TMEM lane quarter this warp may touch
     const int r = wq * 32 + lane;      // row within the tile
-    const int q_tile = qt0 + i;
+    const bool has_seg = p.q_seg != nullptr;
+    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
+    const uint32_t t_s = tmem + lane_addr + i * kTile;
+    const uint32_t t_o = tmem + lane_addr + 2 * kTile + i * kTile;
+    uint32_t cnt = 0;
+    uint32_t stepped = 0;  // rows with steps so far
+    bool ok = true;
+    int4 work;
+    while (ok && next_work(work, true)) {
+    const int head = work.y % p.q_heads, batch = work.y / p.q_heads, eend = work.w;
+    const int kv_head = head / (p.q_heads / p.kv_heads);
+    const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
+    const PartWalk<kSplit> walk(entries, work.z, eend, p.n_split);
+    const int efirst = walk.first(walk.offset((int)rank));
+    const int q_tile = 2 * work.x + i;
     const bool valid = q_tile < p.n_q_tiles;
     const int q_row = valid ? q_tile * kTile + r : 0;
     const int qi = p.q_sequence ? p.q_sequence[q_row] : q_row;
     const RowInterval iv = mask_fn_interval(p.fn, qi);
-    const bool has_seg = p.q_seg != nullptr;
     const int q_seg = has_seg ? p.q_seg[(int64_t)batch * p.q_len + q_row] : 0;
     const int32_t* kv_seg_row = has_seg ? p.kv_seg + (int64_t)batch * p.kv_len : nullptr;
-    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
-    const uint32_t t_s = tmem + lane_addr + i * kTile;
-    const uint32_t t_o = tmem + lane_addr + 2 * kTile + i * kTile;
     // e4m3: scores carry the q tile's and the kv tile's scale; V tiles are weighted relative to
     // the largest V scale of this (batch, kv head).
     float cq = kSoftCap ? p.soft_cap * kLog2e : p.scale_log2;  // score -> log2 units
@@ -432,9 +534,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       m_used = sink2;
       l = 1.f;
     }
-    uint32_t cnt = 0;
     bool started = false;
-    bool ok = true;
 
     int4 ent_next = efirst < eend ? entries[efirst] : make_int4(0, 0, 0, 0);
     float ks_next = 1.f, vs_next = 1.f;
@@ -661,8 +761,8 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
 
     // ---- epilogue: O / l -> bf16, logsumexp, max_logits
-    if (ok) {
-      ok = mbar_wait(&bars->o_done[i], 0, ab, 0x500u + i);
+    if (ok && efirst < eend) {
+      ok = mbar_wait(&bars->o_done[i], stepped & 1u, ab, 0x500u + i);
       ok = __all_sync(0xffffffffu, ok);
     }
     if constexpr (kSplit) {
@@ -739,16 +839,14 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
     } else if (ok && valid) {
       tc_fence_after();
-      __nv_bfloat16* orow = p.o + (int64_t)batch * p.o_sb + (int64_t)head * p.o_sh +
-                            (int64_t)q_row * p.o_ss;
-      uint4* o4 = reinterpret_cast<uint4*>(orow);
-      // context parallelism: the row also goes to the rank that owns it in the sequence-sharded layout
-      uint4* peer4 = p.o_peer.ptrs ? reinterpret_cast<uint4*>(peer_row(p.o_peer, batch, head, q_row)) : nullptr;
+      // (context parallelism: the rows also go to the ranks that own them in the sequence-sharded layout)
+      __nv_bfloat16* row0 = p.o + (int64_t)batch * p.o_sb + (int64_t)head * p.o_sh + (int64_t)(q_row - lane) * p.o_ss;
       // e4m3: O accumulated P * 2^shift * (v scale / v_ref) times the stored V values
       const bool live = l > 0.f;  // a row that met a live key, or has a sink
       const float inv = live ? (kFp8 ? v_ref * 0.015625f / l : 1.0f / l) : 0.f;
 #pragma unroll
       for (int g = 0; g < 4; ++g) {
+        if (g * 32 >= p.d_v) break;
         uint32_t v[32];
         if (started) {
           tmem_ld32(t_o + g * 32, v);
@@ -757,20 +855,16 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = 0u;
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          uint4 w;
-          w.x = pack_bf16(__uint_as_float(v[8 * j + 0]) * inv, __uint_as_float(v[8 * j + 1]) * inv);
-          w.y = pack_bf16(__uint_as_float(v[8 * j + 2]) * inv, __uint_as_float(v[8 * j + 3]) * inv);
-          w.z = pack_bf16(__uint_as_float(v[8 * j + 4]) * inv, __uint_as_float(v[8 * j + 5]) * inv);
-          w.w = pack_bf16(__uint_as_float(v[8 * j + 6]) * inv, __uint_as_float(v[8 * j + 7]) * inv);
-          if ((g * 4 + j) * 8 < p.d_v) {
-            o4[g * 4 + j] = w;
-            if (peer4) peer4[g * 4 + j] = w;
-          }
-        }
+        store_rows32_peer(row0, p.o_ss, p.o_peer, batch, head, q_row - lane, v, inv, g * 32, p.d_v);
       }
       store_row_stats<kFp8, kSoftCap>(p, batch, head, q_row, live, m_used, l, m_true, sink2, fixed_max);
+    }
+    if (!kSplit && efirst < eend) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars->o_free[i]);
+      ++stepped;
+    }
     }
   }
 
