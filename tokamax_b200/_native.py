@@ -16,6 +16,7 @@ _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_PKG_DIR, "csrc")
 _LIB_DIR = os.path.join(_PKG_DIR, "lib")
 LIB_PATH = os.path.join(_LIB_DIR, "libsplash_b200.so")
+HOST_PATH = os.path.join(_LIB_DIR, "_splash_torch.so")
 
 SOURCES = (
     "splash_fwd_sm100.cu",
@@ -31,6 +32,8 @@ SOURCES = (
     "exchange.cu",
     "splash_xla_ffi.cc",  # handlers compile only where xla/ffi/api/ffi.h is on the include path
 )
+
+HOST_SOURCE = "splash_torch.cc"  # the host side of a call: tensors in, tensors out (needs torch's headers)
 
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -252,25 +255,40 @@ _lock = threading.Lock()
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-  """Compiles the CUDA/C++ sources into ``lib/libsplash_b200.so`` (sm_100a). Returns its path."""
+  """Compiles the CUDA/C++ sources into ``lib/libsplash_b200.so`` (sm_100a), and its host side into
+  ``lib/_splash_torch.so``. Returns the former's path."""
   srcs = [os.path.join(_CSRC, s) for s in SOURCES if os.path.exists(os.path.join(_CSRC, s))]
-  deps = srcs + [os.path.join(_CSRC, f) for f in os.listdir(_CSRC) if f.endswith(".cuh")]
-  deps.append(os.path.join(os.path.dirname(_PKG_DIR), "include", "splash_b200.h"))
-  if not force and os.path.exists(LIB_PATH):
-    newest = max(os.path.getmtime(d) for d in deps)
-    if os.path.getmtime(LIB_PATH) >= newest:
-      return LIB_PATH
+  header = os.path.join(os.path.dirname(_PKG_DIR), "include", "splash_b200.h")
+  deps = srcs + [os.path.join(_CSRC, f) for f in os.listdir(_CSRC) if f.endswith(".cuh")] + [header]
   os.makedirs(_LIB_DIR, exist_ok=True)
-  nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-  cmd = [nvcc, *NVCC_FLAGS, "-o", LIB_PATH, *srcs]
-  if verbose:
-    cmd.insert(1, "-Xptxas")
-    cmd.insert(2, "-v")
-  res = subprocess.run(cmd, capture_output=True, text=True)
-  if res.returncode != 0:
-    raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
-  if verbose:
-    print(res.stderr)
+
+  def stale(path, sources):
+    return force or not os.path.exists(path) or os.path.getmtime(path) < max(os.path.getmtime(d) for d in sources)
+
+  def run(cmd):
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+      raise RuntimeError(f"{cmd[0]} failed:\n" + res.stdout + res.stderr)
+    if verbose:
+      print(res.stderr)
+
+  host_src = os.path.join(_CSRC, HOST_SOURCE)
+  if stale(HOST_PATH, [host_src, header]):
+    import sysconfig
+
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    include = (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               os.path.join(cuda, "include"), sysconfig.get_paths()["include"])
+    run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{d}" for d in include),
+         "-o", HOST_PATH, host_src, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
+         "-lc10_cuda"])
+  if stale(LIB_PATH, deps):
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    run([nvcc, *(("-Xptxas", "-v") if verbose else ()), *NVCC_FLAGS, "-o", LIB_PATH, *srcs])
   return LIB_PATH
 
 
@@ -288,6 +306,29 @@ def lib() -> C.CDLL:
         fn.argtypes = argtypes
       _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+  """The module of ``csrc/splash_torch.cc``, bound to the library (built first if absent)."""
+  global _host
+  if _host is None:
+    handle = lib()
+    with _lock:
+      if _host is None:
+        import importlib.util
+
+        if not os.path.exists(HOST_PATH):
+          build()
+        spec = importlib.util.spec_from_file_location("_splash_torch", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind_library(*(C.cast(getattr(handle, name), C.c_void_p).value for name in (
+            "splash_fwd_shard", "splash_bwd_shard", "splash_bwd_workspace_bytes", "splash_bwd_fused_workspace_bytes")))
+        _host = module
+  return _host
 
 
 def exported_symbols() -> tuple[str, ...]:

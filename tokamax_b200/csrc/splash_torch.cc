@@ -1,0 +1,155 @@
+// The host side of a call in native code: reads the tensors' addresses, sizes and strides, allocates the results
+// and fills the C ABI's argument structs (include/splash_b200.h), which python did field by field through ctypes.
+// A forward spent 20 us of its host time there and a backward 35; they take 6 and 8 here.  The autograd function, the
+// checks of arguments and the schedules stay where they were, in splash_attention_kernel.py.
+#include <torch/csrc/utils/pybind.h>
+#include <torch/csrc/Exceptions.h>
+
+#include <ATen/ATen.h>
+#include <c10/core/DeviceGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <optional>
+#include <tuple>
+
+#include "../../include/splash_b200.h"
+
+namespace {
+
+// entry points of libsplash_b200.so, as ctypes resolved them
+struct Library {
+  int (*fwd)(const SplashFwdArgs*, const SplashShards*, void*) = nullptr;
+  int (*bwd)(const SplashBwdArgs*, const SplashShards*, void*) = nullptr;
+  size_t (*workspace_bytes)(int64_t, int64_t, int64_t) = nullptr;
+  size_t (*fused_workspace_bytes)(int64_t, int64_t, int64_t) = nullptr;
+} lib;
+
+void bind_library(uintptr_t fwd, uintptr_t bwd, uintptr_t workspace_bytes, uintptr_t fused_workspace_bytes) {
+  lib.fwd = reinterpret_cast<decltype(lib.fwd)>(fwd);
+  lib.bwd = reinterpret_cast<decltype(lib.bwd)>(bwd);
+  lib.workspace_bytes = reinterpret_cast<decltype(lib.workspace_bytes)>(workspace_bytes);
+  lib.fused_workspace_bytes = reinterpret_cast<decltype(lib.fused_workspace_bytes)>(fused_workspace_bytes);
+}
+
+// `t` if the kernels can read it in place, else a contiguous copy
+at::Tensor usable(const at::Tensor& t) {
+  TORCH_CHECK(t.dim() == 4, "expected a tensor of rank 4, got rank ", t.dim());
+  bool ok = t.stride(3) == 1 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  for (int i = 0; i < 3; ++i) ok = ok && t.stride(i) % 8 == 0;
+  return ok ? t : t.contiguous();
+}
+
+SplashTensor describe(const at::Tensor& t) {
+  TORCH_CHECK(t.dim() == 4, "expected a tensor of rank 4, got rank ", t.dim());
+  SplashTensor d{};
+  d.data = t.data_ptr();
+  d.dtype = SPLASH_BF16;
+  for (int i = 0; i < 4; ++i) d.size[i] = t.size(i), d.stride[i] = t.stride(i);
+  return d;
+}
+
+template <typename T>
+T* pointer(const std::optional<at::Tensor>& t) {
+  return t.has_value() ? static_cast<T*>(t->data_ptr()) : nullptr;
+}
+
+template <typename T>
+const T& at_address(uintptr_t a) {
+  return *reinterpret_cast<const T*>(a);
+}
+
+using Maybe = std::optional<at::Tensor>;
+
+// `sched`, `mask_fn`, `o_peer`: addresses of the structs (o_peer: 0 for none).  Returns the status, the operands as
+// the kernel read them, and the results.
+std::tuple<int, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor> forward(
+    const at::Tensor& q_in, const at::Tensor& k_in, const at::Tensor& v_in, const Maybe& q_seg, const Maybe& kv_seg,
+    const Maybe& q_sequence, const Maybe& sinks, const Maybe& max_logit, const at::Tensor& error_record, uintptr_t sched,
+    uintptr_t mask_fn, double scale, double mask_value, double soft_cap, int head_shards, int q_shards, uintptr_t o_peer) {
+  const at::Tensor q = usable(q_in), k = usable(k_in), v = usable(v_in);
+  const int64_t b = q.size(0), hq = q.size(1), sq = q.size(2);
+  // (like q, it keeps q's dense stride order, e.g. [B,T,H,D] storage stays [B,T,H,D])
+  const at::Tensor o = v.size(3) == q.size(3) ? at::empty_like(q) : at::empty({b, hq, sq, v.size(3)}, q.options());
+  const auto f32 = q.options().dtype(at::kFloat);
+  const at::Tensor lse = at::empty({b, hq, sq}, f32), max_logits = at::empty({b, hq, sq}, f32);
+  SplashFwdArgs a{};
+  a.q = describe(q);
+  a.k = describe(k);
+  a.v = describe(v);
+  a.o = describe(o);
+  a.logsumexp = static_cast<float*>(lse.data_ptr());
+  a.max_logits = static_cast<float*>(max_logits.data_ptr());
+  a.q_segment_ids = pointer<int32_t>(q_seg);
+  a.kv_segment_ids = pointer<int32_t>(kv_seg);
+  a.q_sequence = pointer<int32_t>(q_sequence);
+  a.sched = at_address<SplashDeviceSchedule>(sched);
+  a.mask_fn = at_address<SplashMaskFn>(mask_fn);
+  a.scale = (float)scale;
+  a.mask_value = (float)mask_value;
+  a.error_record = static_cast<uint32_t*>(error_record.data_ptr());
+  a.sinks = pointer<float>(sinks);
+  a.max_logit_value = pointer<float>(max_logit);
+  a.soft_cap = (float)soft_cap;
+  if (o_peer != 0) a.o_peer = at_address<SplashPeerOutput>(o_peer);
+  const SplashShards shards{head_shards, q_shards};
+  int status;
+  {
+    pybind11::gil_scoped_release release;
+    const c10::OptionalDeviceGuard guard(q.device());
+    status = lib.fwd(&a, &shards, c10::cuda::getCurrentCUDAStream(q.device().index()).stream());
+  }
+  return {status, q, k, v, o, lse, max_logits};
+}
+
+// `peers`: addresses of three SplashPeerOutput, or zeros.  Returns the status, the gradients and the workspace.
+std::tuple<int, at::Tensor, at::Tensor, at::Tensor, at::Tensor> backward(
+    const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& o, const at::Tensor& lse,
+    const at::Tensor& d_o_in, const Maybe& q_seg, const Maybe& kv_seg, const Maybe& q_sequence, const at::Tensor& error_record,
+    uintptr_t sched_dq, uintptr_t sched_dkv, uintptr_t mask_fn, double scale, double soft_cap, bool fused, int head_shards,
+    int q_shards, uintptr_t dq_peer, uintptr_t dk_peer, uintptr_t dv_peer) {
+  const at::Tensor d_o = usable(d_o_in);
+  const at::Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
+  SplashBwdArgs a{};
+  a.q = describe(q);
+  a.k = describe(k);
+  a.v = describe(v);
+  a.o = describe(o);
+  a.d_o = describe(d_o);
+  a.dq = describe(dq);
+  a.dk = describe(dk);
+  a.dv = describe(dv);
+  const size_t bytes = (fused ? lib.fused_workspace_bytes : lib.workspace_bytes)(q.size(0), q.size(1), q.size(2));
+  const at::Tensor workspace = at::empty({(int64_t)bytes}, q.options().dtype(at::kByte));
+  a.flags = fused ? SPLASH_BWD_FUSED_DQ : 0;
+  a.logsumexp = static_cast<float*>(lse.data_ptr());
+  a.q_segment_ids = pointer<int32_t>(q_seg);
+  a.kv_segment_ids = pointer<int32_t>(kv_seg);
+  a.q_sequence = pointer<int32_t>(q_sequence);
+  a.sched_dq = at_address<SplashDeviceSchedule>(sched_dq);
+  a.sched_dkv = at_address<SplashDeviceSchedule>(sched_dkv);
+  a.mask_fn = at_address<SplashMaskFn>(mask_fn);
+  a.scale = (float)scale;
+  a.workspace = workspace.data_ptr();
+  a.workspace_bytes = bytes;
+  a.error_record = static_cast<uint32_t*>(error_record.data_ptr());
+  a.soft_cap = (float)soft_cap;
+  if (dq_peer != 0) a.dq_peer = at_address<SplashPeerOutput>(dq_peer);
+  if (dk_peer != 0) a.dk_peer = at_address<SplashPeerOutput>(dk_peer);
+  if (dv_peer != 0) a.dv_peer = at_address<SplashPeerOutput>(dv_peer);
+  const SplashShards shards{head_shards, q_shards};
+  int status;
+  {
+    pybind11::gil_scoped_release release;
+    const c10::OptionalDeviceGuard guard(q.device());
+    status = lib.bwd(&a, &shards, c10::cuda::getCurrentCUDAStream(q.device().index()).stream());
+  }
+  return {status, dq, dk, dv, workspace};
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_splash_torch, m) {
+  m.def("bind_library", &bind_library);
+  m.def("forward", torch::wrap_pybind_function(forward));
+  m.def("backward", torch::wrap_pybind_function(backward));
+}

@@ -306,10 +306,8 @@ def _on(device: torch.device):
   return _ALREADY if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
-def _usable(t: torch.Tensor) -> torch.Tensor:
-  """Returns ``t`` if the kernels can read it in place, else a contiguous copy."""
-  ok = t.stride(-1) == 1 and all(s % 8 == 0 for s in t.stride()[:-1]) and t.data_ptr() % 16 == 0
-  return t if ok else t.contiguous()
+def _address(struct_or_none) -> int:
+  return 0 if struct_or_none is None else C.addressof(struct_or_none)
 
 
 def _shards(kernel, tables):
@@ -336,38 +334,15 @@ def splash_forward(kernel, q, k, v, q_seg, kv_seg, scale, sinks, max_logit, shar
   """
   _require_cuda(q)
   tables = kernel._tables(q.device, q.shape[0], shard)  # pylint: disable=protected-access
-  q, k, v = _usable(q), _usable(k), _usable(v)
-  b, hq, sq, d = q.shape
-  if v.shape[-1] == d:
-    o = torch.empty_like(q)  # keeps q's (dense) stride order, e.g. [B,T,H,D] storage stays [B,T,H,D]
-  else:
-    o = torch.empty((b, hq, sq, v.shape[-1]), dtype=q.dtype, device=q.device)
-  lse = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device)
-  max_logits = torch.empty((b, hq, sq), dtype=torch.float32, device=q.device)
-  args = _native.SplashFwdArgs()
-  args.q, args.k, args.v, args.o = map(_tensor_desc, (q, k, v, o))
-  args.logsumexp = lse.data_ptr()
-  args.max_logits = max_logits.data_ptr()
-  args.q_segment_ids = q_seg.data_ptr() if q_seg is not None else None
-  args.kv_segment_ids = kv_seg.data_ptr() if kv_seg is not None else None
-  args.q_sequence = tables.q_sequence.data_ptr() if tables.q_sequence is not None else None
-  keep = []
-  args.sched = tables.fwd
-  if q_seg is not None and not tables.fwd.row_end:  # device-built schedules are not filtered further
-    args.sched, ws = _segment_schedule(tables.fwd, 0, q_seg, kv_seg, q.shape[2], k.shape[2])
-    keep.append(ws)
-  args.mask_fn = kernel._mask_fn  # pylint: disable=protected-access
-  args.scale = scale
-  args.mask_value = max(kernel.mask_value, -3.0e38)
-  args.error_record = tables.error_record.data_ptr()
+  sched = tables.fwd
+  if q_seg is not None and not sched.row_end:  # device-built schedules are not filtered further
+    sched, keep = _segment_schedule(sched, 0, q_seg, kv_seg, q.shape[2], k.shape[2])  # (`keep`: until the launch below)
   sinks_f32 = None if sinks is None else sinks.detach().to(torch.float32).contiguous()
-  args.sinks = None if sinks_f32 is None else sinks_f32.data_ptr()
-  args.soft_cap = float(kernel.config.attn_logits_soft_cap or 0.0)
-  args.max_logit_value = None if max_logit is None else max_logit.data_ptr()
-  if o_peer is not None:
-    args.o_peer = o_peer
-  with _on(q.device):
-    _native.check(_native.lib().splash_fwd_shard(C.byref(args), _shards(kernel, tables), _raw_stream(q.device)), "splash_fwd")
+  status, q, k, v, o, lse, max_logits = _native.host().forward(
+      q, k, v, q_seg, kv_seg, tables.q_sequence, sinks_f32, max_logit, tables.error_record, C.addressof(sched),
+      C.addressof(kernel._mask_fn), scale, max(kernel.mask_value, -3.0e38),  # pylint: disable=protected-access
+      float(kernel.config.attn_logits_soft_cap or 0.0), kernel.head_shards, tables.q_shards, _address(o_peer))
+  _native.check(status, "splash_fwd")
   return q, k, v, o, lse, max_logits, sinks_f32
 
 
@@ -391,7 +366,8 @@ class _SplashFunction(torch.autograd.Function):
     q, k, v, o, lse, q_seg, kv_seg, sinks = ctx.saved_tensors
     if d_o is None:  # an undefined gradient of o is zero
       d_o = torch.zeros_like(o)
-    dq, dk, dv, neg_di = splash_backward(ctx.kernel, q, k, v, o, lse, d_o, q_seg, kv_seg, ctx.scale, ctx.shard)
+    dq, dk, dv, neg_di = splash_backward(ctx.kernel, q, k, v, o, lse, d_o, q_seg, kv_seg, ctx.scale, ctx.shard,
+                                         with_di=sinks is not None)
     dsinks = None
     if sinks is not None:
       # reference kernel.py:1928-1935: dsinks[h] = -sum_rows exp(sink - lse) * sum_d(o * do)
@@ -400,7 +376,7 @@ class _SplashFunction(torch.autograd.Function):
 
 
 def splash_backward(kernel: "SplashAttentionKernel", q, k, v, o, lse, d_o, q_seg=None, kv_seg=None,
-                    scale: float = 1.0, shard: int = 0, peers=None):
+                    scale: float = 1.0, shard: int = 0, peers=None, with_di: bool = True):
   """One `splash_bwd` call: ``(dq, dk, dv, neg_di)`` for batched ``[B, H, S, 128]`` bf16 tensors.
 
   ``peers``: optional ``(dq_peer, dk_peer, dv_peer)`` of `_native.SplashPeerOutput`, second
@@ -410,44 +386,27 @@ def splash_backward(kernel: "SplashAttentionKernel", q, k, v, o, lse, d_o, q_seg
   softmax over more keys than ``k`` holds (ring attention passes the merged values, reference
   ring_attention_kernel.py:228-262), in which case dq / dk / dv are this key shard's share.
   ``neg_di`` is ``-sum_d(o * do)`` (fp32 ``[B, Hq, Sq]``), a view of the backward's workspace, which
-  keeps the row sums negated.
+  keeps the row sums negated (None without ``with_di``).
   """
   tables = kernel._tables(q.device, q.shape[0], shard)  # pylint: disable=protected-access
-  d_o = _usable(d_o)
-  dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-  lib = _native.lib()
-  # head dims above 128 run three separate passes (dq, dk, dv), each repeatable bit for bit
+  # head dims above 128 run separate passes, each repeatable bit for bit
   fused = not kernel.repeatable_dq and q.shape[-1] <= _HEAD_DIM and v.shape[-1] <= _HEAD_DIM
-  size_fn = lib.splash_bwd_fused_workspace_bytes if fused else lib.splash_bwd_workspace_bytes
-  ws_bytes = size_fn(q.shape[0], q.shape[1], q.shape[2])
-  workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-  args = _native.SplashBwdArgs()
-  args.flags = _native.BWD_FUSED_DQ if fused else 0
-  args.q, args.k, args.v, args.o, args.d_o = map(_tensor_desc, (q, k, v, o, d_o))
-  args.dq, args.dk, args.dv = map(_tensor_desc, (dq, dk, dv))
-  args.logsumexp = lse.data_ptr()
-  args.q_segment_ids = q_seg.data_ptr() if q_seg is not None else None
-  args.kv_segment_ids = kv_seg.data_ptr() if kv_seg is not None else None
-  args.q_sequence = tables.q_sequence.data_ptr() if tables.q_sequence is not None else None
-  keep = []
-  args.sched_dq = tables.dq
-  args.sched_dkv = tables.dkv
-  if q_seg is not None and not tables.dq.row_end:
+  sched_dq, sched_dkv = tables.dq, tables.dkv
+  keep = []  # until the launch below
+  if q_seg is not None and not sched_dq.row_end:
     if not fused:  # the fused form walks the dkv schedule only
-      args.sched_dq, ws1 = _segment_schedule(tables.dq, 1, q_seg, kv_seg, q.shape[2], k.shape[2])
+      sched_dq, ws1 = _segment_schedule(sched_dq, 1, q_seg, kv_seg, q.shape[2], k.shape[2])
       keep.append(ws1)
-    args.sched_dkv, ws2 = _segment_schedule(tables.dkv, 2, q_seg, kv_seg, q.shape[2], k.shape[2])
+    sched_dkv, ws2 = _segment_schedule(sched_dkv, 2, q_seg, kv_seg, q.shape[2], k.shape[2])
     keep.append(ws2)
-  args.mask_fn = kernel._mask_fn  # pylint: disable=protected-access
-  args.scale = scale
-  args.workspace = workspace.data_ptr()
-  args.workspace_bytes = ws_bytes
-  args.soft_cap = float(kernel.config.attn_logits_soft_cap or 0.0)
-  args.error_record = tables.error_record.data_ptr()
-  if peers is not None:
-    args.dq_peer, args.dk_peer, args.dv_peer = peers
-  with _on(q.device):
-    _native.check(lib.splash_bwd_shard(C.byref(args), _shards(kernel, tables), _raw_stream(q.device)), "splash_bwd")
+  status, dq, dk, dv, workspace = _native.host().backward(
+      q, k, v, o, lse, d_o, q_seg, kv_seg, tables.q_sequence, tables.error_record, C.addressof(sched_dq),
+      C.addressof(sched_dkv), C.addressof(kernel._mask_fn), scale,  # pylint: disable=protected-access
+      float(kernel.config.attn_logits_soft_cap or 0.0), fused, kernel.head_shards, tables.q_shards,
+      *map(_address, peers if peers is not None else (None, None, None)))
+  _native.check(status, "splash_bwd")
+  if not with_di:
+    return dq, dk, dv, None
   n = q.shape[0] * q.shape[1] * q.shape[2]
   neg_di = workspace[:4 * n].view(torch.float32).view(q.shape[0], q.shape[1], q.shape[2])
   return dq, dk, dv, neg_di
