@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 import torch
 
+from tokamax_b200 import fp8
 from tokamax_b200 import splash_attention_kernel as splash
 from tokamax_b200 import splash_attention_mask as mask_lib
 
@@ -64,3 +65,59 @@ def test_heads_above_128_of_a_large_call_are_those_of_small_calls(d_qk, d_v, kin
     for name in part:
       mine = whole[name][:, heads if name in ("out", "lse", "dq") else slice(h, h + 1)]
       assert torch.equal(mine, part[name]), (name, h)
+
+
+# 7 schedule rows of 44 (batch, q head) pairs; the second tile of every head's last row does not exist
+@pytest.mark.parametrize("d", [128, 64, 80])
+@pytest.mark.parametrize("kind,soft_cap,segments,sinks", [("causal", None, False, True), ("window", 20.0, True, False),
+                                                          ("table", None, False, False)])
+def test_heads_up_to_128_of_a_large_call_are_those_of_its_shares(d, kind, soft_cap, segments, sinks):
+  b, hkv, group, s = 2, 11, 2, 1664
+  g = torch.Generator(device=DEV).manual_seed(d)
+  mk = lambda h: torch.randn(b, h, s, d, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v, do = mk(hkv * group), mk(hkv), mk(hkv), mk(hkv * group)
+  seg = None
+  if segments:
+    ids = torch.zeros((b, s), dtype=torch.int32, device=DEV)
+    ids[0, 700:], ids[1, 130:], ids[1, 1500:] = 1, 1, 2
+    seg = splash.SegmentIds(q=ids, kv=ids)
+  config = splash.SplashConfig.get_default()
+  if soft_cap:
+    config = splash.dataclasses.replace(config, attn_logits_soft_cap=soft_cap)
+  kernel = splash.make_splash_mha(_mask(kind, s), config=config, q_seq_shards=1, save_residuals=True, repeatable_dq=True)
+  sink = torch.randn(hkv * group, generator=g, device=DEV) if sinks else None
+  scale = 1 / math.sqrt(d)
+
+  def run(kern, q, k, v, do, sink):
+    q, k, v = (t.detach().requires_grad_(True) for t in (q, k, v))
+    out, res = kern(q, k, v, seg, sink, logits_scale=scale)
+    dq, dk, dv = torch.autograd.grad(out, (q, k, v), do)
+    return {"out": out.detach(), "lse": res["logsumexp"], "max": res["max_logits"], "dq": dq, "dk": dk, "dv": dv}
+
+  whole = run(kernel, q, k, v, do, sink)
+  kernel.check_errors()
+  share = kernel.head_shard(hkv)  # cut as the whole call is, whatever its size
+  for h in range(0, hkv, 5):
+    heads = slice(h * group, (h + 1) * group)
+    part = run(share, q[:, heads].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous(),
+               do[:, heads].contiguous(), sink[heads] if sinks else None)
+    share.check_errors()
+    for name in part:
+      mine = whole[name][:, slice(h, h + 1) if name in ("dk", "dv") else heads]
+      assert torch.equal(mine, part[name]), (name, h)
+
+
+@pytest.mark.parametrize("p_format", ["e4m3", "f16"])
+def test_e4m3_heads_of_a_large_call_are_those_of_its_shares(p_format):
+  b, hkv, group, s = 2, 11, 2, 1664
+  g = torch.Generator(device=DEV).manual_seed(3)
+  mk = lambda h: torch.randn(b, h, s, 128, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v = mk(hkv * group), mk(hkv), mk(hkv)
+  kernel = splash.make_splash_mha(_mask("causal", s), q_seq_shards=1)
+  run = lambda kern, *t: fp8.splash_fwd_fp8(kern, *(fp8.quantize_e4m3(x) for x in t), logits_scale=0.09, p_format=p_format)
+  whole = run(kernel, q, k, v)
+  for h in range(0, hkv, 5):
+    heads = slice(h * group, (h + 1) * group)
+    part = run(kernel.head_shard(hkv), q[:, heads].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous())
+    kernel.check_errors()
+    assert torch.equal(whole[:, heads], part), h
