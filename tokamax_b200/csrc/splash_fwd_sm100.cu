@@ -151,6 +151,19 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int eend = p.row_end ? p.row_end[(int64_t)(work.group / p.q_heads) * p.n_rows + work.row] : p.row_ptr[work.row + 1];
     return make_int4(work.row, work.group, ebeg, eend < ebeg ? ebeg : eend);
   };
+  auto list_of = [&](const int4& w) { return p.entries + (int64_t)(w.y / p.q_heads) * p.entries_per_batch; };
+  // the entries of this CTA in a row, and the first of them (a cluster's row: looked up here, under the set-up of
+  // barriers and TMEM)
+  int4 own = make_int4(0, 0, 0, 0);
+  if constexpr (kSplit) own = row_of(blockIdx.x / p.n_split);
+  const PartWalk<kSplit> own_walk(list_of(own), own.z, own.w, p.n_split);
+  int own_first = 0;
+  if constexpr (kSplit) own_first = own_walk.first(own_walk.offset((int)rank));
+  auto walk_of = [&](const int4& w) {
+    if constexpr (kSplit) return own_walk;
+    return PartWalk<kSplit>(list_of(w), w.z, w.w, p.n_split);
+  };
+  auto first_of = [&](const int4& w) { return kSplit ? own_first : w.z; };
 
   if (threadIdx.x == 0) {
     bars->early_exit = *reinterpret_cast<volatile uint32_t*>(p.err);
@@ -199,12 +212,9 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   // The rows this CTA works on, in order: its own, then those it takes over (the producer posts both).  A CTA of a
   // cluster has the cluster's row and no other.
   RingPos work_pos{0, 0};
-  bool first_work = true;
   auto next_work = [&](int4& w, bool warp_wide) {  // by a whole warp, or by a thread for its warp
-    if constexpr (kSplit) {
-      if (!first_work) return false;
-      first_work = false;
-      w = row_of(blockIdx.x / p.n_split);
+    if constexpr (kSplit) {  // (whose loops end behind it)
+      w = own;
       return true;
     }
     bool ok = mbar_wait(&bars->work_full[work_pos.slot], work_pos.phase, ab, 0x700u + work_pos.slot);
@@ -232,8 +242,8 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       int4 w;
       while (ok && next_work(w, true)) {
        const int eend = w.w;
-       const PartWalk<kSplit> walk(p.entries + (int64_t)(w.y / p.q_heads) * p.entries_per_batch, w.z, eend, p.n_split);
-       for (int e = walk.first(walk.offset((int)rank)); e < eend; e = walk.next(e), ++n) {
+       const PartWalk<kSplit> walk = walk_of(w);
+       for (int e = first_of(w); e < eend; e = walk.next(e), ++n) {
         const uint32_t it = 2 * n + 1, s = it % kFwdStages, j = n & 1u;
         ok = mbar_wait(&bars->kv_full[s], (it / kFwdStages) & 1u, ab, 0x600u + s);
         if (ok) ok = mbar_wait(&bars->vc_empty[j], ((n >> 1) & 1u) ^ 1u, ab, 0x610u + j);
@@ -262,6 +272,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           mbar_arrive(&bars->kv_empty[s]);
         }
        }
+       if (kSplit) break;
       }
     }
    } else if (warp == 8) {
@@ -274,23 +285,23 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint32_t stepped = 0;  // rows with steps so far
       uint32_t asked = 0;
       bool ok = true;
-      int block = (int)(kSplit ? blockIdx.x / p.n_split : blockIdx.x);
+      int block = (int)blockIdx.x;
       for (;;) {
-        int4 w = make_int4(-1, 0, 0, 0);
-        if (block >= 0) w = row_of((unsigned)block);
+        int4 w = own;
         if constexpr (!kSplit) {
+          w = block >= 0 ? row_of((unsigned)block) : make_int4(-1, 0, 0, 0);
           ok = mbar_wait(&bars->work_empty[work_pos.slot], work_pos.phase ^ 1u, ab, 0x710u + work_pos.slot);
           if (!ok) break;
           bars->work[work_pos.slot] = w;
           mbar_arrive(&bars->work_full[work_pos.slot]);
           work_pos.advance(1, 2);
+          if (block < 0) break;
         }
-        if (block < 0) break;
         const int qt0 = 2 * w.x, head = w.y % p.q_heads, batch = w.y / p.q_heads, eend = w.w;
         const int kv_head = head / (p.q_heads / p.kv_heads);
-        const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
-        const PartWalk<kSplit> walk(entries, w.z, eend, p.n_split);  // the entries of this CTA
-        const int efirst = walk.first(walk.offset((int)rank));
+        const int4* entries = list_of(w);
+        const PartWalk<kSplit> walk = walk_of(w);
+        const int efirst = first_of(w);
         if (efirst < eend) {
           if (stepped > 0) ok = mbar_wait(&bars->q_free, (stepped - 1) & 1u, ab, 0x110u);
           if (!ok) break;
@@ -404,11 +415,14 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       bool ok = true;
       int4 w;
       while (ok && next_work(w, false)) {
-        const int4* entries = p.entries + (int64_t)(w.y / p.q_heads) * p.entries_per_batch;
+        const int4* entries = list_of(w);
         const int ebeg = w.z, eend = w.w;
-        const PartWalk<kSplit> walk(entries, ebeg, eend, p.n_split);
-        const int efirst = walk.first(walk.offset((int)rank));
-        if (efirst >= eend) continue;
+        const PartWalk<kSplit> walk = walk_of(w);
+        const int efirst = first_of(w);
+        if (efirst >= eend) {
+          if (kSplit) break;
+          continue;
+        }
         const int n_ent = eend - ebeg;
         int e = efirst;
         bool started[2] = {false, false};
@@ -468,6 +482,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
         it0 += 2 * n;
         ++stepped;
+        if (kSplit) break;
       }
     }
    }
@@ -488,9 +503,9 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     while (ok && next_work(work, true)) {
     const int head = work.y % p.q_heads, batch = work.y / p.q_heads, eend = work.w;
     const int kv_head = head / (p.q_heads / p.kv_heads);
-    const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
-    const PartWalk<kSplit> walk(entries, work.z, eend, p.n_split);
-    const int efirst = walk.first(walk.offset((int)rank));
+    const int4* entries = list_of(work);
+    const PartWalk<kSplit> walk = walk_of(work);
+    const int efirst = first_of(work);
     const int q_tile = 2 * work.x + i;
     const bool valid = q_tile < p.n_q_tiles;
     const int q_row = valid ? q_tile * kTile + r : 0;
@@ -865,6 +880,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       if (lane == 0) mbar_arrive(&bars->o_free[i]);
       ++stepped;
     }
+    if (kSplit) break;
     }
   }
 
