@@ -53,23 +53,6 @@ __device__ __forceinline__ uint32_t packed_a_col(int k) {
   return (uint32_t)((k >> 2) * 64 + (k & 3) * 8);
 }
 
-// 32 columns of a row, starting at column `col0` of a tensor that has `cols` columns: chunks of
-// eight that lie beyond the tensor's last column (head dims below 128) are not stored.
-__device__ __forceinline__ void store_row_half(__nv_bfloat16* dst, const uint32_t (&v)[32],
-                                               float mul, int col0 = 0, int cols = kHeadDim) {
-  uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    if (col0 + 8 * j >= cols) break;
-    uint4 w;
-    w.x = pack_bf16(__uint_as_float(v[8 * j + 0]) * mul, __uint_as_float(v[8 * j + 1]) * mul);
-    w.y = pack_bf16(__uint_as_float(v[8 * j + 2]) * mul, __uint_as_float(v[8 * j + 3]) * mul);
-    w.z = pack_bf16(__uint_as_float(v[8 * j + 4]) * mul, __uint_as_float(v[8 * j + 5]) * mul);
-    w.w = pack_bf16(__uint_as_float(v[8 * j + 6]) * mul, __uint_as_float(v[8 * j + 7]) * mul);
-    d4[j] = w;
-  }
-}
-
 // Backward for head dims above 128 (defined in splash_bwd_wide_sm100.cu).  `p` carries the fields
 // that do not depend on the pass; the launcher fills outputs and schedules per pass.
 // The tensor maps have boxes of kSub rows.

@@ -428,8 +428,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     }
 
     // epilogue
-    __nv_bfloat16* dst = p.out0 + (int64_t)batch * p.out0_sb + (int64_t)head * p.out0_sh +
-                         (int64_t)q_row * p.out0_ss + w * 64;
+    __nv_bfloat16* row0 = p.out0 + (int64_t)batch * p.out0_sb + (int64_t)head * p.out0_sh + (int64_t)(q_row - lane) * p.out0_ss;
     if (n_ent > 0) {
       if (ok) {
         ok = mbar_wait(&bars->acc_done, 0, ab, 0x1500u);
@@ -442,15 +441,15 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           uint32_t v[32];
           tmem_ld32(tmem + lane_addr + 3 * kTile + w * 64 + g * 32, v);
           tmem_ld_wait();
-          store_row_half(dst + g * 32, v, p.scale, w * 64 + g * 32, p.d_qk);
+          store_rows32(row0, p.out0_ss, v, p.scale, w * 64 + g * 32, p.d_qk);
         }
       }
     } else {
       uint32_t v[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) v[j] = 0u;
-      store_row_half(dst, v, 0.f, w * 64, p.d_qk);
-      store_row_half(dst + 32, v, 0.f, w * 64 + 32, p.d_qk);
+      store_rows32(row0, p.out0_ss, v, 0.f, w * 64, p.d_qk);
+      store_rows32(row0, p.out0_ss, v, 0.f, w * 64 + 32, p.d_qk);
     }
   }
 
@@ -1020,32 +1019,28 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           if (peer.ptrs) *reinterpret_cast<uint4*>(peer_row(peer, batch, kv_head, kv_row) + col) = w;
         }
       }
-    } else if (n_steps > 0) {
-      if (ok) {
+    } else {
+      if (n_steps > 0 && ok) {
         ok = mbar_wait(&bars->acc_done, 0, ab, 0x3500u);
         ok = __all_sync(0xffffffffu, ok);
       }
       if (ok) {
         tc_fence_after();
-        uint32_t v[32];
-        tmem_ld32(tmem + lane_addr + 2 * kTile + cq * 32, v);
-        tmem_ld_wait();
-        store_row_half(dk, v, p.scale, cq * 32, p.d_qk);
-        // context parallelism: the row also goes to the rank that owns it in the sequence-sharded layout
-        if (p.out0_peer.ptrs) store_row_half(peer_row(p.out0_peer, batch, kv_head, kv_row) + cq * 32, v, p.scale, cq * 32, p.d_qk);
-        tmem_ld32(tmem + lane_addr + 3 * kTile + cq * 32, v);
-        tmem_ld_wait();
-        store_row_half(dv, v, 1.0f, cq * 32, p.d_v);
-        if (p.out1_peer.ptrs) store_row_half(peer_row(p.out1_peer, batch, kv_head, kv_row) + cq * 32, v, 1.0f, cq * 32, p.d_v);
-      }
-    } else {
-      uint32_t v[32];
+        // (context parallelism: the rows also go to the ranks that own them in the sequence-sharded layout)
 #pragma unroll
-      for (int j = 0; j < 32; ++j) v[j] = 0u;
-      store_row_half(dk, v, 0.f, cq * 32, p.d_qk);
-      store_row_half(dv, v, 0.f, cq * 32, p.d_v);
-      if (p.out0_peer.ptrs) store_row_half(peer_row(p.out0_peer, batch, kv_head, kv_row) + cq * 32, v, 0.f, cq * 32, p.d_qk);
-      if (p.out1_peer.ptrs) store_row_half(peer_row(p.out1_peer, batch, kv_head, kv_row) + cq * 32, v, 0.f, cq * 32, p.d_v);
+        for (int which = 0; which < 2; ++which) {
+          uint32_t v[32];
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = 0u;  // (a kv tile that no step touches gets zeros)
+          if (n_steps > 0) {
+            tmem_ld32(tmem + lane_addr + (2 + which) * kTile + cq * 32, v);
+            tmem_ld_wait();
+          }
+          const int64_t ss = which ? p.out1_ss : p.out0_ss;
+          store_rows32_peer((which ? dv : dk) - cq * 32 - (int64_t)lane * ss, ss, which ? p.out1_peer : p.out0_peer, batch, kv_head,
+                            kv_row - lane, v, which ? 1.0f : p.scale, cq * 32, which ? p.d_v : p.d_qk);
+        }
+      }
     }
   }
 
