@@ -33,7 +33,7 @@ SOURCES = (
     "splash_xla_ffi.cc",  # handlers compile only where xla/ffi/api/ffi.h is on the include path
 )
 
-HOST_SOURCE = "splash_torch.cc"  # the host side of a call: tensors in, tensors out (needs torch's headers)
+HOST_SOURCE = "splash_torch.cpp"  # the host side of a call: tensors in, tensors out (needs torch's headers)
 
 NVCC_FLAGS = (
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -312,7 +312,7 @@ _host = None
 
 
 def host():
-  """The module of ``csrc/splash_torch.cc``, bound to the library (built first if absent)."""
+  """The module of ``csrc/splash_torch.cpp``, bound to the library (built first if absent)."""
   global _host
   if _host is None:
     handle = lib()
