@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 import torch
 
+from oracle import attention_ref
 from tokamax_b200 import fp8
 from tokamax_b200 import splash_attention_kernel as splash
 from tokamax_b200 import splash_attention_mask as mask_lib
@@ -121,3 +122,63 @@ def test_e4m3_heads_of_a_large_call_are_those_of_its_shares(p_format):
     part = run(kernel.head_shard(hkv), q[:, heads].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous())
     kernel.check_errors()
     assert torch.equal(whole[:, heads], part), h
+
+
+def _pairs_with_a_dead_tile(s):
+  """A causal table that leaves out one tile of the pairs of a schedule row (256 query rows), or none.
+
+  The warps of a tile that is dead in several of a CTA's rows have nothing to do in them, and may be rows behind the
+  others when the tile is live again.  The last pair's second tile does not exist (its row is then empty).
+  """
+  m = np.tril(np.ones((s, s), np.bool_))
+  for pair, dead in enumerate((1, 1, 0, 1, None, 1, 0)):
+    if dead is not None:
+      m[pair * 256 + dead * 128:pair * 256 + dead * 128 + 128] = False
+  return m
+
+
+# eight rows a CTA and more.  q_len 128: no row has its second tile
+@pytest.mark.parametrize("variant", ["bf16", "soft_cap", "e4m3", "f16"])
+@pytest.mark.parametrize("q_len,kv_len", [(1664, 1664), (128, 128), (128, 640)])
+def test_rows_with_a_dead_tile_of_a_large_call(variant, q_len, kv_len):
+  b, hkv, group = (2, 11, 8) if q_len > 128 else (8, 20, 8)
+  g = torch.Generator(device=DEV).manual_seed(q_len + kv_len)
+  mk = lambda h, s: torch.randn(b, h, s, 128, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v = mk(hkv * group, q_len), mk(hkv, kv_len), mk(hkv, kv_len)
+  dense = _pairs_with_a_dead_tile(q_len) if q_len > 128 else np.tril(np.ones((q_len, kv_len), np.bool_), kv_len - q_len)
+  cap = 20.0 if variant == "soft_cap" else None
+  config = splash.dataclasses.replace(splash.SplashConfig.get_default(), attn_logits_soft_cap=cap)
+  kernel = splash.make_splash_mha(mask_lib.NumpyMask(dense), config=config, q_seq_shards=1,
+                                  save_residuals=variant in ("bf16", "soft_cap"))
+  scale = 1 / math.sqrt(128)
+
+  def run(kern, q, k, v):
+    if variant in ("e4m3", "f16"):
+      t = fp8.splash_fwd_fp8(kern, *(fp8.quantize_e4m3(x) for x in (q, k, v)), logits_scale=scale, p_format=variant)
+      return {"out": t}
+    with torch.no_grad():
+      out, res = kern(q, k, v, logits_scale=scale)
+    return {"out": out, "lse": res["logsumexp"], "max": res["max_logits"]}
+
+  whole = run(kernel, q, k, v)
+  kernel.check_errors()
+  share = kernel.head_shard(hkv)
+  for h in range(0, hkv, 5):
+    heads = slice(h * group, (h + 1) * group)
+    part = run(share, q[:, heads].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous())
+    share.check_errors()
+    for name in part:
+      assert torch.equal(whole[name][:, heads], part[name]), (name, h)
+  live = torch.from_numpy(dense.any(1))
+  assert not whole["out"][:, :, ~live].any()
+  if "lse" not in whole:
+    return
+  for at, h in ((0, 3), (b - 1, hkv * group - 1)):
+    kv = slice(h // group, h // group + 1)
+    ro, rlse, rmax = attention_ref.attention_reference(q[at, h:h + 1].cpu(), k[at, kv].cpu(), v[at, kv].cpu(), dense, scale=scale,
+                                                       attn_logits_soft_cap=cap)
+    # P and the output are rounded to 8 bits, half an ulp (2^-9) each: at most 2^-8 of the largest |v| of a row's keys
+    bound = 2.0 ** -8 * v[at, kv].float().abs().max().item()
+    assert (whole["out"][at, h].float().cpu() - ro[0])[live].abs().max().item() <= bound
+    assert (whole["lse"][at, h].cpu() - rlse[0])[live].abs().max().item() <= 1e-4  # fp32 sums of up to 1664 terms
+    assert (whole["max"][at, h].cpu() - rmax[0])[live].abs().max().item() <= 1e-4

@@ -56,8 +56,9 @@ struct FwdBarriers {
   uint64_t s_full[2];
   uint64_t p_half[2];    // the first 64 key columns of P are in TMEM (the first half of the p v MMAs may go)
   uint64_t p_full[2];
+  // a tile's O is complete: one phase a row in which the tile is live (rows shared by a cluster: one phase).  A phase for
+  // rows that pass the tile by would have nothing to wait for: the issuing thread could complete the next one unseen
   uint64_t o_done[2];
-  uint64_t o_free[2];    // a tile's O has been read
   uint64_t vc_full[2];   // e4m3 with f16 P: a V tile has been converted to f16
   uint64_t vc_empty[2];  //                  the p v MMAs that read it have completed
   uint32_t tmem_base;
@@ -174,7 +175,6 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       mbar_init(&bars->p_half[i], 4);  // one arrival per softmax warp
       mbar_init(&bars->p_full[i], 4);
       mbar_init(&bars->o_done[i], 1);
-      mbar_init(&bars->o_free[i], 4);
       mbar_init(&bars->work_full[i], 1);
       mbar_init(&bars->work_empty[i], kP16 ? 11 : 9);  // softmax warps, the issuing and the converting ones
       mbar_init(&bars->vc_full[i], 2);   // one arrival per converting warp
@@ -411,7 +411,6 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       uint32_t pcnt[2] = {0, 0};
       uint32_t qcnt[2] = {0, 0};   // Q tiles so far
       uint32_t it0 = 0;            // ring slots of the rows before this one
-      uint32_t stepped = 0;        // rows with steps so far
       bool ok = true;
       int4 w;
       while (ok && next_work(w, false)) {
@@ -457,9 +456,8 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           if (!kSplit && !has_next) tc_commit(&bars->q_free);
           for (int i = 0; i < 2 && ok; ++i) {
             if ((cur.y >> (2 * i)) & 3) {
-              if (!kSplit && !started[i] && stepped > 0)  // the previous row's O has left its columns
-                ok = mbar_wait(&bars->o_free[i], (stepped - 1) & 1u, ab, 0x360u + i);
-              ok = ok && mbar_wait(&bars->p_half[i], pcnt[i] & 1u, ab, 0x350u + i);
+              // (its softmax warps have read the previous row's O by then: they come to this row's P behind it)
+              ok = mbar_wait(&bars->p_half[i], pcnt[i] & 1u, ab, 0x350u + i);
               if (!ok) break;
               mma_issue_fence();
               issue_pv(i, kP16 ? vc : vslot, started[i], 0);
@@ -471,7 +469,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               started[i] = true;
             }
             if (i == 1) tc_commit(kP16 ? &bars->vc_empty[vc] : &bars->kv_empty[vslot]);
-            if (!kSplit && !has_next) tc_commit(&bars->o_done[i]);
+            if (!kSplit && !has_next && started[i]) tc_commit(&bars->o_done[i]);
             if (has_next && ((nxt.y >> (2 * i)) & 3)) issue_qk(i, kslot);
           }
           if (ok && has_next) tc_commit(&bars->kv_empty[kslot]);
@@ -481,7 +479,6 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           tc_commit(&bars->o_done[1]);
         }
         it0 += 2 * n;
-        ++stepped;
         if (kSplit) break;
       }
     }
@@ -497,7 +494,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const uint32_t t_s = tmem + lane_addr + i * kTile;
     const uint32_t t_o = tmem + lane_addr + 2 * kTile + i * kTile;
     uint32_t cnt = 0;
-    uint32_t stepped = 0;  // rows with steps so far
+    uint32_t live_rows = 0;  // rows so far in which this tile was live
     bool ok = true;
     int4 work;
     while (ok && next_work(work, true)) {
@@ -776,8 +773,8 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
 
     // ---- epilogue: O / l -> bf16, logsumexp, max_logits
-    if (ok && efirst < eend) {
-      ok = mbar_wait(&bars->o_done[i], stepped & 1u, ab, 0x500u + i);
+    if (ok && (kSplit ? efirst < eend : started)) {
+      ok = mbar_wait(&bars->o_done[i], live_rows++ & 1u, ab, 0x500u + i);
       ok = __all_sync(0xffffffffu, ok);
     }
     if constexpr (kSplit) {
@@ -874,12 +871,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
       store_row_stats<kFp8, kSoftCap>(p, batch, head, q_row, live, m_used, l, m_true, sink2, fixed_max);
     }
-    if (!kSplit && efirst < eend) {
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&bars->o_free[i]);
-      ++stepped;
-    }
+    tc_fence_before();  // O has been read, ahead of the next row's P
     if (kSplit) break;
     }
   }
