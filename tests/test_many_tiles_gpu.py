@@ -182,3 +182,30 @@ def test_rows_with_a_dead_tile_of_a_large_call(variant, q_len, kv_len):
     assert (whole["out"][at, h].float().cpu() - ro[0])[live].abs().max().item() <= bound
     assert (whole["lse"][at, h].cpu() - rlse[0])[live].abs().max().item() <= 1e-4  # fp32 sums of up to 1664 terms
     assert (whole["max"][at, h].cpu() - rmax[0])[live].abs().max().item() <= 1e-4
+
+
+@pytest.mark.parametrize("d_qk,d_v", [(256, 256), (192, 128), (128, 128)])
+@pytest.mark.parametrize("raised", [False, True])
+def test_the_largest_weight_of_a_row_is_not_rounded(d_qk, d_v, raised):
+  # Every row sees key r of its last 128 keys' first half with logit 0 (base 2) and key r of the second half with logit
+  # x < 8: under the maximum of the 128 the second weighs 1, under that of 64 keys the rounded 2^x.  `raised`: 128 keys
+  # of logit -20 come before, so that the maximum in use rises there.
+  n = 256 if raised else 128
+  g = torch.Generator().manual_seed(d_qk)
+  x = (0.5 + 7 * torch.rand(128, generator=g)).to(torch.bfloat16)
+  r = torch.arange(128)
+  dense = np.zeros((128, n), np.bool_)
+  dense[r, n - 128 + r % 64] = dense[r, n - 64 + r % 64] = True
+  dense[:, :n - 128] = True
+  q, k, v = torch.zeros(1, 1, 128, d_qk), torch.zeros(1, 1, n, d_qk), torch.zeros(1, 1, n, d_v)
+  q[..., 0], q[..., 1] = x.float(), 1.0
+  k[0, 0, n - 64:, 0], k[0, 0, :n - 128, 1] = 1.0, -20.0
+  v[0, 0, n - 64:] = 1.0
+  kernel = splash.make_splash_mha(mask_lib.NumpyMask(dense), q_seq_shards=1)
+  q, k, v = (t.to(DEV, torch.bfloat16) for t in (q, k, v))
+  out = kernel(q, k, v, logits_scale=math.log(2.0)).double().cpu()[0, 0]
+  kernel.check_errors()
+  w = torch.exp2(x.double())
+  exact = (w / (w + 1 + (n - 128) * 2.0 ** -20))[:, None]
+  # the output's rounding (2^-9 of a value below 1, half that above 1/2), and fp32 arithmetic on logits up to 20
+  assert (out - exact).abs().max().item() <= 2.0 ** -9 + 20 * 2.0 ** -23

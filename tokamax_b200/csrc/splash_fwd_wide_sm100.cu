@@ -19,15 +19,19 @@
 // A row's maximum in use passes from step to step: a warpgroup takes the maximum of its 64 scores, waits for the
 // maximum that the step before left in shared memory, raises it if it has to (by more than 2^8; O is then rescaled once
 // p v of the step before has completed, a rare wait) and leaves it for the step behind, all ahead of its
-// exponentials.  Each warpgroup sums its own steps' P, relative to the maximum it last saw; the two sums meet at the end.
+// exponentials.  An even step that raises it looks at the odd step's scores too: the first maximum of a row is that of
+// 128 keys, its largest weight 1 and not rounded, as in the 128-wide forward.  Each warpgroup sums its own steps' P,
+// relative to the maximum it last saw; the two sums meet at the end.
 // The schedule is the 128-wide forward's (rows = pairs of q tiles); a tile follows the entries in which it is live.
 //
 // What bounds it: the chain softmax -> q k^T -> softmax of a warpgroup's steps, 1400 cycles a step at (192, 128) and
 // 1800 at 256 for 640 and 1024 of tensor time, and 6000 cycles between two tiles.  Before (steps of 128 keys, both
 // warpgroups on one step, Q in shared memory, room for one step's K and V, a CTA a tile) -> this (us): causal 8192,
-// 16 / 8 heads, head dim 256: 681 -> 429; causal 4096, 32 heads, (192, 128): 275 -> 195.  Measured beside it: P over its
+// 16 / 8 heads, head dim 256: 681 -> 433; causal 4096, 32 heads, (192, 128): 275 -> 200.  (The first step of a
+// tile waits for the second one's scores: 5 us of each.  Raised by 64 keys alone, the maximum left the output 0.6 %
+// further from its value in 64 bits.)  Measured beside it, without that wait: P over its
 // scores in TMEM, rings of their own for K and V 441 / 209; the same with P in shared memory 475 / 206; that with q k^T
-// and p v issued by two threads 454 / 196.
+// and p v issued by two threads 454 / 196; this 429 / 195.
 #include <mutex>
 
 #include "splash_common.cuh"
@@ -51,6 +55,7 @@ struct WideFwdBarriers {
   uint64_t o_done;     // a tile's O is complete,
   uint64_t o_free;     //   and has been read
   uint64_t m_full[4];  // per lane quarter, one phase per step: the step's maximum in use is in shared memory
+  uint64_t x_full[4];  // per lane quarter, one phase per odd step: its scores' maximum is
   uint64_t l_full[4];  // per lane quarter, one phase per tile: both warpgroups' sums are
   uint32_t tmem_base;
   uint32_t abort_flag;
@@ -108,6 +113,7 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     }
     for (int i = 0; i < 4; ++i) {
       mbar_init(&bars->m_full[i], 1);
+      mbar_init(&bars->x_full[i], 1);
       mbar_init(&bars->l_full[i], 2);
     }
     mbar_init(&bars->o_done, 1);
@@ -317,6 +323,7 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
     float* m_row = xchg + r;                     // the row's maximum in use, as the last step left it
     float* l_row = xchg + kTile + r;             // [warpgroup]: its share of the row's sum
     float* true_row = xchg + 3 * kTile + r;      // [warpgroup]: the largest score it saw
+    float* x_row = true_row + kTile;             // until then: the maximum of an odd step's scores
     RingPos base{0, 0};     // stage at which the next tile begins
     uint32_t ph = 0;        // parity of this warpgroup's steps
     uint32_t stepped = 0;   // tiles with steps so far
@@ -456,6 +463,12 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
         const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
         m_true = fmaxf(m_true, mx);
         if (!fixed_max) {
+          float m_new = fmaxf(mx * c, kLogitFloor);
+          if (set == 1) {
+            *x_row = m_new;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->x_full[wq]);
+          }
           // the maximum in use of the step before (the steps of a tile are an even number: phase n of the barrier has
           // parity n & 1, and step n belongs to warpgroup n & 1)
           float m_in = m_used;
@@ -465,15 +478,25 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             if (!ok) break;
             m_in = *m_row;
           }
-          const float m_new = fmaxf(mx * c, kLogitFloor);
-          const bool need = m_new > m_in + kRescaleThreshold;
-          const float m_next = need ? m_new : m_in;
+          const bool raise = __any_sync(0xffffffffu, m_new > m_in + kRescaleThreshold);
+          float m_next = m_in;
+          if (raise) {
+            if (set == 0) {
+              // (an odd step leaves its scores' maximum, then waits for the even one's m_full: neither the phase before
+              // this one nor the one behind it can be in progress)
+              ok = mbar_wait(&bars->x_full[wq], ph, ab, 0xB80u);
+              ok = __all_sync(0xffffffffu, ok);
+              if (!ok) break;
+              m_new = fmaxf(m_new, *x_row);
+            }
+            m_next = fmaxf(m_in, m_new);
+          }
           *m_row = m_next;
           __syncwarp();
           if (lane == 0) mbar_arrive(&bars->m_full[wq]);
           if (m_next != m_used) l *= ex2(m_used - m_next);
           m_used = m_next;
-          if (__any_sync(0xffffffffu, need) && !first) {
+          if (raise && !first) {
             // O still receives p v of the step before, the other warpgroup's: wait for it before touching O
             RingPos other = last;
             other.advance(1, stages);
@@ -481,7 +504,7 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const float alpha = need ? ex2(m_in - m_next) : 1.f;
+            const float alpha = m_in != m_next ? ex2(m_in - m_next) : 1.f;
             for (int g = 0; g < o_groups; ++g) {
               uint32_t v[32];
               tmem_ld32(t_o + g * 32, v);
