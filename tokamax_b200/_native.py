@@ -10,13 +10,13 @@ from __future__ import annotations
 import ctypes as C
 import os
 import subprocess
+import sys
 import threading
 
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_PKG_DIR, "csrc")
 _LIB_DIR = os.path.join(_PKG_DIR, "lib")
 LIB_PATH = os.path.join(_LIB_DIR, "libsplash_b200.so")
-HOST_PATH = os.path.join(_LIB_DIR, "_splash_torch.so")
 
 SOURCES = (
     "splash_fwd_sm100.cu",
@@ -254,42 +254,71 @@ _lib = None
 _lock = threading.Lock()
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-  """Compiles the CUDA/C++ sources into ``lib/libsplash_b200.so`` (sm_100a), and its host side into
-  ``lib/_splash_torch.so``. Returns the former's path."""
-  srcs = [os.path.join(_CSRC, s) for s in SOURCES if os.path.exists(os.path.join(_CSRC, s))]
-  header = os.path.join(os.path.dirname(_PKG_DIR), "include", "splash_b200.h")
-  deps = srcs + [os.path.join(_CSRC, f) for f in os.listdir(_CSRC) if f.endswith(".cuh")] + [header]
+def _stale(path: str, sources) -> bool:
+  return not os.path.exists(path) or os.path.getmtime(path) < max(os.path.getmtime(d) for d in sources)
+
+
+def _compile(cmd, path: str, verbose: bool) -> None:
+  """Runs a compiler; its output takes the place of ``path`` in one step (other processes may be loading it)."""
   os.makedirs(_LIB_DIR, exist_ok=True)
+  part = f"{path}.{os.getpid()}"
+  res = subprocess.run([*cmd, "-o", part], capture_output=True, text=True)
+  if res.returncode != 0:
+    raise RuntimeError(f"{cmd[0]} failed:\n" + res.stdout + res.stderr)
+  os.replace(part, path)
+  if verbose:
+    print(res.stderr)
 
-  def stale(path, sources):
-    return force or not os.path.exists(path) or os.path.getmtime(path) < max(os.path.getmtime(d) for d in sources)
 
-  def run(cmd):
-    res = subprocess.run(cmd, capture_output=True, text=True)
-    if res.returncode != 0:
-      raise RuntimeError(f"{cmd[0]} failed:\n" + res.stdout + res.stderr)
-    if verbose:
-      print(res.stderr)
+_HEADER = os.path.join(os.path.dirname(_PKG_DIR), "include", "splash_b200.h")
 
-  host_src = os.path.join(_CSRC, HOST_SOURCE)
-  if stale(HOST_PATH, [host_src, header]):
-    import sysconfig
 
-    import torch
+def _library_sources():
+  srcs = [os.path.join(_CSRC, s) for s in SOURCES if os.path.exists(os.path.join(_CSRC, s))]
+  return srcs, srcs + [os.path.join(_CSRC, f) for f in os.listdir(_CSRC) if f.endswith(".cuh")] + [_HEADER]
 
+
+def build(force: bool = False, verbose: bool = False) -> str:
+  """Compiles the CUDA/C++ sources into ``lib/libsplash_b200.so`` (sm_100a). Returns its path.
+
+  Needs nvcc alone: the library serves programs without torch too (mask tables, the C ABI, XLA)."""
+  srcs, deps = _library_sources()
+  if force or _stale(LIB_PATH, deps):
+    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
+    _compile([nvcc, *(("-Xptxas", "-v") if verbose else ()), *NVCC_FLAGS, *srcs], LIB_PATH, verbose)
+  return LIB_PATH
+
+
+def host_path() -> str:
+  """Where the host side of torch calls lies: a file for each python, torch and C++ ABI that it is compiled against."""
+  import torch
+
+  abi = int(torch.compiled_with_cxx11_abi())
+  return os.path.join(_LIB_DIR, f"_splash_torch.{sys.implementation.cache_tag}-torch{torch.__version__}-abi{abi}.so")
+
+
+def build_host(force: bool = False, verbose: bool = False) -> str:
+  """Compiles ``csrc/splash_torch.cpp`` against the torch in use (g++, torch's and python's headers). Returns its path."""
+  import sysconfig
+
+  import torch
+
+  path = host_path()
+  src = os.path.join(_CSRC, HOST_SOURCE)
+  if force or _stale(path, [src, _HEADER]):
+    # it fills the structs of the header as it is now: the library that takes them must not be an older one
+    if os.path.exists(LIB_PATH) and _stale(LIB_PATH, [_HEADER]):
+      if _lib is not None:
+        raise RuntimeError(f"{LIB_PATH} is older than {_HEADER} and already loaded: rebuild it and start again")
+      build()
     root = os.path.dirname(torch.__file__)
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     include = (os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
                os.path.join(cuda, "include"), sysconfig.get_paths()["include"])
-    run([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{d}" for d in include),
-         "-o", HOST_PATH, host_src, "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10",
-         "-lc10_cuda"])
-  if stale(LIB_PATH, deps):
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    run([nvcc, *(("-Xptxas", "-v") if verbose else ()), *NVCC_FLAGS, "-o", LIB_PATH, *srcs])
-  return LIB_PATH
+    _compile([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{d}" for d in include), src,
+              "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"], path, verbose)
+  return path
 
 
 def lib() -> C.CDLL:
@@ -315,14 +344,16 @@ def host():
   """The module of ``csrc/splash_torch.cpp``, bound to the library (built first if absent)."""
   global _host
   if _host is None:
+    import importlib.util
+
+    path = host_path()
+    if not os.path.exists(path):
+      with _lock:
+        build_host()  # (before the library is loaded, where it is not yet)
     handle = lib()
     with _lock:
       if _host is None:
-        import importlib.util
-
-        if not os.path.exists(HOST_PATH):
-          build()
-        spec = importlib.util.spec_from_file_location("_splash_torch", HOST_PATH)
+        spec = importlib.util.spec_from_file_location("_splash_torch", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         module.bind_library(*(C.cast(getattr(handle, name), C.c_void_p).value for name in (
