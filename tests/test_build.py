@@ -71,3 +71,24 @@ def test_the_host_side_is_not_built_beside_an_older_library_in_use(monkeypatch, 
 
 def test_the_host_side_loads():
   assert {"bind_library", "forward", "backward"} <= set(dir(_native.host()))
+
+
+def test_errors_of_the_host_side_are_exceptions():
+  # in a process of its own: a module with another C++ runtime than torch's ends it
+  program = """
+import torch
+from tokamax_b200 import _native
+host = _native.host()
+t, f, rec = torch.zeros(1, 2, 128, 64, dtype=torch.bfloat16), torch.zeros(1, 2, 128), torch.zeros(4, dtype=torch.int32)
+huge = t[:, :1, :1].expand(1 << 20, 1 << 20, 1, 64)
+forward = lambda q, k, v: host.forward(q, k, v, None, None, None, None, None, rec, 0, 0, 1.0, 0.0, 0.0, 1, 1, 0)
+backward = lambda q, d_o: host.backward(q, t, t, t, f, d_o, None, None, None, rec, 0, 0, 0, 1.0, 0.0, True, 1, 1, 0, 0, 0)
+for call in (lambda: forward(t, t, t[0]), lambda: backward(t, t[0]), lambda: forward(huge, t, t), lambda: backward(huge, t)):
+  try:
+    call()
+  except RuntimeError as e:
+    print("RuntimeError", str(e).splitlines()[0])
+"""
+  out = subprocess.run([sys.executable, "-c", program], cwd=ROOT, capture_output=True, text=True)
+  assert out.returncode == 0, (out.returncode, out.stderr[-500:])
+  assert out.stdout.count("RuntimeError") == 4 and out.stdout.count("rank 4") == 2, out.stdout

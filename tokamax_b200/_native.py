@@ -318,7 +318,10 @@ def build_host(force: bool = False, verbose: bool = False) -> str:
                os.path.join(cuda, "include"), sysconfig.get_paths()["include"])
     _compile([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *(f"-I{d}" for d in include), src,
-              "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"], path, verbose)
+              "-L" + os.path.join(root, "lib"), "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda",
+              # torch's C++ runtime, named: a compiler that brings only a static one would put a second runtime into the
+              # process, and an exception that crosses from one to the other (out of memory, say) ends it
+              "-l:libstdc++.so.6"], path, verbose)
   return path
 
 
