@@ -306,6 +306,18 @@ def _on(device: torch.device):
   return _ALREADY if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
+def _in_class_of(source: torch.Tensor, result: torch.Tensor) -> torch.Tensor:
+  """``result`` in ``source``'s class, where that passes itself on to what torch makes of its tensors."""
+  cls = type(source)
+  if cls.__torch_function__ is torch._C._disabled_torch_function_impl or type(result) is cls:  # pylint: disable=protected-access
+    return result
+  return result.as_subclass(cls)
+
+
+def _plain(q, k, v, _tensor=torch.Tensor) -> bool:
+  return type(q) is _tensor and type(k) is _tensor and type(v) is _tensor
+
+
 def _address(struct_or_none) -> int:
   return 0 if struct_or_none is None else C.addressof(struct_or_none)
 
@@ -338,11 +350,14 @@ def splash_forward(kernel, q, k, v, q_seg, kv_seg, scale, sinks, max_logit, shar
   if q_seg is not None and not sched.row_end:  # device-built schedules are not filtered further
     sched, keep = _segment_schedule(sched, 0, q_seg, kv_seg, q.shape[2], k.shape[2])  # (`keep`: until the launch below)
   sinks_f32 = None if sinks is None else sinks.detach().to(torch.float32).contiguous()
+  given = None if _plain(q, k, v) else (q, k, v)
   status, q, k, v, o, lse, max_logits = _native.host().forward(
       q, k, v, q_seg, kv_seg, tables.q_sequence, sinks_f32, max_logit, tables.error_record, C.addressof(sched),
       C.addressof(kernel._mask_fn), scale, max(kernel.mask_value, -3.0e38),  # pylint: disable=protected-access
       float(kernel.config.attn_logits_soft_cap or 0.0), kernel.head_shards, tables.q_shards, _address(o_peer))
   _native.check(status, "splash_fwd")
+  if given is not None:
+    q, k, v, o = map(_in_class_of, (*given, given[0]), (q, k, v, o))
   return q, k, v, o, lse, max_logits, sinks_f32
 
 
@@ -405,6 +420,8 @@ def splash_backward(kernel: "SplashAttentionKernel", q, k, v, o, lse, d_o, q_seg
       float(kernel.config.attn_logits_soft_cap or 0.0), fused, kernel.head_shards, tables.q_shards,
       *map(_address, peers if peers is not None else (None, None, None)))
   _native.check(status, "splash_bwd")
+  if not _plain(q, k, v):
+    dq, dk, dv = map(_in_class_of, (q, k, v), (dq, dk, dv))
   if not with_di:
     return dq, dk, dv, None
   n = q.shape[0] * q.shape[1] * q.shape[2]
