@@ -11,6 +11,7 @@ import pytest
 import torch
 
 from oracle import attention_ref
+from tokamax_b200 import _native
 from tokamax_b200 import fp8
 from tokamax_b200 import splash_attention_kernel as splash
 from tokamax_b200 import splash_attention_mask as mask_lib
@@ -209,3 +210,89 @@ def test_the_largest_weight_of_a_row_is_not_rounded(d_qk, d_v, raised):
   exact = (w / (w + 1 + (n - 128) * 2.0 ** -20))[:, None]
   # the output's rounding (2^-9 of a value below 1, half that above 1/2), and fp32 arithmetic on logits up to 20
   assert (out - exact).abs().max().item() <= 2.0 ** -9 + 20 * 2.0 ** -23
+
+
+# 286 tiles and more, as above.  A fixed maximum drops the exchange of maxima between the warpgroups; a sink is counted once
+@pytest.mark.parametrize("d_qk,d_v", [(192, 128), (256, 256)])
+@pytest.mark.parametrize("fixed,sinks", [(True, False), (True, True), (False, True)])
+def test_heads_above_128_with_a_fixed_maximum_or_sinks_of_a_large_call(d_qk, d_v, fixed, sinks):
+  b, hkv, group, s = 2, 11, 2, 1664
+  g = torch.Generator(device=DEV).manual_seed(d_qk)
+  mk = lambda h, d: torch.randn(b, h, s, d, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v = mk(hkv * group, d_qk), mk(hkv, d_qk), mk(hkv, d_v)
+  sink = torch.randn(hkv * group, generator=g, device=DEV) if sinks else None
+  top = 6 + torch.rand(hkv * group, generator=g, device=DEV) if fixed else None
+  kernel = splash.make_splash_mha(_mask("causal", s), q_seq_shards=1, save_residuals=True)
+
+  def run(heads, q, k, v):
+    with torch.no_grad():
+      out, res = kernel(q, k, v, None, sink[heads] if sinks else None, max_logit_value=top[heads] if fixed else None,
+                        logits_scale=1 / math.sqrt(d_qk))
+    kernel.check_errors()
+    return {"out": out, "lse": res["logsumexp"], "max": res["max_logits"]}
+
+  whole = run(slice(None), q, k, v)
+  for h in range(0, hkv, 5):
+    heads = slice(h * group, (h + 1) * group)
+    part = run(heads, q[:, heads].contiguous(), k[:, h:h + 1].contiguous(), v[:, h:h + 1].contiguous())
+    for name in part:
+      assert torch.equal(whole[name][:, heads], part[name]), (name, h)
+  h = hkv * group - 1
+  ro, rlse, _ = attention_ref.attention_reference(q[1, h:].cpu(), k[1, -1:].cpu(), v[1, -1:].cpu(), np.tril(np.ones((s, s), np.bool_)),
+                                                  scale=1 / math.sqrt(d_qk), sinks=sink[h:].cpu() if sinks else None)
+  # P and the output are rounded to 8 bits, half an ulp each
+  assert (whole["out"][1, h].float().cpu() - ro[0]).abs().max().item() <= 2.0 ** -8 * v[1, -1].float().abs().max().item()
+  assert (whole["lse"][1, h].cpu() - rlse[0]).abs().max().item() <= 1e-4
+
+
+@pytest.mark.parametrize("d_qk,d_v", [(128, 128), (64, 64), (192, 128), (256, 256)])
+def test_device_masks_of_a_large_call(d_qk, d_v):
+  # schedules built on the device (an end for each row of each batch row) against the host's tables; the fused backward
+  # up to 128, and its dq against the repeatable one
+  b, hkv, group, s = 2, 11, 2, 1664
+  g = torch.Generator(device=DEV).manual_seed(d_qk)
+  mk = lambda h, d: torch.randn(b, h, s, d, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v, do = mk(hkv * group, d_qk), mk(hkv, d_qk), mk(hkv, d_v), mk(hkv * group, d_v)
+  dense = _pairs_with_a_dead_tile(s)
+  dense[:, 300:900] &= np.random.default_rng(d_qk).random((s, 600)) < 0.5
+  kernels = [splash.make_dynamic_splash_mha(torch.from_numpy(dense).to(DEV), save_residuals=True),
+             splash.make_splash_mha(mask_lib.NumpyMask(dense), q_seq_shards=1, save_residuals=True),
+             splash.make_splash_mha(mask_lib.NumpyMask(dense), q_seq_shards=1, save_residuals=True, repeatable_dq=True)]
+  device, host, repeatable = (_run(kernel, q, k, v, do, None, 1 / math.sqrt(d_qk)) for kernel in kernels)
+  for kernel in kernels:
+    kernel.check_errors()
+  for name in ("out", "lse", "dk", "dv") if d_qk <= 128 else device:
+    assert torch.equal(device[name], host[name]), name
+  for name in ("dq", "dk", "dv"):
+    want = repeatable[name].float()
+    # the same products summed in another order (fp32), rounded to bf16 where they differ in the last bits
+    for other in (device, host):
+      assert ((other[name].float() - want).norm() / want.norm()).item() <= 1e-3, name
+
+
+def test_peer_outputs_of_a_large_call():
+  # rows that CTAs take over, stored twice: in the call's own tensor and in the buffer of the rank that owns them
+  b, hq, hkv, s, d, world, rank = 2, 44, 22, 1536, 128, 2, 1
+  g = torch.Generator(device=DEV).manual_seed(5)
+  mk = lambda h: torch.randn(b, h, s, d, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v, do = mk(hq), mk(hkv), mk(hkv), mk(hq)
+  kernel = splash.make_splash_mha(_mask("causal", s), q_seq_shards=1)
+  s_loc = s // world
+
+  def receive(heads):
+    bufs = [torch.full((b, heads * world, s_loc, d), 7.0, dtype=torch.bfloat16, device=DEV) for _ in range(world)]
+    ptrs = torch.tensor([t.data_ptr() for t in bufs], dtype=torch.int64, device=DEV)
+    po = _native.SplashPeerOutput()
+    po.ptrs, po.base_bytes, po.rows_per_peer = ptrs.data_ptr(), 0, s_loc
+    po.stride_b, po.stride_h, po.stride_s, po.head0 = heads * world * s_loc * d, s_loc * d, d, rank * heads
+    return bufs, ptrs, po
+
+  recv = [receive(h) for h in (hq, hq, hkv, hkv)]
+  _, _, _, o, lse, _, _ = splash.splash_forward(kernel, q, k, v, None, None, 0.09, None, None, 0, o_peer=recv[0][2])
+  dq, dk, dv, _ = splash.splash_backward(kernel, q, k, v, o, lse, do, None, None, 0.09, 0, peers=tuple(r[2] for r in recv[1:]))
+  kernel.check_errors()
+  assert torch.equal(o, kernel(q, k, v, logits_scale=0.09))
+  for (bufs, _, _), local, heads in zip(recv, (o, dq, dk, dv), (hq, hq, hkv, hkv)):
+    for peer in range(world):
+      assert torch.equal(bufs[peer][:, rank * heads:], local[:, :, peer * s_loc:(peer + 1) * s_loc])
+      assert (bufs[peer][:, :rank * heads] == 7.0).all()
