@@ -77,7 +77,7 @@ def test_row_parts_refuses_what_it_cannot_read():
   assert row_parts(mask, 0, 8, 4, 2048, 2048, clusters=CAPACITIES[0]) == (-1, -1)
   assert row_parts(mask, 1, 8, 4, 2000, 2048, clusters=CAPACITIES[0]) == (-1, -1)
   assert row_parts(mask, 1, 8, 4, 2048, 2048, clusters=[0] * 9) == (-1, -1)
-  assert row_parts(mask, 1, 8, 4, 2048, 2048, d=192, clusters=CAPACITIES[0]) == (1, 1)  # two-panel kernels
+  assert row_parts(mask, 1, 8, 4, 2048, 2048, d=192, clusters=CAPACITIES[0]) == (1, 1)  # the kernels above 128
   kernel = splash.make_splash_mha(mask, q_seq_shards=1)
   assert kernel.head_shards == 1 and kernel.head_shard(4).head_shard(2).head_shards == 8
   for bad in (0, -1, 1 << 16):

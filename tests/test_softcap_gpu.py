@@ -28,7 +28,7 @@ def _rel(a, ref):
                                             (4.0, 1 / 16, (256, 256))])
 @pytest.mark.parametrize("kind", ["causal", "local_segments"])
 def test_soft_cap_forward_backward(cap, scale, dims, kind):
-  """(128, 128), and the head dims above 128 that run the two-panel kernels."""
+  """(128, 128), and the head dims above 128 that run kernels of their own."""
   b, hq, hkv, s = 1, 4, 2, 512
   d_qk, d_v = dims
   g = torch.Generator().manual_seed(int(cap * 10) + len(kind) + d_qk)

@@ -36,8 +36,8 @@
 // What bounds it: the shared-memory pipe (operand reads of the 128 x 64 score MMAs, the streamed tiles coming in,
 // statistics) together with the tensor core, at 1500 (dq), 1950 (dkv) cycles a step for (192, 128), 2150 (dq), 2250
 // (dk), 1300 (dv) for 256.  Measured, three passes over 128 x 128 tiles that a CTA each computed one after the
-// other -> this (us): causal 4096, 32 heads, (192, 128): dq 394 -> 235, dk and dv 721 -> 317; causal 8192, 16 / 8
-// heads, head dim 256: dq 762 -> 612, dk 909 -> 641, dv 594 -> 393.
+// other -> this (us, a pause before each pass): causal 4096, 32 heads, (192, 128): dq 403 -> 244, dk and dv 727 -> 323;
+// causal 8192, 16 / 8 heads, head dim 256: dq 781 -> 636, dk 925 -> 649, dv 603 -> 399.
 #include <mutex>
 
 #include "splash_common.cuh"

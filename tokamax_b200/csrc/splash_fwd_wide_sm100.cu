@@ -27,7 +27,7 @@
 // What bounds it: the chain softmax -> q k^T -> softmax of a warpgroup's steps, 1400 cycles a step at (192, 128) and
 // 1800 at 256 for 640 and 1024 of tensor time, and 6000 cycles between two tiles.  Before (steps of 128 keys, both
 // warpgroups on one step, Q in shared memory, room for one step's K and V, a CTA a tile) -> this (us): causal 8192,
-// 16 / 8 heads, head dim 256: 681 -> 433; causal 4096, 32 heads, (192, 128): 275 -> 200.  (The first step of a
+// 16 / 8 heads, head dim 256: 671 -> 431; causal 4096, 32 heads, (192, 128): 272 -> 203.  (The first step of a
 // tile waits for the second one's scores: 5 us of each.  Raised by 64 keys alone, the maximum left the output 0.6 %
 // further from its value in 64 bits.)  Measured beside it, without that wait: P over its
 // scores in TMEM, rings of their own for K and V 441 / 209; the same with P in shared memory 475 / 206; that with q k^T

@@ -1,7 +1,8 @@
 // The host side of a call in native code: reads the tensors' addresses, sizes and strides, allocates the results
 // and fills the C ABI's argument structs (include/splash_b200.h), which python did field by field through ctypes.
-// A forward spent 20 us of its host time there and a backward 35; they take 6 and 8 here.  The autograd function, the
-// checks of arguments and the schedules stay where they were, in splash_attention_kernel.py.
+// forward() takes 12 us and backward() 25 (three launches), launches included; a whole forward pass of 256 tokens went
+// from 39 to 21 us, a training step of 2 x 1024 from 176 to 114.  The autograd function, the checks of arguments and the
+// schedules stay where they were, in splash_attention_kernel.py.
 #include <torch/csrc/utils/pybind.h>
 #include <torch/csrc/Exceptions.h>
 

@@ -39,7 +39,7 @@ partial = functools.partial
 
 _TILE = 128
 _HEAD_DIM = 128
-_MAX_HEAD_DIM = 256  # above _HEAD_DIM: the kernels that work on two 128-column panels
+_MAX_HEAD_DIM = 256  # above _HEAD_DIM: kernels of their own
 
 
 def get_kernel_name(is_mqa: bool, save_residuals: bool, is_segmented: bool, phase: str) -> str:
@@ -589,7 +589,7 @@ class SplashAttentionKernel:
     # read in place: the kernels' TMA boxes reach past the end of a row and get zeros there, which
     # change neither q k^T nor p v, and only the real columns of outputs and gradients are stored.
     # No copy is made.  Head dims above 128, up to 256 (the reference's (192, 128) and (256, 256)),
-    # run kernels that work on two 128-column panels.
+    # run kernels of their own, in steps of 64 rows.
     d_qk, d_v = q.shape[-1], v.shape[-1]
     if k.shape[-1] != d_qk:
       raise ValueError(f"q and k head dims differ: {d_qk} vs {k.shape[-1]}")
