@@ -103,6 +103,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const 
   return false;
 }
 
+// Before a CTA leaves whose waits have run out: its copies, MMAs and answers from cluster launch control may still be in
+// flight towards shared memory and TMEM that are another CTA's next.  They land within microseconds.
+constexpr long long kDrainCycles = 1000000ll;  // ~0.5 ms
+__device__ __forceinline__ void drain_after_give_up(const volatile uint32_t* cta_flag) {
+  if (*cta_flag == 0u) return;
+  const long long start = clock64();
+  while (clock64() - start < kDrainCycles) {
+  }
+}
+
 // ----------------------------------------------------------------------------------------
 // thread-block clusters: barrier over all threads of the cluster, loads from a peer CTA's shared memory
 // ----------------------------------------------------------------------------------------

@@ -457,6 +457,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   __syncthreads();
   if (warp == 9) {
     __syncwarp();
+    drain_after_give_up(&bars->abort_flag);
     tmem_dealloc(tmem, 512);
   }
 }
@@ -1052,6 +1053,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   __syncthreads();
   if (warp == kDkvMmaWarp) {
     __syncwarp();
+    drain_after_give_up(&bars->abort_flag);
     tmem_dealloc(tmem, 512);
   }
 }

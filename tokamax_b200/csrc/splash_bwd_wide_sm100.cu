@@ -683,6 +683,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
   __syncthreads();
   if (warp == kWideMmaWarp) {
     __syncwarp();
+    drain_after_give_up(&bars->abort_flag);
     tmem_dealloc(tmem, 512);
   }
 }

@@ -500,6 +500,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   __syncthreads();
   if (warp == 9) {
     __syncwarp();
+    drain_after_give_up(&bars->abort_flag);
     tmem_dealloc(tmem, 512);
   }
 }

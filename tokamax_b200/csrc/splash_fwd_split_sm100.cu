@@ -434,6 +434,7 @@ splash_fwd_split_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_c
   __syncthreads();
   if (warp == 9) {
     __syncwarp();
+    drain_after_give_up(&bars->abort_flag);
     tmem_dealloc(tmem, 512);
   }
 }
