@@ -204,6 +204,19 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, 
       : "memory");
 }
 
+// Bulk reduction shared -> global: adds `bytes` of fp32 to what is there (both addresses 16-byte aligned, size a multiple of
+// 16).  A bulk group of its own; the shared memory may be written again behind bulk_wait_read().
+__device__ __forceinline__ void bulk_reduce_add(float* gmem_dst, const void* smem_src, uint32_t bytes) {
+  asm volatile(
+      "cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;\n\t"
+      "cp.async.bulk.commit_group;"
+      :
+      : "l"(gmem_dst), "r"(smem_u32(smem_src)), "r"(bytes)
+      : "memory");
+}
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 __device__ __forceinline__ void tma_store_4d(const void* tmap, const void* smem_src, int c0,
                                              int c1, int c2, int c3) {
   asm volatile(
@@ -430,13 +443,6 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
-}
-
-// Four-wide fp32 reduction into global memory (16-byte aligned address); no return value, so the
-// issuing warp does not wait for it.
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d)
-               : "memory");
 }
 
 // Register reallocation between warpgroups (all four warps of a warpgroup must execute it).

@@ -41,7 +41,8 @@ struct BwdParams {
   float scale, scale_log2;
   uint32_t* err;
   // fused form only: fp32 dQ image, one 128 x 128 tile per (batch, q head, q tile), each tile
-  // stored as [col / 4][row][col % 4] so that one warp's vector red covers 512 contiguous bytes
+  // stored as [col / 32][row / 32][col / 4 % 8][row % 32][col % 4]: a warp's 32 rows (TMEM lanes) of 32 columns
+  // are 4 KiB in one piece
   float* dq_acc;
 };
 

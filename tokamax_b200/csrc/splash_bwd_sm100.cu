@@ -13,7 +13,7 @@
 // five matmuls per live block (splash_attention_kernel.py:1234-1459, dq partials :1395-1410
 // reduced at :1864): the dkv kernel also forms dQ_partial = dS K for every (q tile, kv tile) pair
 // it visits, from the dS^T tile it already holds in shared memory, and adds it into an fp32 dQ
-// image in global memory (vector red.add from four drain warps); a last HBM-bound pass scales
+// image in global memory (bulk reductions, sent by eight drain warps); a last HBM-bound pass scales
 // and casts that image to bf16.  S and dP are then computed once per pair instead of twice (5
 // tile-MMAs instead of 7).  dK / dV stay atomic-free and repeatable; dQ's fp32 sums arrive in an
 // order that varies from run to run, so its last bits are not repeatable in this form.
@@ -49,8 +49,8 @@ struct DeltaParams {
   float* nlse2;      // [B, Hq, Sq]  -lse * log2(e): the exponent offset the MMA kernels subtract
   int q_heads, q_len;
   int d_v;  // columns of o / do
-  // fused backward: the fp32 dQ image (one 128 x 128 tile per 128 rows, [col / 4][row][col % 4])
-  // that the reds of the dkv kernel add into; this pass clears it on the way.  nullptr: none.
+  // fused backward: the fp32 dQ image (one 128 x 128 tile per 128 rows, see BwdParams::dq_acc)
+  // that the reductions of the dkv kernel add into; this pass clears it on the way.  nullptr: none.
   float* dq_image;
 };
 
@@ -85,16 +85,13 @@ __global__ void __launch_bounds__(256) splash_delta_kernel(const DeltaParams p) 
       }
     }
     if (c0 == 0 && p.dq_image != nullptr) {
-      // The block's 64 rows are half of one image tile: for each of the 32 four-column groups a run of
-      // 64 rows x 16 bytes.  256 threads x 8 stores of 16 bytes, issued under the loads.
-      float* tile = p.dq_image + (first / kTile) * (int64_t)(kTile * kHeadDim) + (first % kTile) * 4;
+      // The block's 64 rows are half of one image tile: in each 32-column chunk a run of 8 KiB.  256 threads x 8 stores
+      // of 16 bytes, issued under the loads.
+      float* tile = p.dq_image + (first / kTile) * (int64_t)(kTile * kHeadDim) + (first % kTile) * 32;
       const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int idx = i * 256 + threadIdx.x;  // 0 .. 2047: (column group, row) of the half tile
-        const int cg = idx >> 6, r = idx & 63;
-        *reinterpret_cast<uint4*>(tile + (int64_t)cg * (kTile * 4) + r * 4) = zero;
-      }
+      for (int i = 0; i < 8; ++i)
+        *reinterpret_cast<uint4*>(tile + (i >> 1) * (kTile * 32) + (((i & 1) * 256 + (int)threadIdx.x) << 2)) = zero;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -471,15 +468,24 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 constexpr int kDkvThreads = 640;
 constexpr int kDkvTmaWarp = 16;
 constexpr int kDkvMmaWarp = 17;
-// Fused form: warps 20-23 drain the per-pair dQ tile from TMEM into the fp32 image.  768 threads
-// start at 80 registers.  Registers live in four banks, one per scheduler, and warp w draws on bank
-// w mod 4, so every bank serves four compute warps, one warp of the issuing warpgroup and one
-// drain warp: 6 x 80 at launch, 4 x 88 + 80 + 48 after the hand-over (the sum per bank has to stay
-// at what the launch gave it, or the increase never completes).
-constexpr int kFusedThreads = 768;
+// Fused form: warps 20-27 drain the per-pair dQ tile from TMEM, each 32 lanes of 64 columns: half of that goes through
+// 4 KiB of shared memory at once, the other half waits in registers until those have been read, so that the TMEM columns
+// are free for the next step's dP^T after two loads.  The image is added to by bulk reductions: an SM sends
+// 25 bytes a cycle whichever way (64 KiB a step: 2570 cycles; 3100 beside the step's loads), but vector reds from
+// registers, which four warps issued before, stand in the queue that every mbarrier and shared-memory access of the SM goes
+// through (the issuing thread saw a finished barrier 1400 cycles late).  4 x 8192, 32 / 8 heads: 5500 -> 4600 cycles a
+// step of a CTA in mid-grid, whole pass 7.63 -> 7.35 ms; 8 x 16384, 16 heads, window 4096: 6.99 -> 6.68.  The staging
+// takes the slot that a second dO tile had: dO(n) is last read by dV(n), two thousand cycles before dP^T(n + 1) wants the
+// next one.  896 threads start at 72 registers.  Registers live in four banks, one per scheduler, and warp w draws on bank
+// w mod 4, so every bank serves four compute warps, one warp of the issuing warpgroup and two drain warps: 7 x 72 at
+// launch, 4 x 88 + 56 + 2 x 48 after the hand-over (the sum per bank has to stay at what the launch gave it, or the
+// increase never completes).
+constexpr int kFusedThreads = 896;
 constexpr int kDkvDrainWarp = 20;
 constexpr int kFusedComputeRegs = 88;
+constexpr int kFusedIssueRegs = 56;
 constexpr int kFusedDrainRegs = 48;
+constexpr int kDqBlockBytes = 32 * 32 * 4;  // a drain warp's share of 32 columns
 constexpr int kDqTileFloats = kTile * kHeadDim;
 // No register hand-over here: at 640 threads every thread gets 96 registers, which the compute
 // warps fit in, and the MMA / TMA threads keep their loop state in registers instead of spilling
@@ -555,6 +561,12 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + kv_tile] : p.row_ptr[kv_tile + 1];
   const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
   const int n_ent = eend - ebeg;
+  // Q and dO of step n in the ring: slots 0, 2 and 1, 3 by turns.  The fused form parks dQ in slot 3: dO then keeps to
+  // slot 1, whose two halves take turns where dO has one half.
+  const bool one_do = kFuseDq && p.d_v > 64;
+  auto do_bar = [&](uint32_t n) { return one_do ? 1u : 1u + 2u * (n & 1u); };
+  auto do_phase = [&](uint32_t n) { return (one_do ? n : n >> 1) & 1u; };
+  auto do_offset = [&](uint32_t n) { return kTileBytes + (one_do ? 0u : (n & 1u) * (kFuseDq ? kHalfBytes : 2 * kTileBytes)); };
   // steps of this CTA: (q head g of the group, entry e) pairs in that order
   const PartWalk<kSplit> walk(entries, ebeg, eend, p.n_split);
   const int offset0 = walk.offset((int)rank);  // of head 0's part; a tile less for each further head
@@ -589,7 +601,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_init(&bars->ds_free, 1);
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->dq_full, 1);
-    mbar_init(&bars->dq_free, 4);
+    mbar_init(&bars->dq_free, kFusedThreads / 32 - kDkvDrainWarp);
     mbar_fence_init();
   }
   __syncthreads();
@@ -622,45 +634,59 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
   if (kFuseDq && warp >= kDkvDrainWarp) {
     // ------------------------------------------------------------------ dQ drain (fused form)
-    // Thread = q row of the pair's dQ tile (TMEM lane) x all 128 head-dim columns, read 32 at a
-    // time and added to the fp32 image with four-wide reds.  The TMEM columns are handed back
-    // to the issuing thread as soon as the last load has completed, before the last reds go out.
+    // Thread = q row of the pair's dQ tile (TMEM lane) x 64 head-dim columns, 32 at a time.
     setmaxnreg_dec<kFusedDrainRegs>();
     const int wq = warp & 3;
-    const int r = wq * 32 + lane;
-    const uint32_t t_dq = tmem + ((uint32_t)(wq * 32) << 16) + kTile;
+    const int half = (warp - kDkvDrainWarp) >> 2;
+    const bool two = p.d_qk > 64;  // columns 64 half .. + 63; with at most 64 of them in all, 32 half .. + 31
+    const int chunk = two ? 2 * half : half;
+    const uint32_t t_dq = tmem + ((uint32_t)(wq * 32) << 16) + kTile + chunk * 32;
+    uint8_t* stage = ring + 3 * kTileBytes + (warp - kDkvDrainWarp) * kDqBlockBytes;
     const int n_q_tiles = p.q_len / kTile;
     bool ok = true;
     uint32_t n = 0;
+    uint32_t v[32];
+    // v -> the image: through the warp's own 4 KiB of shared memory, once what it held before has been read
+    auto park = [&]() {
+      if (lane == 0) bulk_wait_read();
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint4*>(stage + j * 512 + lane * 16) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    };
+    auto send = [&](float* dst) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) bulk_reduce_add(dst, stage, kDqBlockBytes);
+    };
     for (int g = 0, o = offset0; n < (uint32_t)n_steps && ok; ++g, o = offset_behind(o)) {
       const int head = kv_head * group + g;
-      float* head_base = p.dq_acc + ((int64_t)batch * p.q_heads + head) * n_q_tiles * (int64_t)kDqTileFloats + r * 4;
+      float* head_base = p.dq_acc + ((int64_t)batch * p.q_heads + head) * n_q_tiles * (int64_t)kDqTileFloats +
+                         (chunk * 4 + wq) * (kDqBlockBytes / 4);
       for (int e = walk.first(o); e < eend && ok; e = walk.next(e), ++n) {
         float* dst = head_base + (int64_t)entries[e].x * kDqTileFloats;
         ok = mbar_wait(&bars->dq_full, n & 1u, ab, 0x3600u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const int last = p.d_qk <= 64 ? 1 : 3;  // 32-column chunks beyond dq's columns hold nothing
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (c > last) break;
-          uint32_t v[32];
-          tmem_ld32(t_dq + c * 32, v);
+        tmem_ld32(t_dq, v);
+        tmem_ld_wait();
+        if (two) {
+          park();
+          tmem_ld32(t_dq + 32, v);
+          send(dst);
           tmem_ld_wait();
-          if (c == last) {
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->dq_free);
-          }
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            red_add_v4(dst + (c * 8 + j) * (kTile * 4), __uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                       __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars->dq_free);
+        park();
+        send(two ? dst + 4 * (kDqBlockBytes / 4) : dst);
       }
     }
+    if (lane == 0) bulk_wait_all();
   } else if (warp >= 16) {
+   if constexpr (kFuseDq) setmaxnreg_dec<kFusedIssueRegs>();
    if (warp == kDkvTmaWarp) {
     if (n_steps > 0 && elect_one()) {
       tma_prefetch_desc(&tm_q);
@@ -675,30 +701,35 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       mbar_arrive_expect_tx(&bars->stat_full[1], v2 ? kTileBytes : kHalfBytes);
       tma_load_4d(v_smem, &tm_v, &bars->stat_full[1], 0, kv_tile * kTile, kv_head, batch);
       if (v2) tma_load_4d(v_smem + kHalfBytes, &tm_v, &bars->stat_full[1], 64, kv_tile * kTile, kv_head, batch);
-      uint32_t it = 0;
+      uint32_t n = 0;
       bool ok = true;
-      for (int g = 0, o = offset0; it < 2u * (uint32_t)n_steps && ok; ++g, o = offset_behind(o)) {
+      for (int g = 0, o = offset0; n < (uint32_t)n_steps && ok; ++g, o = offset_behind(o)) {
         const int head = kv_head * group + g;
         const int64_t stat_base = ((int64_t)batch * p.q_heads + head) * p.q_len;
-        for (int e = walk.first(o); e < eend && ok; e = walk.next(e)) {
+        for (int e = walk.first(o); e < eend && ok; e = walk.next(e), ++n) {
           const int qt = entries[e].x;
-          for (int which = 0; which < 2 && ok; ++which, ++it) {
-            const uint32_t s = it % kBwdStages;
-            ok = mbar_wait(&bars->ring_empty[s], ((it / kBwdStages) & 1u) ^ 1u, ab, 0x3100u + s);
+          {
+            const uint32_t s = 2u * (n & 1u);
+            ok = mbar_wait(&bars->ring_empty[s], ((n >> 1) & 1u) ^ 1u, ab, 0x3100u + s);
             if (!ok) break;
             uint8_t* dst = ring + s * kTileBytes;
-            const CUtensorMap* tm = which == 0 ? &tm_q : &tm_do;
-            const bool two = which == 0 ? qk2 : v2;
-            const uint32_t tile_bytes = two ? kTileBytes : kHalfBytes;
-            if (kSplit && which == 0) bars->step[s / 2] = entries[e];
-            mbar_arrive_expect_tx(&bars->ring_full[s], which == 0 ? tile_bytes + 2 * kTile * 4 : tile_bytes);
-            tma_load_4d(dst, tm, &bars->ring_full[s], 0, qt * kTile, head, batch);
-            if (two) tma_load_4d(dst + kHalfBytes, tm, &bars->ring_full[s], 64, qt * kTile, head, batch);
-            if (which == 0) {  // the step's statistics ride on the Q slot's barrier
-              float* sdst = stats + (s / 2) * 2 * kTile;
-              bulk_load(sdst, p.nlse2 + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
-              bulk_load(sdst + kTile, p.delta + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
-            }
+            if (kSplit) bars->step[s / 2] = entries[e];
+            mbar_arrive_expect_tx(&bars->ring_full[s], (qk2 ? kTileBytes : kHalfBytes) + 2 * kTile * 4);
+            tma_load_4d(dst, &tm_q, &bars->ring_full[s], 0, qt * kTile, head, batch);
+            if (qk2) tma_load_4d(dst + kHalfBytes, &tm_q, &bars->ring_full[s], 64, qt * kTile, head, batch);
+            // the step's statistics ride on the Q slot's barrier
+            float* sdst = stats + (s / 2) * 2 * kTile;
+            bulk_load(sdst, p.nlse2 + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
+            bulk_load(sdst + kTile, p.delta + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
+          }
+          {
+            const uint32_t s = do_bar(n);
+            ok = mbar_wait(&bars->ring_empty[s], do_phase(n) ^ 1u, ab, 0x3100u + s);
+            if (!ok) break;
+            uint8_t* dst = ring + do_offset(n);
+            mbar_arrive_expect_tx(&bars->ring_full[s], v2 ? kTileBytes : kHalfBytes);
+            tma_load_4d(dst, &tm_do, &bars->ring_full[s], 0, qt * kTile, head, batch);
+            if (v2) tma_load_4d(dst + kHalfBytes, &tm_do, &bars->ring_full[s], 64, qt * kTile, head, batch);
           }
         }
       }
@@ -712,10 +743,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const uint32_t k_addr = smem_u32(k_smem), v_addr = smem_u32(v_smem), ds_addr = smem_u32(ds_smem);
       const uint32_t ring_addr = smem_u32(ring);
       const uint32_t t_st = tmem, t_dpt = tmem + kTile, t_dk = tmem + 2 * kTile, t_dv = tmem + 3 * kTile;
-      auto slot_addr = [&](uint32_t it) { return ring_addr + (it % kBwdStages) * kTileBytes; };
-      auto ring_wait = [&](uint32_t it, uint32_t tag) {
-        return mbar_wait(&bars->ring_full[it % kBwdStages], (it / kBwdStages) & 1u, ab, tag);
-      };
+      auto q_addr = [&](uint32_t n) { return ring_addr + 2 * (n & 1u) * kTileBytes; };
+      auto do_addr = [&](uint32_t n) { return ring_addr + do_offset(n); };
+      auto q_wait = [&](uint32_t n, uint32_t tag) { return mbar_wait(&bars->ring_full[2 * (n & 1u)], (n >> 1) & 1u, ab, tag); };
+      auto do_wait = [&](uint32_t n, uint32_t tag) { return mbar_wait(&bars->ring_full[do_bar(n)], do_phase(n), ab, tag); };
       // D = A B^T with both operands K-major (head_dim contiguous), K = head_dim
       auto issue_score = [&](uint32_t d, SmemDesc da, uint32_t b0, int nk) {
         const SmemDesc db = make_smem_desc_sw128(b0, 16, 1024);
@@ -734,19 +765,19 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const SmemDesc ds_mn_desc = make_smem_desc_sw128(ds_addr, kHalfBytes, 1024);
       const SmemDesc k_mn_desc = make_smem_desc_sw128(k_addr, kHalfBytes, 1024);
       bool ok = mbar_wait(&bars->stat_full[0], 0, ab, 0x3200u) && mbar_wait(&bars->stat_full[1], 0, ab, 0x3201u);
-      ok = ok && ring_wait(0, 0x3210u);
+      ok = ok && q_wait(0, 0x3210u);
       if (ok) {
-        issue_score(t_st, k_desc, slot_addr(0), p.nk_qk);
+        issue_score(t_st, k_desc, q_addr(0), p.nk_qk);
         tc_commit(&bars->st_full);
       }
-      ok = ok && ring_wait(1, 0x3211u);
+      ok = ok && do_wait(0, 0x3211u);
       if (ok) {
-        issue_score(t_dpt, v_desc, slot_addr(1), p.nk_v);
+        issue_score(t_dpt, v_desc, do_addr(0), p.nk_v);
         tc_commit(&bars->dpt_full);
       }
       for (int n = 0; n < n_steps && ok; ++n) {
         const uint32_t ph = (uint32_t)n & 1u;
-        const uint32_t q_slot = slot_addr(2 * n), do_slot = slot_addr(2 * n + 1);
+        const uint32_t q_slot = q_addr(n), do_slot = do_addr(n);
         const bool more = n + 1 < n_steps;
         ok = mbar_wait(&bars->p_full, ph, ab, 0x3220u);
         if (!ok) break;
@@ -758,10 +789,11 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         for (int k = 0; k < 8; ++k)
           umma_ts(t_dv, t_st + (k >> 1) * 32 + (k & 1) * 8, desc_at(do_mn, k * 2048), idesc_dv,
                   (n > 0 || k > 0) ? 1u : 0u);
+        tc_commit(&bars->ring_empty[do_bar(n)]);
         if (more) {
-          ok = ring_wait(2 * (n + 1), 0x3240u);
+          ok = q_wait(n + 1, 0x3240u);
           if (!ok) break;
-          issue_score(t_st, k_desc, slot_addr(2 * (n + 1)), p.nk_qk);
+          issue_score(t_st, k_desc, q_addr(n + 1), p.nk_qk);
           tc_commit(&bars->st_full);
         }
         ok = mbar_wait(&bars->ds_full, ph, ab, 0x3230u);
@@ -786,17 +818,16 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           umma_ss(t_dk, desc_at(ds_desc, off), desc_at(q_mn, k * 2048), idesc_dk, (n > 0 || k > 0) ? 1u : 0u);
         }
         tc_commit(&bars->ds_free);
-        tc_commit(&bars->ring_empty[(2 * n) % kBwdStages]);
-        tc_commit(&bars->ring_empty[(2 * n + 1) % kBwdStages]);
+        tc_commit(&bars->ring_empty[2 * (n & 1)]);
         if (more) {
-          ok = ring_wait(2 * (n + 1) + 1, 0x3241u);
+          ok = do_wait(n + 1, 0x3241u);
           if (!ok) break;
           if constexpr (kFuseDq) {  // the dP^T columns still hold dQ_partial(n) until it is drained
             ok = mbar_wait(&bars->dq_free, ph, ab, 0x3250u);
             if (!ok) break;
             mma_issue_fence();
           }
-          issue_score(t_dpt, v_desc, slot_addr(2 * (n + 1) + 1), p.nk_v);
+          issue_score(t_dpt, v_desc, do_addr(n + 1), p.nk_v);
           tc_commit(&bars->dpt_full);
         }
       }
@@ -1062,7 +1093,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 // fused form: fp32 dQ image -> bf16 dQ
 // ------------------------------------------------------------------------------------------
 // One CTA per 128 x 128 tile.  A warp instruction reads eight 64-byte runs of the image (four rows
-// of one 4-column group each) and writes four 64-byte runs of bf16 rows, so both sides move whole
+// of one 4-column group each, see BwdParams::dq_acc) and writes four 64-byte runs of bf16 rows, so both sides move whole
 // 32-byte sectors; HBM-bound: 512 + 256 bytes per q row.
 struct DqConvertParams {
   const float* acc;
@@ -1088,7 +1119,7 @@ __global__ void __launch_bounds__(256) splash_dq_convert_kernel(const DqConvertP
 #pragma unroll
   for (int it = 0; it < 4; ++it)
 #pragma unroll
-    for (int jg = 0; jg < 4; ++jg) v[it * 4 + jg] = __ldcs(src + (jg * 8 + jj) * kTile + warp * 16 + it * 4 + rr);
+    for (int jg = 0; jg < 4; ++jg) v[it * 4 + jg] = __ldcs(src + ((jg * 4 + warp / 2) * 8 + jj) * 32 + (warp & 1) * 16 + it * 4 + rr);
 #pragma unroll
   for (int it = 0; it < 4; ++it) {
     const int r = warp * 16 + it * 4 + rr;
@@ -1212,7 +1243,7 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   float* delta = static_cast<float*>(a.workspace);
   float* nlse2 = reinterpret_cast<float*>(static_cast<uint8_t*>(a.workspace) + bwd_workspace_bytes(B, Hq, Sq) / 2);
   float* dq_acc = reinterpret_cast<float*>(static_cast<uint8_t*>(a.workspace) + bwd_workspace_bytes(B, Hq, Sq));
-  // (fused form: the image the reds add into starts at zero; the di pass clears it while it streams)
+  // (fused form: the image the reductions add into starts at zero; the di pass clears it while it streams)
   if (mask & 1u) {
     DeltaParams dp;
     dp.o = static_cast<const __nv_bfloat16*>(a.o.data);
@@ -1329,7 +1360,7 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   p.n_rows = a.sched_dkv.n_rows;
   // dkv: the kv tiles of one (batch, kv head) stream the same Q / dO of its q-head group
   p.n_groups = (int)(Hkv * B);
-  // (fused: plus the fp32 dQ image of those heads, which the reds keep in L2)
+  // (fused: plus the fp32 dQ image of those heads, which the reductions keep in L2)
   p.chunk_groups = chunk_groups_for((Hq / Hkv) * Sq * kHeadDim * (fused ? 8 : 4), p.n_groups, 1);
   if ((int64_t)p.n_rows * p.n_groups > 0x7fffffffll) return SPLASH_ERR_TOO_LARGE;
   if (mask & 4u) {
