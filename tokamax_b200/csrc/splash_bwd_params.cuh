@@ -36,6 +36,7 @@ struct BwdParams {
   int nk_qk, nk_v;             // K = 16 slices with real columns in contractions over d_qk / d_v
   int n_split;                 // dkv kernel: CTAs of a cluster that share a kv tile (1: no clusters)
   int n_groups, chunk_groups;  // (batch, head) pairs of the grid; how many share a launch chunk
+  int main_groups;             // dkv kernel: the groups behind these are the last chunk, see last_chunk()
   // soft-cap variants: logits = cap * tanh(scale * q k^T / cap); dS gains the factor 1 - tanh^2
   float soft_cap, softcap_a;   // cap; scale / cap
   float scale, scale_log2;

@@ -551,8 +551,14 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const unsigned rank = kSplit ? cluster_rank() : 0u;
-  const CtaWork work = cta_work_at(kSplit ? blockIdx.x / p.n_split : blockIdx.x, p.row_order, p.n_rows, p.n_groups,
-                                   p.chunk_groups, false);
+  const CtaWork work = [&] {
+    const unsigned block = kSplit ? blockIdx.x / p.n_split : blockIdx.x, main = (unsigned)(p.main_groups * p.n_rows);
+    if (block < main) return cta_work_at(block, p.row_order, p.n_rows, p.main_groups, p.chunk_groups, false);
+    const int rest = p.n_groups - p.main_groups;
+    CtaWork w = cta_work_at(block - main, p.row_order, p.n_rows, rest, rest, false);
+    w.group += p.main_groups;
+    return w;
+  }();
   const int kv_tile = work.row;
   const int kv_head = work.group % p.kv_heads;
   const int batch = work.group / p.kv_heads;
@@ -1163,6 +1169,17 @@ static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap) {
   return kernels[split][fused][soft_cap];
 }
 
+// The groups of a dkv launch that come chunk by chunk; the others are its last chunk.  A chunk's rows fill the SMs only
+// while the next chunk follows; behind the last one they wait for its longest row, which in a triangle of rows takes as
+// long as several chunks of one group together.  So the last chunk has groups enough for a row an SM, longest first over
+// all of them (prefix mask 2 x 4096, 16 / 4 heads, 8 groups of 32 rows: 682 -> 617 us a pass; causal 4 x 8192, 32 / 8:
+// 7302 -> 7243; two or four rows an SM: 617 and 7284 .. 7527, the dQ images of those groups no longer stay in L2).
+static int last_chunk(int64_t n_groups, int64_t chunk_groups, int64_t n_rows) {
+  constexpr int64_t kSms = 148;
+  const int64_t last = (kSms + n_rows - 1) / n_rows;
+  return n_groups > last ? (int)((n_groups - last) / chunk_groups * chunk_groups) : 0;
+}
+
 // CTAs that share a kv tile of this call's dkv kernel (head dims up to 128)
 static int dkv_split(const SplashBwdArgs& a, const SplashShards& shards, bool fused, const int32_t* clusters) {
   if (a.q_segment_ids != nullptr || a.q_sequence != nullptr) return 1;
@@ -1362,6 +1379,7 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   p.n_groups = (int)(Hkv * B);
   // (fused: plus the fp32 dQ image of those heads, which the reductions keep in L2)
   p.chunk_groups = chunk_groups_for((Hq / Hkv) * Sq * kHeadDim * (fused ? 8 : 4), p.n_groups, 1);
+  p.main_groups = last_chunk(p.n_groups, p.chunk_groups, p.n_rows);
   if ((int64_t)p.n_rows * p.n_groups > 0x7fffffffll) return SPLASH_ERR_TOO_LARGE;
   if (mask & 4u) {
     const int64_t n_ctas = (int64_t)p.n_rows * p.n_groups;
