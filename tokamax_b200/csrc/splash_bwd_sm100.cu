@@ -501,7 +501,7 @@ constexpr int kDqTileFloats = kTile * kHeadDim;
 // dS^T goes to shared memory in the K-major 128-byte-swizzled layout of an operand tile (A operand
 // of dK += dS^T Q), which frees the dP^T columns for the next step as soon as they have been
 // read.  Issue order of step n:  wait P^T(n) | dV(n) | S^T(n+1) | wait dS^T(n) | dK(n) | dP^T(n+1)
-// — the tensor pipe executes in order, so S^T(n+1) cannot overtake dV(n)'s read of P^T(n), and
+// (fused: dQ_partial(n) ahead of dK(n), and in most cases S^T(n+1) between the two) — the tensor pipe executes in order, so S^T(n+1) cannot overtake dV(n)'s read of P^T(n), and
 // dP^T(n+1) is issued only after the compute warps have consumed dP^T(n).
 constexpr int kDkvStatsBytes = (kBwdStages / 2) * 2 * kTile * 4;
 constexpr int kDkvSmemBytes = (3 + kBwdStages) * kTileBytes + kDkvStatsBytes + 512;
@@ -526,6 +526,9 @@ struct DkvBarriers {
 };
 static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 
+// kLateS (fused form): S^T(n+1) is issued behind dQ(n).  Right behind dV(n) it takes all of the shared memory's rate from
+// the compute warps, which read dP^T's statistics and write dS^T then; behind dQ(n) it runs under the drain.  late_scores() has
+// the rule.
 //
 // kSplit: a cluster of 2 .. 8 CTAs shares one kv tile, each taking its part of the steps (q head, q tile), see PartWalk.
 // At the end every CTA leaves its dK and dV (fp32) in its own shared memory and the cluster adds them
@@ -534,7 +537,7 @@ static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 constexpr int kDkvPartWords = 2 * kHeadDim / 4 * kTile;  // 16-byte words: [dk, dv column / 4][kv row]
 static_assert(kDkvPartWords * 16 <= (3 + kBwdStages) * kTileBytes, "the parts lie over the operand tiles");
 
-template <bool kSoftCap, bool kFuseDq, bool kSplit>
+template <bool kSoftCap, bool kFuseDq, bool kSplit, bool kLateS>
 __global__ void __launch_bounds__(kFuseDq ? kFusedThreads : kDkvThreads, 1)
 splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -781,6 +784,12 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         issue_score(t_dpt, v_desc, do_addr(0), p.nk_v);
         tc_commit(&bars->dpt_full);
       }
+      auto next_scores = [&](int n) {
+        if (!q_wait(n + 1, 0x3240u)) return false;
+        issue_score(t_st, k_desc, q_addr(n + 1), p.nk_qk);
+        tc_commit(&bars->st_full);
+        return true;
+      };
       for (int n = 0; n < n_steps && ok; ++n) {
         const uint32_t ph = (uint32_t)n & 1u;
         const uint32_t q_slot = q_addr(n), do_slot = do_addr(n);
@@ -796,11 +805,9 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           umma_ts(t_dv, t_st + (k >> 1) * 32 + (k & 1) * 8, desc_at(do_mn, k * 2048), idesc_dv,
                   (n > 0 || k > 0) ? 1u : 0u);
         tc_commit(&bars->ring_empty[do_bar(n)]);
-        if (more) {
-          ok = q_wait(n + 1, 0x3240u);
+        if (more && !kLateS) {
+          ok = next_scores(n);
           if (!ok) break;
-          issue_score(t_st, k_desc, q_addr(n + 1), p.nk_qk);
-          tc_commit(&bars->st_full);
         }
         ok = mbar_wait(&bars->ds_full, ph, ab, 0x3230u);
         if (!ok) break;
@@ -814,6 +821,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           for (int k = 0; k < 8; ++k)
             umma_ss(t_dpt, desc_at(ds_mn_desc, k * 2048), desc_at(k_mn_desc, k * 2048), idesc_dq, k > 0 ? 1u : 0u);
           tc_commit(&bars->dq_full);
+          if (more && kLateS) {
+            ok = next_scores(n);
+            if (!ok) break;
+          }
         }
         // dK += dS^T Q: A = dS^T from shared memory (K-major, two 64-column halves), B = the Q
         // tile read MN-major
@@ -1160,13 +1171,23 @@ size_t bwd_fused_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len) 
 }
 
 using DkvKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
-static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap) {
+static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap, bool late) {
   static const DkvKernel kernels[2][2][2] = {
-      {{splash_dkv_kernel<false, false, false>, splash_dkv_kernel<true, false, false>},
-       {splash_dkv_kernel<false, true, false>, splash_dkv_kernel<true, true, false>}},
-      {{splash_dkv_kernel<false, false, true>, splash_dkv_kernel<true, false, true>},
-       {splash_dkv_kernel<false, true, true>, splash_dkv_kernel<true, true, true>}}};
+      {{splash_dkv_kernel<false, false, false, false>, splash_dkv_kernel<true, false, false, false>},
+       {splash_dkv_kernel<false, true, false, false>, splash_dkv_kernel<true, true, false, false>}},
+      {{splash_dkv_kernel<false, false, true, false>, splash_dkv_kernel<true, false, true, false>},
+       {splash_dkv_kernel<false, true, true, false>, splash_dkv_kernel<true, true, true, false>}}};
+  if (late) return split ? splash_dkv_kernel<false, true, true, true> : splash_dkv_kernel<false, true, false, true>;
   return kernels[split][fused][soft_cap];
+}
+// Whether S^T of the next step is issued behind dQ of this one instead of behind dV.  d 128: causal 4 x 8192, 32 / 8 heads
+// 7198 -> 7038 us a pass, 2 x 4096 1022 -> 999, 4 x 2048, 16 / 16 366 -> 358; full 1 x 4096, 32 / 8 991 -> 958; packed windows
+// 8 x 16384 6678 -> 6598.  Where forming P^T takes longer it wants its scores early: partial blocks read from a table (prefix 2 x
+// 4096, 16 / 4: 623 -> 641), a soft cap (187 -> 193); so it does where the scores are half as long (d 64, 2 x 8192, 16 / 4:
+// 1270 -> 1479).  Without dQ there is nothing to put them behind (4 x 4096, 16 / 8: behind dS^T's arrival 1097 -> 1158).
+static bool late_scores(const SplashBwdArgs& a, bool fused) {
+  const bool table = a.mask_fn.kind == SPLASH_MASK_TABLE && a.sched_dkv.partial_mask_blocks != nullptr;
+  return fused && a.soft_cap == 0.f && a.q.size[3] > 64 && !table;
 }
 
 // The groups of a dkv launch that come chunk by chunk; the others are its last chunk.  A chunk's rows fill the SMs only
@@ -1191,9 +1212,10 @@ static int dkv_split(const SplashBwdArgs& a, const SplashShards& shards, bool fu
                                  n_rows * a.k.size[0] * a.k.size[1] * (shards.head_shards > 1 ? shards.head_shards : 1), true);
   rw.longest *= (float)(a.q.size[1] / a.k.size[1]);  // a kv tile walks every q head of its group
   rw.mean *= (float)(a.q.size[1] / a.k.size[1]);
-  const bool soft_cap = a.soft_cap != 0.f;
+  const bool soft_cap = a.soft_cap != 0.f, late = late_scores(a, fused);
   return row_parts(rw, clusters, [&] {
-    return cluster_capacity((const void*)dkv_kernel_for(true, fused, soft_cap), 4 + (soft_cap ? 1 : 0) + (fused ? 2 : 0),
+    return cluster_capacity((const void*)dkv_kernel_for(true, fused, soft_cap, late),
+                            4 + (soft_cap ? 1 : 0) + (fused ? 2 : 0) + (late ? 4 : 0),
                             fused ? kFusedThreads : kDkvThreads, kDkvSmemBytes);
   });
 }
@@ -1286,16 +1308,17 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   const bool soft_cap = a.soft_cap != 0.f;
   if (soft_cap && !(a.soft_cap > 0.f)) return SPLASH_ERR_INVALID_ARGUMENT;
   auto* dq_kernel = soft_cap ? splash_dq_kernel<true> : splash_dq_kernel<false>;
-  DkvKernel dkv_kernel = dkv_kernel_for(false, fused, soft_cap);
+  const bool late = late_scores(a, fused);
+  DkvKernel dkv_kernel = dkv_kernel_for(false, fused, soft_cap, late);
   const int dkv_smem = kDkvSmemBytes;
   // function attributes are per device: remember which devices have been set up
   {
     static std::mutex attr_mu;
-    static bool attr_done[64][4] = {};
+    static bool attr_done[64][8] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SPLASH_ERR_CUDA;
     std::lock_guard<std::mutex> lock(attr_mu);
-    bool& done = attr_done[dev][(soft_cap ? 1 : 0) + (fused ? 2 : 0)];
+    bool& done = attr_done[dev][(soft_cap ? 1 : 0) + (fused ? 2 : 0) + (late ? 4 : 0)];
     if (!done) {
       if (cudaFuncSetAttribute(dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmemBytes) !=
               cudaSuccess ||
@@ -1386,7 +1409,7 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
     const int threads = fused ? kFusedThreads : kDkvThreads;
     p.n_split = dkv_split(a, shards, fused, nullptr);
     if (p.n_split < 0) return p.n_split;
-    if (p.n_split > 1) dkv_kernel = dkv_kernel_for(true, fused, soft_cap);
+    if (p.n_split > 1) dkv_kernel = dkv_kernel_for(true, fused, soft_cap, late);
     if (launch_clusters(dkv_kernel, (unsigned)n_ctas, p.n_split, threads, dkv_smem, stream, tm_q, tm_do, tm_k, tm_v, p) !=
         cudaSuccess)
       return SPLASH_ERR_CUDA;
