@@ -109,6 +109,31 @@ def test_heads_up_to_128_of_a_large_call_are_those_of_its_shares(d, kind, soft_c
       assert torch.equal(mine, part[name]), (name, h)
 
 
+# 13 kv tiles of 24 (batch, kv head) pairs: 312 CTAs, two tiles and more for an SM, with a soft cap too.  The two forms of
+# the backward compute dk and dv by the same products in the same order; dq's are summed in another one.
+@pytest.mark.parametrize("d_qk,d_v", [(128, 128), (64, 64), (80, 128), (128, 64)])
+@pytest.mark.parametrize("kind,soft_cap,segments", [("causal", None, False), ("window", 20.0, True), ("window", None, True),
+                                                    ("table", None, False), ("full", None, False)])
+def test_both_backward_forms_of_a_large_call(d_qk, d_v, kind, soft_cap, segments):
+  b, hkv, group, s = 2, 12, 2, 1664
+  g = torch.Generator(device=DEV).manual_seed(d_qk + d_v)
+  mk = lambda h, d: torch.randn(b, h, s, d, generator=g, device=DEV).to(torch.bfloat16)
+  q, k, v, do = mk(hkv * group, d_qk), mk(hkv, d_qk), mk(hkv, d_v), mk(hkv * group, d_v)
+  seg = None
+  if segments:  # the second row's queries see no key of its last 164 tokens: kv tiles with steps that come to nothing
+    ids = torch.zeros((b, s), dtype=torch.int32, device=DEV)
+    ids[0, 700:], ids[1, 130:], ids[1, 1500:] = 1, 1, 2
+    seg = splash.SegmentIds(q=ids.clamp(max=1) if kind == "window" else ids, kv=ids)
+  config = splash.dataclasses.replace(splash.SplashConfig.get_default(), attn_logits_soft_cap=soft_cap)
+  mask = mask_lib.FullMask((s, s)) if kind == "full" else _mask(kind, s)
+  fused, split = (_run(splash.make_splash_mha(mask, config=config, q_seq_shards=1, save_residuals=True, repeatable_dq=r),
+                       q, k, v, do, seg, 1 / math.sqrt(d_qk)) for r in (False, True))
+  for name in ("out", "lse", "dk", "dv"):
+    assert torch.equal(fused[name], split[name]), name
+  # fp32 sums of the same products in another order, rounded to bf16 where they differ in the last bits
+  assert ((fused["dq"].float() - split["dq"].float()).norm() / split["dq"].float().norm()).item() <= 1e-3
+
+
 @pytest.mark.parametrize("p_format", ["e4m3", "f16"])
 def test_e4m3_heads_of_a_large_call_are_those_of_its_shares(p_format):
   b, hkv, group, s = 2, 11, 2, 1664

@@ -175,6 +175,16 @@ __device__ __forceinline__ int clc_block(const void* answer) {
   return block;
 }
 
+// 16 bytes of shared memory, whether or not they have been read before
+__device__ __forceinline__ int4 ld_again(const int4* p) {
+  int4 v;
+  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(smem_u32(p))
+               : "memory");
+  return v;
+}
+
 // ----------------------------------------------------------------------------------------
 // TMA (tiled, no multicast)
 // ----------------------------------------------------------------------------------------

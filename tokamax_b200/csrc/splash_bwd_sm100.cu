@@ -506,7 +506,15 @@ constexpr int kDqTileFloats = kTile * kHeadDim;
 constexpr int kDkvStatsBytes = (kBwdStages / 2) * 2 * kTile * 4;
 constexpr int kDkvSmemBytes = (3 + kBwdStages) * kTileBytes + kDkvStatsBytes + 512;
 
+constexpr uint32_t kDkvWork = 2;
+
 struct DkvBarriers {
+  uint64_t answer[2];  // cluster launch control: what the request for the next tile returned
+  // tiles in the order they are worked on: kv tile (-1: none left), (batch, kv head), first and last entry
+  int4 work[kDkvWork];
+  uint64_t answer_full;
+  uint64_t work_full[kDkvWork], work_empty[kDkvWork];
+  uint64_t out_free;  // a tile's dK and dV have been read from TMEM (16 arrivals)
   uint64_t stat_full[2];
   uint64_t ring_full[kBwdStages];
   uint64_t ring_empty[kBwdStages];
@@ -530,6 +538,13 @@ static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 // the compute warps, which read dP^T's statistics and write dS^T then; behind dQ(n) it runs under the drain.  late_scores() has
 // the rule.
 //
+// CTAs stay for several tiles: the producer takes over CTAs that have not been launched yet (cluster launch control) when all
+// loads of its tile are on their way, posts their tiles and goes on loading; the next tile's first scores are computed while
+// the compute warps store dK and dV.  A tile a CTA spent about 20000 cycles between its last step and its successor's
+// first.  One tile a CTA -> this, us a pass: 8 x 16384, 16 heads, window 4096 and documents (some 12 steps a tile) 6584 -> 6260,
+// causal 4 x 2048, 16 / 16 359 -> 334, 4 x 8192, 32 / 8 6974 -> 6842, prefix 2 x 4096, 16 / 4 617 -> 597 (with the drain
+// below, 604 before).  kOneTile: its own tile only, see one_tile_ctas().
+//
 // kSplit: a cluster of 2 .. 8 CTAs shares one kv tile, each taking its part of the steps (q head, q tile), see PartWalk.
 // At the end every CTA leaves its dK and dV (fp32) in its own shared memory and the cluster adds them
 // up over distributed shared memory in rank order, each CTA a share of the columns: no atomics, still
@@ -537,7 +552,7 @@ static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 constexpr int kDkvPartWords = 2 * kHeadDim / 4 * kTile;  // 16-byte words: [dk, dv column / 4][kv row]
 static_assert(kDkvPartWords * 16 <= (3 + kBwdStages) * kTileBytes, "the parts lie over the operand tiles");
 
-template <bool kSoftCap, bool kFuseDq, bool kSplit, bool kLateS>
+template <bool kSoftCap, bool kFuseDq, bool kSplit, bool kLateS, bool kOneTile = kSplit>
 __global__ void __launch_bounds__(kFuseDq ? kFusedThreads : kDkvThreads, 1)
 splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -554,33 +569,34 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const unsigned rank = kSplit ? cluster_rank() : 0u;
-  const CtaWork work = [&] {
-    const unsigned block = kSplit ? blockIdx.x / p.n_split : blockIdx.x, main = (unsigned)(p.main_groups * p.n_rows);
-    if (block < main) return cta_work_at(block, p.row_order, p.n_rows, p.main_groups, p.chunk_groups, false);
-    const int rest = p.n_groups - p.main_groups;
-    CtaWork w = cta_work_at(block - main, p.row_order, p.n_rows, rest, rest, false);
-    w.group += p.main_groups;
-    return w;
-  }();
-  const int kv_tile = work.row;
-  const int kv_head = work.group % p.kv_heads;
-  const int batch = work.group / p.kv_heads;
   const int group = p.q_heads / p.kv_heads;
-  const int ebeg = p.row_ptr[kv_tile];
-  const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + kv_tile] : p.row_ptr[kv_tile + 1];
-  const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
-  const int n_ent = eend - ebeg;
+  // kv tile, (batch, kv head), first and last entry of a block of the grid
+  auto tile_of = [&](unsigned block) {
+    const unsigned main = (unsigned)(p.main_groups * p.n_rows);
+    CtaWork t;
+    if (block < main) {
+      t = cta_work_at(block, p.row_order, p.n_rows, p.main_groups, p.chunk_groups, false);
+    } else {
+      const int rest = p.n_groups - p.main_groups;
+      t = cta_work_at(block - main, p.row_order, p.n_rows, rest, rest, false);
+      t.group += p.main_groups;
+    }
+    const int beg = p.row_ptr[t.row];
+    const int end = p.row_end ? p.row_end[(int64_t)(t.group / p.kv_heads) * p.n_rows + t.row] : p.row_ptr[t.row + 1];
+    return make_int4(t.row, t.group, beg, end < beg ? beg : end);
+  };
+  auto list_of = [&](const int4& w) { return p.entries + (int64_t)(w.y / p.kv_heads) * p.entries_per_batch; };
   // Q and dO of step n in the ring: slots 0, 2 and 1, 3 by turns.  The fused form parks dQ in slot 3: dO then keeps to
   // slot 1, whose two halves take turns where dO has one half.
   const bool one_do = kFuseDq && p.d_v > 64;
   auto do_bar = [&](uint32_t n) { return one_do ? 1u : 1u + 2u * (n & 1u); };
   auto do_phase = [&](uint32_t n) { return (one_do ? n : n >> 1) & 1u; };
   auto do_offset = [&](uint32_t n) { return kTileBytes + (one_do ? 0u : (n & 1u) * (kFuseDq ? kHalfBytes : 2 * kTileBytes)); };
-  // steps of this CTA: (q head g of the group, entry e) pairs in that order
-  const PartWalk<kSplit> walk(entries, ebeg, eend, p.n_split);
-  const int offset0 = walk.offset((int)rank);  // of head 0's part; a tile less for each further head
+  // steps of a tile: (q head g of the group, entry e) pairs in that order; `offset` (kSplit): of head g's part, a tile less
+  // for each further head
+  int4 own = kOneTile ? tile_of(kSplit ? blockIdx.x / p.n_split : blockIdx.x) : make_int4(0, 0, 0, 0);
+  auto walk_of = [&](const int4& w) { return PartWalk<kSplit>(list_of(w), w.z, w.w, p.n_split); };
   auto offset_behind = [&](int offset) { return kSplit ? (offset == 0 ? p.n_split : offset) - 1 : 0; };
-  int n_steps = n_ent * group;  // (kSplit: counted below)
 
   if (threadIdx.x == 0) {
     // The operand tiles need a 1024-byte aligned base for the 128-byte swizzle; there is no
@@ -597,6 +613,12 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     bars->early_exit = bad;
     bars->abort_flag = kSplit ? bad : 0u;  // (read by the other CTAs of the cluster)
     bars->n_steps = 0;
+    for (uint32_t i = 0; i < kDkvWork; ++i) {
+      mbar_init(&bars->work_full[i], 1);
+      mbar_init(&bars->work_empty[i], 17 + (kFuseDq ? kFusedThreads / 32 - kDkvDrainWarp : 0));  // compute, MMA, drain warps
+    }
+    mbar_init(&bars->answer_full, 1);
+    mbar_init(&bars->out_free, 16);
     mbar_init(&bars->stat_full[0], 1);
     mbar_init(&bars->stat_full[1], 1);
     for (int s = 0; s < kBwdStages; ++s) {
@@ -622,13 +644,23 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     return;
   }
   if constexpr (kSplit) {
+    const PartWalk<kSplit> walk = walk_of(own);
     unsigned mine = 0;
-    for (int e = ebeg + (int)threadIdx.x; e < eend; e += (int)blockDim.x) {
-      const int part = (entries[e].x - walk.first_tile) % p.n_split;
-      for (int g = 0, o = offset0; g < group; ++g, o = offset_behind(o)) mine += part == o;
+    for (int e = own.z + (int)threadIdx.x; e < own.w; e += (int)blockDim.x) {
+      const int part = (list_of(own)[e].x - walk.first_tile) % p.n_split;
+      for (int g = 0, o = walk.offset((int)rank); g < group; ++g, o = offset_behind(o)) mine += part == o;
     }
     mine = __reduce_add_sync(0xffffffffu, mine);
     if (lane == 0) atomicAdd(&bars->n_steps, mine);
+  }
+  if (!kOneTile && warp == kDkvTmaWarp) {  // looked up beside the allocation; the others hear of it from the queue
+    own = tile_of(blockIdx.x);
+    if (lane == 0) {
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_do);
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+    }
   }
   if (warp == kDkvMmaWarp) {
     tmem_alloc(&bars->tmem_base, 512);
@@ -637,9 +669,38 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if constexpr (kSplit) n_steps = (int)bars->n_steps;
   const uint32_t tmem = bars->tmem_base;
   AbortCtx ab{&bars->abort_flag, p.err};
+  auto steps_of = [&](const int4& w) { return kSplit ? bars->n_steps : (uint32_t)((w.w - w.z) * group); };
+
+  // The tiles this CTA works on, in order: its own, then those it takes over (the producer posts both).  kOneTile: its own.
+  uint32_t taken = 0;  // tiles so far: slot and phase of the next one
+  auto work_slot = [&]() { return taken % kDkvWork; };
+  auto work_phase = [&]() { return (taken / kDkvWork) & 1u; };
+  // Calls body(tile) for each, until it returns false: by a whole warp, or by a thread for its warp.  `hold`: the tile's
+  // slot is kept to the end, for body to read it again.
+  auto each_tile = [&](bool warp_wide, bool hold, auto body) {
+    if constexpr (kOneTile) {
+      body(own);
+    } else {
+      auto release = [&]() {
+        if (warp_wide) __syncwarp();
+        if (!warp_wide || lane == 0) mbar_arrive(&bars->work_empty[work_slot()]);
+        ++taken;
+      };
+      for (;;) {
+        bool ok = mbar_wait(&bars->work_full[work_slot()], work_phase(), ab, 0x3700u + work_slot());
+        if (warp_wide) ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        const int4 w = bars->work[work_slot()];
+        if (w.x < 0) break;
+        if (!hold) release();
+        if (!body(w)) break;
+        asm volatile("" : "+r"(taken));  // (the slot's addresses are worked out again, not kept over the tile)
+        if (hold) release();
+      }
+    }
+  };
 
   if (kFuseDq && warp >= kDkvDrainWarp) {
     // ------------------------------------------------------------------ dQ drain (fused form)
@@ -668,83 +729,118 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       __syncwarp();
       if (lane == 0) bulk_reduce_add(dst, stage, kDqBlockBytes);
     };
-    for (int g = 0, o = offset0; n < (uint32_t)n_steps && ok; ++g, o = offset_behind(o)) {
-      const int head = kv_head * group + g;
-      float* head_base = p.dq_acc + ((int64_t)batch * p.q_heads + head) * n_q_tiles * (int64_t)kDqTileFloats +
-                         (chunk * 4 + wq) * (kDqBlockBytes / 4);
-      for (int e = walk.first(o); e < eend && ok; e = walk.next(e), ++n) {
-        float* dst = head_base + (int64_t)entries[e].x * kDqTileFloats;
-        ok = mbar_wait(&bars->dq_full, n & 1u, ab, 0x3600u);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        tmem_ld32(t_dq, v);
-        tmem_ld_wait();
-        if (two) {
-          park();
-          tmem_ld32(t_dq + 32, v);
-          send(dst);
+    each_tile(true, false, [&](const int4& w) {
+      const PartWalk<kSplit> walk = walk_of(w);
+      const int4* entries = list_of(w);
+      const uint32_t last = n + steps_of(w);
+      for (int g = 0, o = walk.offset((int)rank); n < last && ok; ++g, o = offset_behind(o)) {
+        // (w.y * group: batch * q heads + first q head of the group)
+        float* head_base = p.dq_acc + ((int64_t)w.y * group + g) * n_q_tiles * (int64_t)kDqTileFloats +
+                           (chunk * 4 + wq) * (kDqBlockBytes / 4);
+        for (int e = walk.first(o); e < w.w && ok; e = walk.next(e), ++n) {
+          float* dst = head_base + (int64_t)entries[e].x * kDqTileFloats;
+          ok = mbar_wait(&bars->dq_full, n & 1u, ab, 0x3600u);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+          tmem_ld32(t_dq, v);
           tmem_ld_wait();
+          if (two) {
+            park();
+            tmem_ld32(t_dq + 32, v);
+            if (kLateS) send(dst);
+            tmem_ld_wait();
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->dq_free);
+          if (two && !kLateS) send(dst);  // (dP^T waits for these columns more often: prefix 2 x 4096 618 -> 604 us)
+          park();
+          send(two ? dst + 4 * (kDqBlockBytes / 4) : dst);
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars->dq_free);
-        park();
-        send(two ? dst + 4 * (kDqBlockBytes / 4) : dst);
       }
-    }
+      return ok;
+    });
     if (lane == 0) bulk_wait_all();
   } else if (warp >= 16) {
    if constexpr (kFuseDq) setmaxnreg_dec<kFusedIssueRegs>();
    if (warp == kDkvTmaWarp) {
-    if (n_steps > 0 && elect_one()) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_do);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
+    if (elect_one()) {
       // tiles are two 64-column halves; with at most 64 real columns the second is never read
       const bool qk2 = p.d_qk > 64, v2 = p.d_v > 64;
-      mbar_arrive_expect_tx(&bars->stat_full[0], qk2 ? kTileBytes : kHalfBytes);
-      tma_load_4d(k_smem, &tm_k, &bars->stat_full[0], 0, kv_tile * kTile, kv_head, batch);
-      if (qk2) tma_load_4d(k_smem + kHalfBytes, &tm_k, &bars->stat_full[0], 64, kv_tile * kTile, kv_head, batch);
-      mbar_arrive_expect_tx(&bars->stat_full[1], v2 ? kTileBytes : kHalfBytes);
-      tma_load_4d(v_smem, &tm_v, &bars->stat_full[1], 0, kv_tile * kTile, kv_head, batch);
-      if (v2) tma_load_4d(v_smem + kHalfBytes, &tm_v, &bars->stat_full[1], 64, kv_tile * kTile, kv_head, batch);
       uint32_t n = 0;
+      uint32_t stepped = 0;  // tiles with steps so far
+      uint32_t asked = 0;
       bool ok = true;
-      for (int g = 0, o = offset0; n < (uint32_t)n_steps && ok; ++g, o = offset_behind(o)) {
-        const int head = kv_head * group + g;
-        const int64_t stat_base = ((int64_t)batch * p.q_heads + head) * p.q_len;
-        for (int e = walk.first(o); e < eend && ok; e = walk.next(e), ++n) {
-          const int qt = entries[e].x;
-          {
-            const uint32_t s = 2u * (n & 1u);
-            ok = mbar_wait(&bars->ring_empty[s], ((n >> 1) & 1u) ^ 1u, ab, 0x3100u + s);
-            if (!ok) break;
-            uint8_t* dst = ring + s * kTileBytes;
-            if (kSplit) bars->step[s / 2] = entries[e];
-            mbar_arrive_expect_tx(&bars->ring_full[s], (qk2 ? kTileBytes : kHalfBytes) + 2 * kTile * 4);
-            tma_load_4d(dst, &tm_q, &bars->ring_full[s], 0, qt * kTile, head, batch);
-            if (qk2) tma_load_4d(dst + kHalfBytes, &tm_q, &bars->ring_full[s], 64, qt * kTile, head, batch);
-            // the step's statistics ride on the Q slot's barrier
-            float* sdst = stats + (s / 2) * 2 * kTile;
-            bulk_load(sdst, p.nlse2 + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
-            bulk_load(sdst + kTile, p.delta + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
-          }
-          {
-            const uint32_t s = do_bar(n);
-            ok = mbar_wait(&bars->ring_empty[s], do_phase(n) ^ 1u, ab, 0x3100u + s);
-            if (!ok) break;
-            uint8_t* dst = ring + do_offset(n);
-            mbar_arrive_expect_tx(&bars->ring_full[s], v2 ? kTileBytes : kHalfBytes);
-            tma_load_4d(dst, &tm_do, &bars->ring_full[s], 0, qt * kTile, head, batch);
-            if (v2) tma_load_4d(dst + kHalfBytes, &tm_do, &bars->ring_full[s], 64, qt * kTile, head, batch);
+      int4 w = own;
+      while (ok) {
+        if constexpr (!kOneTile) {
+          ok = mbar_wait(&bars->work_empty[work_slot()], work_phase() ^ 1u, ab, 0x3710u + work_slot());
+          if (!ok) break;
+          bars->work[work_slot()] = w;
+          mbar_arrive(&bars->work_full[work_slot()]);
+          ++taken;
+          if (w.x < 0) break;
+        }
+        const PartWalk<kSplit> walk = walk_of(w);
+        const int4* entries = list_of(w);
+        const int kv_head = w.y % p.kv_heads, batch = w.y / p.kv_heads;
+        const uint32_t first = n, last = n + steps_of(w);
+        for (int g = 0, o = walk.offset((int)rank); n < last && ok; ++g, o = offset_behind(o)) {
+          const int head = kv_head * group + g;
+          const int64_t stat_base = ((int64_t)batch * p.q_heads + head) * p.q_len;
+          for (int e = walk.first(o); e < w.w && ok; e = walk.next(e), ++n) {
+            const int qt = entries[e].x;
+            {
+              const uint32_t s = 2u * (n & 1u);
+              ok = mbar_wait(&bars->ring_empty[s], ((n >> 1) & 1u) ^ 1u, ab, 0x3100u + s);
+              if (!ok) break;
+              uint8_t* dst = ring + s * kTileBytes;
+              if (kSplit) bars->step[s / 2] = entries[e];
+              mbar_arrive_expect_tx(&bars->ring_full[s], (qk2 ? kTileBytes : kHalfBytes) + 2 * kTile * 4);
+              tma_load_4d(dst, &tm_q, &bars->ring_full[s], 0, qt * kTile, head, batch);
+              if (qk2) tma_load_4d(dst + kHalfBytes, &tm_q, &bars->ring_full[s], 64, qt * kTile, head, batch);
+              // the step's statistics ride on the Q slot's barrier
+              float* sdst = stats + (s / 2) * 2 * kTile;
+              bulk_load(sdst, p.nlse2 + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
+              bulk_load(sdst + kTile, p.delta + stat_base + (int64_t)qt * kTile, kTile * 4, &bars->ring_full[s]);
+            }
+            if (n == first) {  // K and V of the tile, once the MMAs of the last one have read theirs
+              if (stepped > 0) ok = mbar_wait(&bars->acc_done, (stepped - 1) & 1u, ab, 0x3120u);
+              if (!ok) break;
+              mbar_arrive_expect_tx(&bars->stat_full[0], qk2 ? kTileBytes : kHalfBytes);
+              tma_load_4d(k_smem, &tm_k, &bars->stat_full[0], 0, w.x * kTile, kv_head, batch);
+              if (qk2) tma_load_4d(k_smem + kHalfBytes, &tm_k, &bars->stat_full[0], 64, w.x * kTile, kv_head, batch);
+              mbar_arrive_expect_tx(&bars->stat_full[1], v2 ? kTileBytes : kHalfBytes);
+              tma_load_4d(v_smem, &tm_v, &bars->stat_full[1], 0, w.x * kTile, kv_head, batch);
+              if (v2) tma_load_4d(v_smem + kHalfBytes, &tm_v, &bars->stat_full[1], 64, w.x * kTile, kv_head, batch);
+              ++stepped;
+            }
+            {
+              const uint32_t s = do_bar(n);
+              ok = mbar_wait(&bars->ring_empty[s], do_phase(n) ^ 1u, ab, 0x3100u + s);
+              if (!ok) break;
+              uint8_t* dst = ring + do_offset(n);
+              mbar_arrive_expect_tx(&bars->ring_full[s], v2 ? kTileBytes : kHalfBytes);
+              tma_load_4d(dst, &tm_do, &bars->ring_full[s], 0, qt * kTile, head, batch);
+              if (v2) tma_load_4d(dst + kHalfBytes, &tm_do, &bars->ring_full[s], 64, qt * kTile, head, batch);
+            }
           }
         }
+        if (kOneTile || !ok) break;
+        // The next tile.  Asked for when all of this one is on its way, and no earlier: what a CTA has taken over, no other
+        // can take that is done before it.
+        mbar_arrive_expect_tx(&bars->answer_full, 16);
+        clc_request(bars->answer, &bars->answer_full);
+        ok = mbar_wait(&bars->answer_full, asked & 1u, ab, 0x3720u);
+        ++asked;
+        const int block = ok ? clc_block(bars->answer) : -1;
+        fence_proxy_async_smem();  // read before the next answer overwrites it
+        w = block >= 0 ? tile_of((unsigned)block) : make_int4(-1, 0, 0, 0);
       }
     }
   } else if (warp == kDkvMmaWarp) {
-    if (n_steps > 0 && elect_one()) {
+    if (elect_one()) {
       constexpr uint32_t idesc_s = make_idesc_bf16(kTile, kTile, false, false);
       // N of the accumulating MMAs = the gradient's columns: 128, or 64 when the tensor has at most 64
       const uint32_t idesc_dv = make_idesc_bf16(kTile, p.d_v <= 64 ? 64 : kHeadDim, false, true);
@@ -773,27 +869,37 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       const uint32_t idesc_dq = make_idesc_bf16(kTile, p.d_qk <= 64 ? 64 : kHeadDim, true, true);
       const SmemDesc ds_mn_desc = make_smem_desc_sw128(ds_addr, kHalfBytes, 1024);
       const SmemDesc k_mn_desc = make_smem_desc_sw128(k_addr, kHalfBytes, 1024);
-      bool ok = mbar_wait(&bars->stat_full[0], 0, ab, 0x3200u) && mbar_wait(&bars->stat_full[1], 0, ab, 0x3201u);
-      ok = ok && q_wait(0, 0x3210u);
-      if (ok) {
-        issue_score(t_st, k_desc, q_addr(0), p.nk_qk);
-        tc_commit(&bars->st_full);
-      }
-      ok = ok && do_wait(0, 0x3211u);
-      if (ok) {
-        issue_score(t_dpt, v_desc, do_addr(0), p.nk_v);
-        tc_commit(&bars->dpt_full);
-      }
-      auto next_scores = [&](int n) {
+      uint32_t n = 0;      // steps so far
+      uint32_t tiles = 0;  // tiles with steps so far
+      auto next_scores = [&]() {
         if (!q_wait(n + 1, 0x3240u)) return false;
         issue_score(t_st, k_desc, q_addr(n + 1), p.nk_qk);
         tc_commit(&bars->st_full);
         return true;
       };
-      for (int n = 0; n < n_steps && ok; ++n) {
-        const uint32_t ph = (uint32_t)n & 1u;
+      each_tile(false, false, [&](const int4& w) {
+      const uint32_t first = n, last = n + steps_of(w);
+      if (first == last) return true;
+      bool ok = mbar_wait(&bars->stat_full[0], tiles & 1u, ab, 0x3200u) && q_wait(n, 0x3210u);
+      if (ok) {
+        mma_issue_fence();
+        issue_score(t_st, k_desc, q_addr(n), p.nk_qk);
+        tc_commit(&bars->st_full);
+      }
+      ok = ok && mbar_wait(&bars->stat_full[1], tiles & 1u, ab, 0x3201u) && do_wait(n, 0x3211u);
+      if (kFuseDq && n > 0) ok = ok && mbar_wait(&bars->dq_free, (n - 1) & 1u, ab, 0x3251u);
+      if (ok) {
+        mma_issue_fence();
+        issue_score(t_dpt, v_desc, do_addr(n), p.nk_v);
+        tc_commit(&bars->dpt_full);
+      }
+      // the outputs of the tile before have been read
+      if (tiles > 0) ok = ok && mbar_wait(&bars->out_free, (tiles - 1) & 1u, ab, 0x3260u);
+      ++tiles;
+      for (; n < last && ok; ++n) {
+        const uint32_t ph = n & 1u;
         const uint32_t q_slot = q_addr(n), do_slot = do_addr(n);
-        const bool more = n + 1 < n_steps;
+        const bool more = n + 1 < last, begun = n > first;
         ok = mbar_wait(&bars->p_full, ph, ab, 0x3220u);
         if (!ok) break;
         mma_issue_fence();
@@ -803,10 +909,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
         for (int k = 0; k < 8; ++k)
           umma_ts(t_dv, t_st + (k >> 1) * 32 + (k & 1) * 8, desc_at(do_mn, k * 2048), idesc_dv,
-                  (n > 0 || k > 0) ? 1u : 0u);
+                  (begun || k > 0) ? 1u : 0u);
         tc_commit(&bars->ring_empty[do_bar(n)]);
         if (more && !kLateS) {
-          ok = next_scores(n);
+          ok = next_scores();
           if (!ok) break;
         }
         ok = mbar_wait(&bars->ds_full, ph, ab, 0x3230u);
@@ -822,7 +928,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             umma_ss(t_dpt, desc_at(ds_mn_desc, k * 2048), desc_at(k_mn_desc, k * 2048), idesc_dq, k > 0 ? 1u : 0u);
           tc_commit(&bars->dq_full);
           if (more && kLateS) {
-            ok = next_scores(n);
+            ok = next_scores();
             if (!ok) break;
           }
         }
@@ -832,7 +938,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t off = (k >> 2) * kHalfBytes + (k & 3) * 32;
-          umma_ss(t_dk, desc_at(ds_desc, off), desc_at(q_mn, k * 2048), idesc_dk, (n > 0 || k > 0) ? 1u : 0u);
+          umma_ss(t_dk, desc_at(ds_desc, off), desc_at(q_mn, k * 2048), idesc_dk, (begun || k > 0) ? 1u : 0u);
         }
         tc_commit(&bars->ds_free);
         tc_commit(&bars->ring_empty[2 * (n & 1)]);
@@ -849,6 +955,8 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
       }
       tc_commit(&bars->acc_done);
+      return ok;
+      });
     }
    }
   } else {
@@ -857,10 +965,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int cq = warp >> 2;      // column quarter 0..3
     const int wq = warp & 3;       // TMEM lane quarter
     const int r = wq * 32 + lane;  // kv row within the tile
-    const int kv_row = kv_tile * kTile + r;
     const bool has_seg = p.q_seg != nullptr;
-    const int kv_seg = has_seg ? p.kv_seg[(int64_t)batch * p.kv_len + kv_row] : 0;
-    const int32_t* q_seg_row = has_seg ? p.q_seg + (int64_t)batch * p.q_len : nullptr;
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
     const uint32_t t_st = tmem + lane_addr + cq * 32;
     const uint32_t t_dpt = tmem + lane_addr + kTile + cq * 32;
@@ -869,18 +974,26 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     uint8_t* ds_row = ds_smem + (cq >> 1) * kHalfBytes + r * 128;
     const int chunk0 = (cq & 1) * 4;
     const float c = kSoftCap ? p.soft_cap * kLog2e : p.scale_log2;
+    uint32_t n = 0;      // steps so far
+    uint32_t tiles = 0;  // tiles with steps so far
+    each_tile(true, true, [&](const int4& w) {
+    const int kv_row = w.x * kTile + r;
+    const int kv_seg = has_seg ? p.kv_seg[(int64_t)(w.y / p.kv_heads) * p.kv_len + kv_row] : 0;
+    const int32_t* q_seg_row = has_seg ? p.q_seg + (int64_t)(w.y / p.kv_heads) * p.q_len : nullptr;
+    const int4* entries = list_of(w);
+    const int ebeg = w.z, eend = w.w;
+    const uint32_t first = n, last = n + steps_of(w);
     bool ok = true;
-    int n = 0;
 
     // (kSplit: one run through this CTA's steps, whose entries the TMA warp leaves in shared memory)
-    for (int g = 0; n < n_steps && ok; ++g) {
+    while (n < last && ok) {
       int4 ent_next = make_int4(0, 0, 0, 0);
       if constexpr (!kSplit) ent_next = entries[ebeg];
-      for (int e = ebeg; (kSplit ? n < n_steps : e < eend) && ok; ++e, ++n) {
+      for (int e = ebeg; (kSplit ? n < last : e < eend) && ok; ++e, ++n) {
         int4 ent = ent_next;
         if (!kSplit && e + 1 < eend) ent_next = entries[e + 1];
-        const uint32_t ph = (uint32_t)n & 1u;
-        const uint32_t itq = 2u * (uint32_t)n;
+        const uint32_t ph = n & 1u;
+        const uint32_t itq = 2u * n;
         ok = mbar_wait(&bars->ring_full[itq % kBwdStages], (itq / kBwdStages) & 1u, ab, 0x3420u);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -1000,7 +1113,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           }
         }
         if (n > 0) {  // the previous step's dK must have finished reading the tile
-          ok = mbar_wait(&bars->ds_free, (uint32_t)(n - 1) & 1u, ab, 0x3430u);
+          ok = mbar_wait(&bars->ds_free, (n - 1) & 1u, ab, 0x3430u);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
         }
@@ -1016,6 +1129,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
 
     // epilogue: dK (scaled) and dV, 32 columns per thread
+    {  // (the tile's place is read again: the loop over the steps needs the registers)
+    const int4 again = kOneTile ? own : ld_again(&bars->work[work_slot()]);
+    const int batch = again.y / p.kv_heads, kv_head = again.y % p.kv_heads, kv_row = again.x * kTile + r;
+    const uint32_t n_steps = last - first;
     __nv_bfloat16* dk = p.out0 + (int64_t)batch * p.out0_sb + (int64_t)kv_head * p.out0_sh +
                         (int64_t)kv_row * p.out0_ss + cq * 32;
     __nv_bfloat16* dv = p.out1 + (int64_t)batch * p.out1_sb + (int64_t)kv_head * p.out1_sh +
@@ -1070,7 +1187,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       }
     } else {
       if (n_steps > 0 && ok) {
-        ok = mbar_wait(&bars->acc_done, 0, ab, 0x3500u);
+        ok = mbar_wait(&bars->acc_done, tiles++ & 1u, ab, 0x3500u);
         ok = __all_sync(0xffffffffu, ok);
       }
       if (ok) {
@@ -1085,12 +1202,20 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             tmem_ld32(tmem + lane_addr + (2 + which) * kTile + cq * 32, v);
             tmem_ld_wait();
           }
+          if (which == 1 && n_steps > 0) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->out_free);
+          }
           const int64_t ss = which ? p.out1_ss : p.out0_ss;
           store_rows32_peer((which ? dv : dk) - cq * 32 - (int64_t)lane * ss, ss, which ? p.out1_peer : p.out0_peer, batch, kv_head,
                             kv_row - lane, v, which ? 1.0f : p.scale, cq * 32, which ? p.d_v : p.d_qk);
         }
       }
     }
+    }
+    return ok;
+    });
   }
 
   if constexpr (kSplit) {
@@ -1171,14 +1296,22 @@ size_t bwd_fused_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len) 
 }
 
 using DkvKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
-static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap, bool late) {
+static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap, bool late, bool one_tile = false) {
   static const DkvKernel kernels[2][2][2] = {
       {{splash_dkv_kernel<false, false, false, false>, splash_dkv_kernel<true, false, false, false>},
        {splash_dkv_kernel<false, true, false, false>, splash_dkv_kernel<true, true, false, false>}},
       {{splash_dkv_kernel<false, false, true, false>, splash_dkv_kernel<true, false, true, false>},
        {splash_dkv_kernel<false, true, true, false>, splash_dkv_kernel<true, true, true, false>}}};
+  if (one_tile && !split) return fused ? splash_dkv_kernel<true, true, false, false, true> : splash_dkv_kernel<true, false, false, false, true>;
   if (late) return split ? splash_dkv_kernel<false, true, true, true> : splash_dkv_kernel<false, true, false, true>;
   return kernels[split][fused][soft_cap];
+}
+// Whether a CTA keeps to its own kv tile (with a soft cap; the other kernels take over tiles in grids of any size).  What the
+// loop over tiles keeps in registers costs the soft cap's steps 4 %, which grids of one wave and a bit don't get back: 156
+// tiles (3 x 1664, 12 / 4 heads, window 768, d 80) 95.4 us alone, 99.5 with tiles taken over; 1024 tiles (4 x 4096, 16 / 8,
+// window 768) 772 us a pass, 755.
+static bool one_tile_ctas(const SplashBwdArgs& a) {
+  return a.soft_cap != 0.f && a.k.size[2] / kTile * a.k.size[0] * a.k.size[1] < 2 * kSms;
 }
 // Whether S^T of the next step is issued behind dQ of this one instead of behind dV.  d 128: causal 4 x 8192, 32 / 8 heads
 // 7198 -> 7038 us a pass, 2 x 4096 1022 -> 999, 4 x 2048, 16 / 16 366 -> 358; full 1 x 4096, 32 / 8 991 -> 958; packed windows
@@ -1196,7 +1329,6 @@ static bool late_scores(const SplashBwdArgs& a, bool fused) {
 // all of them (prefix mask 2 x 4096, 16 / 4 heads, 8 groups of 32 rows: 682 -> 617 us a pass; causal 4 x 8192, 32 / 8:
 // 7302 -> 7243; two or four rows an SM: 617 and 7284 .. 7527, the dQ images of those groups no longer stay in L2).
 static int last_chunk(int64_t n_groups, int64_t chunk_groups, int64_t n_rows) {
-  constexpr int64_t kSms = 148;
   const int64_t last = (kSms + n_rows - 1) / n_rows;
   return n_groups > last ? (int)((n_groups - last) / chunk_groups * chunk_groups) : 0;
 }
@@ -1309,16 +1441,17 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   if (soft_cap && !(a.soft_cap > 0.f)) return SPLASH_ERR_INVALID_ARGUMENT;
   auto* dq_kernel = soft_cap ? splash_dq_kernel<true> : splash_dq_kernel<false>;
   const bool late = late_scores(a, fused);
-  DkvKernel dkv_kernel = dkv_kernel_for(false, fused, soft_cap, late);
+  const bool one_tile = one_tile_ctas(a);
+  DkvKernel dkv_kernel = dkv_kernel_for(false, fused, soft_cap, late, one_tile);
   const int dkv_smem = kDkvSmemBytes;
   // function attributes are per device: remember which devices have been set up
   {
     static std::mutex attr_mu;
-    static bool attr_done[64][8] = {};
+    static bool attr_done[64][16] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SPLASH_ERR_CUDA;
     std::lock_guard<std::mutex> lock(attr_mu);
-    bool& done = attr_done[dev][(soft_cap ? 1 : 0) + (fused ? 2 : 0) + (late ? 4 : 0)];
+    bool& done = attr_done[dev][(soft_cap ? 1 : 0) + (fused ? 2 : 0) + (late ? 4 : 0) + (one_tile ? 8 : 0)];
     if (!done) {
       if (cudaFuncSetAttribute(dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmemBytes) !=
               cudaSuccess ||

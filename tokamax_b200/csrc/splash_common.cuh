@@ -11,6 +11,7 @@
 
 namespace sb {
 
+constexpr int kSms = 148;           // of a B200
 constexpr int kTile = 128;          // q and kv tile edge the MMAs work on
 constexpr int kHeadDim = 128;       // head dimension of the bf16 kernels
 constexpr int kTileBytes = kTile * kHeadDim * 2;   // one bf16 operand tile: 32 KiB

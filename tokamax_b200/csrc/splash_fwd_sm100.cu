@@ -72,16 +72,6 @@ struct FwdBarriers {
   uint32_t early_exit;
 };
 
-// 16 bytes of shared memory, whether or not they have been read before
-__device__ __forceinline__ int4 ld_again(const int4* p) {
-  int4 v;
-  asm volatile("ld.shared.v4.s32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "r"(smem_u32(p))
-               : "memory");
-  return v;
-}
-
 // kFp8: e4m3 q / k / v with one scale per 128-token tile.  kP16 (with kFp8): the probabilities stay
 // 16 bits wide — q k^T runs on the e4m3 tiles as they are, each V tile is converted once to f16 in
 // shared memory (exact: e4m3 values are f16 values) by the two otherwise idle warps, and p v runs as
