@@ -68,20 +68,29 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
   return w;
 }
 
-// CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (prologue, epilogue; one more
-// for the addition across the cluster).  While everything is resident the longest row sets the time; beyond that the
-// total work over the slots, and half a row for the uneven end.  Rows below 16 steps stay whole although the
+// CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (prologue, epilogue; more for the addition across the
+// cluster).  While everything is resident the longest row sets the time.  Beyond that, rows of different length, longest
+// first, end together but for a tenth of the longest, unless that alone takes as long; rows of one length go in whole waves.  (All
+// numbers tried, us of the kernel, the rule's own marked *, that of the rule before it, which counted half a row for the end
+// of every grid and less for a CTA, in brackets.  dkv, causal: 2 x 4096, 16 / 1 heads, d 64: 733 375 260 *223 254 (249) 315 278,
+// d 128 837 438 307 *259 296 (291) 371 328; 1 x 4096, 8 / 2, fused: 310 173 128 *115 139 (142) 195 185; 2 x 2048, 16 / 4,
+// d 64: 105 *(74) 96 100; window 1000, 1 x 8192, 8 / 1: 193 *(110) 153 128.  Forward: 512 x 16384, 32 / 8: 238 *(137) 184 153;
+// causal 4096, 8 / 2: (65) *55 75 88, d 64 (61) *47 64; 4096, 16 / 2: *(75) 106.)
+// Rows below 16 steps stay whole although the
 // rule would share some (causal 2 x 1024, 8 heads, 64 CTAs of 2 .. 8 steps: 24.7 us, 20.9 with two CTAs a row),
 // so that the bits of short rows do not depend on the batch and the heads beside them: in the forward those
 // of fewer than 2048 keys, in dkv kv tiles of fewer than 16 (q tile, q head of the group) steps.
 inline int split_for(const RowWork& w, const ClusterCapacity& cap) {
-  constexpr float kFixed = 3.f, kMerge = 1.f, kFewest = 16.f;
+  constexpr float kFixed = 4.f, kMerge = 3.f, kFewest = 16.f;
   if (w.longest < kFewest) return 1;
   auto time = [&](int n) {
     const float fixed = kFixed + (n > 1 ? kMerge : 0.f);
-    const float longest = w.longest / n + fixed, mean = w.mean / n + fixed;
-    if (w.ctas <= cap.clusters[n]) return longest;
-    return (float)w.ctas * mean / cap.clusters[n] + 0.5f * longest;
+    const float longest = w.longest / n, mean = w.mean / n + fixed;
+    const int64_t room = cap.clusters[n];
+    if (w.ctas <= room) return longest + fixed;
+    if (w.mean > 0.9f * w.longest) return (float)((w.ctas + room - 1) / room) * mean;
+    const float all = (float)w.ctas * mean / room + 0.1f * longest;
+    return all > longest + fixed ? all : longest + fixed;
   };
   int best = 1;
   float least = 0.9f * time(1);  // a split has to gain a tenth
