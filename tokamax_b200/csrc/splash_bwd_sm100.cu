@@ -124,13 +124,20 @@ __global__ void __launch_bounds__(256) splash_delta_kernel(const DeltaParams p) 
 // ------------------------------------------------------------------------------------------
 // shared pieces of the two MMA kernels
 // ------------------------------------------------------------------------------------------
+constexpr uint32_t kBwdWork = 2;
+
 struct BwdBarriers {
+  uint64_t answer[2];  // cluster launch control: what the request for the next tile returned
+  // tiles in the order they are worked on: q tile (-1: none left), (batch, q head), first and last entry
+  int4 work[kBwdWork];
+  uint64_t answer_full;
+  uint64_t work_full[kBwdWork], work_empty[kBwdWork];
+  uint64_t out_free;                  // a tile's dQ has been read from TMEM (8 arrivals)
   uint64_t stat_full[2];              // stationary operand tiles
   uint64_t ring_full[kDqStages];
   uint64_t ring_empty[kDqStages];
   uint64_t s_full[2];
   uint64_t dp_full;
-  uint64_t p_full;                    // dkv: P^T ready; dq: unused
   uint64_t ds_full;
   uint64_t acc_done;
   uint32_t tmem_base;
@@ -144,6 +151,8 @@ constexpr int kDqSmemBytes = (2 + kDqStages) * kTileBytes + 1024 + 1024;
 // dq kernel
 // ------------------------------------------------------------------------------------------
 // TMEM: S0 [0,128) | S1 [128,256) | dP [256,384) | dQ [384,512)
+// CTAs stay for several tiles, as the dkv kernel's do: a whole pass of causal 2 x 4096, 16 / 1 heads
+// takes 497 -> 493 us at d 64, 576 -> 566 at d 128; 4 x 4096, 16 / 8: 1107 -> 1089.
 template <bool kSoftCap>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
@@ -159,15 +168,14 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const CtaWork work = cta_work(p.row_order, p.n_rows, p.n_groups, p.chunk_groups, true);
-  const int q_tile = work.row;
-  const int head = work.group % p.q_heads;
-  const int batch = work.group / p.q_heads;
-  const int kv_head = head / (p.q_heads / p.kv_heads);
-  const int ebeg = p.row_ptr[q_tile];
-  const int eend = p.row_end ? p.row_end[(int64_t)batch * p.n_rows + q_tile] : p.row_ptr[q_tile + 1];
-  const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
-  const int n_ent = eend - ebeg;
+  // q tile, (batch, q head), first and last entry of a block of the grid
+  auto tile_of = [&](unsigned block) {
+    const CtaWork t = cta_work_at(block, p.row_order, p.n_rows, p.n_groups, p.chunk_groups, true);
+    const int beg = p.row_ptr[t.row];
+    const int end = p.row_end ? p.row_end[(int64_t)(t.group / p.q_heads) * p.n_rows + t.row] : p.row_ptr[t.row + 1];
+    return make_int4(t.row, t.group, beg, end < beg ? beg : end);
+  };
+  auto list_of = [&](const int4& w) { return p.entries + (int64_t)(w.y / p.q_heads) * p.entries_per_batch; };
 
   if (threadIdx.x == 0) {
     bars->early_exit = *reinterpret_cast<volatile uint32_t*>(p.err);
@@ -181,13 +189,28 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     mbar_init(&bars->s_full[0], 1);
     mbar_init(&bars->s_full[1], 1);
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->p_full, 8);
+    for (uint32_t i = 0; i < kBwdWork; ++i) {
+      mbar_init(&bars->work_full[i], 1);
+      mbar_init(&bars->work_empty[i], 9);  // compute warps and the issuing one
+    }
+    mbar_init(&bars->answer_full, 1);
+    mbar_init(&bars->out_free, 8);
     mbar_init(&bars->ds_full, 8);  // one arrival per compute warp
     mbar_init(&bars->acc_done, 1);
     mbar_fence_init();
   }
   __syncthreads();
   if (bars->early_exit != 0) return;
+  int4 own = make_int4(0, 0, 0, 0);
+  if (warp == 8) {  // looked up beside the allocation; the others hear of it from the queue
+    own = tile_of(blockIdx.x);
+    if (lane == 0) {
+      tma_prefetch_desc(&tm_q);
+      tma_prefetch_desc(&tm_do);
+      tma_prefetch_desc(&tm_k);
+      tma_prefetch_desc(&tm_v);
+    }
+  }
   if (warp == 9) {
     tmem_alloc(&bars->tmem_base, 512);
     tmem_relinquish();
@@ -198,41 +221,84 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const uint32_t tmem = bars->tmem_base;
   AbortCtx ab{&bars->abort_flag, p.err};
 
+  // The tiles this CTA works on, in order: its own, then those it takes over (the producer posts both).
+  uint32_t taken = 0;  // tiles so far: slot and phase of the next one
+  auto work_slot = [&]() { return taken % kBwdWork; };
+  auto work_phase = [&]() { return (taken / kBwdWork) & 1u; };
+  // Calls body(tile) for each, until it returns false: by a whole warp, or by a thread for its warp.
+  auto each_tile = [&](bool warp_wide, auto body) {
+    for (;;) {
+      bool ok = mbar_wait(&bars->work_full[work_slot()], work_phase(), ab, 0x1700u + work_slot());
+      if (warp_wide) ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      const int4 w = bars->work[work_slot()];
+      if (w.x < 0) break;
+      if (warp_wide) __syncwarp();
+      if (!warp_wide || lane == 0) mbar_arrive(&bars->work_empty[work_slot()]);
+      ++taken;
+      if (!body(w)) break;
+    }
+  };
+
   if (warp >= 8) {
    setmaxnreg_dec<kIssueRegs>();
    if (warp == 8) {
-    if (n_ent > 0 && elect_one()) {
-      tma_prefetch_desc(&tm_q);
-      tma_prefetch_desc(&tm_do);
-      tma_prefetch_desc(&tm_k);
-      tma_prefetch_desc(&tm_v);
+    if (elect_one()) {
       // tiles are two 64-column halves; with at most 64 real columns the second is never read
       const bool qk2 = p.d_qk > 64, v2 = p.d_v > 64;
-      mbar_arrive_expect_tx(&bars->stat_full[0], qk2 ? kTileBytes : kHalfBytes);
-      tma_load_4d(q_smem, &tm_q, &bars->stat_full[0], 0, q_tile * kTile, head, batch);
-      if (qk2) tma_load_4d(q_smem + kHalfBytes, &tm_q, &bars->stat_full[0], 64, q_tile * kTile, head, batch);
-      mbar_arrive_expect_tx(&bars->stat_full[1], v2 ? kTileBytes : kHalfBytes);
-      tma_load_4d(do_smem, &tm_do, &bars->stat_full[1], 0, q_tile * kTile, head, batch);
-      if (v2) tma_load_4d(do_smem + kHalfBytes, &tm_do, &bars->stat_full[1], 64, q_tile * kTile, head, batch);
       uint32_t it = 0;
+      uint32_t stepped = 0;  // tiles with steps so far
+      uint32_t asked = 0;
       bool ok = true;
-      for (int e = ebeg; e < eend && ok; ++e) {
-        const int col = entries[e].x;
-        for (int kv = 0; kv < 2 && ok; ++kv, ++it) {
-          const uint32_t s = it % kDqStages;
-          ok = mbar_wait(&bars->ring_empty[s], ((it / kDqStages) & 1u) ^ 1u, ab, 0x1100u + s);
-          if (!ok) break;
-          uint8_t* dst = ring + s * kTileBytes;
-          const CUtensorMap* tm = kv == 0 ? &tm_k : &tm_v;
-          const bool two = kv == 0 ? qk2 : v2;
-          mbar_arrive_expect_tx(&bars->ring_full[s], two ? kTileBytes : kHalfBytes);
-          tma_load_4d(dst, tm, &bars->ring_full[s], 0, col * kTile, kv_head, batch);
-          if (two) tma_load_4d(dst + kHalfBytes, tm, &bars->ring_full[s], 64, col * kTile, kv_head, batch);
+      int4 w = own;
+      while (ok) {
+        ok = mbar_wait(&bars->work_empty[work_slot()], work_phase() ^ 1u, ab, 0x1710u + work_slot());
+        if (!ok) break;
+        bars->work[work_slot()] = w;
+        mbar_arrive(&bars->work_full[work_slot()]);
+        ++taken;
+        if (w.x < 0) break;
+        const int4* entries = list_of(w);
+        const int head = w.y % p.q_heads, batch = w.y / p.q_heads, kv_head = head / (p.q_heads / p.kv_heads);
+        for (int e = w.z; e < w.w && ok; ++e) {
+          const int col = entries[e].x;
+          for (int kv = 0; kv < 2 && ok; ++kv, ++it) {
+            const uint32_t s = it % kDqStages;
+            ok = mbar_wait(&bars->ring_empty[s], ((it / kDqStages) & 1u) ^ 1u, ab, 0x1100u + s);
+            if (!ok) break;
+            uint8_t* dst = ring + s * kTileBytes;
+            const CUtensorMap* tm = kv == 0 ? &tm_k : &tm_v;
+            const bool two = kv == 0 ? qk2 : v2;
+            mbar_arrive_expect_tx(&bars->ring_full[s], two ? kTileBytes : kHalfBytes);
+            tma_load_4d(dst, tm, &bars->ring_full[s], 0, col * kTile, kv_head, batch);
+            if (two) tma_load_4d(dst + kHalfBytes, tm, &bars->ring_full[s], 64, col * kTile, kv_head, batch);
+            if (kv == 0 && e == w.z) {  // Q and dO of the tile, once the MMAs of the last one have read theirs
+              if (stepped > 0) ok = mbar_wait(&bars->acc_done, (stepped - 1) & 1u, ab, 0x1120u);
+              if (!ok) break;
+              mbar_arrive_expect_tx(&bars->stat_full[0], qk2 ? kTileBytes : kHalfBytes);
+              tma_load_4d(q_smem, &tm_q, &bars->stat_full[0], 0, w.x * kTile, head, batch);
+              if (qk2) tma_load_4d(q_smem + kHalfBytes, &tm_q, &bars->stat_full[0], 64, w.x * kTile, head, batch);
+              mbar_arrive_expect_tx(&bars->stat_full[1], v2 ? kTileBytes : kHalfBytes);
+              tma_load_4d(do_smem, &tm_do, &bars->stat_full[1], 0, w.x * kTile, head, batch);
+              if (v2) tma_load_4d(do_smem + kHalfBytes, &tm_do, &bars->stat_full[1], 64, w.x * kTile, head, batch);
+              ++stepped;
+            }
+          }
         }
+        if (!ok) break;
+        // The next tile.  Asked for when all of this one is on its way, and no earlier: what a CTA has taken over, no other
+        // can take that is done before it.
+        mbar_arrive_expect_tx(&bars->answer_full, 16);
+        clc_request(bars->answer, &bars->answer_full);
+        ok = mbar_wait(&bars->answer_full, asked & 1u, ab, 0x1720u);
+        ++asked;
+        const int block = ok ? clc_block(bars->answer) : -1;
+        fence_proxy_async_smem();  // read before the next answer overwrites it
+        w = block >= 0 ? tile_of((unsigned)block) : make_int4(-1, 0, 0, 0);
       }
     }
   } else if (warp == 9) {
-    if (n_ent > 0 && elect_one()) {
+    if (elect_one()) {
       constexpr uint32_t idesc_kk = make_idesc_bf16(kTile, kTile, false, false);
       // N of dQ += dS K: dq's columns — 128, or 64 when q / k have at most 64
       const uint32_t idesc_mn = make_idesc_bf16(kTile, p.d_qk <= 64 ? 64 : kHeadDim, false, true);
@@ -250,23 +316,30 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       auto ring_wait = [&](uint32_t it, uint32_t tag) {
         return mbar_wait(&bars->ring_full[it % kDqStages], (it / kDqStages) & 1u, ab, tag);
       };
-      bool ok = mbar_wait(&bars->stat_full[0], 0, ab, 0x1200u) && mbar_wait(&bars->stat_full[1], 0, ab, 0x1201u);
-      // prologue: S_0, dP_0
-      ok = ok && ring_wait(0, 0x1210u);
+      uint32_t n = 0;      // steps so far
+      uint32_t tiles = 0;  // tiles with steps so far
+      each_tile(false, [&](const int4& w) {
+      const uint32_t first = n, last = n + (uint32_t)(w.w - w.z);
+      if (first == last) return true;
+      // S and dP of the first step
+      bool ok = mbar_wait(&bars->stat_full[0], tiles & 1u, ab, 0x1200u) && ring_wait(2 * n, 0x1210u);
       if (ok) {
         mma_issue_fence();
-        ss_kmajor(tmem, q_addr, ring_addr, p.nk_qk);
-        tc_commit(&bars->s_full[0]);
+        ss_kmajor(tmem + (n & 1u) * kTile, q_addr, ring_addr + (2 * n % kDqStages) * kTileBytes, p.nk_qk);
+        tc_commit(&bars->s_full[n & 1u]);
       }
-      ok = ok && ring_wait(1, 0x1211u);
+      ok = ok && mbar_wait(&bars->stat_full[1], tiles & 1u, ab, 0x1201u) && ring_wait(2 * n + 1, 0x1211u);
       if (ok) {
         mma_issue_fence();
-        ss_kmajor(t_dp, do_addr, ring_addr + kTileBytes, p.nk_v);
+        ss_kmajor(t_dp, do_addr, ring_addr + ((2 * n + 1) % kDqStages) * kTileBytes, p.nk_v);
         tc_commit(&bars->dp_full);
-        tc_commit(&bars->ring_empty[1]);
+        tc_commit(&bars->ring_empty[(2 * n + 1) % kDqStages]);
       }
-      for (int n = 0; n < n_ent && ok; ++n) {
-        const bool has_next = n + 1 < n_ent;
+      // the output of the tile before has been read
+      if (tiles > 0) ok = ok && mbar_wait(&bars->out_free, (tiles - 1) & 1u, ab, 0x1260u);
+      ++tiles;
+      for (; n < last && ok; ++n) {
+        const bool has_next = n + 1 < last;
         const uint32_t it_k = 2 * n, it_kn = 2 * n + 2, it_vn = 2 * n + 3;
         if (has_next) {
           ok = ring_wait(it_kn, 0x1220u);
@@ -284,7 +357,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           const SmemDesc db = make_smem_desc_sw128(ring_addr + (it_k % kDqStages) * kTileBytes, kHalfBytes, 1024);
 #pragma unroll
           for (int k = 0; k < 8; ++k)
-            umma_ts(t_dq, a_base + packed_a_col(k), desc_at(db, k * 2048), idesc_mn, (n > 0 || k > 0) ? 1u : 0u);
+            umma_ts(t_dq, a_base + packed_a_col(k), desc_at(db, k * 2048), idesc_mn, (n > first || k > 0) ? 1u : 0u);
           tc_commit(&bars->ring_empty[it_k % kDqStages]);
         }
         if (has_next) {
@@ -297,6 +370,8 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       }
       tc_commit(&bars->acc_done);
+      return ok;
+      });
     }
    }
   } else {
@@ -305,23 +380,29 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const int w = warp >> 2;       // column half this warpgroup owns
     const int wq = warp & 3;
     const int r = wq * 32 + lane;  // q row within the tile
-    const int q_row = q_tile * kTile + r;
+    const bool has_seg = p.q_seg != nullptr;
+    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
+    const float c = kSoftCap ? p.soft_cap * kLog2e : p.scale_log2;
+    uint32_t n = 0;      // steps so far
+    uint32_t tiles = 0;  // tiles with steps so far
+    each_tile(true, [&](const int4& work) {
+    const int head = work.y % p.q_heads, batch = work.y / p.q_heads;
+    const int4* entries = list_of(work);
+    const int n_ent = work.w - work.z;
+    const int q_row = work.x * kTile + r;
     const int qi = p.q_sequence ? p.q_sequence[q_row] : q_row;
     const RowInterval iv = mask_fn_interval(p.fn, qi);
-    const bool has_seg = p.q_seg != nullptr;
     const int q_seg = has_seg ? p.q_seg[(int64_t)batch * p.q_len + q_row] : 0;
     const int32_t* kv_seg_row = has_seg ? p.kv_seg + (int64_t)batch * p.kv_len : nullptr;
     const int64_t stat = ((int64_t)batch * p.q_heads + head) * p.q_len + q_row;
     const float nlse2 = p.nlse2[stat];
     const float ndelta = p.delta[stat];  // -di
-    const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
-    const float c = kSoftCap ? p.soft_cap * kLog2e : p.scale_log2;
     bool ok = true;
 
-    int4 ent_next = n_ent > 0 ? entries[ebeg] : make_int4(0, 0, 0, 0);
-    for (int n = 0; n < n_ent; ++n) {
+    int4 ent_next = n_ent > 0 ? entries[work.z] : make_int4(0, 0, 0, 0);
+    for (int e = work.z; e < work.w; ++e, ++n) {
       const int4 ent = ent_next;
-      if (n + 1 < n_ent) ent_next = entries[ebeg + n + 1];  // fetched a step ahead of its use
+      if (e + 1 < work.w) ent_next = entries[e + 1];  // fetched a step ahead of its use
       const int st = ent.y & 3;
       const int kv0 = ent.x * kTile + w * 64;
       const uint32_t t_s = tmem + lane_addr + (n & 1) * kTile;
@@ -428,7 +509,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     __nv_bfloat16* row0 = p.out0 + (int64_t)batch * p.out0_sb + (int64_t)head * p.out0_sh + (int64_t)(q_row - lane) * p.out0_ss;
     if (n_ent > 0) {
       if (ok) {
-        ok = mbar_wait(&bars->acc_done, 0, ab, 0x1500u);
+        ok = mbar_wait(&bars->acc_done, tiles++ & 1u, ab, 0x1500u);
         ok = __all_sync(0xffffffffu, ok);
       }
       if (ok) {
@@ -438,6 +519,11 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
           uint32_t v[32];
           tmem_ld32(tmem + lane_addr + 3 * kTile + w * 64 + g * 32, v);
           tmem_ld_wait();
+          if (g == 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bars->out_free);
+          }
           store_rows32(row0, p.out0_ss, v, p.scale, w * 64 + g * 32, p.d_qk);
         }
       }
@@ -448,6 +534,8 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       store_rows32(row0, p.out0_ss, v, 0.f, w * 64, p.d_qk);
       store_rows32(row0, p.out0_ss, v, 0.f, w * 64 + 32, p.d_qk);
     }
+    return ok;
+    });
   }
 
   tc_fence_before();
