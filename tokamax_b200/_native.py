@@ -362,6 +362,7 @@ def host():
         spec.loader.exec_module(module)
         module.bind_library(*(C.cast(getattr(handle, name), C.c_void_p).value for name in (
             "splash_fwd_shard", "splash_bwd_shard", "splash_bwd_workspace_bytes", "splash_bwd_fused_workspace_bytes")))
+        module.bind_check(check)
         _host = module
   return _host
 

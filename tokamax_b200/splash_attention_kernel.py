@@ -164,6 +164,8 @@ def _build_schedule(state: np.ndarray, pid: np.ndarray, block_q: int, block_kv: 
 class _DeviceTables:
   """Schedules, partial-mask blocks and the error record of one kernel object on one device."""
 
+  native = None  # the same for calls whose autograd function is native, made by the first of them
+
   def __init__(self, kernel: "SplashAttentionKernel", device: torch.device, shard: int = 0):
     cfg = kernel.config
     fwd, dkv = kernel.fwd_mask_info, kernel.dkv_mask_info
@@ -226,6 +228,8 @@ class _DynamicDeviceTables:
   The 128x128 tile states come from one pass over the mask, the three schedules from one small
   kernel each, and partial tiles are read from the mask itself (its transpose for dkv).
   """
+
+  native = None
 
   def __init__(self, mask: torch.Tensor, batch: int):
     lib = _native.lib()
@@ -316,6 +320,13 @@ def _in_class_of(source: torch.Tensor, result: torch.Tensor) -> torch.Tensor:
 
 def _plain(q, k, v, _tensor=torch.Tensor) -> bool:
   return type(q) is _tensor and type(k) is _tensor and type(v) is _tensor
+
+
+def _transformed() -> bool:
+  """Whether the call is traced or transformed: those see python's autograd function, and refuse it in their own words."""
+  # pylint: disable=protected-access
+  return (torch.compiler.is_compiling() or torch._C._get_tracing_state() is not None
+          or torch._C._functorch.peek_interpreter_stack() is not None)
 
 
 def _address(struct_or_none) -> int:
@@ -524,6 +535,20 @@ class SplashAttentionKernel:
       self._device_tables[key] = _DeviceTables(self, device, shard)
     return self._device_tables[key]
 
+  def _attention(self, q, k, v, scale: float, shard: int):
+    """`_SplashFunction` on these arguments, its forward and backward in native code."""
+    _require_cuda(q)
+    tables = self._tables(q.device, q.shape[0], shard)
+    host = _native.host()
+    native = tables.native
+    if native is None:
+      native = tables.native = host.Tables(C.addressof(tables.fwd), C.addressof(tables.dq), C.addressof(tables.dkv), tables.keep,
+                                           tables.error_record, tables.q_sequence, tables.q_shards)
+    # (the backward's form: head dims above 128 run separate passes, each repeatable bit for bit)
+    return host.attention(native, q, k, v, C.addressof(self._mask_fn), scale, max(self.mask_value, -3.0e38),
+                          float(self.config.attn_logits_soft_cap or 0.0),
+                          not self.repeatable_dq and q.shape[-1] <= _HEAD_DIM and v.shape[-1] <= _HEAD_DIM, self.head_shards)
+
   def check_errors(self) -> None:
     """Synchronises and raises if a kernel reported a device-side fault (bounded wait ran out).
 
@@ -619,8 +644,11 @@ class SplashAttentionKernel:
       if tuple(value.shape) not in ((), (1,), (hq,)):
         raise ValueError(f"max_logit_value should have shape (), (1,) or ({hq},), got {tuple(value.shape)}")
       max_logit = value.reshape(-1).expand(hq).contiguous()
-    apply = _function if _function is not None else _SplashFunction.apply
-    o, lse, max_logits = apply(q, k, v, q_seg, kv_seg, self, float(logits_scale), sinks, max_logit, int(q_shard))
+    if _function is None and q_seg is None and sinks is None and max_logit is None and _plain(q, k, v) and not _transformed():
+      o, lse, max_logits = self._attention(q, k, v, float(logits_scale), int(q_shard))
+    else:
+      apply = _function if _function is not None else _SplashFunction.apply
+      o, lse, max_logits = apply(q, k, v, q_seg, kv_seg, self, float(logits_scale), sinks, max_logit, int(q_shard))
     if not batched:
       o, lse, max_logits = o[0], lse[0], max_logits[0]
     if save_residuals:
