@@ -429,6 +429,12 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
       }
       const float c = fmaxf(kFp8 ? cq * ks : cq, kMinScaleLog2);
+      float v_share = 1.f, log_share = 0.f;
+      if constexpr (kFp8) {
+        v_share = fmaxf(__fdividef(vs, v_ref), 5.9604645e-8f);  // (so that a tile of zeros, scale 0, still counts in l)
+        log_share = __log2f(v_share);
+        asm volatile("" : "+f"(v_share), "+f"(log_share));  // (ahead of the wait for the scores)
+      }
       const int st = (ent.y >> (2 * i)) & 3;
       if (st == 0) continue;
       ok = mbar_wait(&bars->s_full[i], cnt & 1u, ab, 0x400u + i);
@@ -437,7 +443,7 @@ splash_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       ++cnt;
       tc_fence_after();
 
-      fwd_softmax_step<kFp8, kSoftCap, kP16>(p, &bars->p_half[i], &bars->p_full[i], t_s, t_o, i, lane, ent, st, c, vs, v_ref, iv,
+      fwd_softmax_step<kFp8, kSoftCap, kP16>(p, &bars->p_half[i], &bars->p_full[i], t_s, t_o, i, lane, ent, st, c, v_share, log_share, iv,
                                              q_row, has_seg, q_seg, kv_seg_row, fixed_max, started, m_used, m_true, l);
       started = true;
     }
