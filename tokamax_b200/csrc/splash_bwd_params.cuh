@@ -45,6 +45,7 @@ struct BwdParams {
   // stored as [col / 32][row / 32][col / 4 % 8][row % 32][col % 4]: a warp's 32 rows (TMEM lanes) of 32 columns
   // are 4 KiB in one piece
   float* dq_acc;
+  int dq_pairs;  // halves of its columns whose second chunk of 32 holds columns of dq too
 };
 
 // Column offset (32-bit TMEM columns) at which compute warpgroup w stores its 32 packed bf16

@@ -52,6 +52,7 @@ struct DeltaParams {
   // fused backward: the fp32 dQ image (one 128 x 128 tile per 128 rows, see BwdParams::dq_acc)
   // that the reductions of the dkv kernel add into; this pass clears it on the way.  nullptr: none.
   float* dq_image;
+  int dq_chunks;  // 32-column chunks of the image that hold columns of dq
 };
 
 // 64 rows per block: a warp takes eight rows, half a warp per row (16 lanes x 16 bytes = one row of
@@ -85,13 +86,21 @@ __global__ void __launch_bounds__(256) splash_delta_kernel(const DeltaParams p) 
       }
     }
     if (c0 == 0 && p.dq_image != nullptr) {
-      // The block's 64 rows are half of one image tile: in each 32-column chunk a run of 8 KiB.  256 threads x 8 stores
-      // of 16 bytes, issued under the loads.
+      // The block's 64 rows are half of one image tile: in each 32-column chunk a run of 8 KiB.  256 threads x two stores
+      // of 16 bytes for each, issued under the loads.
       float* tile = p.dq_image + (first / kTile) * (int64_t)(kTile * kHeadDim) + (first % kTile) * 32;
       const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+      auto clear = [&](int chunk) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-        *reinterpret_cast<uint4*>(tile + (i >> 1) * (kTile * 32) + (((i & 1) * 256 + (int)threadIdx.x) << 2)) = zero;
+        for (int i = 0; i < 2; ++i)
+          *reinterpret_cast<uint4*>(tile + chunk * (kTile * 32) + ((i * 256 + (int)threadIdx.x) << 2)) = zero;
+      };
+      if (p.dq_chunks == 4) {  // (a straight run of stores: tests between them cost this pass a fifth)
+#pragma unroll
+        for (int chunk = 0; chunk < 4; ++chunk) clear(chunk);
+      } else {
+        for (int chunk = 0; chunk < p.dq_chunks; ++chunk) clear(chunk);
+      }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -796,8 +805,10 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     setmaxnreg_dec<kFusedDrainRegs>();
     const int wq = warp & 3;
     const int half = (warp - kDkvDrainWarp) >> 2;
-    const bool two = p.d_qk > 64;  // columns 64 half .. + 63; with at most 64 of them in all, 32 half .. + 31
-    const int chunk = two ? 2 * half : half;
+    // Columns 64 half .. + 63; with at most 64 of them in all, 32 half .. + 31.  (Where dq has 96 at most the last 32 hold zeros
+    // and need not go; with late scores they do, for the registers: without them causal 4 x 8192 6941 -> 7004 us.)
+    const bool two = kLateS ? p.d_qk > 64 : p.dq_pairs > half;
+    const int chunk = p.d_qk > 64 ? 2 * half : half;
     const uint32_t t_dq = tmem + ((uint32_t)(wq * 32) << 16) + kTile + chunk * 32;
     uint8_t* stage = ring + 3 * kTileBytes + (warp - kDkvDrainWarp) * kDqBlockBytes;
     const int n_q_tiles = p.q_len / kTile;
@@ -1322,9 +1333,11 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 // ------------------------------------------------------------------------------------------
 // fused form: fp32 dQ image -> bf16 dQ
 // ------------------------------------------------------------------------------------------
-// One CTA per 128 x 128 tile.  A warp instruction reads eight 64-byte runs of the image (four rows
-// of one 4-column group each, see BwdParams::dq_acc) and writes four 64-byte runs of bf16 rows, so both sides move whole
-// 32-byte sectors; HBM-bound: 512 + 256 bytes per q row.
+// One CTA per 128 x 128 tile, a warp for 32 rows x 64 columns: a warp instruction reads 512 bytes of the image in one
+// piece (lane = row, as the rows came from TMEM) and writes 64-byte runs of eight bf16 rows; HBM-bound: 16 + 8 bytes for
+// four columns of a row.  32768 rows x 32 117 us = 6.9 TB/s, 1.05 of the measured copy rate (139 with 64-byte reads);
+// 32768 x 128 at a window: 314 -> 233.  Chunks beyond dq's columns are neither cleared nor read: 2 x 8192, 16 heads, d 64
+// 1243 -> 1216 us a pass.
 struct DqConvertParams {
   const float* acc;
   __nv_bfloat16* dq;
@@ -1341,30 +1354,24 @@ __global__ void __launch_bounds__(256) splash_dq_convert_kernel(const DqConvertP
   const int64_t bh = tile / p.n_q_tiles;
   const int h = (int)(bh % p.q_heads);
   const int64_t b = bh / p.q_heads;
-  const float4* src = reinterpret_cast<const float4*>(p.acc + tile * kDqTileFloats);
-  __nv_bfloat16* dst = p.dq + b * p.dq_sb + h * p.dq_sh + (int64_t)qt * kTile * p.dq_ss;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int jj = lane & 7, rr = lane >> 3;
-  float4 v[16];
+  const int wq = (threadIdx.x >> 5) & 3, half = threadIdx.x >> 7, lane = threadIdx.x & 31;
+  const int row = qt * kTile + wq * 32;
+  const uint4* src = reinterpret_cast<const uint4*>(p.acc + tile * kDqTileFloats) + lane;
+  uint4 x[2][8];
 #pragma unroll
-  for (int it = 0; it < 4; ++it)
+  for (int c = 0; c < 2; ++c)
+    if ((half * 2 + c) * 32 < p.d_qk)
 #pragma unroll
-    for (int jg = 0; jg < 4; ++jg) v[it * 4 + jg] = __ldcs(src + ((jg * 4 + warp / 2) * 8 + jj) * 32 + (warp & 1) * 16 + it * 4 + rr);
+      for (int j = 0; j < 8; ++j) x[c][j] = __ldcs(src + (((half * 2 + c) * 4 + wq) * 8 + j) * 32);
+  __nv_bfloat16* row0 = p.dq + b * p.dq_sb + h * p.dq_sh + (int64_t)row * p.dq_ss;
 #pragma unroll
-  for (int it = 0; it < 4; ++it) {
-    const int r = warp * 16 + it * 4 + rr;
+  for (int c = 0; c < 2; ++c) {
+    const int col0 = (half * 2 + c) * 32;
+    if (col0 >= p.d_qk) break;
+    uint32_t v[32];
 #pragma unroll
-    for (int jg = 0; jg < 4; ++jg) {
-      const float4 x = v[it * 4 + jg];
-      uint2 w;
-      w.x = pack_bf16(x.x * p.scale, x.y * p.scale);
-      w.y = pack_bf16(x.z * p.scale, x.w * p.scale);
-      if ((jg * 8 + jj) * 4 < p.d_qk) {
-        *reinterpret_cast<uint2*>(dst + (int64_t)r * p.dq_ss + (jg * 8 + jj) * 4) = w;
-        if (p.dq_peer.ptrs)
-          *reinterpret_cast<uint2*>(peer_row(p.dq_peer, (int)b, h, qt * kTile + r) + (jg * 8 + jj) * 4) = w;
-      }
-    }
+    for (int j = 0; j < 8; ++j) v[4 * j] = x[c][j].x, v[4 * j + 1] = x[c][j].y, v[4 * j + 2] = x[c][j].z, v[4 * j + 3] = x[c][j].w;
+    store_rows32_peer(row0, p.dq_ss, p.dq_peer, (int)b, h, row, v, p.scale, col0, p.d_qk);
   }
 }
 
@@ -1520,6 +1527,7 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
     dp.q_len = (int)Sq;
     dp.d_v = (int)Dv;
     dp.dq_image = fused ? dq_acc : nullptr;
+    dp.dq_chunks = (int)((D + 31) / 32);
     const unsigned blocks = (unsigned)(B * Hq * Sq / kDeltaRowsPerBlock);
     splash_delta_kernel<<<blocks, 256, 0, stream>>>(dp);
     if (cudaGetLastError() != cudaSuccess) return SPLASH_ERR_CUDA;
@@ -1572,6 +1580,7 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   p.soft_cap = a.soft_cap;
   p.softcap_a = soft_cap ? a.scale / a.soft_cap : 0.f;
   p.dq_acc = fused ? dq_acc : nullptr;
+  p.dq_pairs = D > 96 ? 2 : D > 64 ? 1 : 0;
   if (wide) return launch_bwd_wide(tm_q, tm_do, tm_k, tm_v, p, a, soft_cap, mask, stream);
 
   // dq (split form)
