@@ -61,6 +61,42 @@ def test_soft_cap_forward_backward(cap, scale, dims, kind):
     assert _rel(got, ref) <= 1e-2
 
 
+# A warp whose arguments of tanh are all at most 1/2 takes a polynomial, any other the special functions.  A tile has warps of
+# either kind here: queries grow in runs of 16 rows until the largest argument of a run lies at `top` and around it.  Of rows
+# 0 and 64 .. the arguments are zero and tiny.
+@pytest.mark.parametrize("repeatable", [False, True])
+@pytest.mark.parametrize("d,kind", [(128, "full"), (128, "causal"), (64, "full"), (256, "full"), (192, "causal")])
+@pytest.mark.parametrize("top", [0.49, 0.5, 0.51, 40.0])
+def test_both_forms_of_tanh_in_one_tile(d, kind, top, repeatable):
+  s, cap, scale = 256, 20.0, 1 / math.sqrt(d)
+  g = torch.Generator().manual_seed(d)
+  q, k, v, do = (torch.randn(1, 1, s, d, generator=g, dtype=torch.float64) for _ in range(4))
+  largest = (q @ k.transpose(-1, -2)).abs().amax(-1, keepdim=True) * scale / cap
+  grow = torch.tensor([0.0, 1e-4, 0.1, 0.5, 0.9, 1.0, 1.0, 1.2]).repeat_interleave(16).repeat(2).view(1, 1, s, 1)
+  q, k, v, do = (t.to(torch.bfloat16) for t in (q / largest * top * grow, k, v, do))
+  mask = mask_lib.FullMask((s, s)) if kind == "full" else mask_lib.CausalMask((s, s))
+  dense = np.tril(np.ones((s, s), np.bool_)) if kind == "causal" else np.ones((s, s), np.bool_)
+  cfg = dataclasses.replace(splash.SplashConfig.get_default(), attn_logits_soft_cap=cap)
+  kernel = splash.make_splash_mha(mask, config=cfg, q_seq_shards=1, save_residuals=True, repeatable_dq=repeatable)
+  ts = [t.to(DEV).requires_grad_(True) for t in (q, k, v)]
+  out, res = kernel(*ts, logits_scale=scale)
+  grads = torch.autograd.grad(out, ts, do.to(DEV))
+  kernel.check_errors()
+  wide = [t.double().requires_grad_(True) for t in (q, k, v)]
+  x = cap * torch.tanh(wide[0] @ wide[1].transpose(-1, -2) * (scale / cap))
+  x = x.masked_fill(~torch.from_numpy(dense), -math.inf)
+  ro = torch.softmax(x, -1) @ wide[2]
+  rgrads = torch.autograd.grad(ro, wide, do.double())
+  # tanh to 1e-6 absolute times the cap, and fp32 sums of d products and of s weights
+  bound = cap * 1e-6 + 1e-5
+  assert (res["logsumexp"].cpu().double() - torch.logsumexp(x, -1)).abs().max().item() <= bound
+  assert (res["max_logits"].cpu().double() - x.amax(-1)).abs().max().item() <= bound
+  # P and the output are rounded to 8 bits, half an ulp (2^-9) each
+  assert (out.cpu().double() - ro).abs().max().item() <= 2.0 ** -8 * v.double().abs().max().item()
+  for got, want in zip(grads, rgrads):
+    assert ((got.cpu().double() - want).norm() / want.norm()).item() <= 1e-2
+
+
 def test_soft_cap_changes_the_result_and_rejects_bad_values():
   s = 256
   g = torch.Generator().manual_seed(3)

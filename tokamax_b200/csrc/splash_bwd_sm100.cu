@@ -432,8 +432,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
         }
       }
       if constexpr (kSoftCap) {  // pr <- tanh(scale * s / cap), capped before it is masked
-#pragma unroll
-        for (int j = 0; j < 64; ++j) pr[j] = tanh_ex2(pr[j] * p.softcap_a);
+        tanh_all(pr, p.softcap_a);
       }
       if (st == 1) {
         if (p.fn.kind != SPLASH_MASK_TABLE) {
@@ -1114,9 +1113,13 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 #pragma unroll
           for (int j = 0; j < 32; ++j) pr[j] = __uint_as_float(v[j]);
         }
+        // Soft cap: tiles without a mask take tanh beside the exponentials (one pass behind the other keeps the FMA units waiting
+        // for the special-function ones and these for them)
+        bool beside = false;
         if constexpr (kSoftCap) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) pr[j] = tanh_ex2(pr[j] * p.softcap_a);
+          const bool small = tanh_is_small(pr, p.softcap_a);
+          beside = small && st != 1 && !(has_seg && !((ent.y >> 4) & 1));
+          if (!beside) tanh_all(pr, p.softcap_a, small);
         }
         if (st == 1) {
           if (p.fn.kind != SPLASH_MASK_TABLE) {
@@ -1158,7 +1161,32 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             if (sv.w != kv_seg) pr[t * 4 + 3] = kMaskedLogit;
           }
         }
-        {
+        auto send_p = [&](const uint32_t (&pk)[16]) {
+          tmem_st16(t_st, pk);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars->p_full);
+        };
+        if (kSoftCap && beside) {
+          uint32_t pk[16];
+          const float2 a2 = make_float2(p.softcap_a, p.softcap_a), c2 = make_float2(c, c);
+#pragma unroll
+          for (int t = 0; t < 8; ++t) {
+            const float4 nl = nl4[t];
+            const float2 ta = tanh_small(__fmul2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]), a2));
+            const float2 tb = tanh_small(__fmul2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]), a2));
+            const float2 xa = __ffma2_rn(ta, c2, make_float2(nl.x, nl.y)), xb = __ffma2_rn(tb, c2, make_float2(nl.z, nl.w));
+            const float p0 = ex2(xa.x), p1 = ex2(xa.y), p2 = ex2(xb.x), p3 = ex2(xb.y);
+            pk[2 * t] = pack_bf16(p0, p1);
+            pk[2 * t + 1] = pack_bf16(p2, p3);
+            pr[4 * t + 0] = p0 * fmaf(-ta.x, ta.x, 1.0f);
+            pr[4 * t + 1] = p1 * fmaf(-ta.y, ta.y, 1.0f);
+            pr[4 * t + 2] = p2 * fmaf(-tb.x, tb.x, 1.0f);
+            pr[4 * t + 3] = p3 * fmaf(-tb.y, tb.y, 1.0f);
+          }
+          send_p(pk);
+        } else {
           uint32_t pk[16];
 #pragma unroll
           for (int t = 0; t < 8; ++t) {
@@ -1183,11 +1211,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
               for (int u = 0; u < 4; ++u) pr[4 * t + u] *= fmaf(-th[u], th[u], 1.0f);
             }
           }
-          tmem_st16(t_st, pk);
-          tmem_st_wait();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&bars->p_full);
+          send_p(pk);
         }
         ok = mbar_wait(&bars->dpt_full, ph, ab, 0x3410u);
         ok = __all_sync(0xffffffffu, ok);

@@ -526,8 +526,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
             if (lane == 0) mbar_arrive(&bars->s_free[set]);
           }
           if constexpr (kSoftCap) {  // pr <- tanh(scale * s / cap), capped before it is masked
-#pragma unroll
-            for (int j = 0; j < 32; ++j) pr[j] = tanh_ex2(pr[j] * p.softcap_a);
+            tanh_all(pr, p.softcap_a);
           }
           if (st == 1) {
             if (p.fn.kind != SPLASH_MASK_TABLE) {

@@ -146,8 +146,7 @@ __device__ __forceinline__ void fwd_softmax_step(const FwdParams& p, uint64_t* p
   if constexpr (kSoftCap) {
     // s <- tanh(scale * s / cap) before masking (reference :202-296 caps, then masks); the
     // factor cap * log2(e) that follows is `c`.
-#pragma unroll
-    for (int j = 0; j < kTile; ++j) s[j] = tanh_ex2(s[j] * p.softcap_a);
+    tanh_all(s, p.softcap_a);
   }
   const int kv0 = ent.x * kTile;
   if (st == 1) {

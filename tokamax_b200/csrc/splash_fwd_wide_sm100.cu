@@ -412,8 +412,7 @@ splash_fwd_wide_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_co
           }
         }
         if constexpr (kSoftCap) {
-#pragma unroll
-          for (int j = 0; j < kSub; ++j) s[j] = tanh_ex2(s[j] * p.softcap_a);
+          tanh_all(s, p.softcap_a);
         }
         const int kv0 = ent.x * kTile + set * kSub;  // first key of this step
         if (st == 1) {
