@@ -79,3 +79,29 @@ def test_rows_with_no_live_key_anywhere(scale):
   assert torch.count_nonzero(dq[:, :, dead]) == 0
   assert _rel(dq[:, :, alive], rdq[:, :, alive]) <= 1e-2
   assert _rel(kd.grad, rdk) <= 1e-2 and _rel(vd.grad, rdv) <= 1e-2
+
+
+@pytest.mark.parametrize("dims", [(64, 64), (128, 128), (192, 128), (256, 256)])
+@pytest.mark.parametrize("repeatable", [False, True])
+@pytest.mark.parametrize("kind", ["table", "segments", "window"])
+def test_one_key_a_row(kind, repeatable, dims):
+  """Every mask form of the backward at every place of a tile: row i sees key perm[i] alone, so o = v[perm] and
+  dv[perm] = do.  Equal to the bit: p differs from 1 by the rounding of an exponent below 32 in 32 bits, under 1e-5, and
+  is 1 in bf16; a key moved by one row or column would be another row of do."""
+  s = 256
+  d_qk, d_v = dims
+  g = torch.Generator().manual_seed(83 + d_qk)
+  mk = lambda d: torch.randn(1, 2, s, d, generator=g).to(torch.bfloat16)
+  q, k, v, do = mk(d_qk), mk(d_qk), mk(d_v), mk(d_v)
+  perm = torch.arange(s) if kind == "window" else torch.randperm(s, generator=g)
+  dense = np.zeros((s, s), bool)
+  dense[np.arange(s), perm.numpy()] = True
+  mask = {"table": dense, "segments": mask_lib.FullMask((s, s)), "window": mask_lib.LocalMask((s, s), (0, 0), 0)}[kind]
+  seg = splash.SegmentIds(torch.arange(s, dtype=torch.int32, device=DEV), torch.argsort(perm).to(torch.int32).to(DEV)) if kind == "segments" else None
+  qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+  kernel = splash.make_splash_mha_single_device(mask, repeatable_dq=repeatable)
+  out = kernel(qd, kd, vd, seg, logits_scale=1 / math.sqrt(d_qk))
+  out.backward(do.to(DEV))
+  kernel.check_errors()
+  assert torch.equal(out.cpu(), v[:, :, perm])
+  assert torch.equal(vd.grad.cpu()[:, :, perm], do)

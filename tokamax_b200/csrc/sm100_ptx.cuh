@@ -424,6 +424,33 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
         "r"(r[14]), "r"(r[15])
       : "memory");
 }
+// 16x256b / 16x128b: 16 lanes of TMEM (the lane in taddr and the 15 behind it), in the fragments of the matrix instructions:
+// thread t holds rows t / 4 and t / 4 + 8.  A load brings 32-bit columns 8 k + 2 (t % 4) and the one behind it as
+// r[4 k + 2 h], r[4 k + 2 h + 1] (h: which of the two rows); a store takes column 4 k + t % 4 from r[2 k + h], so that the
+// 16-bit pairs of a load's columns go back as they lie.
+__device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_frag(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+      : "memory");
+}
+// Four 8 x 8 matrices of 16-bit values from such fragments to shared memory: thread t gives the address of row t % 8 of
+// matrix t / 8.
+__device__ __forceinline__ void stmatrix_x4(uint32_t saddr, uint32_t m0, uint32_t m1, uint32_t m2, uint32_t m3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(m0), "r"(m1), "r"(m2),
+               "r"(m3)
+               : "memory");
+}
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }

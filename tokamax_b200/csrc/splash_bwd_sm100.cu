@@ -558,7 +558,7 @@ splash_dq_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 // ------------------------------------------------------------------------------------------
 // dkv kernel
 // ------------------------------------------------------------------------------------------
-// 16 compute warps (thread = kv row x one 32-column quarter of the q tile) keep the P^T / dS^T
+// 16 compute warps (32 kv rows x one 32-column quarter of the q tile each) keep the P^T / dS^T
 // phases short; warp 16 feeds TMA, warp 17 issues MMAs, warps 18-19 are idle (they complete the
 // fifth warpgroup).
 constexpr int kDkvThreads = 640;
@@ -603,6 +603,7 @@ constexpr int kDkvStatsBytes = (kBwdStages / 2) * 2 * kTile * 4;
 constexpr int kDkvSmemBytes = (3 + kBwdStages) * kTileBytes + kDkvStatsBytes + 512;
 
 constexpr uint32_t kDkvWork = 2;
+constexpr uint32_t kLanes16 = 16u << 16;  // 16 lanes on in a TMEM address
 
 struct DkvBarriers {
   uint64_t answer[2];  // cluster launch control: what the request for the next tile returned
@@ -647,6 +648,12 @@ static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 // bitwise repeatable.  For grids that leave SMs idle; split_for() holds the rule.
 constexpr int kDkvPartWords = 2 * kHeadDim / 4 * kTile;  // 16-byte words: [dk, dv column / 4][kv row]
 static_assert(kDkvPartWords * 16 <= (3 + kBwdStages) * kTileBytes, "the parts lie over the operand tiles");
+
+// Bit i: byte i of w is not 0.  (The product brings the four bits, 8 apart, side by side.)
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
+  const uint32_t top = (((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) & 0x80808080u;
+  return (top >> 7) * 0x01020408u >> 24;
+}
 
 template <bool kSoftCap, bool kFuseDq, bool kSplit, bool kLateS, bool kOneTile = kSplit>
 __global__ void __launch_bounds__(kFuseDq ? kFusedThreads : kDkvThreads, 1)
@@ -1058,7 +1065,14 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     }
    }
   } else {
-    // 16 warps on one 128 x 128 tile: thread = kv row (TMEM lane) x one 32-column quarter.
+    // 16 warps on one 128 x 128 tile: a warp has 32 kv rows (TMEM lanes) x one 32-column quarter, which its threads hold as
+    // matrix fragments (tmem_ld_frag): four rows x eight columns each.  The statistics belong to columns.  With a row
+    // and 32 columns a thread, every warp read 32 columns' pairs in 16 LDS.128, all lanes the same address: 837 of some
+    // 4600 cycles a step of the shared-memory data pipe, which the kernel kept 99 % busy (MMAs 51 %, loads and stores 48 %).
+    // In fragments they are eight LDS.64, and dS^T goes out by stmatrix without bank conflicts.  A row a thread -> this,
+    // us a pass: 4 x 8192, 32 / 8 6977 -> 6860, 8 x 16384, 16 heads, window 4096 6315 -> 6118, 4 x 2048, 16 / 16 330 -> 313,
+    // 2 x 8192, 16 / 4, d 64 1209 -> 1185, repeatable 2 x 4096, 16 / 1 496 -> 480, soft cap 4 x 4096, 16 / 8, window 768
+    // 641 -> 589.
     if constexpr (kFuseDq) setmaxnreg_inc<kFusedComputeRegs>();
     const int cq = warp >> 2;      // column quarter 0..3
     const int wq = warp & 3;       // TMEM lane quarter
@@ -1067,16 +1081,20 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const uint32_t lane_addr = (uint32_t)(wq * 32) << 16;
     const uint32_t t_st = tmem + lane_addr + cq * 32;
     const uint32_t t_dpt = tmem + lane_addr + kTile + cq * 32;
-    // dS^T row r, columns cq*32 .. +31: 64 bytes = four 16-byte chunks of the row's 128-byte
-    // segment in swizzle half cq / 2; chunk c sits at position c ^ (r mod 8)
-    uint8_t* ds_row = ds_smem + (cq >> 1) * kHalfBytes + r * 128;
-    const int chunk0 = (cq & 1) * 4;
+    // Element at(k, hq) + u: kv row row0 + 8 hq, q column col0 + 8 k + u of the quarter.
+    auto at = [](int k, int hq) { return 16 * (hq >> 1) + 4 * k + 2 * (hq & 1); };
+    const int row0 = wq * 32 + (lane >> 2);
+    const int col0 = 2 * (lane & 3);
+    // dS^T rows row.., columns cq*32 .. +31: 64 bytes = four 16-byte chunks of the row's 128-byte
+    // segment in swizzle half cq / 2; chunk c sits at position c ^ (row mod 8).  Lane: row lane % 8, chunk lane / 8.
+    const uint32_t ds_addr = smem_u32(ds_smem) + (cq >> 1) * kHalfBytes + (wq * 32 + (lane & 7)) * 128 +
+                             ((((cq & 1) * 4 + (lane >> 3)) ^ (lane & 7)) << 4);
     const float c = kSoftCap ? p.soft_cap * kLog2e : p.scale_log2;
     uint32_t n = 0;      // steps so far
     uint32_t tiles = 0;  // tiles with steps so far
     each_tile(true, true, [&](const int4& w) {
-    const int kv_row = w.x * kTile + r;
-    const int kv_seg = has_seg ? p.kv_seg[(int64_t)(w.y / p.kv_heads) * p.kv_len + kv_row] : 0;
+    const int kv_row = w.x * kTile + row0;
+    const int32_t* kv_seg_row = has_seg ? p.kv_seg + (int64_t)(w.y / p.kv_heads) * p.kv_len + kv_row : nullptr;
     const int32_t* q_seg_row = has_seg ? p.q_seg + (int64_t)(w.y / p.kv_heads) * p.q_len : nullptr;
     const int4* entries = list_of(w);
     const int ebeg = w.z, eend = w.w;
@@ -1097,9 +1115,22 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         if (!ok) break;
         if constexpr (kSplit) ent = bars->step[(itq % kBwdStages) / 2];
         const int st = ent.y & 3;
-        const int q0 = ent.x * kTile + cq * 32;  // first q column of this thread's 32
-        const float4* nl4 = reinterpret_cast<const float4*>(stats + ((itq % kBwdStages) / 2) * 2 * kTile + cq * 32);
-        const float4* dl4 = nl4 + kTile / 4;
+        const int q0 = ent.x * kTile + cq * 32 + col0;  // first q column of this thread
+        // columns 8 k + 0, 1: word 4 k
+        const float2* nl2 = reinterpret_cast<const float2*>(stats + ((itq % kBwdStages) / 2) * 2 * kTile + cq * 32 + col0);
+        const float2* dl2 = nl2 + kTile / 2;
+        // table: a lane reads eight columns of its four rows and keeps a bit for each of them, row by row (two columns at a
+        // time, as they are used, took 16 loads: prefix 2 x 4096, 16 / 4 631 us a pass instead of 577)
+        uint32_t mask_bits = 0;
+        if (st == 1 && p.fn.kind == SPLASH_MASK_TABLE) {
+          const int8_t* mrow = p.pmb + ((int64_t)ent.z * p.pm_bkv + (kv_row % p.pm_bkv)) * p.pm_bq +
+                               ((ent.x * kTile + cq * 32) % p.pm_bq) + 8 * (lane & 3);
+#pragma unroll
+          for (int hq = 0; hq < 4; ++hq) {
+            const int2 m = __ldg(reinterpret_cast<const int2*>(mrow + (int64_t)(8 * hq) * p.pm_bq));
+            mask_bits |= (nonzero_bytes((uint32_t)m.x) | nonzero_bytes((uint32_t)m.y) << 4) << (8 * hq);
+          }
+        }
 
         ok = mbar_wait(&bars->st_full, ph, ab, 0x3400u);
         ok = __all_sync(0xffffffffu, ok);
@@ -1108,7 +1139,8 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         float pr[32];
         {
           uint32_t v[32];
-          tmem_ld32(t_st, v);
+          tmem_ld_frag(t_st, v);
+          tmem_ld_frag(t_st + kLanes16, v + 16);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) pr[j] = __uint_as_float(v[j]);
@@ -1123,46 +1155,45 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         }
         if (st == 1) {
           if (p.fn.kind != SPLASH_MASK_TABLE) {
-            if (p.q_sequence == nullptr) {
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const RowInterval iv = mask_fn_interval(p.fn, q0 + j);
-                if (kv_row < iv.lo || kv_row > iv.hi) pr[j] = kMaskedLogit;
-              }
-            } else {
+            for (int k = 0; k < 4; ++k)
 #pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const RowInterval iv = mask_fn_interval(p.fn, __ldg(p.q_sequence + q0 + j));
-                if (kv_row < iv.lo || kv_row > iv.hi) pr[j] = kMaskedLogit;
+              for (int u = 0; u < 2; ++u) {
+                const int q = q0 + 8 * k + u;
+                const RowInterval iv = mask_fn_interval(p.fn, p.q_sequence == nullptr ? q : __ldg(p.q_sequence + q));
+#pragma unroll
+                for (int hq = 0; hq < 4; ++hq)
+                  if (kv_row + 8 * hq < iv.lo || kv_row + 8 * hq > iv.hi) pr[at(k, hq) + u] = kMaskedLogit;
               }
-            }
           } else {
-            const int8_t* mrow = p.pmb + ((int64_t)ent.z * p.pm_bkv + (kv_row % p.pm_bkv)) * p.pm_bq +
-                                 (q0 % p.pm_bq);
-            const int4* m4 = reinterpret_cast<const int4*>(mrow);
 #pragma unroll
-            for (int t = 0; t < 2; ++t) {
-              const int4 mv = __ldg(m4 + t);
-              const uint32_t wd[4] = {(uint32_t)mv.x, (uint32_t)mv.y, (uint32_t)mv.z, (uint32_t)mv.w};
+            for (int k = 0; k < 4; ++k) {  // lane 4 i + k of the four that share the rows holds columns 8 k .. + 7
+              const uint32_t mine = __shfl_sync(0xffffffffu, mask_bits, k, 4) >> col0;
 #pragma unroll
-              for (int j = 0; j < 16; ++j)
-                if (((wd[j >> 2] >> ((j & 3) * 8)) & 0xffu) == 0u) pr[t * 16 + j] = kMaskedLogit;
+              for (int hq = 0; hq < 4; ++hq)
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+                  if (((mine >> (8 * hq + u)) & 1u) == 0u) pr[at(k, hq) + u] = kMaskedLogit;
             }
           }
         }
         if (has_seg && !((ent.y >> 4) & 1)) {  // (bit set: the whole tile lies inside one segment)
-          const int4* sg4 = reinterpret_cast<const int4*>(q_seg_row + q0);
+          int kv_seg[4];
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const int4 sv = __ldg(sg4 + t);
-            if (sv.x != kv_seg) pr[t * 4 + 0] = kMaskedLogit;
-            if (sv.y != kv_seg) pr[t * 4 + 1] = kMaskedLogit;
-            if (sv.z != kv_seg) pr[t * 4 + 2] = kMaskedLogit;
-            if (sv.w != kv_seg) pr[t * 4 + 3] = kMaskedLogit;
+          for (int hq = 0; hq < 4; ++hq) kv_seg[hq] = __ldg(kv_seg_row + 8 * hq);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int2 sv = __ldg(reinterpret_cast<const int2*>(q_seg_row + q0) + 4 * k);
+#pragma unroll
+            for (int hq = 0; hq < 4; ++hq) {
+              if (sv.x != kv_seg[hq]) pr[at(k, hq)] = kMaskedLogit;
+              if (sv.y != kv_seg[hq]) pr[at(k, hq) + 1] = kMaskedLogit;
+            }
           }
         }
         auto send_p = [&](const uint32_t (&pk)[16]) {
-          tmem_st16(t_st, pk);
+          tmem_st_frag(t_st, pk);
+          tmem_st_frag(t_st + kLanes16, pk + 8);
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
@@ -1172,43 +1203,37 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           uint32_t pk[16];
           const float2 a2 = make_float2(p.softcap_a, p.softcap_a), c2 = make_float2(c, c);
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const float4 nl = nl4[t];
-            const float2 ta = tanh_small(__fmul2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]), a2));
-            const float2 tb = tanh_small(__fmul2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]), a2));
-            const float2 xa = __ffma2_rn(ta, c2, make_float2(nl.x, nl.y)), xb = __ffma2_rn(tb, c2, make_float2(nl.z, nl.w));
-            const float p0 = ex2(xa.x), p1 = ex2(xa.y), p2 = ex2(xb.x), p3 = ex2(xb.y);
-            pk[2 * t] = pack_bf16(p0, p1);
-            pk[2 * t + 1] = pack_bf16(p2, p3);
-            pr[4 * t + 0] = p0 * fmaf(-ta.x, ta.x, 1.0f);
-            pr[4 * t + 1] = p1 * fmaf(-ta.y, ta.y, 1.0f);
-            pr[4 * t + 2] = p2 * fmaf(-tb.x, tb.x, 1.0f);
-            pr[4 * t + 3] = p3 * fmaf(-tb.y, tb.y, 1.0f);
+          for (int k = 0; k < 4; ++k) {
+            const float2 nl = nl2[4 * k];
+#pragma unroll
+            for (int hq = 0; hq < 4; ++hq) {
+              const int j = at(k, hq);
+              const float2 th = tanh_small(__fmul2_rn(make_float2(pr[j], pr[j + 1]), a2));
+              const float2 x = __ffma2_rn(th, c2, nl);
+              const float p0 = ex2(x.x), p1 = ex2(x.y);
+              pk[j / 2] = pack_bf16(p0, p1);
+              pr[j] = p0 * fmaf(-th.x, th.x, 1.0f);
+              pr[j + 1] = p1 * fmaf(-th.y, th.y, 1.0f);
+            }
           }
           send_p(pk);
         } else {
           uint32_t pk[16];
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const float4 nl = nl4[t];
-            float th[4];
-            if constexpr (kSoftCap) {
+          for (int k = 0; k < 4; ++k) {
+            const float2 nl = nl2[4 * k];
 #pragma unroll
-              for (int u = 0; u < 4; ++u) th[u] = fmaxf(pr[4 * t + u], -1.0f);
-            }
-            const float2 xa = __ffma2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]), make_float2(c, c),
-                                         make_float2(nl.x, nl.y));
-            const float2 xb = __ffma2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]), make_float2(c, c),
-                                         make_float2(nl.z, nl.w));
-            pr[4 * t + 0] = ex2(xa.x);
-            pr[4 * t + 1] = ex2(xa.y);
-            pr[4 * t + 2] = ex2(xb.x);
-            pr[4 * t + 3] = ex2(xb.y);
-            pk[2 * t] = pack_bf16(pr[4 * t + 0], pr[4 * t + 1]);
-            pk[2 * t + 1] = pack_bf16(pr[4 * t + 2], pr[4 * t + 3]);
-            if constexpr (kSoftCap) {
-#pragma unroll
-              for (int u = 0; u < 4; ++u) pr[4 * t + u] *= fmaf(-th[u], th[u], 1.0f);
+            for (int hq = 0; hq < 4; ++hq) {
+              const int j = at(k, hq);
+              const float2 th = make_float2(fmaxf(pr[j], -1.0f), fmaxf(pr[j + 1], -1.0f));
+              const float2 x = __ffma2_rn(make_float2(pr[j], pr[j + 1]), make_float2(c, c), nl);
+              pr[j] = ex2(x.x);
+              pr[j + 1] = ex2(x.y);
+              pk[j / 2] = pack_bf16(pr[j], pr[j + 1]);
+              if constexpr (kSoftCap) {
+                pr[j] *= fmaf(-th.x, th.x, 1.0f);
+                pr[j + 1] *= fmaf(-th.y, th.y, 1.0f);
+              }
             }
           }
           send_p(pk);
@@ -1220,19 +1245,19 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
         uint32_t pk[16];
         {
           uint32_t v[32];
-          tmem_ld32(t_dpt, v);
+          tmem_ld_frag(t_dpt, v);
+          tmem_ld_frag(t_dpt + kLanes16, v + 16);
           tmem_ld_wait();
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const float4 nd = dl4[t];  // -di of the four query columns
-            const float2 a = __fmul2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]),
-                                        __fadd2_rn(make_float2(__uint_as_float(v[4 * t + 0]), __uint_as_float(v[4 * t + 1])),
-                                                   make_float2(nd.x, nd.y)));
-            const float2 b = __fmul2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]),
-                                        __fadd2_rn(make_float2(__uint_as_float(v[4 * t + 2]), __uint_as_float(v[4 * t + 3])),
-                                                   make_float2(nd.z, nd.w)));
-            pk[2 * t] = pack_bf16(a.x, a.y);
-            pk[2 * t + 1] = pack_bf16(b.x, b.y);
+          for (int k = 0; k < 4; ++k) {
+            const float2 nd = dl2[4 * k];  // -di of the two query columns
+#pragma unroll
+            for (int hq = 0; hq < 4; ++hq) {
+              const int j = at(k, hq);
+              const float2 a = __fmul2_rn(make_float2(pr[j], pr[j + 1]),
+                                          __fadd2_rn(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), nd));
+              pk[j / 2] = pack_bf16(a.x, a.y);
+            }
           }
         }
         if (n > 0) {  // the previous step's dK must have finished reading the tile
@@ -1241,9 +1266,9 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
           if (!ok) break;
         }
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
-          const uint4 w = make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]);
-          *reinterpret_cast<uint4*>(ds_row + (((chunk0 + ch) ^ (r & 7)) << 4)) = w;
+        for (int hq = 0; hq < 4; ++hq) {
+          const int j = 8 * (hq >> 1) + (hq & 1);
+          stmatrix_x4(ds_addr + hq * 1024, pk[j], pk[j + 2], pk[j + 4], pk[j + 6]);
         }
         fence_proxy_async_smem();  // generic-proxy stores -> visible to the MMA's async-proxy reads
         __syncwarp();
