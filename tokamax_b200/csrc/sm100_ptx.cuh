@@ -428,6 +428,7 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 // thread t holds rows t / 4 and t / 4 + 8.  A load brings 32-bit columns 8 k + 2 (t % 4) and the one behind it as
 // r[4 k + 2 h], r[4 k + 2 h + 1] (h: which of the two rows); a store takes column 4 k + t % 4 from r[2 k + h], so that the
 // 16-bit pairs of a load's columns go back as they lie.
+constexpr uint32_t kLanes16 = 16u << 16;  // 16 lanes on in a TMEM address
 __device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
@@ -524,6 +525,12 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
+}
+
+// Bit i: byte i of w is not 0.  (The product brings the four bits, 8 apart, side by side.)
+__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
+  const uint32_t top = (((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) & 0x80808080u;
+  return (top >> 7) * 0x01020408u >> 24;
 }
 
 // Register reallocation between warpgroups (all four warps of a warpgroup must execute it).

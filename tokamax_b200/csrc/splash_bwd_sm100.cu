@@ -603,7 +603,6 @@ constexpr int kDkvStatsBytes = (kBwdStages / 2) * 2 * kTile * 4;
 constexpr int kDkvSmemBytes = (3 + kBwdStages) * kTileBytes + kDkvStatsBytes + 512;
 
 constexpr uint32_t kDkvWork = 2;
-constexpr uint32_t kLanes16 = 16u << 16;  // 16 lanes on in a TMEM address
 
 struct DkvBarriers {
   uint64_t answer[2];  // cluster launch control: what the request for the next tile returned
@@ -648,12 +647,6 @@ static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 // bitwise repeatable.  For grids that leave SMs idle; split_for() holds the rule.
 constexpr int kDkvPartWords = 2 * kHeadDim / 4 * kTile;  // 16-byte words: [dk, dv column / 4][kv row]
 static_assert(kDkvPartWords * 16 <= (3 + kBwdStages) * kTileBytes, "the parts lie over the operand tiles");
-
-// Bit i: byte i of w is not 0.  (The product brings the four bits, 8 apart, side by side.)
-__device__ __forceinline__ uint32_t nonzero_bytes(uint32_t w) {
-  const uint32_t top = (((w & 0x7f7f7f7fu) + 0x7f7f7f7fu) | w) & 0x80808080u;
-  return (top >> 7) * 0x01020408u >> 24;
-}
 
 template <bool kSoftCap, bool kFuseDq, bool kSplit, bool kLateS, bool kOneTile = kSplit>
 __global__ void __launch_bounds__(kFuseDq ? kFusedThreads : kDkvThreads, 1)
@@ -1459,9 +1452,10 @@ static bool one_tile_ctas(const SplashBwdArgs& a) {
 }
 // Whether S^T of the next step is issued behind dQ of this one instead of behind dV.  d 128: causal 4 x 8192, 32 / 8 heads
 // 7198 -> 7038 us a pass, 2 x 4096 1022 -> 999, 4 x 2048, 16 / 16 366 -> 358; full 1 x 4096, 32 / 8 991 -> 958; packed windows
-// 8 x 16384 6678 -> 6598.  Where forming P^T takes longer it wants its scores early: partial blocks read from a table (prefix 2 x
-// 4096, 16 / 4: 623 -> 641), a soft cap (187 -> 193); so it does where the scores are half as long (d 64, 2 x 8192, 16 / 4:
-// 1270 -> 1479).  Without dQ there is nothing to put them behind (4 x 4096, 16 / 8: behind dS^T's arrival 1097 -> 1158).
+// 8 x 16384 6678 -> 6598.  Where forming P^T takes longer it wants its scores early: partial blocks read from a table (prefix
+// 1 x 8192, 16 / 16, d 96 928 -> 960, 4 x 1024, 32 / 8 282 -> 289, if 2 x 4096, 16 / 4 575 -> 569), a soft cap (187 -> 193); so it
+// does where the scores are half as long (d 64, 2 x 8192, 16 / 4: 1181 -> 1356).  Without dQ there is nothing to put them behind
+// (4 x 4096, 16 / 8: behind dS^T's arrival 1097 -> 1158).
 static bool late_scores(const SplashBwdArgs& a, bool fused) {
   const bool table = a.mask_fn.kind == SPLASH_MASK_TABLE && a.sched_dkv.partial_mask_blocks != nullptr;
   return fused && a.soft_cap == 0.f && a.q.size[3] > 64 && !table;

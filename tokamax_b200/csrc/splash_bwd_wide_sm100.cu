@@ -467,24 +467,47 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
     };
 
     bool ok = take_work(cur);
+    // The dkv pass holds scores as matrix fragments, as the dkv kernel of the narrower heads does: statistics belong to columns
+    // there, and a thread then needs those of 8 instead of 32.  (192, 128): causal 2 x 2048, 16 / 16
+    // 256 -> 247 us a pass, 4096, 32 / 32 754 -> 751.  The dk and dv passes of wider heads lose by it: causal 8192, 16 / 8, 256
+    // 2140 -> 2164.
+    constexpr bool kFrag = kPass == kWideDkv;
+    auto frag_at = [](int k, int hq) { return 16 * (hq >> 1) + 4 * k + 2 * (hq & 1); };  // columns 8 k, row 8 hq on
+    auto load_scores = [&](uint32_t t, uint32_t (&v)[32]) {
+      if constexpr (kFrag) {
+        tmem_ld_frag(t, v);
+        tmem_ld_frag(t + kLanes16, v + 16);
+      } else {
+        tmem_ld32(t, v);
+      }
+    };
+    auto store_scores = [&](uint32_t t, const uint32_t (&pk)[16]) {
+      if constexpr (kFrag) {
+        tmem_st_frag(t, pk);
+        tmem_st_frag(t + kLanes16, pk + 8);
+      } else {
+        tmem_st16(t, pk);
+      }
+    };
     while (ok && cur.x >= 0) {
       const int tile = cur.x, batch = cur.y / n_own, own_head = cur.y % n_own, ebeg = cur.z, eend = cur.w;
       [[maybe_unused]] const int kv_head = kPass == kWideDq ? own_head / group : own_head;
       const int4* entries = p.entries + (int64_t)batch * p.entries_per_batch;
       const uint32_t n_steps = 2u * (uint32_t)(eend - ebeg) * (uint32_t)heads_here;
-      const int row = tile * kTile + r;
-      int own_seg = 0;
+      const int row = tile * kTile + (kFrag ? wq * 32 + (lane >> 2) : r);  // kFrag: the first of four, 8 apart
+      int own_seg[kFrag ? 4 : 1] = {};
       RowInterval iv{INT32_MIN, INT32_MAX};
       float row_nlse2 = 0.f, row_ndelta = 0.f;
       if (kPass == kWideDq) {  // everything per row is fixed for the tile
         const int qi = p.q_sequence ? p.q_sequence[row] : row;
         iv = mask_fn_interval(p.fn, qi);
-        own_seg = has_seg ? p.q_seg[(int64_t)batch * p.q_len + row] : 0;
+        own_seg[0] = has_seg ? p.q_seg[(int64_t)batch * p.q_len + row] : 0;
         const int64_t stat = ((int64_t)batch * p.q_heads + own_head) * p.q_len + row;
         row_nlse2 = p.nlse2[stat];
         row_ndelta = p.delta[stat];
-      } else {
-        own_seg = has_seg ? p.kv_seg[(int64_t)batch * p.kv_len + row] : 0;
+      } else if (has_seg) {
+#pragma unroll
+        for (int hq = 0; hq < (kFrag ? 4 : 1); ++hq) own_seg[hq] = p.kv_seg[(int64_t)batch * p.kv_len + row + 8 * hq];
       }
       const int32_t* other_seg = has_seg ? (kPass == kWideDq ? p.kv_seg + (int64_t)batch * p.kv_len
                                                                : p.q_seg + (int64_t)batch * p.q_len)
@@ -501,8 +524,11 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
           if (e + 1 < eend) ent_next = entries[e + 1];
           const int st = ent.y & 3;
           const int c0 = ent.x * kTile + set * kSub + cw * 32;  // first column: a key (dq pass) or a query row
-          const float4* nl4 = reinterpret_cast<const float4*>(stats + held.slot * 2 * kSub + cw * 32);
-          const float4* dl4 = nl4 + kSub / 4;
+          // (kFrag: this thread's first two; the next are 4 words on)
+          const float2* nl2 = reinterpret_cast<const float2*>(stats + held.slot * 2 * kSub + cw * 32 + (kFrag ? 2 * (lane & 3) : 0));
+          const float2* dl2 = nl2 + kSub / 2;
+          [[maybe_unused]] const float4* nl4 = reinterpret_cast<const float4*>(nl2);
+          [[maybe_unused]] const float4* dl4 = nl4 + kSub / 4;
           ok = mbar_wait(&bars->s_full[set], ph, ab, 0xE00u);
           if (kPass != kWideDq) {
             // (behind s_full: only then has the slot's previous use, another set's perhaps, surely completed)
@@ -515,7 +541,7 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
           float pr[32];
           {
             uint32_t v[32];
-            tmem_ld32(t_s, v);
+            load_scores(t_s, v);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; ++j) pr[j] = __uint_as_float(v[j]);
@@ -536,45 +562,87 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
 #pragma unroll
                 for (int j = 0; j < 32; ++j)
                   if (j < lo_rel || j > hi_rel) pr[j] = kMaskedLogit;
-              } else if (p.q_sequence == nullptr) {
+              } else if (!kFrag && p.q_sequence == nullptr) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                   const RowInterval ivj = mask_fn_interval(p.fn, c0 + j);
                   if (row < ivj.lo || row > ivj.hi) pr[j] = kMaskedLogit;
                 }
-              } else {
+              } else if (!kFrag) {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                   const RowInterval ivj = mask_fn_interval(p.fn, __ldg(p.q_sequence + c0 + j));
                   if (row < ivj.lo || row > ivj.hi) pr[j] = kMaskedLogit;
                 }
+              } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                  for (int u = 0; u < 2; ++u) {
+                    const int q = c0 + 2 * (lane & 3) + 8 * k + u;
+                    const RowInterval ivj = mask_fn_interval(p.fn, p.q_sequence == nullptr ? q : __ldg(p.q_sequence + q));
+#pragma unroll
+                    for (int hq = 0; hq < 4; ++hq)
+                      if (row + 8 * hq < ivj.lo || row + 8 * hq > ivj.hi) pr[frag_at(k, hq) + u] = kMaskedLogit;
+                  }
               }
             } else {
               // partial blocks: [id][q][kv] for the dq pass, stored transposed ([id][kv][q]) for dk / dv
-              const int8_t* mrow =
-                  kPass == kWideDq
-                      ? p.pmb + ((int64_t)ent.z * p.pm_bq + (row % p.pm_bq)) * p.pm_bkv + (c0 % p.pm_bkv)
-                      : p.pmb + ((int64_t)ent.z * p.pm_bkv + (row % p.pm_bkv)) * p.pm_bq + (c0 % p.pm_bq);
-              const int4* m4 = reinterpret_cast<const int4*>(mrow);
+              if constexpr (kFrag) {
+                const int8_t* mrow = p.pmb + ((int64_t)ent.z * p.pm_bkv + (row % p.pm_bkv)) * p.pm_bq + (c0 % p.pm_bq) + 8 * (lane & 3);
+                uint32_t bits = 0;  // a lane's four rows, eight columns each
 #pragma unroll
-              for (int t = 0; t < 2; ++t) {
-                const int4 mv = __ldg(m4 + t);
-                const uint32_t wd[4] = {(uint32_t)mv.x, (uint32_t)mv.y, (uint32_t)mv.z, (uint32_t)mv.w};
+                for (int hq = 0; hq < 4; ++hq) {
+                  const int2 m = __ldg(reinterpret_cast<const int2*>(mrow + (int64_t)(8 * hq) * p.pm_bq));
+                  bits |= (nonzero_bytes((uint32_t)m.x) | nonzero_bytes((uint32_t)m.y) << 4) << (8 * hq);
+                }
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                  if (((wd[j >> 2] >> ((j & 3) * 8)) & 0xffu) == 0u) pr[t * 16 + j] = kMaskedLogit;
+                for (int k = 0; k < 4; ++k) {  // lane 4 i + k of the four that share the rows holds columns 8 k .. + 7
+                  const uint32_t mine = __shfl_sync(0xffffffffu, bits, k, 4) >> (2 * (lane & 3));
+#pragma unroll
+                  for (int hq = 0; hq < 4; ++hq)
+#pragma unroll
+                    for (int u = 0; u < 2; ++u)
+                      if (((mine >> (8 * hq + u)) & 1u) == 0u) pr[frag_at(k, hq) + u] = kMaskedLogit;
+                }
+              } else {
+                const int8_t* mrow =
+                    kPass == kWideDq
+                        ? p.pmb + ((int64_t)ent.z * p.pm_bq + (row % p.pm_bq)) * p.pm_bkv + (c0 % p.pm_bkv)
+                        : p.pmb + ((int64_t)ent.z * p.pm_bkv + (row % p.pm_bkv)) * p.pm_bq + (c0 % p.pm_bq);
+                const int4* m4 = reinterpret_cast<const int4*>(mrow);
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                  const int4 mv = __ldg(m4 + t);
+                  const uint32_t wd[4] = {(uint32_t)mv.x, (uint32_t)mv.y, (uint32_t)mv.z, (uint32_t)mv.w};
+#pragma unroll
+                  for (int j = 0; j < 16; ++j)
+                    if (((wd[j >> 2] >> ((j & 3) * 8)) & 0xffu) == 0u) pr[t * 16 + j] = kMaskedLogit;
+                }
               }
             }
           }
           if (has_seg && !((ent.y >> 4) & 1)) {  // (bit set: the whole tile lies inside one segment)
-            const int4* sg4 = reinterpret_cast<const int4*>(other_seg + c0);
+            if constexpr (kFrag) {
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const int4 sv = __ldg(sg4 + t);
-              if (sv.x != own_seg) pr[t * 4 + 0] = kMaskedLogit;
-              if (sv.y != own_seg) pr[t * 4 + 1] = kMaskedLogit;
-              if (sv.z != own_seg) pr[t * 4 + 2] = kMaskedLogit;
-              if (sv.w != own_seg) pr[t * 4 + 3] = kMaskedLogit;
+              for (int k = 0; k < 4; ++k) {
+                const int2 sv = __ldg(reinterpret_cast<const int2*>(other_seg + c0) + (lane & 3) + 4 * k);
+#pragma unroll
+                for (int hq = 0; hq < 4; ++hq) {
+                  if (sv.x != own_seg[hq]) pr[frag_at(k, hq)] = kMaskedLogit;
+                  if (sv.y != own_seg[hq]) pr[frag_at(k, hq) + 1] = kMaskedLogit;
+                }
+              }
+            } else {
+              const int4* sg4 = reinterpret_cast<const int4*>(other_seg + c0);
+#pragma unroll
+              for (int t = 0; t < 8; ++t) {
+                const int4 sv = __ldg(sg4 + t);
+                if (sv.x != own_seg[0]) pr[t * 4 + 0] = kMaskedLogit;
+                if (sv.y != own_seg[0]) pr[t * 4 + 1] = kMaskedLogit;
+                if (sv.z != own_seg[0]) pr[t * 4 + 2] = kMaskedLogit;
+                if (sv.w != own_seg[0]) pr[t * 4 + 3] = kMaskedLogit;
+              }
             }
           }
           // P = exp2(c * s - lse * log2 e); with a soft cap dS carries the factor 1 - tanh^2, which goes into
@@ -582,29 +650,46 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
           // finite, their p is 0)
           {
             uint32_t pk[16];
+            if constexpr (kFrag) {
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const float4 nl = kPass == kWideDq ? make_float4(row_nlse2, row_nlse2, row_nlse2, row_nlse2) : nl4[t];
-              float th[4];
+            for (int i = 0; i < 16; ++i) {
+              const int j = frag_at(i >> 2, i & 3);
+              const float2 nl = nl2[4 * (i >> 2)];
+              const float2 th = make_float2(fmaxf(pr[j], -1.0f), fmaxf(pr[j + 1], -1.0f));
+              const float2 x = __ffma2_rn(make_float2(pr[j], pr[j + 1]), make_float2(c, c), nl);
+              pr[j] = ex2(x.x);
+              pr[j + 1] = ex2(x.y);
+              pk[j / 2] = pack_bf16(pr[j], pr[j + 1]);
               if constexpr (kSoftCap && kHasDp) {
-#pragma unroll
-                for (int u = 0; u < 4; ++u) th[u] = fmaxf(pr[4 * t + u], -1.0f);
+                pr[j] *= fmaf(-th.x, th.x, 1.0f);
+                pr[j + 1] *= fmaf(-th.y, th.y, 1.0f);
               }
-              const float2 xa = __ffma2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]), make_float2(c, c), make_float2(nl.x, nl.y));
-              const float2 xb = __ffma2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]), make_float2(c, c), make_float2(nl.z, nl.w));
-              pr[4 * t + 0] = ex2(xa.x);
-              pr[4 * t + 1] = ex2(xa.y);
-              pr[4 * t + 2] = ex2(xb.x);
-              pr[4 * t + 3] = ex2(xb.y);
-              pk[2 * t] = pack_bf16(pr[4 * t + 0], pr[4 * t + 1]);
-              pk[2 * t + 1] = pack_bf16(pr[4 * t + 2], pr[4 * t + 3]);
-              if constexpr (kSoftCap && kHasDp) {
+            }
+            } else {
 #pragma unroll
-                for (int u = 0; u < 4; ++u) pr[4 * t + u] *= fmaf(-th[u], th[u], 1.0f);
+              for (int t = 0; t < 8; ++t) {
+                const float4 nl = kPass == kWideDq ? make_float4(row_nlse2, row_nlse2, row_nlse2, row_nlse2) : nl4[t];
+                float th[4];
+                if constexpr (kSoftCap && kHasDp) {
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) th[u] = fmaxf(pr[4 * t + u], -1.0f);
+                }
+                const float2 xa = __ffma2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]), make_float2(c, c), make_float2(nl.x, nl.y));
+                const float2 xb = __ffma2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]), make_float2(c, c), make_float2(nl.z, nl.w));
+                pr[4 * t + 0] = ex2(xa.x);
+                pr[4 * t + 1] = ex2(xa.y);
+                pr[4 * t + 2] = ex2(xb.x);
+                pr[4 * t + 3] = ex2(xb.y);
+                pk[2 * t] = pack_bf16(pr[4 * t + 0], pr[4 * t + 1]);
+                pk[2 * t + 1] = pack_bf16(pr[4 * t + 2], pr[4 * t + 3]);
+                if constexpr (kSoftCap && kHasDp) {
+#pragma unroll
+                  for (int u = 0; u < 4; ++u) pr[4 * t + u] *= fmaf(-th[u], th[u], 1.0f);
+                }
               }
             }
             if constexpr (kHasP) {
-              tmem_st16(t_s, pk);
+              store_scores(t_s, pk);
               tmem_st_wait();
               tc_fence_before();
               __syncwarp();
@@ -617,21 +702,32 @@ splash_bwd_wide_kernel(const __grid_constant__ CUtensorMap tm_a1, const __grid_c
             if (!ok) break;
             tc_fence_after();
             uint32_t v[32], pk[16];
-            tmem_ld32(t_dp, v);
+            load_scores(t_dp, v);
             tmem_ld_wait();
+            if constexpr (kFrag) {
 #pragma unroll
-            for (int t = 0; t < 8; ++t) {
-              const float4 nd = kPass == kWideDq ? make_float4(row_ndelta, row_ndelta, row_ndelta, row_ndelta) : dl4[t];  // -di
-              const float2 da = __fmul2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]),
-                                           __fadd2_rn(make_float2(__uint_as_float(v[4 * t + 0]), __uint_as_float(v[4 * t + 1])),
-                                                      make_float2(nd.x, nd.y)));
-              const float2 db = __fmul2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]),
-                                           __fadd2_rn(make_float2(__uint_as_float(v[4 * t + 2]), __uint_as_float(v[4 * t + 3])),
-                                                      make_float2(nd.z, nd.w)));
-              pk[2 * t] = pack_bf16(da.x, da.y);
-              pk[2 * t + 1] = pack_bf16(db.x, db.y);
+            for (int i = 0; i < 16; ++i) {
+              const int j = frag_at(i >> 2, i & 3);
+              const float2 nd = dl2[4 * (i >> 2)];  // -di
+              const float2 ds = __fmul2_rn(make_float2(pr[j], pr[j + 1]),
+                                           __fadd2_rn(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), nd));
+              pk[j / 2] = pack_bf16(ds.x, ds.y);
             }
-            tmem_st16(kOneS ? t_dp : t_s + kDsOffset, pk);
+            } else {
+#pragma unroll
+              for (int t = 0; t < 8; ++t) {
+                const float4 nd = kPass == kWideDq ? make_float4(row_ndelta, row_ndelta, row_ndelta, row_ndelta) : dl4[t];  // -di
+                const float2 da = __fmul2_rn(make_float2(pr[4 * t + 0], pr[4 * t + 1]),
+                                             __fadd2_rn(make_float2(__uint_as_float(v[4 * t + 0]), __uint_as_float(v[4 * t + 1])),
+                                                        make_float2(nd.x, nd.y)));
+                const float2 db = __fmul2_rn(make_float2(pr[4 * t + 2], pr[4 * t + 3]),
+                                             __fadd2_rn(make_float2(__uint_as_float(v[4 * t + 2]), __uint_as_float(v[4 * t + 3])),
+                                                        make_float2(nd.z, nd.w)));
+                pk[2 * t] = pack_bf16(da.x, da.y);
+                pk[2 * t + 1] = pack_bf16(db.x, db.y);
+              }
+            }
+            store_scores(kOneS ? t_dp : t_s + kDsOffset, pk);
             tmem_st_wait();
             tc_fence_before();
             __syncwarp();
