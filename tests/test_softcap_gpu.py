@@ -97,6 +97,40 @@ def test_both_forms_of_tanh_in_one_tile(d, kind, top, repeatable):
     assert ((got.cpu().double() - want).norm() / want.norm()).item() <= 1e-2
 
 
+# tanh is a function of its argument alone: the polynomial up to 1/2, the special functions above, whatever a row's neighbours
+# and its masked keys hold.  The middle document shares tiles and warps with the others; once its arguments are tiny, once
+# they run far beyond 1/2, its products with the other documents' tokens too.
+@pytest.mark.parametrize("repeatable", [False, True])
+@pytest.mark.parametrize("dims", [(64, 64), (80, 80), (128, 128), (192, 128), (256, 256)])
+@pytest.mark.parametrize("kind", ["full", "causal"])
+def test_a_documents_bits_do_not_depend_on_its_neighbours(kind, dims, repeatable):
+  s, cap, ends = 256, 20.0, (48, 200, 256)
+  d_qk, d_v = dims
+  g = torch.Generator().manual_seed(d_qk)
+  q, k, v, do = (torch.randn(1, 2, s, d, generator=g) for d in (d_qk, d_qk, d_v, d_v))
+  ids = torch.repeat_interleave(torch.arange(3, dtype=torch.int32), torch.tensor([ends[0], ends[1] - ends[0], s - ends[1]]))
+  mask = mask_lib.FullMask((s, s)) if kind == "full" else mask_lib.CausalMask((s, s))
+  cfg = dataclasses.replace(splash.SplashConfig.get_default(), attn_logits_soft_cap=cap)
+  kernel = splash.make_splash_mha(mask, config=cfg, q_seq_shards=1, save_residuals=True, repeatable_dq=repeatable)
+
+  def run(factor):
+    grow = torch.ones(s, 1)
+    grow[ends[0]:ends[1]] = factor
+    qd, kd, vd, dod = (t.to(torch.bfloat16).to(DEV) for t in (q * grow, k * grow, v, do))
+    ts = [t.requires_grad_(True) for t in (qd, kd, vd)]
+    seg = splash.SegmentIds(ids[None].to(DEV), ids[None].to(DEV))
+    out, res = kernel(*ts, seg, logits_scale=1 / math.sqrt(d_qk))
+    grads = torch.autograd.grad(out, ts, dod)
+    kernel.check_errors()
+    return (out, res["logsumexp"][..., None], res["max_logits"][..., None], *grads)
+
+  small, large = run(0.01), run(30.0)
+  for name, a, b in zip(("out", "lse", "max", "dq", "dk", "dv"), small, large):
+    for rows in (slice(0, ends[0]), slice(ends[1], s)):
+      assert torch.equal(a[:, :, rows], b[:, :, rows]), name
+    assert not torch.equal(a, b)
+
+
 def test_soft_cap_changes_the_result_and_rejects_bad_values():
   s = 256
   g = torch.Generator().manual_seed(3)

@@ -464,12 +464,10 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// tanh to ~1e-6 absolute: (e - 1) / (e + 1) with e = 2^(2 log2(e) y).  tanh.approx.f32 (relative
-// error 2^-11) is too coarse for logits that must hold 1e-3 after being multiplied by a cap of
-// tens.  Saturates cleanly: e = inf -> 1, e = 0 -> -1.
-__device__ __forceinline__ float tanh_ex2(float y) {
-  const float e = ex2(y * 2.8853900817779268f);
-  return 1.0f - __fdividef(2.0f, e + 1.0f);
+__device__ __forceinline__ float rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 // Three-input maximum (one instruction on sm_100).
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -478,7 +476,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 // tanh of two values of at most 1/2 each: y p(y^2) with p of degree 4 through tanh(y) / y at the Chebyshev nodes of 0 .. 1/4,
-// two-wide in fp32 (error 4.1e-8 absolute, 1.1e-7 relative; tanh_ex2 on the same range 1.7e-7 absolute).  The scores of a soft
+// two-wide in fp32 (error 4.1e-8 absolute, 1.1e-7 relative; 1 - 2 / (e + 1) on the same range 1.7e-7 absolute).  The scores of a soft
 // cap lie far inside it, and it spares two of the three special-function operations a score, which take 3072 of a
 // 128 x 128 tile's cycles: 3 x 1664, 12 / 4 heads, d 80, window 768: forward 63.8 -> 54.2 us, fused dkv 95.7 -> 82.0; 4 x 4096,
 // 16 / 8, d 128: a pass 754 -> 641.
@@ -502,12 +500,29 @@ __device__ __forceinline__ bool tanh_is_small(const float (&x)[N], float a) {
   }
   return !__any_sync(0xffffffffu, fmaxf(top0, top1) * a > 0.5f);
 }
-// x <- tanh(a x), N values a lane, by a whole warp.
+// tanh of two values, in the form that each by itself calls for: tanh_small() up to 1/2, 1 - 2 / (e + 1) above, e = 2^(2 log2(e) y)
+// (e = inf gives 1, e = 0 gives -1; tanh.approx.f32, relative error 2^-11, is too coarse for logits that must hold 1e-3 after
+// being multiplied by a cap of tens).
+__device__ __forceinline__ float2 tanh_each(float2 y) {
+  auto two = [](float c) { return make_float2(c, c); };
+  const float2 t = tanh_small(y), w = __fmul2_rn(y, two(2.8853900817779268f));
+  const float2 d = __fadd2_rn(make_float2(ex2(w.x), ex2(w.y)), two(1.0f));
+  const float2 u = __ffma2_rn(make_float2(rcp(d.x), rcp(d.y)), two(-2.0f), two(1.0f));
+  return make_float2(fabsf(y.x) <= 0.5f ? t.x : u.x, fabsf(y.y) <= 0.5f ? t.y : u.y);
+}
+// x <- tanh(a x), N values a lane, by a whole warp; `small`: tanh_is_small() of them, which spares the second form.  Which of the
+// two a value takes must not hang on the vote: a score's last bits would depend on all else that its warp holds, masked keys
+// and other documents among it.  (Warps of both kinds pay for both forms: scores of 16 times the spread, 444 tiles: forward
+// 8 heads, window 768, 135 -> 148 us, dkv 166 -> 175; causal, d 64, 1371 -> 1475, 1728 -> 1840.)
 template <int N>
 __device__ __forceinline__ void tanh_all(float (&x)[N], float a, bool small) {
   if (!small) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) x[j] = tanh_ex2(x[j] * a);
+    for (int j = 0; j < N; j += 2) {
+      const float2 t = tanh_each(__fmul2_rn(make_float2(x[j], x[j + 1]), make_float2(a, a)));
+      x[j] = t.x;
+      x[j + 1] = t.y;
+    }
     return;
   }
 #pragma unroll
