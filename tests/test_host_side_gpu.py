@@ -92,6 +92,16 @@ def test_results_keep_a_tensor_subclass(copied):
   assert all(type(t) is torch.Tensor for t in params)
 
 
+def test_operands_of_another_device_are_refused():
+  q, k, v, _ = _tensors()
+  kernel = splash.make_splash_mha(mask_lib.CausalMask((S, S)), q_seq_shards=1)
+  want = kernel(q, k, v, logits_scale=0.125)
+  for args in ((q, k.cpu(), v), (q, k, v.cpu())):
+    with pytest.raises(RuntimeError, match="on the device of q"):
+      kernel(*args, logits_scale=0.125)
+  assert torch.equal(kernel(q, k, v, logits_scale=0.125), want)
+
+
 # ---- the autograd function in native code, against the python one, which calls with a fixed maximum and others still take
 def _both(monkeypatch, run):
   native = run()

@@ -44,8 +44,15 @@ at::Tensor usable(const at::Tensor& t) {
   return ok ? t : t.contiguous();
 }
 
-SplashTensor describe(const at::Tensor& t) {
+// The kernels follow every address that they are given: each must be one of their own device, that of `q`.
+void require_beside(const at::Tensor& t, const at::Tensor& q) {
+  TORCH_CHECK(t.device() == q.device(), "expected all tensors on the device of q, ", q.device(), ", got one on ", t.device());
+}
+
+SplashTensor describe(const at::Tensor& t, const at::Tensor& q) {
   TORCH_CHECK(t.dim() == 4, "expected a tensor of rank 4, got rank ", t.dim());
+  TORCH_CHECK(t.scalar_type() == at::kBFloat16, "expected bfloat16 operands, got ", t.scalar_type());
+  require_beside(t, q);
   SplashTensor d{};
   d.data = t.data_ptr();
   d.dtype = SPLASH_BF16;
@@ -54,8 +61,13 @@ SplashTensor describe(const at::Tensor& t) {
 }
 
 template <typename T>
-T* pointer(const std::optional<at::Tensor>& t) {
-  return t.has_value() ? static_cast<T*>(t->data_ptr()) : nullptr;
+T* pointer(const at::Tensor& t, const at::Tensor& q) {
+  require_beside(t, q);
+  return static_cast<T*>(t.data_ptr());
+}
+template <typename T>
+T* pointer(const std::optional<at::Tensor>& t, const at::Tensor& q) {
+  return t.has_value() ? pointer<T>(*t, q) : nullptr;
 }
 
 template <typename T>
@@ -88,22 +100,22 @@ std::tuple<int, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::
   const auto f32 = q.options().dtype(at::kFloat);
   const at::Tensor lse = at::empty({b, hq, sq}, f32), max_logits = at::empty({b, hq, sq}, f32);
   SplashFwdArgs a{};
-  a.q = describe(q);
-  a.k = describe(k);
-  a.v = describe(v);
-  a.o = describe(o);
-  a.logsumexp = static_cast<float*>(lse.data_ptr());
+  a.q = describe(q, q);
+  a.k = describe(k, q);
+  a.v = describe(v, q);
+  a.o = describe(o, q);
+  a.logsumexp = pointer<float>(lse, q);
   a.max_logits = static_cast<float*>(max_logits.data_ptr());
-  a.q_segment_ids = pointer<int32_t>(q_seg);
-  a.kv_segment_ids = pointer<int32_t>(kv_seg);
-  a.q_sequence = pointer<int32_t>(q_sequence);
+  a.q_segment_ids = pointer<int32_t>(q_seg, q);
+  a.kv_segment_ids = pointer<int32_t>(kv_seg, q);
+  a.q_sequence = pointer<int32_t>(q_sequence, q);
   a.sched = at_address<SplashDeviceSchedule>(sched);
   a.mask_fn = at_address<SplashMaskFn>(mask_fn);
   a.scale = (float)scale;
   a.mask_value = (float)mask_value;
-  a.error_record = static_cast<uint32_t*>(error_record.data_ptr());
-  a.sinks = pointer<float>(sinks);
-  a.max_logit_value = pointer<float>(max_logit);
+  a.error_record = pointer<uint32_t>(error_record, q);
+  a.sinks = pointer<float>(sinks, q);
+  a.max_logit_value = pointer<float>(max_logit, q);
   a.soft_cap = (float)soft_cap;
   if (o_peer != 0) a.o_peer = at_address<SplashPeerOutput>(o_peer);
   const SplashShards shards{head_shards, q_shards};
@@ -125,28 +137,28 @@ std::tuple<int, at::Tensor, at::Tensor, at::Tensor, at::Tensor> backward(
   const at::Tensor d_o = usable(d_o_in);
   const at::Tensor dq = at::empty_like(q), dk = at::empty_like(k), dv = at::empty_like(v);
   SplashBwdArgs a{};
-  a.q = describe(q);
-  a.k = describe(k);
-  a.v = describe(v);
-  a.o = describe(o);
-  a.d_o = describe(d_o);
-  a.dq = describe(dq);
-  a.dk = describe(dk);
-  a.dv = describe(dv);
+  a.q = describe(q, q);
+  a.k = describe(k, q);
+  a.v = describe(v, q);
+  a.o = describe(o, q);
+  a.d_o = describe(d_o, q);
+  a.dq = describe(dq, q);
+  a.dk = describe(dk, q);
+  a.dv = describe(dv, q);
   const size_t bytes = (fused ? lib.fused_workspace_bytes : lib.workspace_bytes)(q.size(0), q.size(1), q.size(2));
   const at::Tensor workspace = at::empty({(int64_t)bytes}, q.options().dtype(at::kByte));
   a.flags = fused ? SPLASH_BWD_FUSED_DQ : 0;
-  a.logsumexp = static_cast<float*>(lse.data_ptr());
-  a.q_segment_ids = pointer<int32_t>(q_seg);
-  a.kv_segment_ids = pointer<int32_t>(kv_seg);
-  a.q_sequence = pointer<int32_t>(q_sequence);
+  a.logsumexp = pointer<float>(lse, q);
+  a.q_segment_ids = pointer<int32_t>(q_seg, q);
+  a.kv_segment_ids = pointer<int32_t>(kv_seg, q);
+  a.q_sequence = pointer<int32_t>(q_sequence, q);
   a.sched_dq = at_address<SplashDeviceSchedule>(sched_dq);
   a.sched_dkv = at_address<SplashDeviceSchedule>(sched_dkv);
   a.mask_fn = at_address<SplashMaskFn>(mask_fn);
   a.scale = (float)scale;
   a.workspace = workspace.data_ptr();
   a.workspace_bytes = bytes;
-  a.error_record = static_cast<uint32_t*>(error_record.data_ptr());
+  a.error_record = pointer<uint32_t>(error_record, q);
   a.soft_cap = (float)soft_cap;
   if (dq_peer != 0) a.dq_peer = at_address<SplashPeerOutput>(dq_peer);
   if (dk_peer != 0) a.dk_peer = at_address<SplashPeerOutput>(dk_peer);

@@ -567,14 +567,14 @@ class SplashAttentionKernel:
         tables.error_record.zero_()
         raise _native.SplashError(st, f"device error record {list(rec)}")
 
-  def _reject_unsupported(self, q, k, sinks, max_logit_value):
+  def _reject_unsupported(self, q, k, v, max_logit_value):
     cfg = self.config
     if cfg.max_logit_const is not None and max_logit_value is not None:
       raise ValueError(f"Only one of max_logit_const={cfg.max_logit_const} and {max_logit_value=} can be set.")
     if cfg.attn_logits_soft_cap is not None and not cfg.attn_logits_soft_cap > 0:
       raise ValueError(f"attn_logits_soft_cap must be positive, got {cfg.attn_logits_soft_cap}")
-    if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16:
-      raise NotImplementedError(f"only bfloat16 inputs are built on B200, got {q.dtype}")
+    if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16:
+      raise NotImplementedError(f"only bfloat16 inputs are built on B200, got {q.dtype}, {k.dtype}, {v.dtype}")
 
   def __call__(self, q, k, v, segment_ids: SegmentIds | None = None, sinks=None, *,
                max_logit_value=None, logits_scale: float = 1.0, q_shard: int = 0, _function=None, **overrides):
@@ -582,7 +582,7 @@ class SplashAttentionKernel:
     # context-parallel wrapper passes one whose forward also stores the output into its peers).
     kw = dict(self.kwargs, **overrides)
     save_residuals = kw.get("save_residuals", False)
-    self._reject_unsupported(q, k, sinks, max_logit_value)
+    self._reject_unsupported(q, k, v, max_logit_value)
     # SEQ_MINOR operands ([..., head_dim, seq], reference kernel.py:51-54) are viewed head-dim-minor;
     # the kernels take head_dim-contiguous tiles, so such an operand is copied once on the way in.
     cfg = self.config
