@@ -43,6 +43,13 @@ def test_query_shards_are_shared_out_as_the_whole_call(sq, skv, shards, clusters
     assert whole > 1 and row_parts(mask, 1, 8, 4, sq, skv, q_shards=shards, clusters=clusters)[0] == whole
 
 
+@pytest.mark.parametrize("clusters", CAPACITIES)
+@pytest.mark.parametrize("batch,hq,hkv,s", [(2, 20, 5, 4096), (1, 20, 5, 8192), (2, 30, 5, 4096), (1, 40, 10, 4096), (1, 32, 8, 4096)])
+def test_rows_of_tables_are_not_cut_up_for_waves(batch, hq, hkv, s, clusters):
+  """Two or three kv tiles an SM: rows of a table may have every length, which whole tiles, longest first, even out."""
+  assert row_parts(mask_lib.FullMask((s, s)), batch, hq, hkv, s, s, clusters=clusters)[1] == 1
+
+
 def test_query_shards_say_whether_their_rows_are_in_order():
   s, cpu = 512, torch.device("cpu")
   kernel = splash.make_splash_mha(mask_lib.CausalMask((s, s)), q_seq_shards=2)

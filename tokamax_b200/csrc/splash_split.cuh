@@ -2,8 +2,8 @@
 //
 // The kernels keep one CTA on an SM, so a grid of few long rows leaves SMs idle for the whole launch
 // (512 query rows of 32 heads against 16384 keys: 64 CTAs of 128 steps on 148 SMs).  Measured, one CTA
-// a row -> shared: that forward 240 -> 135 us (two CTAs a row); dkv of causal 2 x 4096, 16 q heads
-// on one kv head, d 64 (64 CTAs of 16 .. 512 steps) 745 -> 244 (eight a tile).
+// a row -> shared: that forward 238 -> 137 us (two CTAs a row); dkv of causal 2 x 4096, 16 q heads
+// on one kv head, d 64 (64 CTAs of 16 .. 512 steps) 733 -> 223 (four a tile).
 #pragma once
 
 #include <mutex>
@@ -21,6 +21,7 @@ constexpr int kMaxSplit = 8;  // portable cluster size
 struct RowWork {
   float longest, mean;  // 0: rows are left whole
   int64_t ctas;         // rows of the call (of all launches that make it up)
+  bool known;           // false: a table, whose rows may have any length up to these
 };
 struct ClusterCapacity {
   int clusters[kMaxSplit + 1];  // [n]: clusters of n CTAs that are resident at the same time; [1]: CTAs
@@ -31,10 +32,10 @@ constexpr int kSplitMaxCtas = 1024;  // grids above this fill the chip several t
 // rows of `row_span` query rows (transposed = false) or key tiles (true) over `n_steps_full` tiles of the other side
 inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_span, int n_tiles,
                                  int64_t n_ctas, bool transposed = false) {
-  RowWork w{0.f, 0.f, n_ctas};
+  RowWork w{0.f, 0.f, n_ctas, fn.kind != SPLASH_MASK_TABLE};
   if (n_ctas > kSplitMaxCtas) return w;
   w.longest = w.mean = (float)n_tiles;
-  if (fn.kind == SPLASH_MASK_TABLE) return w;
+  if (!w.known) return w;
   int64_t sum = 0, most = 0;
   for (int r = 0; r < n_rows; ++r) {
     // the row sees columns lo .. hi of the other side
@@ -71,23 +72,31 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
 // CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (prologue, epilogue; more for the addition across the
 // cluster).  While everything is resident the longest row sets the time.  Beyond that, rows of different length, longest
 // first, end together but for a tenth of the longest, unless that alone takes as long; rows of one length go in whole waves.  (All
-// numbers tried, us of the kernel, the rule's own marked *, that of the rule before it, which counted half a row for the end
-// of every grid and less for a CTA, in brackets.  dkv, causal: 2 x 4096, 16 / 1 heads, d 64: 733 375 260 *223 254 (249) 315 278,
+// numbers tried, us of the kernel, the rule's own marked *, that of a rule that counts half a row for the end
+// of every grid and less for a CTA in brackets.  dkv, causal: 2 x 4096, 16 / 1 heads, d 64: 733 375 260 *223 254 (249) 315 278,
 // d 128 837 438 307 *259 296 (291) 371 328; 1 x 4096, 8 / 2, fused: 310 173 128 *115 139 (142) 195 185; 2 x 2048, 16 / 4,
-// d 64: 105 *(74) 96 100; window 1000, 1 x 8192, 8 / 1: 193 *(110) 153 128.  Forward: 512 x 16384, 32 / 8: 238 *(137) 184 153;
+// d 64: 105 *(74) 96 100; window 1000, 1 x 8192, 8 / 1: 193 *(110) 153 128, 20 / 5, 320 tiles, whole backward: *(286) 319 364 400.
+// Forward: 512 x 16384, 32 / 8: 238 *(137) 184 153, 80 / 8, 160 rows: 455 (374) 348 *348, 160 / 8: 700 *627 686 689;
 // causal 4096, 8 / 2: (65) *55 75 88, d 64 (61) *47 64; 4096, 16 / 2: *(75) 106.)
+//
+// Rows of a table take that other rule, which stands between the two: how long its rows are only the device knows.  Taken as
+// full, they would go in waves, and prefixes and triangles, which have none, would be cut up for it.  (Whole backward, d 128, us with 1 2 3 4 CTAs a tile, waves' choice marked w: 4096, 20 / 5 heads, 160 tiles: prefix 343 *260
+// 288 w301, lower triangle 341 *255 274 w292, full 644 *540 497 w479; 2 x 4096, 20 / 5, 320 tiles: *509 w497 554 588, *466 w484 534
+// 566, *1037 w954 1047 1025; 8192, 20 / 5: *989 w916, *865 w869, *2005 w1795; 2 x 4096, 30 / 5, d 64: *476 w487, *431 w469, *970 w893.)
 // Rows below 16 steps stay whole although the
 // rule would share some (causal 2 x 1024, 8 heads, 64 CTAs of 2 .. 8 steps: 24.7 us, 20.9 with two CTAs a row),
 // so that the bits of short rows do not depend on the batch and the heads beside them: in the forward those
 // of fewer than 2048 keys, in dkv kv tiles of fewer than 16 (q tile, q head of the group) steps.
 inline int split_for(const RowWork& w, const ClusterCapacity& cap) {
-  constexpr float kFixed = 4.f, kMerge = 3.f, kFewest = 16.f;
+  constexpr float kFewest = 16.f;
+  const float own = w.known ? 4.f : 3.f, merge = w.known ? 3.f : 1.f;
   if (w.longest < kFewest) return 1;
   auto time = [&](int n) {
-    const float fixed = kFixed + (n > 1 ? kMerge : 0.f);
+    const float fixed = own + (n > 1 ? merge : 0.f);
     const float longest = w.longest / n, mean = w.mean / n + fixed;
     const int64_t room = cap.clusters[n];
     if (w.ctas <= room) return longest + fixed;
+    if (!w.known) return (float)w.ctas * mean / room + 0.5f * (longest + fixed);
     if (w.mean > 0.9f * w.longest) return (float)((w.ctas + room - 1) / room) * mean;
     const float all = (float)w.ctas * mean / room + 0.1f * longest;
     return all > longest + fixed ? all : longest + fixed;
