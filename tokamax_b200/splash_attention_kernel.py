@@ -415,8 +415,7 @@ def splash_backward(kernel: "SplashAttentionKernel", q, k, v, o, lse, d_o, q_seg
   keeps the row sums negated (None without ``with_di``).
   """
   tables = kernel._tables(q.device, q.shape[0], shard)  # pylint: disable=protected-access
-  # head dims above 128 run separate passes, each repeatable bit for bit
-  fused = not kernel.repeatable_dq and q.shape[-1] <= _HEAD_DIM and v.shape[-1] <= _HEAD_DIM
+  fused = kernel._fused_backward(q, v)  # pylint: disable=protected-access
   sched_dq, sched_dkv = tables.dq, tables.dkv
   keep = []  # until the launch below
   if q_seg is not None and not sched_dq.row_end:
@@ -535,6 +534,10 @@ class SplashAttentionKernel:
       self._device_tables[key] = _DeviceTables(self, device, shard)
     return self._device_tables[key]
 
+  def _fused_backward(self, q, v) -> bool:
+    """Whether dkv forms dq too.  Head dims above 128 run separate passes, each repeatable bit for bit."""
+    return not self.repeatable_dq and q.shape[-1] <= _HEAD_DIM and v.shape[-1] <= _HEAD_DIM
+
   def _attention(self, q, k, v, scale: float, shard: int):
     """`_SplashFunction` on these arguments, its forward and backward in native code."""
     _require_cuda(q)
@@ -544,10 +547,8 @@ class SplashAttentionKernel:
     if native is None:
       native = tables.native = host.Tables(C.addressof(tables.fwd), C.addressof(tables.dq), C.addressof(tables.dkv), tables.keep,
                                            tables.error_record, tables.q_sequence, tables.q_shards)
-    # (the backward's form: head dims above 128 run separate passes, each repeatable bit for bit)
     return host.attention(native, q, k, v, C.addressof(self._mask_fn), scale, max(self.mask_value, -3.0e38),
-                          float(self.config.attn_logits_soft_cap or 0.0),
-                          not self.repeatable_dq and q.shape[-1] <= _HEAD_DIM and v.shape[-1] <= _HEAD_DIM, self.head_shards)
+                          float(self.config.attn_logits_soft_cap or 0.0), self._fused_backward(q, v), self.head_shards)
 
   def check_errors(self) -> None:
     """Synchronises and raises if a kernel reported a device-side fault (bounded wait ran out).
