@@ -639,7 +639,9 @@ static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 // the compute warps store dK and dV.  A tile a CTA spent about 20000 cycles between its last step and its successor's
 // first.  One tile a CTA -> this, us a pass: 8 x 16384, 16 heads, window 4096 and documents (some 12 steps a tile) 6584 -> 6260,
 // causal 4 x 2048, 16 / 16 359 -> 334, 4 x 8192, 32 / 8 6974 -> 6842, prefix 2 x 4096, 16 / 4 617 -> 597 (with the drain
-// below, 604 before).  kOneTile: its own tile only, see one_tile_ctas().
+// below, 604 before).  With a soft cap, whole backward: 156 tiles (3 x 1664, 12 / 4 heads, d 80, window 768)
+// 91.0 -> 89.2, 248 (causal 3968, 32 / 8) 368 -> 368, 256 (causal 2 x 4096, 16 / 4) 378 -> 382, 260 (5 x 1664, 12 / 4, d 80, window
+// 768) 145 -> 141, 1024 (causal 4 x 4096, 16 / 8) 756 -> 738.
 //
 // kSplit: a cluster of 2 .. 8 CTAs shares one kv tile, each taking its part of the steps (q head, q tile), see PartWalk.
 // At the end every CTA leaves its dK and dV (fp32) in its own shared memory and the cluster adds them
@@ -648,7 +650,7 @@ static_assert(sizeof(DkvBarriers) <= 512, "barrier block");
 constexpr int kDkvPartWords = 2 * kHeadDim / 4 * kTile;  // 16-byte words: [dk, dv column / 4][kv row]
 static_assert(kDkvPartWords * 16 <= (3 + kBwdStages) * kTileBytes, "the parts lie over the operand tiles");
 
-template <bool kSoftCap, bool kFuseDq, bool kSplit, bool kLateS, bool kOneTile = kSplit>
+template <bool kSoftCap, bool kFuseDq, bool kSplit, bool kLateS>
 __global__ void __launch_bounds__(kFuseDq ? kFusedThreads : kDkvThreads, 1)
 splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_do,
                        const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
@@ -690,7 +692,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   auto do_offset = [&](uint32_t n) { return kTileBytes + (one_do ? 0u : (n & 1u) * (kFuseDq ? kHalfBytes : 2 * kTileBytes)); };
   // steps of a tile: (q head g of the group, entry e) pairs in that order; `offset` (kSplit): of head g's part, a tile less
   // for each further head
-  int4 own = kOneTile ? tile_of(kSplit ? blockIdx.x / p.n_split : blockIdx.x) : make_int4(0, 0, 0, 0);
+  int4 own = kSplit ? tile_of(blockIdx.x / p.n_split) : make_int4(0, 0, 0, 0);
   auto walk_of = [&](const int4& w) { return PartWalk<kSplit>(list_of(w), w.z, w.w, p.n_split); };
   auto offset_behind = [&](int offset) { return kSplit ? (offset == 0 ? p.n_split : offset) - 1 : 0; };
 
@@ -749,7 +751,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mine = __reduce_add_sync(0xffffffffu, mine);
     if (lane == 0) atomicAdd(&bars->n_steps, mine);
   }
-  if (!kOneTile && warp == kDkvTmaWarp) {  // looked up beside the allocation; the others hear of it from the queue
+  if (!kSplit && warp == kDkvTmaWarp) {  // looked up beside the allocation; the others hear of it from the queue
     own = tile_of(blockIdx.x);
     if (lane == 0) {
       tma_prefetch_desc(&tm_q);
@@ -769,14 +771,14 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
   AbortCtx ab{&bars->abort_flag, p.err};
   auto steps_of = [&](const int4& w) { return kSplit ? bars->n_steps : (uint32_t)((w.w - w.z) * group); };
 
-  // The tiles this CTA works on, in order: its own, then those it takes over (the producer posts both).  kOneTile: its own.
+  // The tiles this CTA works on, in order: its own, then those it takes over (the producer posts both).  kSplit: its own.
   uint32_t taken = 0;  // tiles so far: slot and phase of the next one
   auto work_slot = [&]() { return taken % kDkvWork; };
   auto work_phase = [&]() { return (taken / kDkvWork) & 1u; };
   // Calls body(tile) for each, until it returns false: by a whole warp, or by a thread for its warp.  `hold`: the tile's
   // slot is kept to the end, for body to read it again.
   auto each_tile = [&](bool warp_wide, bool hold, auto body) {
-    if constexpr (kOneTile) {
+    if constexpr (kSplit) {
       body(own);
     } else {
       auto release = [&]() {
@@ -872,7 +874,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
       bool ok = true;
       int4 w = own;
       while (ok) {
-        if constexpr (!kOneTile) {
+        if constexpr (!kSplit) {
           ok = mbar_wait(&bars->work_empty[work_slot()], work_phase() ^ 1u, ab, 0x3710u + work_slot());
           if (!ok) break;
           bars->work[work_slot()] = w;
@@ -925,7 +927,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
             }
           }
         }
-        if (kOneTile || !ok) break;
+        if (kSplit || !ok) break;
         // The next tile.  Asked for when all of this one is on its way, and no earlier: what a CTA has taken over, no other
         // can take that is done before it.
         mbar_arrive_expect_tx(&bars->answer_full, 16);
@@ -1271,7 +1273,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
 
     // epilogue: dK (scaled) and dV, 32 columns per thread
     {  // (the tile's place is read again: the loop over the steps needs the registers)
-    const int4 again = kOneTile ? own : ld_again(&bars->work[work_slot()]);
+    const int4 again = kSplit ? own : ld_again(&bars->work[work_slot()]);
     const int batch = again.y / p.kv_heads, kv_head = again.y % p.kv_heads, kv_row = again.x * kTile + r;
     const uint32_t n_steps = last - first;
     __nv_bfloat16* dk = p.out0 + (int64_t)batch * p.out0_sb + (int64_t)kv_head * p.out0_sh +
@@ -1433,22 +1435,14 @@ size_t bwd_fused_workspace_bytes(int64_t batch, int64_t q_heads, int64_t q_len) 
 }
 
 using DkvKernel = void (*)(CUtensorMap, CUtensorMap, CUtensorMap, CUtensorMap, BwdParams);
-static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap, bool late, bool one_tile = false) {
+static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap, bool late) {
   static const DkvKernel kernels[2][2][2] = {
       {{splash_dkv_kernel<false, false, false, false>, splash_dkv_kernel<true, false, false, false>},
        {splash_dkv_kernel<false, true, false, false>, splash_dkv_kernel<true, true, false, false>}},
       {{splash_dkv_kernel<false, false, true, false>, splash_dkv_kernel<true, false, true, false>},
        {splash_dkv_kernel<false, true, true, false>, splash_dkv_kernel<true, true, true, false>}}};
-  if (one_tile && !split) return fused ? splash_dkv_kernel<true, true, false, false, true> : splash_dkv_kernel<true, false, false, false, true>;
   if (late) return split ? splash_dkv_kernel<false, true, true, true> : splash_dkv_kernel<false, true, false, true>;
   return kernels[split][fused][soft_cap];
-}
-// Whether a CTA keeps to its own kv tile (with a soft cap; the other kernels take over tiles in grids of any size).  What the
-// loop over tiles keeps in registers costs the soft cap's steps 4 %, which grids of one wave and a bit don't get back: 156
-// tiles (3 x 1664, 12 / 4 heads, window 768, d 80) 95.4 us alone, 99.5 with tiles taken over; 1024 tiles (4 x 4096, 16 / 8,
-// window 768) 772 us a pass, 755.
-static bool one_tile_ctas(const SplashBwdArgs& a) {
-  return a.soft_cap != 0.f && a.k.size[2] / kTile * a.k.size[0] * a.k.size[1] < 2 * kSms;
 }
 // Whether S^T of the next step is issued behind dQ of this one instead of behind dV.  d 128: causal 4 x 8192, 32 / 8 heads
 // 7198 -> 7038 us a pass, 2 x 4096 1022 -> 999, 4 x 2048, 16 / 16 366 -> 358; full 1 x 4096, 32 / 8 991 -> 958; packed windows
@@ -1580,17 +1574,16 @@ int launch_bwd(const SplashBwdArgs& a, const SplashShards& shards, cudaStream_t 
   if (soft_cap && !(a.soft_cap > 0.f)) return SPLASH_ERR_INVALID_ARGUMENT;
   auto* dq_kernel = soft_cap ? splash_dq_kernel<true> : splash_dq_kernel<false>;
   const bool late = late_scores(a, fused);
-  const bool one_tile = one_tile_ctas(a);
-  DkvKernel dkv_kernel = dkv_kernel_for(false, fused, soft_cap, late, one_tile);
+  DkvKernel dkv_kernel = dkv_kernel_for(false, fused, soft_cap, late);
   const int dkv_smem = kDkvSmemBytes;
   // function attributes are per device: remember which devices have been set up
   {
     static std::mutex attr_mu;
-    static bool attr_done[64][16] = {};
+    static bool attr_done[64][8] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return SPLASH_ERR_CUDA;
     std::lock_guard<std::mutex> lock(attr_mu);
-    bool& done = attr_done[dev][(soft_cap ? 1 : 0) + (fused ? 2 : 0) + (late ? 4 : 0) + (one_tile ? 8 : 0)];
+    bool& done = attr_done[dev][(soft_cap ? 1 : 0) + (fused ? 2 : 0) + (late ? 4 : 0)];
     if (!done) {
       if (cudaFuncSetAttribute(dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kDqSmemBytes) !=
               cudaSuccess ||
