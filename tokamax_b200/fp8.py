@@ -70,13 +70,14 @@ def splash_fwd_fp8(kernel: _k.SplashAttentionKernel, q: Fp8Tensor, k: Fp8Tensor,
   """
   if p_format not in ("e4m3", "f16"):
     raise ValueError(f"p_format must be 'e4m3' or 'f16', got {p_format!r}")
+  device = q.data.device
   for name, t in (("q", q), ("k", k), ("v", v)):
     if t.data.dtype != torch.float8_e4m3fn or t.scale.dtype != torch.float32:
       raise ValueError(f"{name}: expected float8_e4m3fn values with float32 scales")
     if t.data.dim() != 4 or t.scale.shape != (*t.data.shape[:2], t.data.shape[2] // SCALE_TILE):
       raise ValueError(f"{name}: values {tuple(t.data.shape)} / scales {tuple(t.scale.shape)} do not match")
-    if t.data.device != q.data.device or t.scale.device != q.data.device:
-      raise ValueError(f"{name}: values on {t.data.device}, scales on {t.scale.device}, q on {q.data.device}")
+    if t.data.device != device or t.scale.device != device:
+      raise ValueError(f"{name}: values on {t.data.device}, scales on {t.scale.device}, q on {device}")
   qd, kd, vd = (t.data.contiguous() for t in (q, k, v))
   qs, ks, vs = (t.scale.contiguous() for t in (q, k, v))
   _k._require_cuda(qd)  # pylint: disable=protected-access
