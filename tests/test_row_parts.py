@@ -3,6 +3,7 @@
 GPU (marked), at sizes whose rows are shared: results of calls on a share of the heads are the whole
 call's, bit for bit, and so are o, logsumexp and dq of calls on a share of the query rows.
 """
+import ctypes
 import math
 
 import numpy as np
@@ -12,7 +13,7 @@ import torch
 from tokamax_b200 import _native
 from tokamax_b200 import splash_attention_kernel as splash
 from tokamax_b200 import splash_attention_mask as mask_lib
-from abi_util import row_parts
+from abi_util import _row_args, row_parts
 
 # clusters of n CTAs that 148 SMs hold at a time: in one piece, in GPCs of 16 and 18 SMs, in pairs of SMs lost to each
 CAPACITIES = [
@@ -48,6 +49,16 @@ def test_query_shards_are_shared_out_as_the_whole_call(sq, skv, shards, clusters
 def test_rows_of_tables_are_not_cut_up_for_waves(batch, hq, hkv, s, clusters):
   """Two or three kv tiles an SM: rows of a table may have every length, which whole tiles, longest first, even out."""
   assert row_parts(mask_lib.FullMask((s, s)), batch, hq, hkv, s, s, clusters=clusters)[1] == 1
+
+
+@pytest.mark.parametrize("batch,hq,hkv,s,parts", [(1, 1, 1, 8192, (7, 4, 4)), (1, 2, 1, 4096, (4, 4, 4)), (1, 2, 1, 16384, (4, 4, 4)),
+                                                  (3, 1, 1, 5632, (4, 3, 2)), (1, 8, 8, 4096, (1, 1, 1)), (4, 1, 1, 2432, (3, 3, 3))])
+def test_e4m3_rows_are_cut_up_as_they_were(batch, hq, hkv, s, parts):
+  """Probabilities of 4 bits: with another number of CTAs a row, results differ by more than the order of fp32 sums."""
+  fa, _, shards = _row_args(mask_lib.CausalMask((s, s)), batch, hq, hkv, s, s)
+  fa.q.dtype = 2  # SPLASH_F8E4M3
+  for clusters, want in zip(CAPACITIES, parts):
+    assert _native.lib().splash_fwd_row_parts(ctypes.byref(fa), ctypes.byref(shards), (ctypes.c_int32 * 9)(*clusters)) == want
 
 
 def test_query_shards_say_whether_their_rows_are_in_order():

@@ -126,7 +126,7 @@ __device__ __forceinline__ void fwd_softmax_step(const FwdParams& p, uint64_t* p
   constexpr float kThreshold = (kFp8 && !kP16) ? kFp8RescaleThreshold : kRescaleThreshold;
   // e4m3: P * 2^shift * r with r = v scale / largest v scale in (0, 1]; it and its logarithm come from the caller, which works
   // them out ahead of the wait for the scores (behind it: 32768 keys 13.04 -> 12.93 ms, f16 P 2 x 8192 952 -> 933 us)
-  const float r = v_share, m_shift = kFp8PShift + log_share;
+  const float r = v_share;
   float s[kTile];
   {
     uint32_t v0[32], v1[32], v2[32], v3[32];
@@ -222,7 +222,7 @@ __device__ __forceinline__ void fwd_softmax_step(const FwdParams& p, uint64_t* p
   if constexpr (kP16) {
     // as the e4m3 branch below, but P stays 16 bits wide (f16: 11 significant bits; the factor
     // 2^6 keeps the small weights out of the subnormals, 2^(6+8) is the largest value written)
-    const float m_sub = m_used - m_shift;
+    const float m_sub = m_used - kFp8PShift - log_share;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
       uint32_t pk[16];
@@ -245,7 +245,7 @@ __device__ __forceinline__ void fwd_softmax_step(const FwdParams& p, uint64_t* p
     l += (ls0 + ls1) * __fdividef(0.015625f, r);
   } else if constexpr (kFp8) {
     // P * 2^shift * r, see above
-    const float m_sub = m_used - m_shift;
+    const float m_sub = m_used - kFp8PShift - log_share;
 #pragma unroll
     for (int g = 0; g < 2; ++g) {
       uint32_t pk[16];

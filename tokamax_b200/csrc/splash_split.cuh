@@ -21,7 +21,7 @@ constexpr int kMaxSplit = 8;  // portable cluster size
 struct RowWork {
   float longest, mean;  // 0: rows are left whole
   int64_t ctas;         // rows of the call (of all launches that make it up)
-  bool known;           // false: a table, whose rows may have any length up to these
+  bool known;           // false: a table, whose rows may have any length up to these; and e4m3 P, see fwd_split()
 };
 struct ClusterCapacity {
   int clusters[kMaxSplit + 1];  // [n]: clusters of n CTAs that are resident at the same time; [1]: CTAs
