@@ -51,6 +51,20 @@ def test_rows_of_tables_are_not_cut_up_for_waves(batch, hq, hkv, s, clusters):
   assert row_parts(mask_lib.FullMask((s, s)), batch, hq, hkv, s, s, clusters=clusters)[1] == 1
 
 
+# as a B200 reports them
+B200 = [0, 148, 74, 45, 33, 26, 22, 15, 15]
+
+
+@pytest.mark.parametrize("which,window,batch,hq,hkv,sq,skv,best", [
+    (0, 0, 1, 2, 1, 3328, 3328, 5), (0, 0, 1, 6, 2, 3072, 3072, 2), (0, 0, 1, 4, 4, 1408, 4096, 5), (0, 0, 1, 8, 8, 1408, 3456, 2),
+    (0, 2533, 1, 3, 1, 2816, 2816, 4), (0, 0, 3, 16, 16, 384, 14464, 4), (1, 0, 1, 15, 5, 1152, 1152, 3), (1, 3403, 1, 6, 2, 2304, 2304, 4),
+    (1, 0, 4, 12, 2, 640, 640, 3), (1, 0, 1, 16, 2, 1408, 10240, 1), (1, 1368, 3, 16, 2, 4736, 4736, 2)])
+def test_grids_a_little_above_what_is_resident(which, window, batch, hq, hkv, sq, skv, best):
+  """Calls whose every number of CTAs was measured: the fastest one."""
+  mask = mask_lib.LocalMask((sq, skv), (window, 0), skv - sq) if window else mask_lib.CausalMask((sq, skv), skv - sq)
+  assert row_parts(mask, batch, hq, hkv, sq, skv, clusters=B200)[which] == best
+
+
 @pytest.mark.parametrize("batch,hq,hkv,s,parts", [(1, 1, 1, 8192, (7, 4, 4)), (1, 2, 1, 4096, (4, 4, 4)), (1, 2, 1, 16384, (4, 4, 4)),
                                                   (3, 1, 1, 5632, (4, 3, 2)), (1, 8, 8, 4096, (1, 1, 1)), (4, 1, 1, 2432, (3, 3, 3))])
 def test_e4m3_rows_are_cut_up_as_they_were(batch, hq, hkv, s, parts):

@@ -1474,8 +1474,7 @@ static int dkv_split(const SplashBwdArgs& a, const SplashShards& shards, bool fu
   const int64_t n_rows = a.k.size[2] / kTile;
   RowWork rw = estimate_row_work(a.mask_fn, (int)n_rows, kTile, (int)(a.q.size[2] / kTile),
                                  n_rows * a.k.size[0] * a.k.size[1] * (shards.head_shards > 1 ? shards.head_shards : 1), true);
-  rw.longest *= (float)(a.q.size[1] / a.k.size[1]);  // a kv tile walks every q head of its group
-  rw.mean *= (float)(a.q.size[1] / a.k.size[1]);
+  rw.scale((int)(a.q.size[1] / a.k.size[1]));  // a kv tile walks every q head of its group
   const bool soft_cap = a.soft_cap != 0.f, late = late_scores(a, fused);
   return row_parts(rw, clusters, [&] {
     return cluster_capacity((const void*)dkv_kernel_for(true, fused, soft_cap, late),

@@ -523,7 +523,7 @@ static int fwd_split(const SplashFwdArgs& a, const SplashShards& shards, int var
   // e4m3 P: each CTA rounds its probabilities against the maximum of its own part, so that another number of CTAs moves results
   // by 1.7 % of their norm, the width of that rounding, not by the order of fp32 sums (f16 P: 0.05 %).  These rows keep to the
   // rule that they have had (1 x 4096, 8 / 8 heads: 69 us for 56).
-  if (variant == 1) rw.known = false;
+  if (variant == 1) rw.n_rows = 0;
   return row_parts(rw, clusters, [&] {
     return cluster_capacity((const void*)fwd_split_kernel(variant), variant, kFwdThreads, fwd_split_smem_bytes(variant));
   });

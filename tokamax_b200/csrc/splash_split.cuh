@@ -6,6 +6,8 @@
 // on one kv head, d 64 (64 CTAs of 16 .. 512 steps) 733 -> 223 (four a tile).
 #pragma once
 
+#include <algorithm>
+#include <functional>
 #include <mutex>
 
 #include "splash_common.cuh"
@@ -13,29 +15,39 @@
 namespace sb {
 
 constexpr int kMaxSplit = 8;  // portable cluster size
+constexpr int kSplitMaxCtas = 1024;  // grids above this fill the chip several times over
 
-// Steps (128-column tiles) of the longest row and of the average one, from the mask function; a table
+// Steps (128-column tiles) of the rows, of the longest and of the average one, from the mask function; a table
 // mask counts as full, whether it comes from the host or from the device: so both give the same bits.
 // Not asked for calls whose rows come in an order of their own (q_sequence), nor for calls with segment ids,
 // which cut rows at places that only the device knows.
 struct RowWork {
   float longest, mean;  // 0: rows are left whole
   int64_t ctas;         // rows of the call (of all launches that make it up)
-  bool known;           // false: a table, whose rows may have any length up to these; and e4m3 P, see fwd_split()
+  int n_rows;           // those of one head; 0: a table, whose rows may have any length up to these; and e4m3 P, see fwd_split()
+  int steps[kSplitMaxCtas];  // in any order
+
+  void scale(int n) {
+    longest *= (float)n;
+    mean *= (float)n;
+    for (int r = 0; r < n_rows; ++r) steps[r] *= n;
+  }
 };
 struct ClusterCapacity {
   int clusters[kMaxSplit + 1];  // [n]: clusters of n CTAs that are resident at the same time; [1]: CTAs
 };
 
-constexpr int kSplitMaxCtas = 1024;  // grids above this fill the chip several times over
-
 // rows of `row_span` query rows (transposed = false) or key tiles (true) over `n_steps_full` tiles of the other side
 inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_span, int n_tiles,
                                  int64_t n_ctas, bool transposed = false) {
-  RowWork w{0.f, 0.f, n_ctas, fn.kind != SPLASH_MASK_TABLE};
-  if (n_ctas > kSplitMaxCtas) return w;
+  RowWork w;
+  w.longest = w.mean = 0.f;
+  w.ctas = n_ctas;
+  w.n_rows = 0;
+  if (n_ctas > kSplitMaxCtas || n_rows > kSplitMaxCtas) return w;
   w.longest = w.mean = (float)n_tiles;
-  if (!w.known) return w;
+  if (fn.kind == SPLASH_MASK_TABLE) return w;
+  w.n_rows = n_rows;
   int64_t sum = 0, most = 0;
   for (int r = 0; r < n_rows; ++r) {
     // the row sees columns lo .. hi of the other side
@@ -61,6 +73,7 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
       if (has_left && last - fn.offset + left < hi) hi = last - fn.offset + left;
     }
     const int64_t n = hi < lo ? 0 : hi / kTile - lo / kTile + 1;
+    w.steps[r] = (int)n;
     sum += n;
     if (n > most) most = n;
   }
@@ -69,51 +82,67 @@ inline RowWork estimate_row_work(const SplashMaskFn& fn, int n_rows, int row_spa
   return w;
 }
 
-// CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (prologue, epilogue; more for the addition across the
-// cluster).  While everything is resident the longest row sets the time.  Beyond that, rows of different length, longest
-// first, end together but for a tenth of the longest, unless that alone takes as long; rows of one length go in whole waves.  (All
-// numbers tried, us of the kernel, the rule's own marked *, that of a rule that counts half a row for the end
-// of every grid and less for a CTA in brackets.  dkv, causal: 2 x 4096, 16 / 1 heads, d 64: 733 375 260 *223 254 (249) 315 278,
-// d 128 837 438 307 *259 296 (291) 371 328; 1 x 4096, 8 / 2, fused: 310 173 128 *115 139 (142) 195 185; 2 x 2048, 16 / 4,
-// d 64: 105 *(74) 96 100; window 1000, 1 x 8192, 8 / 1: 193 *(110) 153 128, 20 / 5, 320 tiles, whole backward: *(286) 319 364 400.
-// Forward: 512 x 16384, 32 / 8: 238 *(137) 184 153, 80 / 8, 160 rows: 455 (374) 348 *348, 160 / 8: 700 *627 686 689;
-// causal 4096, 8 / 2: (65) *55 75 88, d 64 (61) *47 64; 4096, 16 / 2: *(75) 106.)
+// CTAs per row.  Time in steps: a CTA costs its steps and a fixed part (launch, prologue, epilogue; more for the addition
+// across the cluster).  While everything is resident the longest row sets the time.  Beyond that the whole work over the slots does,
+// or the longest row, or a slot's turns: of k room + 1 rows, longest first, some slot takes k + 1, each at least as long as the last
+// of them and with a fixed part of its own.  (That is what grids a little above the resident ones pay: causal 3328, 2 / 1 heads, 26 rows, forward,
+// 1 .. 8 CTAs a row: 50.9 33.5 27.4 25.2 *23.8 33.5 36.1 35.5 us, 22 clusters of six are resident.  Rows of one length go in whole
+// waves by it.)  The constants are those of least time over 1240 calls of random sizes, forward and backward, causal and windows, every
+// number of CTAs measured (148 SMs, 74 45 33 26 22 15 15 clusters of 2 .. 8), and were then held against 400 others: 1.006 of the best
+// number's time in the mean.  Rows of different length as a tail of a tenth of the longest, and waves of equal ones, made that 1.014 forward, 1.020
+// backward, up to 1.3 times the time of half a row for every grid's end (1.017, 1.038); this one 1.03 times at most.
+// All numbers tried, us of the kernel, the rule's own marked *.  dkv, causal: 2 x 4096, 16 / 1 heads, d 64: 733 375 260 *223 254 249 315
+// 278, d 128 837 438 307 *259 296 291 371 328; 1 x 4096, 8 / 2, fused: 310 173 128 *115 139 142 195 185; 2 x 2048, 16 / 4,
+// d 64: 105 *74 96 100; window 1000, 1 x 8192, 8 / 1: 193 *110 153 128, 20 / 5, 320 tiles, whole backward: *286 319 364 400.
+// Forward: 512 x 16384, 32 / 8: 238 *137 184 153, 80 / 8, 160 rows: 455 374 348 *348, 160 / 8: 700 *627 686 689;
+// causal 4096, 8 / 2: 65 *55 75 88, d 64 61 *47 64; 4096, 16 / 2: *75 106.
 //
-// Rows of a table take that other rule, which stands between the two: how long its rows are only the device knows.  Taken as
-// full, they would go in waves, and prefixes and triangles, which have none, would be cut up for it.  (Whole backward, d 128, us with 1 2 3 4 CTAs a tile, waves' choice marked w: 4096, 20 / 5 heads, 160 tiles: prefix 343 *260
+// How long the rows of a table are only the device knows.  The whole work as if they were full, and half a row for the end,
+// stands between full rows, which go in waves, and those of prefixes and triangles, which have none.  (Whole backward, d 128, us with 1 2 3 4
+// CTAs a tile, the number by waves marked w: 4096, 20 / 5 heads, 160 tiles: prefix 343 *260
 // 288 w301, lower triangle 341 *255 274 w292, full 644 *540 497 w479; 2 x 4096, 20 / 5, 320 tiles: *509 w497 554 588, *466 w484 534
 // 566, *1037 w954 1047 1025; 8192, 20 / 5: *989 w916, *865 w869, *2005 w1795; 2 x 4096, 30 / 5, d 64: *476 w487, *431 w469, *970 w893.)
+//
 // Rows below 16 steps stay whole although the
 // rule would share some (causal 2 x 1024, 8 heads, 64 CTAs of 2 .. 8 steps: 24.7 us, 20.9 with two CTAs a row),
 // so that the bits of short rows do not depend on the batch and the heads beside them: in the forward those
 // of fewer than 2048 keys, in dkv kv tiles of fewer than 16 (q tile, q head of the group) steps.
-inline int split_for(const RowWork& w, const ClusterCapacity& cap) {
+inline int split_for(RowWork& w, const ClusterCapacity& cap) {
   constexpr float kFewest = 16.f;
-  const float own = w.known ? 4.f : 3.f, merge = w.known ? 3.f : 1.f;
+  const bool known = w.n_rows > 0;
+  const float own = known ? 6.f : 3.f, merge = known ? 2.f : 1.f;
   if (w.longest < kFewest) return 1;
+  bool sorted = false;
   auto time = [&](int n) {
     const float fixed = own + (n > 1 ? merge : 0.f);
-    const float longest = w.longest / n, mean = w.mean / n + fixed;
+    const float longest = w.longest / n + fixed, mean = w.mean / n + fixed;
     const int64_t room = cap.clusters[n];
-    if (w.ctas <= room) return longest + fixed;
-    if (!w.known) return (float)w.ctas * mean / room + 0.5f * (longest + fixed);
-    if (w.mean > 0.9f * w.longest) return (float)((w.ctas + room - 1) / room) * mean;
-    const float all = (float)w.ctas * mean / room + 0.1f * longest;
-    return all > longest + fixed ? all : longest + fixed;
+    if (w.ctas <= room) return longest;
+    const float all = (float)w.ctas * mean / room;
+    if (!known) return all + 0.5f * longest;
+    if (!sorted) std::sort(w.steps, w.steps + w.n_rows, std::greater<int>());
+    sorted = true;
+    float least = std::max(longest, all + 0.05f * w.longest / n);
+    for (int64_t k = 1; k * room < w.ctas; ++k)
+      least = std::max(least, (float)(k + 1) * ((float)w.steps[k * room * w.n_rows / w.ctas] / n + fixed));
+    return least;
   };
   int best = 1;
-  float least = 0.9f * time(1);  // a split has to gain a tenth
-  for (int n = 2; n <= kMaxSplit && n * 2 <= w.longest; ++n)
-    if (cap.clusters[n] > 0 && time(n) < least) {
-      least = time(n);
+  float least = (known ? 0.95f : 0.9f) * time(1);  // a split has to gain that much
+  for (int n = 2; n <= kMaxSplit && n * 2 <= w.longest; ++n) {
+    if (cap.clusters[n] <= 0) continue;
+    const float t = time(n);
+    if (t < least) {
+      least = t;
       best = n;
     }
+  }
   return best;
 }
 
 // The number for a call whose capacity the caller gives (clusters[n], n = 1 .. 8) or `device` knows.
 template <typename Device>
-inline int row_parts(const RowWork& w, const int32_t* clusters, Device device) {
+inline int row_parts(RowWork& w, const int32_t* clusters, Device device) {
   if (!(w.longest > 0.f)) return 1;
   if (clusters == nullptr) {
     const ClusterCapacity* cap = device();
