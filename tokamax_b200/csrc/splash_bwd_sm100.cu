@@ -807,7 +807,8 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     const int wq = warp & 3;
     const int half = (warp - kDkvDrainWarp) >> 2;
     // Columns 64 half .. + 63; with at most 64 of them in all, 32 half .. + 31.  (Where dq has 96 at most the last 32 hold zeros
-    // and need not go; with late scores they do, for the registers: without them causal 4 x 8192 6941 -> 7004 us.)
+    // and stay here.  Late scores are for more than 96, but asking for that at run time, with this test, keeps registers: causal 4 x 8192
+    // 6941 us, 7004 with the other one, 7978 -> 8037 a whole pass with a constant.)
     const bool two = kLateS ? p.d_qk > 64 : p.dq_pairs > half;
     const int chunk = p.d_qk > 64 ? 2 * half : half;
     const uint32_t t_dq = tmem + ((uint32_t)(wq * 32) << 16) + kTile + chunk * 32;
@@ -1444,15 +1445,17 @@ static DkvKernel dkv_kernel_for(bool split, bool fused, bool soft_cap, bool late
   if (late) return split ? splash_dkv_kernel<false, true, true, true> : splash_dkv_kernel<false, true, false, true>;
   return kernels[split][fused][soft_cap];
 }
-// Whether S^T of the next step is issued behind dQ of this one instead of behind dV.  d 128: causal 4 x 8192, 32 / 8 heads
-// 7198 -> 7038 us a pass, 2 x 4096 1022 -> 999, 4 x 2048, 16 / 16 366 -> 358; full 1 x 4096, 32 / 8 991 -> 958; packed windows
-// 8 x 16384 6678 -> 6598.  Where forming P^T takes longer it wants its scores early: partial blocks read from a table (prefix
-// 1 x 8192, 16 / 16, d 96 928 -> 960, 4 x 1024, 32 / 8 282 -> 289, if 2 x 4096, 16 / 4 575 -> 569), a soft cap (187 -> 193); so it
-// does where the scores are half as long (d 64, 2 x 8192, 16 / 4: 1181 -> 1356).  Without dQ there is nothing to put them behind
-// (4 x 4096, 16 / 8: behind dS^T's arrival 1097 -> 1158).
+// Whether S^T of the next step is issued behind dQ of this one instead of behind dV.  Whole backward, d 128: causal 4 x 8192,
+// 32 / 8 heads 5580 -> 5465 us, 2 x 4096 787 -> 759, 4 x 2048, 16 / 16 265 -> 257; full 1 x 4096, 32 / 8 710 -> 691; window 4096,
+// 8 x 16384, 16 / 16 10717 -> 10482.  d 104 .. 120 take the same time either way (causal 2 x 8192, 16 / 4 1354 1360, 1338 1344, 1387 1392).
+// Up to 96 the drain sends three quarters or half of dQ, and there is less to run the scores under: d 96 1164 -> 1265, d 80
+// 1097 -> 1192, d 72 1131 -> 1245, d 64 802 -> 984.  A soft cap, whose P^T takes longer to form, wants its scores early
+// (3 x 1664, 12 / 4, d 80, window 768 89 -> 95, causal 4 x 4096, 16 / 8 738 -> 781); partial blocks read from a table did, but no
+// longer do (prefix 2 x 4096, 16 / 4 394 -> 380, 4 x 1024, 32 / 8 163 -> 159, 8192, 16 / 16, d 96 707 -> 694) and are left as they are.
+// Without dQ there is nothing to put them behind (4 x 4096, 16 / 8: behind dS^T's arrival 1097 -> 1158).
 static bool late_scores(const SplashBwdArgs& a, bool fused) {
   const bool table = a.mask_fn.kind == SPLASH_MASK_TABLE && a.sched_dkv.partial_mask_blocks != nullptr;
-  return fused && a.soft_cap == 0.f && a.q.size[3] > 64 && !table;
+  return fused && a.soft_cap == 0.f && a.q.size[3] > 96 && !table;
 }
 
 // The groups of a dkv launch that come chunk by chunk; the others are its last chunk.  A chunk's rows fill the SMs only
