@@ -577,7 +577,8 @@ constexpr int kDkvMmaWarp = 17;
 // launch, 4 x 88 + 56 + 2 x 48 after the hand-over (the sum per bank has to stay at what the launch gave it, or the
 // increase never completes).
 constexpr int kFusedThreads = 896;
-constexpr int kDkvDrainWarp = 20;
+constexpr int kDkvDrainWarp = 20;  // the first of
+constexpr int kDkvDrainWarps = kFusedThreads / 32 - kDkvDrainWarp;
 constexpr int kFusedComputeRegs = 88;
 constexpr int kFusedIssueRegs = 56;
 constexpr int kFusedDrainRegs = 48;
@@ -621,7 +622,7 @@ struct DkvBarriers {
   uint64_t ds_free;   // dK(n) has finished reading the dS^T tile in shared memory
   uint64_t acc_done;
   uint64_t dq_full;   // fused: dQ_partial(n) is complete in the dP^T columns
-  uint64_t dq_free;   // fused: the drain warps have read it out (4 arrivals)
+  uint64_t dq_free;   // fused: the drain warps have read it out (kDkvDrainWarps arrivals)
   uint32_t tmem_base;
   uint32_t abort_flag;
   uint32_t early_exit;
@@ -713,7 +714,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     bars->n_steps = 0;
     for (uint32_t i = 0; i < kDkvWork; ++i) {
       mbar_init(&bars->work_full[i], 1);
-      mbar_init(&bars->work_empty[i], 17 + (kFuseDq ? kFusedThreads / 32 - kDkvDrainWarp : 0));  // compute, MMA, drain warps
+      mbar_init(&bars->work_empty[i], 17 + (kFuseDq ? kDkvDrainWarps : 0));  // compute, MMA, drain warps
     }
     mbar_init(&bars->answer_full, 1);
     mbar_init(&bars->out_free, 16);
@@ -730,7 +731,7 @@ splash_dkv_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constan
     mbar_init(&bars->ds_free, 1);
     mbar_init(&bars->acc_done, 1);
     mbar_init(&bars->dq_full, 1);
-    mbar_init(&bars->dq_free, kFusedThreads / 32 - kDkvDrainWarp);
+    mbar_init(&bars->dq_free, kDkvDrainWarps);
     mbar_fence_init();
   }
   __syncthreads();

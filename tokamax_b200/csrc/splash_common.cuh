@@ -67,10 +67,6 @@ __device__ __forceinline__ CtaWork cta_work_at(unsigned block, const int32_t* ro
   w.row = row_order ? row_order[pos] : (fallback_reversed ? n_rows - 1 - (int)pos : (int)pos);
   return w;
 }
-__device__ __forceinline__ CtaWork cta_work(const int32_t* row_order, int n_rows, int n_groups,
-                                            int chunk_groups, bool fallback_reversed) {
-  return cta_work_at(blockIdx.x, row_order, n_rows, n_groups, chunk_groups, fallback_reversed);
-}
 // Groups per chunk so that `bytes_per_group` of streamed operands of one chunk fill about half
 // of a 126 MB L2, in whole multiples of `align` (heads sharing a kv head stay together).
 inline int chunk_groups_for(int64_t bytes_per_group, int64_t n_groups, int64_t align) {
